@@ -243,7 +243,10 @@ int collision_f64(vg_plan* p, double* f, cudaStream_t s) {
   }
   VG_CHECK(cuda_status(prof_run(p, PK_FP_MOMENTS, s, [&] { return launch_row_moments_f64(*p, f, spec, p->mom, MOM_STRIDE, s); }),
                        "collision moments"));
-  return cuda_status(prof_run(p, PK_FP_SOLVE, s, [&] { return launch_thomas_f64(*p, f, p->mom, 0, 1, s); }),
+  return cuda_status(prof_run(p, PK_FP_SOLVE, s, [&] {
+                       return launch_thomas_f64(f, p->nx, p->nv, p->v, p->mom, MOM_STRIDE, 0, 1,
+                                                p->collision == VG_COLL_DG, p->nudt, nullptr, p->dv, p->dv_sq, p->bb, s);
+                     }),
                      "tridiagonal solve");
 }
 
@@ -633,7 +636,7 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
   TRY(dev_copy<double>(&p->etmp, nullptr, 4 * nx + 4, "scratch"));
   TRY(dev_copy<int>(&p->flags, nullptr, 1, "status"));
   if (d->precision == VG_F64 && d->collision != VG_COLL_NONE)
-    TRY(dev_copy<double>(&p->bb, nullptr, 2 * nx * nv, "thomas scratch"));
+    TRY(dev_copy<double>(&p->bb, nullptr, 2 * nx * thomas_pad(d->nv), "thomas scratch"));
   if (d->precision == VG_F32_DELTA_F) TRY(setup_f32(p, d));
   TRY(cuda_status(launch_twiddles(*p, 0), "twiddles"));
   TRY(cuda_status(cudaDeviceSynchronize(), "plan setup"));

@@ -68,20 +68,6 @@ __global__ void __launch_bounds__(fft_threads<double>(NX))
                        reinterpret_cast<cx<double>*>(smem_raw), threadIdx.x, flags);
 }
 
-// tridiagonal collision solve, one thread per row of a class; rows of
-// collisionless runs (nudt == 0) are left as they are
-__global__ void k_batch_thomas(double* f, int nrows, int nv, const double* __restrict__ v,
-                               const double* __restrict__ mom, const double* __restrict__ nudt_row,
-                               int dougherty, double dv, double dv_sq, double* __restrict__ bb) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= nrows) return;
-  const double nudt = nudt_row[row];
-  if (nudt == 0.0) return;
-  const double vbar = dougherty ? mom[(size_t)row * 2 + 0] : 0.0;
-  const double vth = mom[(size_t)row * 2 + 1];
-  thomas_row_f64(f + (size_t)row * nv, bb + (size_t)row * 2 * nv, nv, v, vbar, vth, dougherty, nudt, dv, dv_sq);
-}
-
 // e history row and the seven series of one run per CTA: the x-means of n,
 // j, T, e^2, driver^2 (no driver: 0), f^2 and f log f by NumPy's pairwise
 // tree over nx, divided by nx (vlapy/core/step.py:174-229)
@@ -337,10 +323,9 @@ int batch_sequence(vg_batch* b, double* f, double* e, int nsteps, double* e_hist
     B_CHECK(moments(BK_FP_MOMENTS, fp_spec, b->fpmom, 2));
     B_CHECK(cuda_status(prof_call(&b->prof, BK_FP_SOLVE, s, [&] {
                           for (const auto& c : b->cls) {
-                            k_batch_thomas<<<div_up(c.rows, 64), 64, 0, s>>>(
-                                f + c.f_off, c.rows, c.nv, c.v, b->fpmom + (size_t)c.x_off * 2, b->nudt_row + c.x_off,
-                                b->collision == VG_COLL_DG, c.dv, c.dv_sq, b->bb);
-                            cudaError_t err = cudaGetLastError();
+                            const cudaError_t err = launch_thomas_f64(
+                                f + c.f_off, c.rows, c.nv, c.v, b->fpmom + (size_t)c.x_off * 2, 2, 0, 1,
+                                b->collision == VG_COLL_DG, 0.0, b->nudt_row + c.x_off, c.dv, c.dv_sq, b->bb, s);
                             if (err != cudaSuccess) return err;
                           }
                           return cudaSuccess;
@@ -454,7 +439,7 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
     }
     vg_batch::Cls& c = b->cls.back();
     c.rows += d.nx;
-    bb_need = std::max(bb_need, (size_t)c.rows * 2 * (size_t)c.nv);
+    bb_need = std::max(bb_need, (size_t)c.rows * 2 * thomas_pad(c.nv));
     if (!pw_x_of.count(d.nx)) {
       const std::vector<int> tx = pairwise_table(d.nx);
       int* p = nullptr;

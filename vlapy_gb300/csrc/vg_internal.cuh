@@ -135,8 +135,23 @@ struct FieldTime {
 };
 cudaError_t launch_poisson_f64(const vg_plan& p, const double* dens, int dens_is_density,
                                const double* driver, const FieldTime& ft, double* e, cudaStream_t s);
-cudaError_t launch_thomas_f64(const vg_plan& p, double* f, const double* mom, int vbar_col,
-                              int vth_col, cudaStream_t s);
+// tridiagonal solve of rows with scratch of 2 thomas_pad(nv) doubles per row;
+// nudt_row (per row, 0: leave the row as it is) or nudt for all
+cudaError_t launch_thomas_f64(double* f, int nrows, int nv, const double* v, const double* mom, int mstride,
+                              int vbar_col, int vth_col, int dougherty, double nudt, const double* nudt_row, double dv,
+                              double dv_sq, double* scratch, cudaStream_t s);
+// longest row whose chunked solve keeps all its arrays in shared memory, and
+// longest row it takes at all
+constexpr int THOMAS_SMEM_NV = 4096;
+constexpr int THOMAS_CHUNK_NV = 8192;
+// rows from which the one-thread-per-row solve fills the FP64 pipes itself (it
+// spends fewer FP64 instructions, the chunked one needs fewer rows): 8192 x 1024
+// 1.63 ms serial against 0.72 (nu 1e-4) to 1.01 ms (3e-3) in chunks, 16384 x
+// 1024 1.72 against 1.45 to 2.01, 65536 x 1024 4.59 against 5.7 to 7.9; the same
+// rows cross at nv = 256 (0.43 against 0.37 to 0.41 at 16384) and 2048
+constexpr int THOMAS_SERIAL_ROWS = 12288;
+// doubles per scratch array of a row: whole chunks of 32 for a whole number of warps
+__host__ __device__ constexpr size_t thomas_pad(int nv) { return ((size_t)nv + 1023) / 1024 * 1024; }
 cudaError_t launch_storage_f64(const vg_plan& p, const double* f, const double* e, const double* de,
                                const vg_history& h, int i, cudaStream_t s);
 cudaError_t launch_driver(const vg_plan& p, const FieldTime& ft, double* out, cudaStream_t s);

@@ -1,4 +1,4 @@
-// FP64 reductions, field solve, tridiagonal solve and storage step.
+// FP64 reductions, field solve and storage step.
 //
 // Every trapz over v and every mean over x is evaluated with NumPy's pairwise
 // summation tree (a table built at plan creation): leaves of <= 128 terms are
@@ -225,29 +225,6 @@ cudaError_t launch_poisson_f64(const vg_plan& p, const double* dens, int is_dens
   }
   k_poisson_dft_f64<<<1, 256, 0, s>>>(dens, is_density, p.nx, p.inv_kx, driver, ft.use_pulses, p.pulses,
                                       p.n_pulses, p.x, to_dev(ft), p.etmp, e, p.flags);
-  return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
-// implicit Fokker-Planck: vlapy/core/collisions.py:26-160 (diagonals) and
-// :222-265 (Thomas), one thread per x row, operation for operation
-// ---------------------------------------------------------------------------
-
-__global__ void k_thomas_f64(double* __restrict__ f, int nrows, int nv, const double* __restrict__ v,
-                             const double* __restrict__ mom, int mstride, int vbar_col, int vth_col,
-                             int dougherty, double nudt, double dv, double dv_sq,
-                             double* __restrict__ bb) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= nrows) return;
-  const double vbar = dougherty ? mom[(size_t)row * mstride + vbar_col] : 0.0;
-  const double vth = mom[(size_t)row * mstride + vth_col];
-  thomas_row_f64(f + (size_t)row * nv, bb + (size_t)row * 2 * nv, nv, v, vbar, vth, dougherty, nudt, dv, dv_sq);
-}
-
-cudaError_t launch_thomas_f64(const vg_plan& p, double* f, const double* mom, int vbar_col, int vth_col,
-                              cudaStream_t s) {
-  k_thomas_f64<<<div_up(p.nx, 64), 64, 0, s>>>(f, p.nx, p.nv, p.v, mom, MOM_STRIDE, vbar_col, vth_col,
-                                               p.collision == VG_COLL_DG, p.nudt, p.dv, p.dv_sq, p.bb);
   return cudaGetLastError();
 }
 
