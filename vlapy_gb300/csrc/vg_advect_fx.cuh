@@ -1,0 +1,38 @@
+// Launch interface of the fixed-point FP64 advection (vg_edfdv_fx.cu,
+// vg_vdfdx_fx.cu; the arithmetic is in vg_fx.cuh).
+#pragma once
+
+#include "vg_fx.cuh"
+
+namespace vg {
+
+// the twiddle table (FX_TABLE entries), built once per process on the host
+const fxw* fx_table_host();
+// turns per index and unit field or velocity of the phase ((-k) dt) c with k =
+// m k1: A = -k1 dt / (2 pi) to 62 bits; false when it is not finite
+bool fx_make_turn(double k1, double dt, FxTurn* out);
+// true when k[m] is m k[1] to a few roundings for m <= n / 2 (fftfreq's grid):
+// the fixed-point phases step from index to index
+bool fx_uniform(const double* k, int n);
+
+// v-advection of nrows rows of nv (a power of two <= 8192); kv, dt and tw64 for
+// the row pairs that go through doubles
+cudaError_t launch_edfdv_fx(double* f, int nrows, int nv, const double* e, FxTurn turn, const fxw* tw, const double* kv,
+                            double dt, const cx<double>* tw64, cudaStream_t s);
+
+// One run of the x-advection: f[nx][nv] at f + f_off
+struct FxColRun {
+  long long f_off;
+  int nv;
+  const double* v;
+  const double* kx;
+  FxTurn turn;
+};
+// column pairs per CTA for nx (a power of two <= 8192) when `pairs` pairs are advanced together
+int fx_col_pairs(int nx, long long pairs);
+// x-advection: items null: run `one`, all its tiles; else (run, tile) items of
+// one nx over runs, tiles of S pairs
+cudaError_t launch_vdfdx_fx(double* f, int nx, const FxColRun* runs, const int2* items, int n_items, FxColRun one, int S,
+                            double dt, const fxw* tw, const cx<double>* tw64, cudaStream_t s);
+
+}  // namespace vg

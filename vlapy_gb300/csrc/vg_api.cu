@@ -165,7 +165,7 @@ int dev_copy(T** dst, const T* src, size_t n, const char* what) {
 
 void free_plan(vg_plan* p) {
   if (!p) return;
-  void* ptrs[] = {p->x, p->v, p->kx, p->kv, p->inv_kx, p->v_pow, p->f_bg, p->pulses, p->tw64, p->tw32,
+  void* ptrs[] = {p->x, p->v, p->kx, p->kv, p->inv_kx, p->v_pow, p->f_bg, p->pulses, p->tw64, p->tw32, p->tw_fx,
                   p->pw_v, p->pw_x, p->dens, p->mom, p->bb, p->rho, p->etmp, p->sl_m, p->sl_w, p->flags};
   for (void* q : ptrs)
     if (q) cudaFree(q);
@@ -623,6 +623,13 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
   if (d->n_pulses > 0) TRY(dev_copy(&p->pulses, d->pulses, (size_t)d->n_pulses, "pulses"));
   TRY(dev_copy<cx<double>>(&p->tw64, nullptr, FFT_NMAX, "twiddles"));
   TRY(dev_copy<cx<float>>(&p->tw32, nullptr, FFT_NMAX, "twiddles"));
+  if (d->precision == VG_F64) {
+    TRY(dev_copy<fxw>(&p->tw_fx, fx_table_host(), FX_TABLE, "fixed-point twiddles"));
+    p->kv1 = d->kv[1];
+    p->kx1 = d->kx[1];
+    p->kv_uniform = fx_uniform(d->kv, d->nv);
+    p->kx_uniform = fx_uniform(d->kx, d->nx);
+  }
   std::vector<int> tv = pairwise_table(d->nv - 1), tx = pairwise_table(d->nx);
   p->pw_v_leaves = tv[0];
   p->pw_x_leaves = tx[0];

@@ -119,6 +119,8 @@ struct vg_batch {
   BatchRunDev* runs = nullptr;
   cx<double>* tw64 = nullptr;
   cx<float>* tw32 = nullptr;
+  fxw* tw_fx = nullptr;
+  FxColRun* fx_runs = nullptr;  // per run, for the fixed-point x-drift
   double* dens = nullptr;      // [x_points]
   double* mom = nullptr;       // [x_points][BATCH_MOMS]
   double* fpmom = nullptr;     // [x_points][2]
@@ -132,7 +134,8 @@ struct vg_batch {
     long long f_off;
     int x_off, rows;
     int pw_v_leaves;
-    double dv, dv_sq;
+    double dv, dv_sq, kv1;
+    int kv_uniform;
     double *v, *kv, *v_pow;
     int* pw_v;
   };
@@ -140,6 +143,7 @@ struct vg_batch {
   // nx classes: x-drift items and Poisson run lists
   struct XCls {
     int nx, W;
+    bool fx;  // every run's kx is uniform: the fixed-point x-drift
     int2* items;
     int n_items;
     int* ids;
@@ -202,6 +206,9 @@ vg_plan class_view(const vg_batch* b, const vg_batch::Cls& c) {
   v.pw_v_leaves = c.pw_v_leaves;
   v.tw64 = b->tw64;
   v.tw32 = b->tw32;
+  v.tw_fx = b->tw_fx;
+  v.kv1 = c.kv1;
+  v.kv_uniform = c.kv_uniform;
   return v;
 }
 
@@ -233,6 +240,11 @@ cudaError_t batch_poisson_launch(const vg_batch* b, const vg_batch::XCls& xc, do
 cudaError_t batch_vdfdx_all(const vg_batch* b, double* f, double dt, cudaStream_t s) {
   for (const auto& xc : b->xcls) {
     cudaError_t err = cudaErrorInvalidValue;
+    if (xc.fx) {
+      err = launch_vdfdx_fx(f, xc.nx, b->fx_runs, xc.items, xc.n_items, FxColRun{}, xc.W / 2, dt, b->tw_fx, b->tw64, s);
+      if (err != cudaSuccess) return err;
+      continue;
+    }
     switch (xc.nx) {
 #define CASE(NX, ...) \
   case NX: err = batch_vdfdx_launch<NX>(b, xc, f, dt, s); break;
@@ -429,6 +441,8 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
       c.x_off = xoff;
       c.dv = d.dv;
       c.dv_sq = d.dv_sq;
+      c.kv1 = d.kv[1];
+      c.kv_uniform = fx_uniform(d.kv, d.nv);
       B_TRY(b_alloc(b, &c.v, d.nv, d.v, "batch grids"));
       B_TRY(b_alloc(b, &c.kv, d.nv, d.kv, "batch grids"));
       B_TRY(b_alloc(b, &c.v_pow, 5 * (size_t)d.nv, d.v_pow, "batch grids"));
@@ -481,6 +495,7 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
   B_TRY(b_alloc<double>(b, &b->bb, bb_need, nullptr, "batch thomas scratch"));
   B_TRY(b_alloc<cx<double>>(b, &b->tw64, FFT_NMAX, nullptr, "twiddles"));
   B_TRY(b_alloc<cx<float>>(b, &b->tw32, FFT_NMAX, nullptr, "twiddles"));
+  B_TRY(b_alloc<fxw>(b, &b->tw_fx, FX_TABLE, fx_table_host(), "fixed-point twiddles"));
   {
     vg_plan tmp;
     std::memset(&tmp, 0, sizeof(tmp));
@@ -490,9 +505,22 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
   }
   // x classes: (run, column tile) items of the x-drift and the Poisson run lists
   std::map<int, std::pair<std::vector<int2>, std::vector<int>>> by_nx;
+  std::map<int, long long> pairs_of;  // column pairs of each nx class
+  std::map<int, bool> fx_of;
+  std::vector<FxColRun> fx_runs(n_runs);
+  for (int i = 0; i < n_runs; ++i) {
+    const vg_run_desc& d = runs[i];
+    fx_runs[i] = {rd[i].f_off, d.nv, rd[i].v, rd[i].kx, {}};
+    const bool ok = fx_uniform(d.kx, d.nx) && fx_make_turn(d.kx[1], d.dt, &fx_runs[i].turn);
+    if (!fx_of.count(d.nx)) fx_of[d.nx] = true;
+    fx_of[d.nx] = fx_of[d.nx] && ok;
+    pairs_of[d.nx] += (d.nv + 1) / 2;
+  }
+  B_TRY(b_alloc(b, &b->fx_runs, fx_runs.size(), fx_runs.data(), "batch runs"));
+  auto tile_w = [&](int nx) { return 2 * (fx_of[nx] ? fx_col_pairs(nx, pairs_of[nx]) : col_seqs<double>(nx)); };
   for (int i = 0; i < n_runs; ++i) {
     const int nx = rd[i].nx;
-    const int W = 2 * col_seqs<double>(nx);
+    const int W = tile_w(nx);
     auto& e = by_nx[nx];
     for (int t = 0; t * W < rd[i].nv; ++t) e.first.push_back(make_int2(i, t));
     e.second.push_back(i);
@@ -500,7 +528,8 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
   for (auto& kv : by_nx) {
     vg_batch::XCls xc;
     xc.nx = kv.first;
-    xc.W = 2 * col_seqs<double>(kv.first);
+    xc.W = tile_w(kv.first);
+    xc.fx = fx_of[kv.first];
     xc.n_items = (int)kv.second.first.size();
     xc.n_ids = (int)kv.second.second.size();
     B_TRY(b_alloc(b, &xc.items, kv.second.first.size(), kv.second.first.data(), "batch work list"));

@@ -1,0 +1,248 @@
+// Fixed-point v-advection of the FP64 mode (vlapy/core/vlasov.py:113-140): f <-
+// Re IFFT_v(exp(-i kv e dt) FFT_v f) on row pairs, and the host side of the
+// fixed-point tables.
+//
+// One group of N / 8 threads (N / 16 at 8192) owns a pair of rows as one complex
+// sequence; f is read once and written once.
+//
+// Measured against the transforms in doubles (FP64 pipe 84 % busy): 4096 x 8192
+// 4.44 -> 0.88 ms, 2048 x 4096 1.02 -> 0.23 ms, 64 x 1024 70 -> 16 us.  Bound by
+// integer issue: a complex product is 12 wide multiplies at a quarter of the
+// add rate.  Radix 16 (3 passes instead of 4 at 4096) takes 0.21 ms there but
+// 34 us at 64 x 1024, where half as many threads carry the latency.  RMS error
+// against 128-bit FFTs: 1.1e-16 of the line's RMS at 1024 and 2.7e-16 at 8192
+// (smooth lines), in doubles 3.0e-16 and 3.2e-16.
+#include <cmath>
+#include <vector>
+
+#include "vg_advect_fx.cuh"
+#include "vg_internal.cuh"
+
+namespace vg {
+
+namespace {
+
+__host__ __device__ constexpr int fx_row_block(int n) { return fx_threads(n) > 256 ? fx_threads(n) : 256; }
+
+template <int N>
+__global__ void __launch_bounds__(fx_row_block(N), fx_row_block(N) > 256 ? 1 : 2)
+    k_edfdv_fx(double* __restrict__ f, int nrows, const double* __restrict__ e, FxTurn turn,
+               const fxw* __restrict__ tw, const double* __restrict__ kv, double dt, const cx<double>* __restrict__ tw64) {
+  constexpr int R = fx_radix(N), G = fx_threads(N);
+  constexpr int DOWN = ilog2(N) - fx_shift<N>();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ uint2 red[G > 32 ? fx_row_block(N) / 32 : 1];
+  __shared__ FxNorms nred[G > 32 ? fx_row_block(N) / 32 : 1];
+  const int g = threadIdx.x / G, t = threadIdx.x - g * G;
+  fx* s = reinterpret_cast<fx*>(smem_raw) + (size_t)g * sp_len<double>(N);
+  const int ra = 2 * (blockIdx.x * (blockDim.x / G) + g), rb = ra + 1;
+  if (ra >= nrows) return;  // the whole group; its barrier is its own
+  const GroupSync sync = GroupSync::of(g, G);
+  const unsigned mask = G < 32 ? sync.mask : 0xffffffffu;
+  const bool vb = rb < nrows;
+  double* fa = f + (size_t)ra * N;
+  double* fb = f + (size_t)(vb ? rb : ra) * N;
+  const double ea = e[ra], eb = vb ? e[rb] : 0.0;
+  fx io[R];
+  int Ea, Eb;
+  bool bad_a, bad_b, zero_a, zero_b;
+  {
+    double da[R], db[R];
+    unsigned ma = 0, mb = 0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      da[i] = fa[t + i * G];
+      db[i] = vb ? fb[t + i * G] : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      ma = max(ma, fx_exp_bits(da[i]));
+      mb = max(mb, fx_exp_bits(db[i]));
+    }
+    ma = __reduce_max_sync(mask, ma);
+    mb = __reduce_max_sync(mask, mb);
+    if constexpr (G > 32) {
+      if ((t & 31) == 0) red[threadIdx.x >> 5] = make_uint2(ma, mb);
+      sync();
+#pragma unroll
+      for (int w = 0; w < G / 32; ++w) {
+        ma = max(ma, red[g * (G / 32) + w].x);
+        mb = max(mb, red[g * (G / 32) + w].y);
+      }
+    }
+    zero_a = ma == 0;
+    zero_b = mb == 0;
+    Ea = fx_exp(ma);
+    Eb = fx_exp(mb);
+    bad_a = Ea == FX_NONFINITE || !isfinite(ea);
+    bad_b = Eb == FX_NONFINITE || !isfinite(eb);
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      io[i] = {bad_a ? 0 : fx_from_double(da[i], Ea), bad_b ? 0 : fx_from_double(db[i], Eb)};
+  }
+  FxPass<N, false, 1, true, false>::run(s, t, tw, sync, io);
+  FxNorms n = fx_rotate<N, DOWN>(s, t, fx_turn(turn, bad_a ? 0.0 : ea), fx_turn(turn, bad_b ? 0.0 : eb), tw);
+  n.l1 = __reduce_add_sync(mask, n.l1);
+  n.a2 = __reduce_add_sync(mask, n.a2);
+  n.b2 = __reduce_add_sync(mask, n.b2);
+  if constexpr (G > 32) {
+    if ((t & 31) == 0) nred[threadIdx.x >> 5] = n;
+  }
+  sync();
+  if constexpr (G > 32) {
+    n = nred[g * (G / 32)];
+#pragma unroll
+    for (int w = 1; w < G / 32; ++w) {
+      const FxNorms q = nred[g * (G / 32) + w];
+      n.l1 += q.l1;
+      n.a2 += q.a2;
+      n.b2 += q.b2;
+    }
+  }
+  // (exponent field 1: a line of zeros, or of values that small)
+  const int h = fx_shift_back<N>(n, bad_a || Ea == 1, bad_b || Eb == 1);
+  if (h < 0) {
+    sync();
+    fx_pair_f64<N>({fa, ea, Ea, true, bad_a}, {fb, eb, Eb, vb, bad_b}, 1, reinterpret_cast<cx<double>*>(s), t, kv, dt,
+                   tw64, sync);
+    return;
+  }
+  FxPass<N, true, 1, false, true>::run(s, t, tw, sync, io, h);
+  // lines of zeros stay so: the partner's rounding does not reach them
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  const bool set_a = bad_a || zero_a, set_b = bad_b || zero_b;
+  const double val_a = bad_a ? nan : 0.0, val_b = bad_b ? nan : 0.0;
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    fa[t + i * G] = set_a ? val_a : fx_to_double(io[i].x, Ea - FX_SCALE + h);
+    if (vb) fb[t + i * G] = set_b ? val_b : fx_to_double(io[i].y, Eb - FX_SCALE + h);
+  }
+}
+
+template <int N>
+cudaError_t edfdv_fx_n(double* f, int nrows, const double* e, FxTurn turn, const fxw* tw, const double* kv, double dt,
+                       const cx<double>* tw64, cudaStream_t s) {
+  constexpr int G = fx_threads(N);
+  const int pairs = (nrows + 1) / 2;
+  // groups per CTA: fewer when the pairs would not give every SM two CTAs
+  // (a scheduler runs the integer work of one CTA's warps with gaps), whole warps
+  int P = fx_row_block(N) / G;
+  while (P > 1 && (P / 2) * G >= 32 && div_up(pairs, P) < 304) P /= 2;
+  const size_t smem = (size_t)P * sp_len<double>(N) * sizeof(fx);
+  cudaError_t err = ensure_smem((const void*)k_edfdv_fx<N>, smem);
+  if (err != cudaSuccess) return err;
+  k_edfdv_fx<N><<<div_up(pairs, P), P * G, smem, s>>>(f, nrows, e, turn, tw, kv, dt, tw64);
+  return cudaGetLastError();
+}
+
+// ---- host tables -------------------------------------------------------------
+// double-double arithmetic by exact products (fma) and two-sums
+struct dd {
+  double h, l;
+};
+dd dd_norm(double a, double b) {
+  const double s = a + b, t = s - a;
+  return {s, (a - (s - t)) + (b - t)};
+}
+dd dd_mul(dd a, dd b) {
+  const double p = a.h * b.h;
+  return dd_norm(p, std::fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h));
+}
+dd dd_add(dd a, dd b) {
+  const dd s = dd_norm(a.h, b.h);
+  return dd_norm(s.h, s.l + (a.l + b.l));
+}
+const dd kPi = {3.141592653589793116, 1.2246467991473532072e-16};
+const dd kInv2Pi = {0.15915494309189534561, -9.8393383375912127e-18};
+
+// cos and sin of pi j / 4096 for j <= 1024 (an eighth of the circle) by their Taylor series
+void dd_cos_sin(int j, dd* c, dd* s) {
+  const dd x = dd_mul(kPi, {(double)j / 4096.0, 0.0}), x2 = dd_mul(x, x);
+  dd tc = {1.0, 0.0}, ts = x;
+  *c = tc;
+  *s = ts;
+  for (int n = 1; n < 16; ++n) {
+    const dd pc = dd_mul(tc, x2), ps = dd_mul(ts, x2);
+    const double dc = -(2.0 * n - 1.0) * (2.0 * n), ds = -(2.0 * n) * (2.0 * n + 1.0);
+    const double qc = pc.h / dc, qs = ps.h / ds;
+    tc = dd_norm(qc, (std::fma(-qc, dc, pc.h) + pc.l) / dc);
+    ts = dd_norm(qs, (std::fma(-qs, ds, ps.h) + ps.l) / ds);
+    *c = dd_add(*c, tc);
+    *s = dd_add(*s, ts);
+  }
+}
+long long q62(dd a) {
+  return (long long)std::llrint(std::ldexp(a.h, 62)) + (long long)std::llrint(std::ldexp(a.l, 62));
+}
+
+std::vector<fxw> build_table() {
+  std::vector<long long> c(FX_NMAX), s(FX_NMAX);
+  for (int j = 0; j <= FX_NMAX / 8; ++j) {
+    dd cj, sj;
+    dd_cos_sin(j, &cj, &sj);
+    const long long C = q62(cj), S = q62(sj);
+    const int h = FX_NMAX / 4, n = FX_NMAX;
+    // the eight angles +-j, h +- j, 2h +- j, 3h +- j
+    auto put = [&](int k, long long cc, long long ss) {
+      c[(k + n) % n] = cc;
+      s[(k + n) % n] = ss;
+    };
+    put(j, C, S);
+    put(-j, C, -S);
+    put(h - j, S, C);
+    put(h + j, -S, C);
+    put(2 * h - j, -C, S);
+    put(2 * h + j, -C, -S);
+    put(3 * h - j, -S, -C);
+    put(3 * h + j, S, -C);
+  }
+  std::vector<fxw> out(FX_TABLE);
+  for (int L = 2; L <= FX_NMAX; L *= 2)
+    for (int q = 0; q < L; ++q) {
+      const int k = q * (FX_NMAX / L);
+      out[L - 2 + q] = fx_mult(c[k], -s[k]);
+    }
+  return out;
+}
+
+}  // namespace
+
+const fxw* fx_table_host() {
+  static const std::vector<fxw> table = build_table();
+  return table.data();
+}
+
+bool fx_make_turn(double k1, double dt, FxTurn* out) {
+  const double p = k1 * dt;
+  if (!std::isfinite(p) || std::fabs(p) > 1e280 || (p != 0.0 && std::fabs(p) < 1e-280)) return false;
+  const dd a = dd_mul(dd_norm(p, std::fma(k1, dt, -p)), kInv2Pi);
+  int e = 0;
+  const double m = std::frexp(a.h, &e);
+  out->am = -((long long)std::ldexp(m, 62) + (long long)std::llrint(std::ldexp(a.l, 62 - e)));
+  out->ae = e - 62;
+  return true;
+}
+
+bool fx_uniform(const double* k, int n) {
+  for (int m = 0; m <= n / 2; ++m) {
+    const double want = m * k[n > 1 ? 1 : 0], tol = 1e-15 * std::fabs(want);
+    if (!(std::fabs(std::fabs(k[m % n]) - std::fabs(want)) <= tol)) return false;
+    if (2 * m != n && m > 0 && want != 0.0 && (k[m] < 0.0) != (want < 0.0)) return false;
+  }
+  return true;
+}
+
+#define VG_FX_CASES(M) M(1) M(2) M(3) M(4) M(5) M(6) M(7) M(8) M(9) M(10) M(11) M(12) M(13)
+
+cudaError_t launch_edfdv_fx(double* f, int nrows, int nv, const double* e, FxTurn turn, const fxw* tw, const double* kv,
+                            double dt, const cx<double>* tw64, cudaStream_t s) {
+  switch (ilog2(nv)) {
+#define CASE(L) \
+  case L: return edfdv_fx_n<(1 << L)>(f, nrows, e, turn, tw, kv, dt, tw64, s);
+    VG_FX_CASES(CASE)
+#undef CASE
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+}  // namespace vg

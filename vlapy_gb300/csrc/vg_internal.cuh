@@ -4,6 +4,7 @@
 #include <string>
 #include <vector>
 
+#include "vg_advect_fx.cuh"
 #include "vg_common.cuh"
 #include "vg_f32_plan.cuh"
 #include "vg_fft.cuh"
@@ -25,6 +26,11 @@ struct vg_plan {
   vg_pulse* pulses;  // [n_pulses]
   vg::cx<double>* tw64;  // [FFT_NMAX]
   vg::cx<float>* tw32;   // [FFT_NMAX]
+  // fixed-point advection: its table (null: none), kv[1] and kx[1], and whether
+  // each wavenumber grid is uniform (else the transforms in doubles)
+  vg::fxw* tw_fx;
+  double kv1, kx1;
+  int kv_uniform, kx_uniform;
   int* pw_v;   // NumPy pairwise tree over nv-1 trapz terms
   int* pw_x;   // NumPy pairwise tree over nx values (x-means)
   int pw_v_leaves, pw_x_leaves, pw_v_words, pw_x_words;

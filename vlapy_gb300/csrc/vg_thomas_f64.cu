@@ -23,8 +23,8 @@
 // the serial one bit for bit.  The k-th sweep leaves at least k lanes exact,
 // so there are never more sweeps than lanes; contraction makes it two to five
 // (the pivots forget their start by a factor a c / p^2 per element, below 0.6
-// for c = nu dt vth / dv^2 up to 13).  Measured: 64 x 1024 from 1.59 to 0.08 ms,
-// 2048 x 4096 from 6.4 to 1.3 ms, against one thread per row.
+// for c = nu dt vth / dv^2 up to 13).  Measured: 64 x 1024 from 1.59 to 0.09 ms,
+// 2048 x 4096 from 6.4 to 1.2 ms, against one thread per row.
 //
 // Divisions that share a divisor (by 2 dv, by a pivot) go through its
 // correctly rounded reciprocal y and remainder term yl: q = n y + n yl is
