@@ -68,42 +68,36 @@ __global__ void __launch_bounds__(fft_threads<double>(NX))
                        reinterpret_cast<cx<double>*>(smem_raw), threadIdx.x, flags);
 }
 
-// e history row and the seven series of one run per CTA: the x-means of n,
-// j, T, e^2, driver^2 (no driver: 0), f^2 and f log f by NumPy's pairwise
-// tree over nx, divided by nx (vlapy/core/step.py:174-229)
-__global__ void k_batch_store(const BatchRunDev* __restrict__ runs, const double* __restrict__ mom,
-                              const double* __restrict__ e, int n_runs, double* __restrict__ e_row,
-                              double* __restrict__ s_row) {
+// e history row and the seven series of one run per CTA: the x-means of n, j, T,
+// e^2, driver^2 (no driver: 0), f^2 and f log f by NumPy's pairwise tree over nx,
+// divided by nx (vlapy/core/step.py:174-229); one warp per series, as
+// k_fields_series_f64
+__global__ void __launch_bounds__(256) k_batch_store(const BatchRunDev* __restrict__ runs, const double* __restrict__ mom,
+                                                     const double* __restrict__ e, int n_runs,
+                                                     double* __restrict__ e_row, double* __restrict__ s_row) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* leaf = reinterpret_cast<double*>(smem_raw);  // [7][nl]
   const BatchRunDev r = runs[blockIdx.x];
   const int* table = r.pw_x;
-  const int nl = table[0];
-  const int* leaves = table + 2;
+  const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const double* er = e + r.x_off;
   const double* mr = mom + (size_t)r.x_off * BATCH_MOMS;
   if (e_row)
     for (int n = threadIdx.x; n < r.nx; n += blockDim.x) e_row[r.x_off + n] = er[n];
-  for (int idx = threadIdx.x; idx < 7 * nl; idx += blockDim.x) {
-    const int q = idx / nl, L = idx - q * nl;
-    auto term = [&](int n) -> double {
-      switch (q) {
-        case 0: return mr[(size_t)n * BATCH_MOMS + 0];
-        case 1: return mr[(size_t)n * BATCH_MOMS + 1];
-        case 2: return mr[(size_t)n * BATCH_MOMS + 2];
-        case 3: return mul_rn(er[n], er[n]);
-        case 4: return 0.0;
-        case 5: return mr[(size_t)n * BATCH_MOMS + 3];
-        default: return mr[(size_t)n * BATCH_MOMS + 4];
-      }
-    };
-    leaf[q * nl + L] = leaf_sum(leaves[2 * L], leaves[2 * L + 1], term);
+  if (q >= 7 || !s_row) return;
+  double* out = s_row + (size_t)r.run * 7 + q;
+  if (q == 4) {
+    if (lane == 0) *out = 0.0;
+    return;
   }
-  __syncthreads();
-  if (s_row && threadIdx.x < 7) {
-    const int q = threadIdx.x;
-    s_row[(size_t)r.run * 7 + q] = __ddiv_rn(combine_leaves(table, leaf + q * nl), (double)r.nx);
+  double* leaf = reinterpret_cast<double*>(smem_raw) + q * table[0];
+  if (q == 3) {
+    warp_leaf_sums(table, lane, leaf, [&](int n) { return mul_rn(er[n], er[n]); });
+  } else {
+    const double* m = mr + (q < 3 ? q : q - 2);
+    warp_leaf_sums(table, lane, leaf, [&](int n) { return m[(size_t)n * BATCH_MOMS]; });
   }
+  __syncwarp();
+  if (lane == 0) *out = __ddiv_rn(combine_leaves(table, leaf), (double)r.nx);
 }
 
 }  // namespace vg
@@ -350,7 +344,7 @@ int batch_sequence(vg_batch* b, double* f, double* e, int nsteps, double* e_hist
       double* sr = s_hist ? s_hist + (size_t)r * b->n_runs * 7 : nullptr;
       B_CHECK(cuda_status(prof_call(&b->prof, BK_STORE, s, [&] {
                             const size_t smem = (size_t)7 * b->max_pw_x_leaves * sizeof(double);
-                            k_batch_store<<<b->n_runs, 128, smem, s>>>(b->runs, b->mom, e, b->n_runs, er, sr);
+                            k_batch_store<<<b->n_runs, 256, smem, s>>>(b->runs, b->mom, e, b->n_runs, er, sr);
                             return cudaGetLastError();
                           }),
                           "batch store"));

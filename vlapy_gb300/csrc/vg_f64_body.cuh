@@ -13,31 +13,41 @@ namespace vg {
 // pairwise-sum helpers
 // ---------------------------------------------------------------------------
 
-// Sum of leaf (start, len) of terms term(j), NumPy order.
+// The leaf sums of terms term(j) in NumPy's order, for all leaves of a table
+// into leaf[0 .. n_leaves), by a warp:
+// eight lanes are one leaf's eight accumulators (four leaves at a time), each a
+// serial chain; the eight are added pairwise in NumPy's order by shuffles and
+// the leaf's first lane adds the tail.  All 32 lanes must call it.
 template <typename TermFn>
-__device__ __forceinline__ double leaf_sum(int start, int len, TermFn term) {
-  if (len < 8) {
-    double r = 0.0;
-    for (int i = 0; i < len; ++i) r = add_rn(r, term(start + i));
-    return r;
+__device__ __forceinline__ void warp_leaf_sums(const int* __restrict__ table, int lane, double* leaf, TermFn term) {
+  const int nl = table[0];
+  const int* leaves = table + 2;
+  const int a = lane & 7;
+  for (int L0 = 0; L0 < nl; L0 += 4) {
+    const int L = L0 + (lane >> 3);
+    const int st = L < nl ? leaves[2 * L] : 0, len = L < nl ? leaves[2 * L + 1] : 0;
+    const int stop = len - (len % 8);
+    double x = 0.0;
+    if (len < 8) {
+      if (a == 0)
+        for (int i = 0; i < len; ++i) x = add_rn(x, term(st + i));
+    } else {
+      x = term(st + a);
+      for (int i = 8 + a; i < stop; i += 8) x = add_rn(x, term(st + i));
+    }
+    double r = x;
+#pragma unroll
+    for (int m = 1; m < 8; m <<= 1) {
+      const double o = __shfl_down_sync(0xffffffffu, r, m, 8);
+      r = add_rn(r, o);
+    }
+    if (a == 0 && L < nl) {
+      if (len < 8) r = x;
+      else
+        for (int i = stop; i < len; ++i) r = add_rn(r, term(st + i));
+      leaf[L] = r;
+    }
   }
-  double a0 = term(start), a1 = term(start + 1), a2 = term(start + 2), a3 = term(start + 3);
-  double a4 = term(start + 4), a5 = term(start + 5), a6 = term(start + 6), a7 = term(start + 7);
-  int i = 8;
-  const int stop = len - (len % 8);
-  for (; i < stop; i += 8) {
-    a0 = add_rn(a0, term(start + i));
-    a1 = add_rn(a1, term(start + i + 1));
-    a2 = add_rn(a2, term(start + i + 2));
-    a3 = add_rn(a3, term(start + i + 3));
-    a4 = add_rn(a4, term(start + i + 4));
-    a5 = add_rn(a5, term(start + i + 5));
-    a6 = add_rn(a6, term(start + i + 6));
-    a7 = add_rn(a7, term(start + i + 7));
-  }
-  double res = add_rn(add_rn(add_rn(a0, a1), add_rn(a2, a3)), add_rn(add_rn(a4, a5), add_rn(a6, a7)));
-  for (; i < len; ++i) res = add_rn(res, term(start + i));
-  return res;
 }
 
 // Replay the combine program over leaf sums leaf[0..n_leaves).

@@ -232,80 +232,114 @@ cudaError_t launch_poisson_f64(const vg_plan& p, const double* dens, int is_dens
 // storage step, vlapy/core/step.py:116-283
 // ---------------------------------------------------------------------------
 
-// fields[.][i] and the seven x-means; mom holds n, j, T, q, fv4, vN, f^2, f log f per row
-__global__ void k_fields_series_f64(const double* __restrict__ mom, const double* __restrict__ e,
-                                    const double* __restrict__ de, int nx, int i, vg_history h,
-                                    const int* __restrict__ table) {
+// fields[.][i] and the seven x-means; mom holds n, j, T, q, fv4, vN, f^2, f log f
+// per row.  One warp per series (lanes that took different series ran one after
+// the other, 25 us at nx = 64 against 8), the eighth copies the fields.
+__global__ void __launch_bounds__(256) k_fields_series_f64(const double* __restrict__ mom, const double* __restrict__ e,
+                                                           const double* __restrict__ de, int nx, int i, vg_history h,
+                                                           const int* __restrict__ table) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* leaf = reinterpret_cast<double*>(smem_raw);  // [7][nl]
   const int nl = table[0];
-  const int* leaves = table + 2;
+  const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t off = (size_t)i * nx;
-  for (int n = threadIdx.x; n < nx; n += blockDim.x) {
-    if (h.fields[0]) h.fields[0][off + n] = e[n];
-    if (h.fields[1]) h.fields[1][off + n] = de ? de[n] : 0.0;
-    for (int q = 0; q < 6; ++q)
-      if (h.fields[2 + q]) h.fields[2 + q][off + n] = mom[(size_t)n * MOM_STRIDE + q];
+  for (int idx = threadIdx.x; idx < 8 * nx; idx += blockDim.x) {
+    const int k = idx / nx, n = idx - k * nx;
+    if (h.fields[k]) h.fields[k][off + n] = k == 0 ? e[n] : k == 1 ? (de ? de[n] : 0.0) : mom[(size_t)n * MOM_STRIDE + k - 2];
   }
   // series sources: n, j, T, e^2, de^2, f^2, flogf
-  for (int idx = threadIdx.x; idx < 7 * nl; idx += blockDim.x) {
-    const int q = idx / nl, L = idx - q * nl;
-    auto term = [&](int n) -> double {
-      switch (q) {
-        case 0: return mom[(size_t)n * MOM_STRIDE + 0];
-        case 1: return mom[(size_t)n * MOM_STRIDE + 1];
-        case 2: return mom[(size_t)n * MOM_STRIDE + 2];
-        case 3: return mul_rn(e[n], e[n]);
-        case 4: return de ? mul_rn(de[n], de[n]) : 0.0;
-        case 5: return mom[(size_t)n * MOM_STRIDE + 6];
-        default: return mom[(size_t)n * MOM_STRIDE + 7];
-      }
-    };
-    leaf[q * nl + L] = leaf_sum(leaves[2 * L], leaves[2 * L + 1], term);
+  if (q >= 7 || !h.series[q]) return;
+  double* leaf = reinterpret_cast<double*>(smem_raw) + q * nl;
+  if (q == 3) {
+    warp_leaf_sums(table, lane, leaf, [&](int n) { return mul_rn(e[n], e[n]); });
+  } else if (q == 4) {
+    warp_leaf_sums(table, lane, leaf, [&](int n) { return de ? mul_rn(de[n], de[n]) : 0.0; });
+  } else {
+    const double* m = mom + (q < 3 ? q : q + 1);
+    warp_leaf_sums(table, lane, leaf, [&](int n) { return m[(size_t)n * MOM_STRIDE]; });
   }
-  __syncthreads();
-  if (threadIdx.x < 7) {
-    const int q = threadIdx.x;
-    const double m = __ddiv_rn(combine_leaves(table, leaf + q * nl), (double)nx);
-    if (h.series[q]) h.series[q][i] = m;
-  }
+  __syncwarp();
+  if (lane == 0) h.series[q][i] = __ddiv_rn(combine_leaves(table, leaf), (double)nx);
 }
 
-// stored_f[i][slot][v] = complex64(sum_x f[x][v] exp(-2 pi i m x / nx))
-__global__ void k_store_modes_f64(const double* __restrict__ f, int nx, int nv, int n_modes, int n_slots,
-                                  int nx_pow2, const cx<double>* __restrict__ tw, int i,
-                                  cx<float>* __restrict__ out) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= nv) return;
+// stored_f[i][slot][v] = complex64(sum_x f[x][v] exp(-2 pi i m x / nx)).  A CTA
+// takes 32 columns; its eight warps take every eighth row and the partial sums
+// are added in warp order.  MODES_AT_ONCE modes share one pass over f (their
+// cosines and sines come from a table of the nx angles in shared memory, or, for
+// long columns, straight from the plan's table or sincospi).  One thread per
+// column had run 32 CTAs of serial loops: 2.01 ms at 2048 x 4096 with two modes,
+// now bound by the three FP64 operations per cell.
+constexpr int MODES_AT_ONCE = 2;
+constexpr int MODES_TABLE_NX = 4096;
+__device__ __forceinline__ cx<double> mode_angle(int q, int nx, int nx_pow2, const cx<double>* __restrict__ tw) {
+  if (q == 0) return {1.0, 0.0};
+  if (nx_pow2) {
+    // exp(-2 pi i q / nx) from the span-ordered table; q >= nx/2 is the negated
+    // entry q - nx/2
+    const bool hi = 2 * q >= nx;
+    const cx<double> w = tw[tw_index(nx, hi ? q - nx / 2 : q)];
+    return hi ? cx<double>{-w.x, -w.y} : w;
+  }
+  double sn, cs;
+  sincospi(2.0 * (double)q / (double)nx, &sn, &cs);
+  return {cs, -sn};
+}
+__global__ void __launch_bounds__(256) k_store_modes_f64(const double* __restrict__ f, int nx, int nv, int n_modes,
+                                                         int n_slots, int nx_pow2, const cx<double>* __restrict__ tw,
+                                                         int i, cx<float>* __restrict__ out) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double part[2 * MODES_AT_ONCE][8][32];
+  cx<double>* angles = reinterpret_cast<cx<double>*>(smem_raw);
+  const bool table = nx <= MODES_TABLE_NX && n_modes > 1;
+  if (table)
+    for (int q = threadIdx.x; q < nx; q += blockDim.x) angles[q] = mode_angle(q, nx, nx_pow2, tw);
+  __syncthreads();
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int j = blockIdx.x * 32 + lane;
   cx<float>* dst = out + (size_t)i * n_slots * nv;
-  for (int m = 0; m < n_modes && m < n_slots; ++m) {
-    double zr = 0.0, zi = 0.0;
-    for (int xx = 0; xx < nx; ++xx) {
-      const long long q = ((long long)m * xx) % nx;
-      double cs, sn;
-      if (q == 0) {
-        cs = 1.0;
-        sn = 0.0;
-      } else if (nx_pow2) {
-        // exp(-2 pi i q / nx) from the span-ordered table; q >= nx/2 is the
-        // negated entry q - nx/2
-        const bool hi = 2 * q >= nx;
-        const cx<double> w = tw[tw_index(nx, hi ? (int)(q - nx / 2) : (int)q)];
-        cs = hi ? -w.x : w.x;
-        sn = hi ? w.y : -w.y;
-      } else {
-        sincospi(2.0 * (double)q / (double)nx, &sn, &cs);
+  const int nm = min(n_modes, n_slots);
+  for (int m0 = 0; m0 < nm; m0 += MODES_AT_ONCE) {
+    double zr[MODES_AT_ONCE], zi[MODES_AT_ONCE];
+    int at[MODES_AT_ONCE], step[MODES_AT_ONCE];
+#pragma unroll
+    for (int u = 0; u < MODES_AT_ONCE; ++u) {
+      zr[u] = zi[u] = 0.0;
+      at[u] = (int)(((long long)(m0 + u) * w) % nx);
+      step[u] = (int)(((long long)(m0 + u) * 8) % nx);
+    }
+    if (j < nv) {
+#pragma unroll 4
+      for (int x = w; x < nx; x += 8) {
+        const double fv = f[(size_t)x * nv + j];
+#pragma unroll
+        for (int u = 0; u < MODES_AT_ONCE; ++u) {
+          if (m0 + u >= nm) continue;
+          if (m0 + u == 0) {
+            zr[u] += fv;
+          } else {
+            const cx<double> c = table ? angles[at[u]] : mode_angle(at[u], nx, nx_pow2, tw);
+            zr[u] = fma(fv, c.x, zr[u]);
+            zi[u] = fma(fv, c.y, zi[u]);
+          }
+          at[u] += step[u];
+          if (at[u] >= nx) at[u] -= nx;
+        }
       }
-      const double fv = f[(size_t)xx * nv + j];
-      zr += fv * cs;
-      zi -= fv * sn;
     }
-    const cx<float> z = {__double2float_rn(zr), __double2float_rn(zi)};
-    if (n_modes == 1) {
-      for (int sl = 0; sl < n_slots; ++sl) dst[(size_t)sl * nv + j] = z;
-    } else {
-      dst[(size_t)m * nv + j] = z;
+#pragma unroll
+    for (int u = 0; u < MODES_AT_ONCE; ++u) {
+      part[2 * u][w][lane] = zr[u];
+      part[2 * u + 1][w][lane] = zi[u];
     }
+    __syncthreads();
+    if (w < 2 * MODES_AT_ONCE && m0 + w / 2 < nm && j < nv) {
+      double z = part[w][0][lane];
+      for (int q = 1; q < 8; ++q) z += part[w][q][lane];
+      const float zf = __double2float_rn(z);
+      const int m = m0 + w / 2;
+      for (int sl = n_modes == 1 ? 0 : m; sl < (n_modes == 1 ? n_slots : m + 1); ++sl)
+        reinterpret_cast<float*>(dst + (size_t)sl * nv + j)[w & 1] = zf;
+    }
+    __syncthreads();
   }
 }
 
@@ -330,9 +364,12 @@ cudaError_t launch_storage_f64(const vg_plan& p, const double* f, const double* 
       err = cudaMemcpyAsync(static_cast<double*>(h.stored_f) + (size_t)i * p.nx * p.nv, f,
                             (size_t)p.nx * p.nv * sizeof(double), cudaMemcpyDeviceToDevice, s);
     } else {
-      k_store_modes_f64<<<div_up(p.nv, 128), 128, 0, s>>>(f, p.nx, p.nv, h.n_modes, h.n_slots,
-                                                          p.nx_pow2 && p.nx <= FFT_NMAX,
-                                                          p.tw64, i, static_cast<cx<float>*>(h.stored_f));
+      const size_t tab = p.nx <= MODES_TABLE_NX && h.n_modes > 1 ? (size_t)p.nx * sizeof(cx<double>) : 0;
+      err = ensure_smem((const void*)k_store_modes_f64, tab);
+      if (err != cudaSuccess) return err;
+      k_store_modes_f64<<<div_up(p.nv, 32), 256, tab, s>>>(f, p.nx, p.nv, h.n_modes, h.n_slots,
+                                                           p.nx_pow2 && p.nx <= FFT_NMAX, p.tw64, i,
+                                                           static_cast<cx<float>*>(h.stored_f));
       err = cudaGetLastError();
     }
   }
