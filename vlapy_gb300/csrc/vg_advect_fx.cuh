@@ -3,11 +3,21 @@
 #pragma once
 
 #include "vg_fx.cuh"
+#include "vg_moments_fx.cuh"
 
 namespace vg {
 
-// the twiddle table (FX_TABLE entries), built once per process on the host
-const fxw* fx_table_host();
+// The constant tables of the fixed-point kernels on the current device: the
+// twiddles (FX_TABLE entries) and the logarithm's entries.  Plans and batches
+// hold them together: the first to ask uploads them, the last to let go frees
+// them (both under one lock).
+struct FxTables {
+  int device, refs;
+  fxw* tw;
+  FxLogEntry* log;
+};
+cudaError_t fx_tables_acquire(FxTables** out);
+void fx_tables_release(FxTables* t);
 // turns per index and unit field or velocity of the phase ((-k) dt) c with k =
 // m k1: A = -k1 dt / (2 pi) to 62 bits; false when it is not finite
 bool fx_make_turn(double k1, double dt, FxTurn* out);

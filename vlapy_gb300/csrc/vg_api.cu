@@ -165,10 +165,11 @@ int dev_copy(T** dst, const T* src, size_t n, const char* what) {
 
 void free_plan(vg_plan* p) {
   if (!p) return;
-  void* ptrs[] = {p->x, p->v, p->kx, p->kv, p->inv_kx, p->v_pow, p->f_bg, p->pulses, p->tw64, p->tw32, p->tw_fx,
+  void* ptrs[] = {p->x, p->v, p->kx, p->kv, p->inv_kx, p->v_pow, p->f_bg, p->pulses, p->tw64, p->tw32, p->fx_vp,
                   p->pw_v, p->pw_x, p->dens, p->mom, p->bb, p->rho, p->etmp, p->sl_m, p->sl_w, p->flags};
   for (void* q : ptrs)
     if (q) cudaFree(q);
+  fx_tables_release(p->fx_tables);
   if (p->graph_cache) {
     auto* gc = static_cast<GraphCache*>(p->graph_cache);
     for (auto& kv : gc->execs) cudaGraphExecDestroy(kv.second);
@@ -624,11 +625,17 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
   TRY(dev_copy<cx<double>>(&p->tw64, nullptr, FFT_NMAX, "twiddles"));
   TRY(dev_copy<cx<float>>(&p->tw32, nullptr, FFT_NMAX, "twiddles"));
   if (d->precision == VG_F64) {
-    TRY(dev_copy<fxw>(&p->tw_fx, fx_table_host(), FX_TABLE, "fixed-point twiddles"));
+    TRY(cuda_status(fx_tables_acquire(&p->fx_tables), "fixed-point tables"));
+    p->tw_fx = p->fx_tables->tw;
     p->kv1 = d->kv[1];
     p->kx1 = d->kx[1];
     p->kv_uniform = fx_uniform(d->kv, d->nv);
     p->kx_uniform = fx_uniform(d->kx, d->nx);
+    std::vector<int2> vp;
+    if (d->nv <= FX_MOMENTS_NV && fx_powers_host(d->v, d->v_pow, d->nv, &vp, &p->fx_pw)) {
+      TRY(dev_copy(&p->fx_vp, vp.data(), vp.size(), "velocity powers"));
+      p->fx_log = p->fx_tables->log;
+    }
   }
   std::vector<int> tv = pairwise_table(d->nv - 1), tx = pairwise_table(d->nx);
   p->pw_v_leaves = tv[0];

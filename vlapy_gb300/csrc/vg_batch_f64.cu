@@ -113,7 +113,7 @@ struct vg_batch {
   BatchRunDev* runs = nullptr;
   cx<double>* tw64 = nullptr;
   cx<float>* tw32 = nullptr;
-  fxw* tw_fx = nullptr;
+  FxTables* fx_tables = nullptr;
   FxColRun* fx_runs = nullptr;  // per run, for the fixed-point x-drift
   double* dens = nullptr;      // [x_points]
   double* mom = nullptr;       // [x_points][BATCH_MOMS]
@@ -131,6 +131,8 @@ struct vg_batch {
     double dv, dv_sq, kv1;
     int kv_uniform;
     double *v, *kv, *v_pow;
+    int2* fx_vp;  // null: the storage moments in doubles
+    FxPowers fx_pw;
     int* pw_v;
   };
   std::vector<Cls> cls;
@@ -174,6 +176,7 @@ void free_batch(vg_batch* b) {
   for (auto& kv : b->graphs) cudaGraphExecDestroy(kv.second);
   for (void* p : b->owned)
     if (p) cudaFree(p);
+  fx_tables_release(b->fx_tables);
   delete b;
 }
 
@@ -200,9 +203,12 @@ vg_plan class_view(const vg_batch* b, const vg_batch::Cls& c) {
   v.pw_v_leaves = c.pw_v_leaves;
   v.tw64 = b->tw64;
   v.tw32 = b->tw32;
-  v.tw_fx = b->tw_fx;
+  v.tw_fx = b->fx_tables->tw;
   v.kv1 = c.kv1;
   v.kv_uniform = c.kv_uniform;
+  v.fx_vp = c.fx_vp;
+  v.fx_pw = c.fx_pw;
+  v.fx_log = b->fx_tables->log;
   return v;
 }
 
@@ -235,7 +241,7 @@ cudaError_t batch_vdfdx_all(const vg_batch* b, double* f, double dt, cudaStream_
   for (const auto& xc : b->xcls) {
     cudaError_t err = cudaErrorInvalidValue;
     if (xc.fx) {
-      err = launch_vdfdx_fx(f, xc.nx, b->fx_runs, xc.items, xc.n_items, FxColRun{}, xc.W / 2, dt, b->tw_fx, b->tw64, s);
+      err = launch_vdfdx_fx(f, xc.nx, b->fx_runs, xc.items, xc.n_items, FxColRun{}, xc.W / 2, dt, b->fx_tables->tw, b->tw64, s);
       if (err != cudaSuccess) return err;
       continue;
     }
@@ -309,14 +315,6 @@ int batch_sequence(vg_batch* b, double* f, double* e, int nsteps, double* e_hist
     fp_spec.kind[1] = MOM_W;  // v0t^2 = trapz(f v**2.0)
     fp_spec.arg[1] = 0;
   }
-  MomSpec st_spec;
-  st_spec.nm = BATCH_MOMS;
-  const int kinds[BATCH_MOMS] = {MOM_ONE, MOM_V, MOM_W, MOM_SQ, MOM_FLOGF};
-  const int args[BATCH_MOMS] = {0, 0, 1, 0, 0};
-  for (int q = 0; q < BATCH_MOMS; ++q) {
-    st_spec.kind[q] = kinds[q];
-    st_spec.arg[q] = args[q];
-  }
   for (int k = 0; k < nsteps; ++k) {
     // vlapy/core/vlasov_poisson.py:36-58, then the collision step and storage
     B_CHECK(edfdv(0.5 * dt));
@@ -339,7 +337,16 @@ int batch_sequence(vg_batch* b, double* f, double* e, int nsteps, double* e_hist
                         "batch collision solve"));
     const int r = row0 + k;
     if ((e_hist || s_hist) && r >= 0 && r < rows) {
-      B_CHECK(moments(BK_STORE, st_spec, b->mom, BATCH_MOMS));
+      B_CHECK(cuda_status(prof_call(&b->prof, BK_STORE, s, [&] {
+                            for (const auto& c : b->cls) {
+                              const vg_plan view = class_view(b, c);
+                              const cudaError_t err = launch_storage_moments_f64(
+                                  view, f + c.f_off, b->mom + (size_t)c.x_off * BATCH_MOMS, BATCH_MOMS, false, s);
+                              if (err != cudaSuccess) return err;
+                            }
+                            return cudaSuccess;
+                          }),
+                          "batch moments"));
       double* er = e_hist ? e_hist + (size_t)r * b->x_points : nullptr;
       double* sr = s_hist ? s_hist + (size_t)r * b->n_runs * 7 : nullptr;
       B_CHECK(cuda_status(prof_call(&b->prof, BK_STORE, s, [&] {
@@ -437,6 +444,9 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
       c.dv_sq = d.dv_sq;
       c.kv1 = d.kv[1];
       c.kv_uniform = fx_uniform(d.kv, d.nv);
+      std::vector<int2> vp;
+      if (d.nv <= FX_MOMENTS_NV && fx_powers_host(d.v, d.v_pow, d.nv, &vp, &c.fx_pw))
+        B_TRY(b_alloc(b, &c.fx_vp, vp.size(), vp.data(), "batch grids"));
       B_TRY(b_alloc(b, &c.v, d.nv, d.v, "batch grids"));
       B_TRY(b_alloc(b, &c.kv, d.nv, d.kv, "batch grids"));
       B_TRY(b_alloc(b, &c.v_pow, 5 * (size_t)d.nv, d.v_pow, "batch grids"));
@@ -489,7 +499,7 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
   B_TRY(b_alloc<double>(b, &b->bb, bb_need, nullptr, "batch thomas scratch"));
   B_TRY(b_alloc<cx<double>>(b, &b->tw64, FFT_NMAX, nullptr, "twiddles"));
   B_TRY(b_alloc<cx<float>>(b, &b->tw32, FFT_NMAX, nullptr, "twiddles"));
-  B_TRY(b_alloc<fxw>(b, &b->tw_fx, FX_TABLE, fx_table_host(), "fixed-point twiddles"));
+  B_TRY(cuda_status(fx_tables_acquire(&b->fx_tables), "fixed-point tables"));
   {
     vg_plan tmp;
     std::memset(&tmp, 0, sizeof(tmp));

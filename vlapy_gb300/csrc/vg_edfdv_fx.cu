@@ -12,7 +12,9 @@
 // 34 us at 64 x 1024, where half as many threads carry the latency.  RMS error
 // against 128-bit FFTs: 1.1e-16 of the line's RMS at 1024 and 2.7e-16 at 8192
 // (smooth lines), in doubles 3.0e-16 and 3.2e-16.
+#include <algorithm>
 #include <cmath>
+#include <mutex>
 #include <vector>
 
 #include "vg_advect_fx.cuh"
@@ -99,8 +101,8 @@ __global__ void __launch_bounds__(fx_row_block(N), fx_row_block(N) > 256 ? 1 : 2
       n.b2 += q.b2;
     }
   }
-  // (exponent field 1: a line of zeros, or of values that small)
-  const int h = fx_shift_back<N>(n, bad_a || Ea == 1, bad_b || Eb == 1);
+  // (E <= 1: a line of zeros, or of values that small)
+  const int h = fx_shift_back<N>(n, bad_a || Ea <= 1, bad_b || Eb <= 1);
   if (h < 0) {
     sync();
     fx_pair_f64<N>({fa, ea, Ea, true, bad_a}, {fb, eb, Eb, vb, bad_b}, 1, reinterpret_cast<cx<double>*>(s), t, kv, dt,
@@ -205,11 +207,52 @@ std::vector<fxw> build_table() {
   return out;
 }
 
+const std::vector<fxw>& twiddles_host() {
+  static const std::vector<fxw> table = build_table();
+  return table;
+}
+
+std::mutex tables_mu;
+std::vector<FxTables*> tables_held;  // one per device in use
+
 }  // namespace
 
-const fxw* fx_table_host() {
-  static const std::vector<fxw> table = build_table();
-  return table.data();
+cudaError_t fx_tables_acquire(FxTables** out) {
+  *out = nullptr;
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  std::lock_guard<std::mutex> lk(tables_mu);
+  for (FxTables* t : tables_held)
+    if (t->device == dev) {
+      ++t->refs;
+      *out = t;
+      return cudaSuccess;
+    }
+  FxTables t = {dev, 1, nullptr, nullptr};
+  const std::vector<fxw>& tw = twiddles_host();
+  err = cudaMalloc(&t.tw, tw.size() * sizeof(fxw) + FX_LOG_ENTRIES * sizeof(FxLogEntry));
+  if (err != cudaSuccess) return err;
+  t.log = reinterpret_cast<FxLogEntry*>(t.tw + tw.size());
+  err = cudaMemcpy(t.tw, tw.data(), tw.size() * sizeof(fxw), cudaMemcpyHostToDevice);
+  if (err == cudaSuccess)
+    err = cudaMemcpy(t.log, fx_log_host(), FX_LOG_ENTRIES * sizeof(FxLogEntry), cudaMemcpyHostToDevice);
+  if (err != cudaSuccess) {
+    cudaFree(t.tw);
+    return err;
+  }
+  tables_held.push_back(new FxTables(t));
+  *out = tables_held.back();
+  return cudaSuccess;
+}
+
+void fx_tables_release(FxTables* t) {
+  if (!t) return;
+  std::lock_guard<std::mutex> lk(tables_mu);
+  if (--t->refs > 0) return;
+  tables_held.erase(std::find(tables_held.begin(), tables_held.end(), t));
+  cudaFree(t->tw);
+  delete t;
 }
 
 bool fx_make_turn(double k1, double dt, FxTurn* out) {

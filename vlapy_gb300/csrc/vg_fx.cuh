@@ -317,8 +317,9 @@ struct FxPass {
 
 // ---- doubles to fixed point and back ------------------------------------------
 // The largest element of a line decides its scale: element f -> f 2^(1081 - E)
-// with E the exponent field (at least 1), or one less where the largest
-// mantissa is below sqrt(2), so that the largest value is in [2^58.5, 2^59.5).
+// with E the exponent field, or one less where the largest mantissa is below
+// sqrt(2), so that the largest value is in [2^58.5, 2^59.5) (zero and below for
+// lines of subnormal values).
 // (0 for a zero alone)
 __device__ __forceinline__ unsigned fx_exp_bits(double f) {
   return max((unsigned)__double2hiint(f) & 0x7fffffffu, (unsigned)(__double2loint(f) != 0));
@@ -326,7 +327,8 @@ __device__ __forceinline__ unsigned fx_exp_bits(double f) {
 __device__ __forceinline__ int fx_exp(unsigned max_hi) {
   const int e = (int)(max_hi >> 20);
   if (e == 0x7ff) return e;
-  return e < 2 ? 1 : e - ((max_hi & 0xfffff) < 0x6a09e ? 1 : 0);
+  if (e == 0) return max_hi ? __clz(max_hi) == 31 ? -19 : 12 - __clz(max_hi) : 1;  // subnormal: its own leading bit
+  return e == 1 ? 1 : e - ((max_hi & 0xfffff) < 0x6a09e ? 1 : 0);
 }
 constexpr int FX_SCALE = 1081;
 constexpr int FX_NONFINITE = 0x7ff;  // fx_exp of a line with a NaN or infinity

@@ -8,6 +8,7 @@
 #include "vg_common.cuh"
 #include "vg_f32_plan.cuh"
 #include "vg_fft.cuh"
+#include "vg_moments_fx.cuh"
 #include "vlagpu.h"
 
 struct vg_plan {
@@ -28,9 +29,15 @@ struct vg_plan {
   vg::cx<float>* tw32;   // [FFT_NMAX]
   // fixed-point advection: its table (null: none), kv[1] and kx[1], and whether
   // each wavenumber grid is uniform (else the transforms in doubles)
+  vg::FxTables* fx_tables;
   vg::fxw* tw_fx;
   double kv1, kx1;
   int kv_uniform, kx_uniform;
+  // fixed-point storage moments: the velocity powers and the logarithm's table
+  // (null: the moments in doubles)
+  int2* fx_vp;
+  vg::FxPowers fx_pw;
+  vg::FxLogEntry* fx_log;
   int* pw_v;   // NumPy pairwise tree over nv-1 trapz terms
   int* pw_x;   // NumPy pairwise tree over nx values (x-means)
   int pw_v_leaves, pw_x_leaves, pw_v_words, pw_x_words;
@@ -129,6 +136,10 @@ cudaError_t launch_edfdv_sl_f64(const vg_plan& p, const double* fin, const doubl
                                 cudaStream_t s);
 cudaError_t launch_edfdv_cd2_f64(const vg_plan& p, const double* fin, const double* e, double* fout, double dt,
                                  cudaStream_t s);
+// the storage moments of all rows (layout of launch_moments_fx), in fixed point
+// where the plan has its tables, else in doubles
+cudaError_t launch_storage_moments_f64(const vg_plan& p, const double* f, double* out, int stride, bool full,
+                                       cudaStream_t s);
 cudaError_t launch_row_moments_f64(const vg_plan& p, const double* f, const MomSpec& spec,
                                    double* out, int out_stride, cudaStream_t s);
 // e = [driver or pulses(t)] + Re IFFT(i/kx FFT(rho)), rho = 1 - dens (dens_is_density) or dens

@@ -343,17 +343,25 @@ __global__ void __launch_bounds__(256) k_store_modes_f64(const double* __restric
   }
 }
 
-cudaError_t launch_storage_f64(const vg_plan& p, const double* f, const double* e, const double* de,
-                               const vg_history& h, int i, cudaStream_t s) {
+cudaError_t launch_storage_moments_f64(const vg_plan& p, const double* f, double* out, int stride, bool full,
+                                       cudaStream_t s) {
+  if (p.fx_vp && p.nv <= FX_MOMENTS_NV)
+    return launch_moments_fx(f, p.nx, p.nv, p.fx_vp, p.fx_pw, p.fx_log, p.dv, out, stride, full, s);
   MomSpec spec;
-  spec.nm = 8;
   const int kinds[8] = {MOM_ONE, MOM_V, MOM_W, MOM_W, MOM_W, MOM_W, MOM_SQ, MOM_FLOGF};
   const int args[8] = {0, 0, 1, 2, 3, 4, 0, 0};
+  spec.nm = 0;
   for (int q = 0; q < 8; ++q) {
-    spec.kind[q] = kinds[q];
-    spec.arg[q] = args[q];
+    if (!full && q >= 3 && q < 6) continue;
+    spec.kind[spec.nm] = kinds[q];
+    spec.arg[spec.nm++] = args[q];
   }
-  cudaError_t err = launch_row_moments_f64(p, f, spec, p.mom, MOM_STRIDE, s);
+  return launch_row_moments_f64(p, f, spec, out, stride, s);
+}
+
+cudaError_t launch_storage_f64(const vg_plan& p, const double* f, const double* e, const double* de,
+                               const vg_history& h, int i, cudaStream_t s) {
+  cudaError_t err = launch_storage_moments_f64(p, f, p.mom, MOM_STRIDE, true, s);
   if (err != cudaSuccess) return err;
   const size_t smem = (size_t)7 * p.pw_x_leaves * sizeof(double);
   k_fields_series_f64<<<1, 256, smem, s>>>(p.mom, e, de, p.nx, i, h, p.pw_x);

@@ -109,8 +109,8 @@ __global__ void __launch_bounds__(fx_col_block(NX), fx_col_block(NX) > 256 ? 1 :
     __syncthreads();
     n = {red[5 * p + 2], red[5 * p + 3], red[5 * p + 4]};
   }
-  // (exponent field 1: a column of zeros, or of values that small)
-  const int h = fx_shift_back<NX>(n, bad_a || Ea == 1, bad_b || Eb == 1);
+  // (E <= 1: a column of zeros, or of values that small)
+  const int h = fx_shift_back<NX>(n, bad_a || Ea <= 1, bad_b || Eb <= 1);
   if (__syncthreads_or(h < 0)) {
     // a column the fixed-point transform is not exact enough for: the tile's pairs in doubles
     cx<double>* sd = reinterpret_cast<cx<double>*>(smem_raw) + (size_t)p * (sp_len<double>(NX) + COL_PAD);
