@@ -165,7 +165,7 @@ int dev_copy(T** dst, const T* src, size_t n, const char* what) {
 
 void free_plan(vg_plan* p) {
   if (!p) return;
-  void* ptrs[] = {p->x, p->v, p->kx, p->kv, p->inv_kx, p->v_pow, p->f_bg, p->pulses, p->tw64, p->tw32, p->fx_vp,
+  void* ptrs[] = {p->x, p->v, p->kx, p->kv, p->inv_kx, p->v_pow, p->f_bg, p->pulses, p->tw64, p->tw32, p->fx_vp, p->green, p->green_e,
                   p->pw_v, p->pw_x, p->dens, p->mom, p->bb, p->rho, p->etmp, p->sl_m, p->sl_w, p->flags};
   for (void* q : ptrs)
     if (q) cudaFree(q);
@@ -649,6 +649,11 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
   TRY(dev_copy<double>(&p->rho, nullptr, nx, "scratch"));
   TRY(dev_copy<double>(&p->etmp, nullptr, 4 * nx + 4, "scratch"));
   TRY(dev_copy<int>(&p->flags, nullptr, 1, "status"));
+  if (d->nx <= POISSON_FX_NX) {
+    TRY(dev_copy<int2>(&p->green, nullptr, nx, "Green's function"));
+    TRY(dev_copy<int>(&p->green_e, nullptr, 1, "Green's function"));
+    TRY(cuda_status(build_poisson_fx(p->inv_kx, d->nx, 1, p->green, p->green_e, p->etmp, 0), "Green's function"));
+  }
   if (d->precision == VG_F64 && d->collision != VG_COLL_NONE)
     TRY(dev_copy<double>(&p->bb, nullptr, 2 * nx * thomas_pad(d->nv), "thomas scratch"));
   if (d->precision == VG_F32_DELTA_F) TRY(setup_f32(p, d));

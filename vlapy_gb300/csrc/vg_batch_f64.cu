@@ -34,7 +34,6 @@ struct BatchRunDev {
   int x_off;        // x points before this run
   int run;          // index in the caller's order (series row)
   const double* kx;
-  const double* inv_kx;
   const double* v;  // the v grid of the run's nv class
   const int* pw_x;  // pairwise table over nx (x-means)
 };
@@ -50,22 +49,6 @@ __global__ void __launch_bounds__(col_seqs<double>(NX) * fft_threads<double>(NX)
   const int2 it = items[blockIdx.x];
   const BatchRunDev r = runs[it.x];
   vdfdx_tile_body<NX>(f + r.f_off, r.nv, it.y * W, W, r.kx, r.v, dt, tw, smem_raw);
-}
-
-// spectral Poisson of one run per CTA (one kernel per nx class); no driver
-template <int NX>
-__global__ void __launch_bounds__(fft_threads<double>(NX))
-    k_batch_poisson(const BatchRunDev* __restrict__ runs, const int* __restrict__ ids,
-                    const double* __restrict__ dens, const cx<double>* __restrict__ tw, double* e,
-                    int* flags) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const BatchRunDev r = runs[ids[blockIdx.x]];
-  FieldTimeDev ft;
-  ft.t_ptr = nullptr;
-  ft.t_host = 0.0;
-  ft.nadd = 0;
-  poisson_fft_body<NX>(dens + r.x_off, 1, r.inv_kx, nullptr, 0, nullptr, 0, nullptr, ft, tw, e + r.x_off,
-                       reinterpret_cast<cx<double>*>(smem_raw), threadIdx.x, flags);
 }
 
 // e history row and the seven series of one run per CTA: the x-means of n, j, T,
@@ -142,8 +125,11 @@ struct vg_batch {
     bool fx;  // every run's kx is uniform: the fixed-point x-drift
     int2* items;
     int n_items;
-    int* ids;
     int n_ids;
+    // Poisson solve: the runs' x offsets and Green's functions, in list order
+    int* x_offs;
+    int2* green;
+    int* green_e;
   };
   std::vector<XCls> xcls;
   std::map<std::tuple<const void*, const void*, int, const void*, const void*, int, int, cudaStream_t>,
@@ -223,16 +209,6 @@ cudaError_t batch_vdfdx_launch(const vg_batch* b, const vg_batch::XCls& xc, doub
   return cudaGetLastError();
 }
 
-template <int NX>
-cudaError_t batch_poisson_launch(const vg_batch* b, const vg_batch::XCls& xc, double* e, cudaStream_t s) {
-  constexpr int G = fft_threads<double>(NX);
-  const size_t smem = (size_t)sp_len<double>(NX) * sizeof(cx<double>);
-  cudaError_t err = ensure_smem((const void*)k_batch_poisson<NX>, smem);
-  if (err != cudaSuccess) return err;
-  k_batch_poisson<NX><<<xc.n_ids, G, smem, s>>>(b->runs, xc.ids, b->dens, b->tw64, e, b->flags);
-  return cudaGetLastError();
-}
-
 #define VG_BATCH_NX_CASES(M, ...) \
   M(2, __VA_ARGS__) M(4, __VA_ARGS__) M(8, __VA_ARGS__) M(16, __VA_ARGS__) M(32, __VA_ARGS__) \
   M(64, __VA_ARGS__) M(128, __VA_ARGS__) M(256, __VA_ARGS__) M(512, __VA_ARGS__) M(1024, __VA_ARGS__)
@@ -259,14 +235,8 @@ cudaError_t batch_vdfdx_all(const vg_batch* b, double* f, double dt, cudaStream_
 
 cudaError_t batch_poisson_all(const vg_batch* b, double* e, cudaStream_t s) {
   for (const auto& xc : b->xcls) {
-    cudaError_t err = cudaErrorInvalidValue;
-    switch (xc.nx) {
-#define CASE(NX, ...) \
-  case NX: err = batch_poisson_launch<NX>(b, xc, e, s); break;
-      VG_BATCH_NX_CASES(CASE, 0)
-#undef CASE
-      default: break;
-    }
+    const cudaError_t err =
+        launch_poisson_fx_runs(xc.x_offs, xc.n_ids, b->dens, xc.nx, {xc.green, xc.green_e}, e, b->flags, s);
     if (err != cudaSuccess) return err;
   }
   return cudaSuccess;
@@ -427,7 +397,7 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
     }                  \
   } while (0)
   std::vector<BatchRunDev> rd(n_runs);
-  std::vector<double> kx_all, inv_all, nudt_row;
+  std::vector<double> kx_all, nudt_row;
   std::map<int, int*> pw_x_of;
   long long cells = 0;
   int xoff = 0;
@@ -474,7 +444,6 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
     r.v = c.v;
     r.pw_x = pw_x_of[d.nx];
     kx_all.insert(kx_all.end(), d.kx, d.kx + d.nx);
-    inv_all.insert(inv_all.end(), d.one_over_kx, d.one_over_kx + d.nx);
     // nu * dt as vg_plan_create forms it; 0 leaves the run's rows as they are
     const double nudt = (d.collision != VG_COLL_NONE && d.nu > 0.0) ? d.nu * d.dt : 0.0;
     nudt_row.insert(nudt_row.end(), (size_t)d.nx, nudt);
@@ -483,12 +452,10 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
   }
   b->cells = cells;
   b->x_points = xoff;
-  double *kx_d = nullptr, *inv_d = nullptr;
+  double* kx_d = nullptr;
   B_TRY(b_alloc(b, &kx_d, kx_all.size(), kx_all.data(), "batch grids"));
-  B_TRY(b_alloc(b, &inv_d, inv_all.size(), inv_all.data(), "batch grids"));
   for (int i = 0; i < n_runs; ++i) {
     rd[i].kx = kx_d + rd[i].x_off;
-    rd[i].inv_kx = inv_d + rd[i].x_off;
   }
   B_TRY(b_alloc(b, &b->runs, rd.size(), rd.data(), "batch runs"));
   B_TRY(b_alloc(b, &b->nudt_row, nudt_row.size(), nudt_row.data(), "batch runs"));
@@ -537,7 +504,23 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
     xc.n_items = (int)kv.second.first.size();
     xc.n_ids = (int)kv.second.second.size();
     B_TRY(b_alloc(b, &xc.items, kv.second.first.size(), kv.second.first.data(), "batch work list"));
-    B_TRY(b_alloc(b, &xc.ids, kv.second.second.size(), kv.second.second.data(), "batch work list"));
+    // the Green's functions of the class's runs, from their inv_kx in list order
+    std::vector<int> offs;
+    std::vector<double> inv;
+    for (int id : kv.second.second) {
+      offs.push_back(rd[id].x_off);
+      inv.insert(inv.end(), runs[id].one_over_kx, runs[id].one_over_kx + xc.nx);
+    }
+    double *inv_x = nullptr, *work = nullptr;
+    B_TRY(b_alloc(b, &xc.x_offs, offs.size(), offs.data(), "batch work list"));
+    B_TRY(b_alloc(b, &inv_x, inv.size(), inv.data(), "batch grids"));
+    B_TRY(b_alloc<double>(b, &work, inv.size(), nullptr, "batch grids"));
+    B_TRY(b_alloc<int2>(b, &xc.green, inv.size(), nullptr, "batch grids"));
+    B_TRY(b_alloc<int>(b, &xc.green_e, offs.size(), nullptr, "batch grids"));
+    for (int r0 = 0; r0 < xc.n_ids; r0 += 65535)
+      B_TRY(cuda_status(build_poisson_fx(inv_x + (size_t)r0 * xc.nx, xc.nx, std::min(65535, xc.n_ids - r0),
+                                         xc.green + (size_t)r0 * xc.nx, xc.green_e + r0, work + (size_t)r0 * xc.nx, 0),
+                        "batch grids"));
     b->xcls.push_back(xc);
   }
   B_TRY(cuda_status(cudaDeviceSynchronize(), "batch setup"));

@@ -123,6 +123,13 @@ struct FieldTimeDev {
   double add[6];
 };
 
+// the Poisson solve by the plan's Green's function, and of many runs of one nx
+// (vg_poisson_fx.cu)
+cudaError_t launch_poisson_fx(const vg_plan& p, const double* dens, int is_density, const double* driver,
+                              const FieldTimeDev& ft, int use_pulses, double* e, cudaStream_t s);
+cudaError_t launch_poisson_fx_runs(const int* x_off, int n_runs, const double* dens, int nx, const PoissonFx& t,
+                                   double* e, int* flags, cudaStream_t s);
+
 __device__ __forceinline__ double field_time(const FieldTimeDev& ft) {
   double t = ft.t_ptr ? *ft.t_ptr : ft.t_host;
   for (int i = 0; i < ft.nadd; ++i) t = add_rn(t, ft.add[i]);

@@ -98,6 +98,23 @@ __device__ __forceinline__ fx fx_down(fx a) {
   return {fx_down<D>(a.x), fx_down<D>(a.y)};
 }
 
+// A sum in 96 bits, so that products near 2^61 add up exactly
+struct Acc96 {
+  unsigned long long lo;
+  int hi;
+};
+__device__ __forceinline__ void acc_add(Acc96& s, long long x) {
+  asm("add.cc.u64 %0, %0, %2;\n\taddc.s32 %1, %1, %3;" : "+l"(s.lo), "+r"(s.hi) : "l"(x), "r"((int)(x >> 63)));
+}
+__device__ __forceinline__ void acc_add96(Acc96& s, const Acc96& o) {
+  asm("add.cc.u64 %0, %0, %2;\n\taddc.s32 %1, %1, %3;" : "+l"(s.lo), "+r"(s.hi) : "l"(o.lo), "r"(o.hi));
+}
+// rounded once: the sum in two parts of 48 bits
+__device__ __forceinline__ double acc_to_double(const Acc96& s) {
+  const long long up = ((long long)s.hi << 16) | (long long)(s.lo >> 48);
+  return fma((double)up, 281474976710656.0, (double)(long long)(s.lo & 0xffffffffffffull));  // 2^48
+}
+
 // cos(2 pi j / 16), j = 0..4, in Q62
 constexpr long long FX_ONE = 1ll << 62;
 constexpr long long FX_C1 = 4260642322793532497ll;   // cos(pi / 8)

@@ -9,6 +9,7 @@
 #include "vg_f32_plan.cuh"
 #include "vg_fft.cuh"
 #include "vg_moments_fx.cuh"
+#include "vg_poisson_fx.cuh"
 #include "vlagpu.h"
 
 struct vg_plan {
@@ -38,6 +39,9 @@ struct vg_plan {
   int2* fx_vp;
   vg::FxPowers fx_pw;
   vg::FxLogEntry* fx_log;
+  // Green's function of the Poisson solve (null: by transforms)
+  int2* green;
+  int* green_e;
   int* pw_v;   // NumPy pairwise tree over nv-1 trapz terms
   int* pw_x;   // NumPy pairwise tree over nx values (x-means)
   int pw_v_leaves, pw_x_leaves, pw_v_words, pw_x_words;

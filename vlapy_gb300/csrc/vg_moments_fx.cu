@@ -26,14 +26,6 @@ namespace vg {
 
 namespace {
 
-// A thread's sum: 96 bits, so that products at 2^60.5 add up exactly
-struct Acc96 {
-  unsigned long long lo;
-  int hi;
-};
-__device__ __forceinline__ void acc_add(Acc96& s, long long x) {
-  asm("add.cc.u64 %0, %0, %2;\n\taddc.s32 %1, %1, %3;" : "+l"(s.lo), "+r"(s.hi) : "l"(x), "r"((int)(x >> 63)));
-}
 struct Sum96 {
   long long hi, lo;  // hi 2^48 + lo
 };
@@ -231,8 +223,9 @@ bool fx_powers_host(const double* v, const double* v_pow, int nv, std::vector<in
     if (mx == 0.0) e = 0;
     if (e > 900 || e < -900) return false;
     pw->e[p] = e;
+    const double up = std::ldexp(1.0, 62 - e);
     for (int j = 0; j < nv; ++j) {
-      const long long q = (long long)std::llrint(std::ldexp(a[j], 62 - e));
+      const long long q = (long long)std::llrint(a[j] * up);
       (*out)[(size_t)p * nv + j] = make_int2(fx_hi(q), fx_lo(q));
     }
   }

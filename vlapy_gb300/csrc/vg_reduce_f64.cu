@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(fft_threads<double>(NX)) k_poisson_fft_f64(
                        reinterpret_cast<cx<double>*>(smem_raw), threadIdx.x, flags);
 }
 
-// Direct DFT for lengths that are not powers of two (O(nx^2), one CTA).
+// Direct DFT for the other lengths past the Green's function's (O(nx^2), one CTA).
 __global__ void k_poisson_dft_f64(const double* __restrict__ dens, int is_density, int nx,
                                   const double* __restrict__ inv_kx, const double* __restrict__ driver,
                                   int use_pulses, const vg_pulse* __restrict__ P, int np,
@@ -205,24 +205,8 @@ cudaError_t poisson_n(const vg_plan& p, const double* dens, int is_density, cons
 
 cudaError_t launch_poisson_f64(const vg_plan& p, const double* dens, int is_density, const double* driver,
                                const FieldTime& ft, double* e, cudaStream_t s) {
-  if (p.nx_pow2 && p.nx <= 8192) {
-    switch (ilog2(p.nx)) {
-      case 1: return poisson_n<2>(p, dens, is_density, driver, ft, e, s);
-      case 2: return poisson_n<4>(p, dens, is_density, driver, ft, e, s);
-      case 3: return poisson_n<8>(p, dens, is_density, driver, ft, e, s);
-      case 4: return poisson_n<16>(p, dens, is_density, driver, ft, e, s);
-      case 5: return poisson_n<32>(p, dens, is_density, driver, ft, e, s);
-      case 6: return poisson_n<64>(p, dens, is_density, driver, ft, e, s);
-      case 7: return poisson_n<128>(p, dens, is_density, driver, ft, e, s);
-      case 8: return poisson_n<256>(p, dens, is_density, driver, ft, e, s);
-      case 9: return poisson_n<512>(p, dens, is_density, driver, ft, e, s);
-      case 10: return poisson_n<1024>(p, dens, is_density, driver, ft, e, s);
-      case 11: return poisson_n<2048>(p, dens, is_density, driver, ft, e, s);
-      case 12: return poisson_n<4096>(p, dens, is_density, driver, ft, e, s);
-      case 13: return poisson_n<8192>(p, dens, is_density, driver, ft, e, s);
-      default: break;
-    }
-  }
+  if (p.green) return launch_poisson_fx(p, dens, is_density, driver, to_dev(ft), ft.use_pulses, e, s);
+  if (p.nx == 8192) return poisson_n<8192>(p, dens, is_density, driver, ft, e, s);
   k_poisson_dft_f64<<<1, 256, 0, s>>>(dens, is_density, p.nx, p.inv_kx, driver, ft.use_pulses, p.pulses,
                                       p.n_pulses, p.x, to_dev(ft), p.etmp, e, p.flags);
   return cudaGetLastError();
