@@ -205,8 +205,26 @@ cudaError_t poisson_n(const vg_plan& p, const double* dens, int is_density, cons
 
 cudaError_t launch_poisson_f64(const vg_plan& p, const double* dens, int is_density, const double* driver,
                                const FieldTime& ft, double* e, cudaStream_t s) {
+  // (transforms: nx = 8192, and the solve without allocation, which has no table)
   if (p.green) return launch_poisson_fx(p, dens, is_density, driver, to_dev(ft), ft.use_pulses, e, s);
-  if (p.nx == 8192) return poisson_n<8192>(p, dens, is_density, driver, ft, e, s);
+  if (p.nx_pow2 && p.nx <= 8192) {
+    switch (ilog2(p.nx)) {
+      case 1: return poisson_n<2>(p, dens, is_density, driver, ft, e, s);
+      case 2: return poisson_n<4>(p, dens, is_density, driver, ft, e, s);
+      case 3: return poisson_n<8>(p, dens, is_density, driver, ft, e, s);
+      case 4: return poisson_n<16>(p, dens, is_density, driver, ft, e, s);
+      case 5: return poisson_n<32>(p, dens, is_density, driver, ft, e, s);
+      case 6: return poisson_n<64>(p, dens, is_density, driver, ft, e, s);
+      case 7: return poisson_n<128>(p, dens, is_density, driver, ft, e, s);
+      case 8: return poisson_n<256>(p, dens, is_density, driver, ft, e, s);
+      case 9: return poisson_n<512>(p, dens, is_density, driver, ft, e, s);
+      case 10: return poisson_n<1024>(p, dens, is_density, driver, ft, e, s);
+      case 11: return poisson_n<2048>(p, dens, is_density, driver, ft, e, s);
+      case 12: return poisson_n<4096>(p, dens, is_density, driver, ft, e, s);
+      case 13: return poisson_n<8192>(p, dens, is_density, driver, ft, e, s);
+      default: break;
+    }
+  }
   k_poisson_dft_f64<<<1, 256, 0, s>>>(dens, is_density, p.nx, p.inv_kx, driver, ft.use_pulses, p.pulses,
                                       p.n_pulses, p.x, to_dev(ft), p.etmp, e, p.flags);
   return cudaGetLastError();
