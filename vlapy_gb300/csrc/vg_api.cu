@@ -228,21 +228,8 @@ cudaError_t prof_run(vg_plan* p, int kind, cudaStream_t s, Fn fn) {
 // One FP step: moments of the operator, then the tridiagonal solve.
 int collision_f64(vg_plan* p, double* f, cudaStream_t s) {
   if (p->collision == VG_COLL_NONE) return VG_OK;
-  MomSpec spec;
-  if (p->collision == VG_COLL_DG) {
-    spec.nm = 2;
-    spec.kind[0] = MOM_V;   // vbar = trapz(f v)
-    spec.arg[0] = 0;
-    spec.kind[1] = MOM_DG2; // v0t^2 = trapz(f (v - vbar)^2)
-    spec.arg[1] = 0;
-  } else {
-    spec.nm = 2;
-    spec.kind[0] = MOM_ONE;  // unused slot, keeps the column layout of the DG case
-    spec.arg[0] = 0;
-    spec.kind[1] = MOM_W;    // v0t^2 = trapz(f v**2.0)
-    spec.arg[1] = 0;
-  }
-  VG_CHECK(cuda_status(prof_run(p, PK_FP_MOMENTS, s, [&] { return launch_row_moments_f64(*p, f, spec, p->mom, MOM_STRIDE, s); }),
+  const int op = p->collision == VG_COLL_DG ? TRAPZ_DG : TRAPZ_LB;
+  VG_CHECK(cuda_status(prof_run(p, PK_FP_MOMENTS, s, [&] { return launch_trapz_f64(*p, op, f, p->mom, MOM_STRIDE, s); }),
                        "collision moments"));
   return cuda_status(prof_run(p, PK_FP_SOLVE, s, [&] {
                        return launch_thomas_f64(f, p->nx, p->nv, p->v, p->mom, MOM_STRIDE, 0, 1,
@@ -253,11 +240,7 @@ int collision_f64(vg_plan* p, double* f, cudaStream_t s) {
 
 int field_f64(vg_plan* p, const double* f, const double* driver, const FieldTime& ft, double* e,
               cudaStream_t s) {
-  MomSpec spec;
-  spec.nm = 1;
-  spec.kind[0] = MOM_ONE;
-  spec.arg[0] = 0;
-  VG_CHECK(cuda_status(prof_run(p, PK_DENSITY, s, [&] { return launch_row_moments_f64(*p, f, spec, p->dens, 1, s); }),
+  VG_CHECK(cuda_status(prof_run(p, PK_DENSITY, s, [&] { return launch_trapz_f64(*p, TRAPZ_DENSITY, f, p->dens, 1, s); }),
                        "charge density"));
   return cuda_status(prof_run(p, PK_POISSON, s, [&] { return launch_poisson_f64(*p, p->dens, 1, driver, ft, e, s); }),
                      "poisson");
@@ -780,11 +763,7 @@ int vg_charge_density(vg_plan* p, const void* f, double* n, vg_stream stream) {
   if (p->f32)
     return cuda_status(launch_dens_rows_f32(*p, static_cast<const float*>(f), n, 1, (cudaStream_t)stream),
                        "charge density");
-  MomSpec spec;
-  spec.nm = 1;
-  spec.kind[0] = MOM_ONE;
-  spec.arg[0] = 0;
-  return cuda_status(launch_row_moments_f64(*p, static_cast<const double*>(f), spec, n, 1, (cudaStream_t)stream),
+  return cuda_status(launch_trapz_f64(*p, TRAPZ_DENSITY, static_cast<const double*>(f), n, 1, (cudaStream_t)stream),
                      "charge density");
 }
 

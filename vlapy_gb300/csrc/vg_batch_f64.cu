@@ -256,45 +256,29 @@ int batch_sequence(vg_batch* b, double* f, double* e, int nsteps, double* e_hist
                        }),
                        "batch edfdv");
   };
-  auto moments = [&](int kind, const MomSpec& spec, double* out, int stride) {
+  auto moments = [&](int kind, int op, double* out, int stride) {
     return cuda_status(prof_call(&b->prof, kind, s, [&] {
                          for (const auto& c : b->cls) {
                            const vg_plan view = class_view(b, c);
                            cudaError_t err =
-                               launch_row_moments_f64(view, f + c.f_off, spec, out + (size_t)c.x_off * stride, stride, s);
+                               launch_trapz_f64(view, op, f + c.f_off, out + (size_t)c.x_off * stride, stride, s);
                            if (err != cudaSuccess) return err;
                          }
                          return cudaSuccess;
                        }),
                        "batch moments");
   };
-  MomSpec dens_spec;
-  dens_spec.nm = 1;
-  dens_spec.kind[0] = MOM_ONE;
-  dens_spec.arg[0] = 0;
-  MomSpec fp_spec;
-  fp_spec.nm = 2;
-  if (b->collision == VG_COLL_DG) {
-    fp_spec.kind[0] = MOM_V;  // vbar = trapz(f v)
-    fp_spec.arg[0] = 0;
-    fp_spec.kind[1] = MOM_DG2;  // v0t^2 = trapz(f (v - vbar)^2)
-    fp_spec.arg[1] = 0;
-  } else {
-    fp_spec.kind[0] = MOM_ONE;  // unused slot (LB has no drift)
-    fp_spec.arg[0] = 0;
-    fp_spec.kind[1] = MOM_W;  // v0t^2 = trapz(f v**2.0)
-    fp_spec.arg[1] = 0;
-  }
+  const int fp_op = b->collision == VG_COLL_DG ? TRAPZ_DG : TRAPZ_LB;
   for (int k = 0; k < nsteps; ++k) {
     // vlapy/core/vlasov_poisson.py:36-58, then the collision step and storage
     B_CHECK(edfdv(0.5 * dt));
     B_CHECK(cuda_status(prof_call(&b->prof, BK_VDFDX, s, [&] { return batch_vdfdx_all(b, f, dt, s); }),
                         "batch vdfdx"));
-    B_CHECK(moments(BK_DENSITY, dens_spec, b->dens, 1));
+    B_CHECK(moments(BK_DENSITY, TRAPZ_DENSITY, b->dens, 1));
     B_CHECK(cuda_status(prof_call(&b->prof, BK_POISSON, s, [&] { return batch_poisson_all(b, e, s); }),
                         "batch poisson"));
     B_CHECK(edfdv(0.5 * dt));
-    B_CHECK(moments(BK_FP_MOMENTS, fp_spec, b->fpmom, 2));
+    B_CHECK(moments(BK_FP_MOMENTS, fp_op, b->fpmom, 2));
     B_CHECK(cuda_status(prof_call(&b->prof, BK_FP_SOLVE, s, [&] {
                           for (const auto& c : b->cls) {
                             const cudaError_t err = launch_thomas_f64(

@@ -144,6 +144,10 @@ cudaError_t launch_edfdv_cd2_f64(const vg_plan& p, const double* fin, const doub
 // where the plan has its tables, else in doubles
 cudaError_t launch_storage_moments_f64(const vg_plan& p, const double* f, double* out, int stride, bool full,
                                        cudaStream_t s);
+// the density, or the collision operators' moments (columns 0: vbar, 1: v0t^2;
+// column 0 is not written for LB), as NumPy sums them
+enum TrapzOp { TRAPZ_DENSITY = 0, TRAPZ_DG = 1, TRAPZ_LB = 2 };
+cudaError_t launch_trapz_f64(const vg_plan& p, int op, const double* f, double* out, int stride, cudaStream_t s);
 cudaError_t launch_row_moments_f64(const vg_plan& p, const double* f, const MomSpec& spec,
                                    double* out, int out_stride, cudaStream_t s);
 // e = [driver or pulses(t)] + Re IFFT(i/kx FFT(rho)), rho = 1 - dens (dens_is_density) or dens

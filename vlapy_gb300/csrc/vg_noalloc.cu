@@ -192,11 +192,7 @@ extern "C" int vg_field_solve_noalloc(const double* f, int32_t nx, int32_t nv, d
   view.pw_v_leaves = leaves;
   view.dens = reinterpret_cast<double*>(base + NA_DENS_OFF);
   view.etmp = reinterpret_cast<double*>(base + NA_ETMP_OFF);
-  MomSpec spec;
-  spec.nm = 1;
-  spec.kind[0] = MOM_ONE;
-  spec.arg[0] = 0;
-  st = cuda_status(launch_row_moments_f64(view, f, spec, view.dens, 1, s), "no-alloc density");
+  st = cuda_status(launch_trapz_f64(view, TRAPZ_DENSITY, f, view.dens, 1, s), "no-alloc density");
   if (st != VG_OK) return st;
   FieldTime ft{};
   ft.use_pulses = 0;

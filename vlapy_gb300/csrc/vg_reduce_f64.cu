@@ -98,6 +98,135 @@ __global__ void k_row_moments_f64(const double* __restrict__ f, int nv, const do
   }
 }
 
+// ---------------------------------------------------------------------------
+// the density and the collision operator's moments, NumPy's sums bit for bit
+// ---------------------------------------------------------------------------
+
+// sum of the nv - 1 trapz terms dv (p_{j+1} + p_j) / 2 of the products p in NumPy's
+// order, in every thread.  All threads form the terms; eight lanes then run a
+// leaf's eight accumulators, and one thread the combine program, its stack in
+// place of the leaves it has taken.  The halving is left to the end (exact; a
+// factor of two commutes with every rounding above the subnormal range).
+// p: nv products in shared memory, or the row itself in global memory.
+__device__ __forceinline__ double trapz_exact(const double* p, int nv, double dv, const int* __restrict__ table,
+                                              double* term, double* leaf, double* result) {
+  for (int j = threadIdx.x; j < nv - 1; j += blockDim.x) term[j] = mul_rn(dv, add_rn(p[j + 1], p[j]));
+  __syncthreads();
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nl = table[0], np = table[1];
+  const int* leaves = table + 2;
+  const int a = lane & 7;
+  for (int L0 = 4 * w; L0 < nl; L0 += 4 * (blockDim.x >> 5)) {
+    const int L = L0 + (lane >> 3);
+    const int st = L < nl ? leaves[2 * L] : 0, len = L < nl ? leaves[2 * L + 1] : 0;
+    const int stop = len - (len % 8);
+    double x = 0.0;
+    if (len < 8) {
+      if (a == 0)
+        for (int i = 0; i < len; ++i) x = add_rn(x, term[st + i]);
+    } else {
+      x = term[st + a];
+      for (int i = 8 + a; i < stop; i += 8) x = add_rn(x, term[st + i]);
+    }
+    double r = x;
+#pragma unroll
+    for (int m = 1; m < 8; m <<= 1) {
+      const double o = __shfl_down_sync(0xffffffffu, r, m, 8);
+      r = add_rn(r, o);
+    }
+    if (a == 0 && L < nl) {
+      if (len < 8) r = x;
+      else
+        for (int i = stop; i < len; ++i) r = add_rn(r, term[st + i]);
+      leaf[L] = r;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const int* prog = leaves + 2 * nl;
+    int sp = 0;
+    for (int i = 0; i < np; ++i) {
+      const int op = prog[i];
+      if (op >= 0) {
+        leaf[sp++] = leaf[op];  // op >= sp: the stack never passes the leaves taken
+      } else {
+        --sp;
+        leaf[sp - 1] = add_rn(leaf[sp - 1], leaf[sp]);
+      }
+    }
+    *result = nv > 1 ? leaf[0] * 0.5 : 0.0;
+  }
+  __syncthreads();
+  return *result;
+}
+
+// One CTA per row.  DENSITY: out[0] = trapz f.  DG: out[0] = vbar = trapz(f v),
+// out[1] = trapz(f (v - vbar)^2).  LB: out[1] = trapz(f v^2.0).  Three FP64
+// instructions per cell for the sum and one or three for the product; the
+// general kernel above spends one more per moment and leaves the terms to the
+// chains' few threads (2048 x 4096: density 137 -> 79 us, DG 353 -> 260 us;
+// 64 x 1024: DG 19 -> 13 us).
+template <int OP>
+__global__ void __launch_bounds__(256) k_trapz_f64(const double* __restrict__ f, int nv, const double* __restrict__ v,
+                                                   const double* __restrict__ v2, const int* __restrict__ table,
+                                                   double dv, double* __restrict__ out, int stride) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double res[2];
+  double* term = reinterpret_cast<double*>(smem_raw);  // [nv]
+  double* leaf = term + nv;                            // [n_leaves]
+  double* prod = leaf + table[0];                      // [nv] (DG, LB)
+  const double* fr = f + (size_t)blockIdx.x * nv;
+  double* o = out + (size_t)blockIdx.x * stride;
+  if constexpr (OP == TRAPZ_DENSITY) {
+    const double n = trapz_exact(fr, nv, dv, table, term, leaf, &res[0]);
+    if (threadIdx.x == 0) o[0] = n;
+  } else if constexpr (OP == TRAPZ_LB) {
+    for (int j = threadIdx.x; j < nv; j += blockDim.x) prod[j] = mul_rn(fr[j], v2[j]);
+    __syncthreads();
+    const double t = trapz_exact(prod, nv, dv, table, term, leaf, &res[0]);
+    if (threadIdx.x == 0) o[1] = t;
+  } else {
+    for (int j = threadIdx.x; j < nv; j += blockDim.x) prod[j] = mul_rn(fr[j], v[j]);
+    __syncthreads();
+    const double vbar = trapz_exact(prod, nv, dv, table, term, leaf, &res[0]);
+    for (int j = threadIdx.x; j < nv; j += blockDim.x) {
+      const double d = sub_rn(v[j], vbar);
+      prod[j] = mul_rn(fr[j], mul_rn(d, d));
+    }
+    __syncthreads();
+    const double t = trapz_exact(prod, nv, dv, table, term, leaf, &res[1]);
+    if (threadIdx.x == 0) {
+      o[0] = vbar;
+      o[1] = t;
+    }
+  }
+}
+
+cudaError_t launch_trapz_f64(const vg_plan& p, int op, const double* f, double* out, int stride, cudaStream_t s) {
+  const size_t smem = ((op == TRAPZ_DENSITY ? 1 : 2) * (size_t)p.nv + (size_t)p.pw_v_leaves) * sizeof(double);
+  if (smem > ((size_t)220 << 10)) {
+    // longer rows: the general kernel
+    MomSpec spec = {};
+    spec.nm = op == TRAPZ_DENSITY ? 1 : 2;
+    spec.kind[0] = op == TRAPZ_DG ? MOM_V : MOM_ONE;
+    spec.kind[1] = op == TRAPZ_DG ? MOM_DG2 : MOM_W;
+    return launch_row_moments_f64(p, f, spec, out, stride, s);
+  }
+  const void* k = op == TRAPZ_DENSITY ? (const void*)k_trapz_f64<TRAPZ_DENSITY>
+                : op == TRAPZ_DG      ? (const void*)k_trapz_f64<TRAPZ_DG>
+                                      : (const void*)k_trapz_f64<TRAPZ_LB>;
+  cudaError_t err = ensure_smem(k, smem);
+  if (err != cudaSuccess) return err;
+  const int block = p.nv >= 1024 ? 256 : p.nv >= 512 ? 128 : 64;
+  if (op == TRAPZ_DENSITY)
+    k_trapz_f64<TRAPZ_DENSITY><<<p.nx, block, smem, s>>>(f, p.nv, p.v, p.v_pow, p.pw_v, p.dv, out, stride);
+  else if (op == TRAPZ_DG)
+    k_trapz_f64<TRAPZ_DG><<<p.nx, block, smem, s>>>(f, p.nv, p.v, p.v_pow, p.pw_v, p.dv, out, stride);
+  else
+    k_trapz_f64<TRAPZ_LB><<<p.nx, block, smem, s>>>(f, p.nv, p.v, p.v_pow, p.pw_v, p.dv, out, stride);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_row_moments_f64(const vg_plan& p, const double* f, const MomSpec& spec,
                                    double* out, int out_stride, cudaStream_t s) {
   // products of as many moments at once as fit in 64 KB (at least one)
