@@ -174,13 +174,15 @@ cudaError_t vdfdx_n(const vg_plan& p, double* f, double dt, cudaStream_t s) {
   M(6, __VA_ARGS__) M(7, __VA_ARGS__) M(8, __VA_ARGS__) M(9, __VA_ARGS__) M(10, __VA_ARGS__) \
   M(11, __VA_ARGS__) M(12, __VA_ARGS__) M(13, __VA_ARGS__)
 
-// Powers of two on a uniform wavenumber grid (the reference's fftfreq) go
-// through the fixed-point transforms of vg_fx.cuh; a caller's own grid takes
-// the transforms in doubles below.
+// A uniform wavenumber grid (the reference's fftfreq) goes through the
+// fixed-point transforms, powers of two by vg_fx.cuh's and other lengths by
+// vg_dft_fx.cu's; a caller's own grid takes the transforms in doubles below.
 cudaError_t launch_edfdv_f64(const vg_plan& p, double* f, const double* e, double dt, cudaStream_t s) {
   FxTurn turn;
   if (p.nv_pow2 && p.tw_fx && p.kv_uniform && fx_make_turn(p.kv1, dt, &turn))
     return launch_edfdv_fx(f, p.nx, p.nv, e, turn, p.tw_fx, p.kv, dt, p.tw64, s);
+  if (!p.nv_pow2 && p.dft_v && p.kv_uniform && fx_make_turn(p.kv1, dt, &turn))
+    return launch_dft_fx(f, p.nv, p.nx, 1, p.nv, e, turn, p.tw_fx, p.dft_v, p.dft_work, s);
   if (!p.nv_pow2) return dft_advect(f, p.nv, p.nx, 1, p.nv, p.kv, e, dt, s);
   switch (ilog2(p.nv)) {
 #define CASE(L, ...) case L: return edfdv_n<(1 << L)>(p, f, e, dt, s);
@@ -194,6 +196,8 @@ cudaError_t launch_vdfdx_f64(const vg_plan& p, double* f, double dt, cudaStream_
   FxColRun run = {0, p.nv, p.v, p.kx, {}};
   if (p.nx_pow2 && p.tw_fx && p.kx_uniform && fx_make_turn(p.kx1, dt, &run.turn))
     return launch_vdfdx_fx(f, p.nx, nullptr, nullptr, 0, run, fx_col_pairs(p.nx, (p.nv + 1) / 2), dt, p.tw_fx, p.tw64, s);
+  if (!p.nx_pow2 && p.dft_x && p.kx_uniform && fx_make_turn(p.kx1, dt, &run.turn))
+    return launch_dft_fx(f, p.nx, p.nv, p.nv, 1, p.v, run.turn, p.tw_fx, p.dft_x, p.dft_work, s);
   if (!p.nx_pow2) return dft_advect(f, p.nx, p.nv, p.nv, 1, p.kx, p.v, dt, s);
   switch (ilog2(p.nx)) {
 #define CASE(L, ...) case L: return vdfdx_n<(1 << L)>(p, f, dt, s);

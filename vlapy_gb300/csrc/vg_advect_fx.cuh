@@ -45,4 +45,13 @@ int fx_col_pairs(int nx, long long pairs);
 cudaError_t launch_vdfdx_fx(double* f, int nx, const FxColRun* runs, const int2* items, int n_items, FxColRun one, int S,
                             double dt, const fxw* tw, const cx<double>* tw64, cudaStream_t s);
 
+// Lines whose length N is not a power of two (vg_dft_fx.cu): n_lines lines of N
+// elements es apart, line l at l ls with the phase's double c[l]; angles: the N
+// angles' table; scratch: dft_fx_scratch bytes for the larger of the directions
+// a plan uses
+size_t dft_fx_scratch(int nx, int nv, bool x, bool v);
+cudaError_t build_dft_table(int N, const fxw* tw, fxw* out, cudaStream_t s);
+cudaError_t launch_dft_fx(double* f, int N, int n_lines, long long es, long long ls, const double* c, FxTurn turn,
+                          const fxw* tw, const fxw* angles, void* scratch, cudaStream_t s);
+
 }  // namespace vg

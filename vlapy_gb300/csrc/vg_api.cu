@@ -147,28 +147,62 @@ using namespace vg;
 
 namespace {
 
+// A plan's device memory: blocks of a megabyte that are zeroed once and handed
+// out in pieces, so that its twenty-odd arrays cost one or two allocations (they
+// were most of the time of making a small plan)
+struct DevArena {
+  static constexpr size_t BLOCK = (size_t)1 << 20, ALIGN = 256;
+  std::vector<void*> blocks;
+  char* cur = nullptr;
+  size_t left = 0;
+  ~DevArena() {
+    for (void* b : blocks) cudaFree(b);
+  }
+  // bytes (zeroed unless scratch), or null with the error in *err
+  void* take(size_t bytes, bool scratch, cudaError_t* err) {
+    bytes = (bytes + ALIGN - 1) / ALIGN * ALIGN;
+    void* p = nullptr;
+    if (bytes > BLOCK / 2) {
+      *err = cudaMalloc(&p, bytes);
+      if (*err != cudaSuccess) return nullptr;
+      blocks.push_back(p);
+      if (!scratch) *err = cudaMemset(p, 0, bytes);
+      return p;
+    }
+    if (bytes > left) {
+      *err = cudaMalloc(&p, BLOCK);
+      if (*err != cudaSuccess) return nullptr;
+      blocks.push_back(p);
+      cur = static_cast<char*>(p);
+      left = BLOCK;
+      *err = cudaMemset(p, 0, BLOCK);
+      if (*err != cudaSuccess) return nullptr;
+    }
+    p = cur;
+    cur += bytes;
+    left -= bytes;
+    return p;
+  }
+};
+
+// n elements of the plan's memory, copied from src, or zero where src is null
+// (left as they are when scratch)
 template <typename T>
-int dev_copy(T** dst, const T* src, size_t n, const char* what) {
+int dev_copy(vg_plan* p, T** dst, const T* src, size_t n, const char* what, bool scratch = false) {
   *dst = nullptr;
   if (n == 0) return VG_OK;
-  cudaError_t err = cudaMalloc(reinterpret_cast<void**>(dst), n * sizeof(T));
+  cudaError_t err = cudaSuccess;
+  *dst = static_cast<T*>(static_cast<DevArena*>(p->arena)->take(n * sizeof(T), scratch || src, &err));
   if (err != cudaSuccess) return cuda_status(err, what);
-  if (src) {
-    err = cudaMemcpy(*dst, src, n * sizeof(T), cudaMemcpyHostToDevice);
-    if (err != cudaSuccess) return cuda_status(err, what);
-  } else {
-    err = cudaMemset(*dst, 0, n * sizeof(T));
-    if (err != cudaSuccess) return cuda_status(err, what);
-  }
-  return VG_OK;
+  if (src) err = cudaMemcpy(*dst, src, n * sizeof(T), cudaMemcpyHostToDevice);
+  return cuda_status(err, what);
 }
 
 void free_plan(vg_plan* p) {
   if (!p) return;
-  void* ptrs[] = {p->x, p->v, p->kx, p->kv, p->inv_kx, p->v_pow, p->f_bg, p->pulses, p->tw64, p->tw32, p->fx_vp, p->green, p->green_e,
-                  p->pw_v, p->pw_x, p->dens, p->mom, p->bb, p->rho, p->etmp, p->sl_m, p->sl_w, p->flags};
-  for (void* q : ptrs)
-    if (q) cudaFree(q);
+  if (p->sl_m) cudaFree(p->sl_m);
+  if (p->sl_w) cudaFree(p->sl_w);
+  delete static_cast<DevArena*>(p->arena);
   fx_tables_release(p->fx_tables);
   if (p->graph_cache) {
     auto* gc = static_cast<GraphCache*>(p->graph_cache);
@@ -176,13 +210,7 @@ void free_plan(vg_plan* p) {
     delete gc;
   }
   delete static_cast<ProfState*>(p->prof);
-  if (p->f32) {
-    F32Plan* q = p->f32;
-    void* qp[] = {q->F0, q->v32, q->f0_32, q->S, q->Mv, q->D, q->dpart, q->mpart, q->spart, q->vhl, q->e32, q->rc_dev};
-    for (void* x : qp)
-      if (x) cudaFree(x);
-    delete q;
-  }
+  delete p->f32;
   delete p;
 }
 
@@ -353,8 +381,8 @@ void host_fft(std::vector<double>& re, std::vector<double>& im) {
 }
 
 template <typename T>
-int upload(T** dst, const std::vector<T>& src, const char* what) {
-  return dev_copy(dst, src.data(), src.size(), what);
+int upload(vg_plan* p, T** dst, const std::vector<T>& src, const char* what) {
+  return dev_copy(p, dst, src.data(), src.size(), what);
 }
 
 // Constants of the delta-f path: the background f0 in FP32, its collision
@@ -396,14 +424,14 @@ int setup_f32(vg_plan* p, const vg_run_desc* d) {
   host_fft(re, im);
   std::vector<cx<float>> F0(nv / 2 + 1);
   for (int k = 0; k <= nv / 2; ++k) F0[k] = {(float)re[k], (float)im[k]};
-  VG_CHECK(upload(&q->v32, v32, "f32 constants"));
-  VG_CHECK(upload(&q->f0_32, f32v, "f32 constants"));
-  VG_CHECK(upload(&q->S, S, "f32 constants"));
-  VG_CHECK(upload(&q->Mv, Mv, "f32 constants"));
-  VG_CHECK(upload(&q->D, D, "f32 constants"));
-  VG_CHECK(upload(&q->F0, F0, "f32 constants"));
-  VG_CHECK(upload(&q->vhl, vhl, "f32 constants"));
-  VG_CHECK(dev_copy<float>(&q->e32, nullptr, (size_t)nx, "f32 field"));
+  VG_CHECK(upload(p, &q->v32, v32, "f32 constants"));
+  VG_CHECK(upload(p, &q->f0_32, f32v, "f32 constants"));
+  VG_CHECK(upload(p, &q->S, S, "f32 constants"));
+  VG_CHECK(upload(p, &q->Mv, Mv, "f32 constants"));
+  VG_CHECK(upload(p, &q->D, D, "f32 constants"));
+  VG_CHECK(upload(p, &q->F0, F0, "f32 constants"));
+  VG_CHECK(upload(p, &q->vhl, vhl, "f32 constants"));
+  VG_CHECK(dev_copy<float>(p, &q->e32, nullptr, (size_t)nx, "f32 field"));
   q->dkx = nx > 1 ? d->kx[1] : 0.0;
   q->dkv = d->kv[1];
   q->c0 = mom[0] - 1.0;
@@ -423,16 +451,16 @@ int setup_f32(vg_plan* p, const vg_run_desc* d) {
   q->rc.dv2f = split_f2(dv);
   q->rc.idv2f = split_f2(1.0 / dv2);
   for (int k = 0; k < 3; ++k) q->rc.f0m2f[k] = split_f2(mom[k]);
-  VG_CHECK(upload(&q->rc_dev, std::vector<RowConsts>(1, q->rc), "f32 constants"));
+  VG_CHECK(upload(p, &q->rc_dev, std::vector<RowConsts>(1, q->rc), "f32 constants"));
   int dev = 0, nsm = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   q->n_sm = nsm;
   q->col_grid_max = 8 * nsm;
   q->row_grid_max = 8 * nsm;
-  VG_CHECK(dev_copy<float2>(&q->dpart, nullptr, (size_t)q->col_grid_max * nx, "density partials"));
-  VG_CHECK(dev_copy<cx<float>>(&q->mpart, nullptr, (size_t)q->row_grid_max * F32_MAX_MODES * nv, "mode partials"));
-  VG_CHECK(dev_copy<float2>(&q->spart, nullptr, (size_t)F32_STORE_MAX_CTAS * 7, "series partials"));
+  VG_CHECK(dev_copy<float2>(p, &q->dpart, nullptr, (size_t)q->col_grid_max * nx, "density partials"));
+  VG_CHECK(dev_copy<cx<float>>(p, &q->mpart, nullptr, (size_t)q->row_grid_max * F32_MAX_MODES * nv, "mode partials"));
+  VG_CHECK(dev_copy<float2>(p, &q->spart, nullptr, (size_t)F32_STORE_MAX_CTAS * 7, "series partials"));
   return VG_OK;
 }
 
@@ -573,6 +601,7 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
   }
   vg_plan* p = new vg_plan();
   std::memset(p, 0, sizeof(vg_plan));
+  p->arena = new DevArena();
   p->nx = d->nx;
   p->nv = d->nv;
   p->precision = d->precision;
@@ -597,16 +626,16 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
       return st;                          \
     }                                     \
   } while (0)
-  TRY(dev_copy(&p->x, d->x, nx, "x"));
-  TRY(dev_copy(&p->v, d->v, nv, "v"));
-  TRY(dev_copy(&p->kx, d->kx, nx, "kx"));
-  TRY(dev_copy(&p->kv, d->kv, nv, "kv"));
-  TRY(dev_copy(&p->inv_kx, d->one_over_kx, nx, "one_over_kx"));
-  TRY(dev_copy(&p->v_pow, d->v_pow, 5 * nv, "v_pow"));
-  if (d->f_background) TRY(dev_copy(&p->f_bg, d->f_background, nv, "f_background"));
-  if (d->n_pulses > 0) TRY(dev_copy(&p->pulses, d->pulses, (size_t)d->n_pulses, "pulses"));
-  TRY(dev_copy<cx<double>>(&p->tw64, nullptr, FFT_NMAX, "twiddles"));
-  TRY(dev_copy<cx<float>>(&p->tw32, nullptr, FFT_NMAX, "twiddles"));
+  TRY(dev_copy(p, &p->x, d->x, nx, "x"));
+  TRY(dev_copy(p, &p->v, d->v, nv, "v"));
+  TRY(dev_copy(p, &p->kx, d->kx, nx, "kx"));
+  TRY(dev_copy(p, &p->kv, d->kv, nv, "kv"));
+  TRY(dev_copy(p, &p->inv_kx, d->one_over_kx, nx, "one_over_kx"));
+  TRY(dev_copy(p, &p->v_pow, d->v_pow, 5 * nv, "v_pow"));
+  if (d->f_background) TRY(dev_copy(p, &p->f_bg, d->f_background, nv, "f_background"));
+  if (d->n_pulses > 0) TRY(dev_copy(p, &p->pulses, d->pulses, (size_t)d->n_pulses, "pulses"));
+  TRY(dev_copy<cx<double>>(p, &p->tw64, nullptr, FFT_NMAX, "twiddles"));
+  TRY(dev_copy<cx<float>>(p, &p->tw32, nullptr, FFT_NMAX, "twiddles"));
   if (d->precision == VG_F64) {
     TRY(cuda_status(fx_tables_acquire(&p->fx_tables), "fixed-point tables"));
     p->tw_fx = p->fx_tables->tw;
@@ -614,9 +643,21 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
     p->kx1 = d->kx[1];
     p->kv_uniform = fx_uniform(d->kv, d->nv);
     p->kx_uniform = fx_uniform(d->kx, d->nx);
+    const bool dx = !p->nx_pow2 && d->nx <= DFT_ADVECT_NMAX, dv = !p->nv_pow2 && d->nv <= DFT_ADVECT_NMAX;
+    if (dv) {
+      TRY(dev_copy<fxw>(p, &p->dft_v, nullptr, nv, "DFT angles"));
+      TRY(cuda_status(build_dft_table(d->nv, p->tw_fx, p->dft_v, 0), "DFT angles"));
+    }
+    if (dx) {
+      TRY(dev_copy<fxw>(p, &p->dft_x, nullptr, nx, "DFT angles"));
+      TRY(cuda_status(build_dft_table(d->nx, p->tw_fx, p->dft_x, 0), "DFT angles"));
+    }
+    if (dx || dv)
+      TRY(dev_copy<unsigned char>(p, reinterpret_cast<unsigned char**>(&p->dft_work), nullptr,
+                                  dft_fx_scratch(d->nx, d->nv, dx, dv), "DFT scratch", true));
     std::vector<int2> vp;
     if (d->nv <= FX_MOMENTS_NV && fx_powers_host(d->v, d->v_pow, d->nv, &vp, &p->fx_pw)) {
-      TRY(dev_copy(&p->fx_vp, vp.data(), vp.size(), "velocity powers"));
+      TRY(dev_copy(p, &p->fx_vp, vp.data(), vp.size(), "velocity powers"));
       p->fx_log = p->fx_tables->log;
     }
   }
@@ -625,20 +666,20 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
   p->pw_x_leaves = tx[0];
   p->pw_v_words = (int)tv.size();
   p->pw_x_words = (int)tx.size();
-  TRY(dev_copy(&p->pw_v, tv.data(), tv.size(), "pairwise table"));
-  TRY(dev_copy(&p->pw_x, tx.data(), tx.size(), "pairwise table"));
-  TRY(dev_copy<double>(&p->dens, nullptr, nx, "scratch"));
-  TRY(dev_copy<double>(&p->mom, nullptr, nx * MOM_STRIDE, "scratch"));
-  TRY(dev_copy<double>(&p->rho, nullptr, nx, "scratch"));
-  TRY(dev_copy<double>(&p->etmp, nullptr, 4 * nx + 4, "scratch"));
-  TRY(dev_copy<int>(&p->flags, nullptr, 1, "status"));
+  TRY(dev_copy(p, &p->pw_v, tv.data(), tv.size(), "pairwise table"));
+  TRY(dev_copy(p, &p->pw_x, tx.data(), tx.size(), "pairwise table"));
+  TRY(dev_copy<double>(p, &p->dens, nullptr, nx, "scratch"));
+  TRY(dev_copy<double>(p, &p->mom, nullptr, nx * MOM_STRIDE, "scratch"));
+  TRY(dev_copy<double>(p, &p->rho, nullptr, nx, "scratch"));
+  TRY(dev_copy<double>(p, &p->etmp, nullptr, 4 * nx + 4, "scratch"));
+  TRY(dev_copy<int>(p, &p->flags, nullptr, 1, "status"));
   if (d->nx <= POISSON_FX_NX) {
-    TRY(dev_copy<int2>(&p->green, nullptr, nx, "Green's function"));
-    TRY(dev_copy<int>(&p->green_e, nullptr, 1, "Green's function"));
+    TRY(dev_copy<int2>(p, &p->green, nullptr, nx, "Green's function"));
+    TRY(dev_copy<int>(p, &p->green_e, nullptr, 1, "Green's function"));
     TRY(cuda_status(build_poisson_fx(p->inv_kx, d->nx, 1, p->green, p->green_e, p->etmp, 0), "Green's function"));
   }
   if (d->precision == VG_F64 && d->collision != VG_COLL_NONE)
-    TRY(dev_copy<double>(&p->bb, nullptr, 2 * nx * thomas_pad(d->nv), "thomas scratch"));
+    TRY(dev_copy<double>(p, &p->bb, nullptr, 2 * nx * thomas_pad(d->nv), "thomas scratch", true));
   if (d->precision == VG_F32_DELTA_F) TRY(setup_f32(p, d));
   TRY(cuda_status(launch_twiddles(*p, 0), "twiddles"));
   TRY(cuda_status(cudaDeviceSynchronize(), "plan setup"));

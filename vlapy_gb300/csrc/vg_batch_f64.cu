@@ -97,6 +97,7 @@ struct vg_batch {
   cx<double>* tw64 = nullptr;
   cx<float>* tw32 = nullptr;
   FxTables* fx_tables = nullptr;
+  unsigned char* dft_work = nullptr;  // bins of the largest class whose nv is not a power of two
   FxColRun* fx_runs = nullptr;  // per run, for the fixed-point x-drift
   double* dens = nullptr;      // [x_points]
   double* mom = nullptr;       // [x_points][BATCH_MOMS]
@@ -114,6 +115,7 @@ struct vg_batch {
     double dv, dv_sq, kv1;
     int kv_uniform;
     double *v, *kv, *v_pow;
+    fxw* dft_v;  // nv not a power of two: its angles
     int2* fx_vp;  // null: the storage moments in doubles
     FxPowers fx_pw;
     int* pw_v;
@@ -192,6 +194,8 @@ vg_plan class_view(const vg_batch* b, const vg_batch::Cls& c) {
   v.tw_fx = b->fx_tables->tw;
   v.kv1 = c.kv1;
   v.kv_uniform = c.kv_uniform;
+  v.dft_v = c.dft_v;
+  v.dft_work = b->dft_work;
   v.fx_vp = c.fx_vp;
   v.fx_pw = c.fx_pw;
   v.fx_log = b->fx_tables->log;
@@ -451,6 +455,14 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
   B_TRY(b_alloc<cx<double>>(b, &b->tw64, FFT_NMAX, nullptr, "twiddles"));
   B_TRY(b_alloc<cx<float>>(b, &b->tw32, FFT_NMAX, nullptr, "twiddles"));
   B_TRY(cuda_status(fx_tables_acquire(&b->fx_tables), "fixed-point tables"));
+  size_t dft_need = 0;
+  for (auto& c : b->cls)
+    if (!is_pow2(c.nv)) {
+      B_TRY(b_alloc<fxw>(b, &c.dft_v, (size_t)c.nv, nullptr, "batch grids"));
+      B_TRY(cuda_status(build_dft_table(c.nv, b->fx_tables->tw, c.dft_v, 0), "batch grids"));
+      dft_need = std::max(dft_need, dft_fx_scratch(c.rows, c.nv, false, true));
+    }
+  if (dft_need) B_TRY(b_alloc<unsigned char>(b, &b->dft_work, dft_need, nullptr, "batch grids"));
   {
     vg_plan tmp;
     std::memset(&tmp, 0, sizeof(tmp));

@@ -13,6 +13,7 @@
 #include "vlagpu.h"
 
 struct vg_plan {
+  void* arena;  // the plan's device memory (all arrays below but the spline's)
   // scalars of the run
   int nx, nv, precision, collision, integrator, n_pulses;
   double dt, nu, dx, dv, dv_sq, nudt;
@@ -34,6 +35,10 @@ struct vg_plan {
   vg::fxw* tw_fx;
   double kv1, kx1;
   int kv_uniform, kx_uniform;
+  // lengths that are not powers of two: their angle tables and the bins' scratch
+  vg::fxw* dft_v;
+  vg::fxw* dft_x;
+  void* dft_work;
   // fixed-point storage moments: the velocity powers and the logarithm's table
   // (null: the moments in doubles)
   int2* fx_vp;
