@@ -14,7 +14,7 @@
 // A line is scaled so that the sum of its moduli, which bounds every bin, fills the
 // 64 bits of the accumulators, and so are its bins on the way back (they go
 // through scratch between the two kernels).  A step of 48 x 720 (two half kicks, a
-// drift) went from 1.45 to 0.06 ms; the errors stay within twice the bound of a
+// drift) went from 1.45 to 0.07 ms; the errors stay within twice the bound of a
 // power-of-two transform in doubles where the direct sums in doubles were at
 // several times it.
 #include <algorithm>

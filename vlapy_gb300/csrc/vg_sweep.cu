@@ -32,6 +32,7 @@ struct SweepRunDev {
   int x_off;           // x points before this run
   long long dp_off;    // density-partial elements (float2) before this run
   double k, nudt;
+  float2 inv_k;  // 1 / k split (hi, lo)
   float2 nudt2;  // nudt split (hi, lo)
   float2 kdt;          // -k dt split into FP32 (hi, lo): the x-drift angle per unit m and v
   float nudt_f;
@@ -134,7 +135,8 @@ struct SweepConsts {
   RowConsts rc[SWEEP_MAX_CLASSES];
   const cx<float>* F0[SWEEP_MAX_CLASSES];
   const double* v64[SWEEP_MAX_CLASSES];
-  double c0[SWEEP_MAX_CLASSES];
+  float2 c0[SWEEP_MAX_CLASSES];  // trapz(f0) - 1, split
+  float2 inv_m[129];             // 1 / m, split (m <= nx / 2)
 };
 
 // ---------------------------------------------------------------------------
@@ -388,26 +390,45 @@ __global__ void __launch_bounds__(SWEEP_BLOCK, sweep_col_min_blocks(NX)) k_sweep
   }
 }
 
-// field solve of up to SWEEP_FIELD_BLOCK/G runs of one nx per CTA
+// field solve of up to SWEEP_FIELD_BLOCK/G runs of one nx per CTA.  A thread adds
+// the tiles' density partials of its nx / G points side by side, four tiles in
+// flight (one load after another, each an L2 latency, was most of the kernel), and
+// the charge and 1 / kx are formed in double-float: GB300 spends 64 cycles on each
+// FP64 instruction of a warp, a dozen of them on a division.  22 -> 15 us for a
+// 64-run sweep, 33 -> 22 us for 4096 runs (nx 32 .. 128).
 template <int NX>
 __device__ __forceinline__ void sweep_field_runs(const SweepRunDev* __restrict__ runs, int first, int count,
                                                  const SweepConsts& sc, const float2* __restrict__ dpart,
                                                  const cx<float>* __restrict__ tw, double* __restrict__ e,
                                                  float* __restrict__ e32, unsigned char* smem, int* flags) {
   constexpr int G = fft_threads<float>(NX);
+  constexpr int PER = NX / G;
   const int grp = threadIdx.x / G, t = threadIdx.x - grp * G;
   cx<float>* s = reinterpret_cast<cx<float>*>(smem) + (size_t)grp * sp_len<float>(NX);
   const bool valid = grp < count;
   const SweepRunDev r = runs[valid ? first + grp : first];
-  const double dv = sc.rc[r.cls].dv, c0 = sc.c0[r.cls];
-  for (int x = t; x < NX; x += G) {
-    df32 acc = {0.f, 0.f};
-    if (valid)
-      for (int p = 0; p < r.ntiles; ++p) {
-        const float2 q = dpart[r.dp_off + (size_t)p * NX + x];
-        acc = df_add(acc, {q.x, q.y});
-      }
-    s[sp<float>(x)] = {valid ? (float)(-(dv * df_to_double(acc)) - c0) : 0.f, 0.f};
+  const float2 dv2 = sc.rc[r.cls].dv2f, c0 = sc.c0[r.cls];
+  df32 acc[PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i) acc[i] = {0.f, 0.f};
+  if (valid)
+    for (int p0 = 0; p0 < r.ntiles; p0 += 4) {
+      float2 q[4][PER];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int i = 0; i < PER; ++i)
+          q[u][i] = p0 + u < r.ntiles ? dpart[r.dp_off + (size_t)(p0 + u) * NX + t + i * G] : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int i = 0; i < PER; ++i) acc[i] = df_add(acc[i], {q[u][i].x, q[u][i].y});
+    }
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    // 1 - n = -dv sum g - (trapz(f0) - 1)
+    const df32 rho = df_add(df_mul({dv2.x, dv2.y}, acc[i]), {c0.x, c0.y});
+    s[sp<float>(t + i * G)] = {valid ? -df_round(rho) : 0.f, 0.f};
   }
   __syncthreads();
   block_fft<float, NX, false>(s, t, tw);
@@ -415,7 +436,9 @@ __device__ __forceinline__ void sweep_field_runs(const SweepRunDev* __restrict__
   for (int m = t; m < NX; m += G) {
     // 1 / kx with kx = 2 pi fftfreq(nx, dx) = m' k, the zero mode removed
     const int mm = (m < NX / 2) ? m : m - NX;
-    const float ik = (m == 0) ? 0.f : (float)(1.0 / ((double)mm * r.k)) * scale;
+    const float2 im = sc.inv_m[mm < 0 ? -mm : mm];
+    const float a = df_round(df_mul({r.inv_k.x, r.inv_k.y}, {im.x, im.y})) * scale;
+    const float ik = m == 0 ? 0.f : mm < 0 ? -a : a;
     const cx<float> z = s[sp<float>(m)];
     s[sp<float>(m)] = {-ik * z.y, ik * z.x};
   }
@@ -511,11 +534,14 @@ __global__ void __launch_bounds__(sweep_row_block(N), KICK ? (sweep_row_radix(N)
 
 // e history row and the seven series of every run (one CTA per run, one
 // row per thread): each warp adds its rows' double-float sums by
-// transposition, then seven threads add the four warps' totals in order
+// transposition, then seven threads add the four warps' totals in order.  The
+// moments are formed in double-float as well (in FP64 they were some 60
+// instructions a row at 64 cycles each: 42 us for 4096 runs, now 18).
 __global__ void __launch_bounds__(128) k_sweep_store(const SweepRunDev* __restrict__ runs, int n_runs,
                                                      const SweepConsts* __restrict__ scp,
-                                                     const double* __restrict__ mom, const double* __restrict__ e,
-                                                     double* __restrict__ e_row, double* __restrict__ s_row) {
+                                                     const double* __restrict__ mom, const float* __restrict__ e32,
+                                                     const double* __restrict__ e, double* __restrict__ e_row,
+                                                     double* __restrict__ s_row) {
   __shared__ df32 red[4][8];
   const SweepRunDev r = runs[blockIdx.x];
   const RowConsts& rc = scp->rc[r.cls];
@@ -524,16 +550,16 @@ __global__ void __launch_bounds__(128) k_sweep_store(const SweepRunDev* __restri
 #pragma unroll
   for (int q = 0; q < 8; ++q) acc[q] = {0.f, 0.f};
   for (int x = threadIdx.x; x < r.nx; x += blockDim.x) {
-    const double ex = e[r.x_off + x];
-    if (e_row) e_row[r.x_off + x] = ex;
+    if (e_row) e_row[r.x_off + x] = e[r.x_off + x];
+    const float ex = e32[r.x_off + x];
     const double* slots = mom + (size_t)(r.x_off + x) * MOM_STRIDE;
-    const double src[7] = {row_moment(slots, 0, rc), row_moment(slots, 1, rc), row_moment(slots, 2, rc), ex * ex,
-                           0.0, row_moment(slots, 6, rc), row_moment(slots, 7, rc)};
+    // e^2 exactly (the field is an FP32 value); no driver
+    const float e2 = ex * ex;
+    const df32 src[7] = {row_moment_df(slots, 0, rc), row_moment_df(slots, 1, rc), row_moment_df(slots, 2, rc),
+                         {e2, fmaf(ex, ex, -e2)},     {0.f, 0.f},                  row_moment_df(slots, 6, rc),
+                         row_moment_df(slots, 7, rc)};
 #pragma unroll
-    for (int q = 0; q < 7; ++q) {
-      const float hi = (float)src[q];
-      acc[q] = df_add(acc[q], {hi, (float)(src[q] - (double)hi)});
-    }
+    for (int q = 0; q < 7; ++q) acc[q] = df_add(acc[q], src[q]);
   }
   int idx;
   bool writer;
@@ -847,10 +873,10 @@ int sweep_class(vg_sweep* s, int cls, int nv) {
   for (int k = 0; k < 7; ++k) rc.f0m[k] = mom[k];
   rc.dv2f = split_f2(dv);
   rc.idv2f = split_f2(1.0 / dv2);
-  for (int k = 0; k < 3; ++k) rc.f0m2f[k] = split_f2(mom[k]);
+  for (int k = 0; k < 7; ++k) rc.f0m2f[k] = split_f2(mom[k]);
   s->consts_h.F0[cls] = dF0;
   s->consts_h.v64[cls] = dv64;
-  s->consts_h.c0[cls] = mom[0] - 1.0;
+  s->consts_h.c0[cls] = split_f2(mom[0] - 1.0);
   s->f0d[cls] = df064;
   return VG_OK;
 }
@@ -1029,7 +1055,7 @@ int sweep_sequence(vg_sweep* s, int nsteps, double* e_hist, double* s_hist, int 
       double* er = e_hist ? e_hist + (size_t)r * s->x_points : nullptr;
       double* sr = s_hist ? s_hist + (size_t)r * s->n_runs * 7 : nullptr;
       SW_CHECK(cuda_status(prof_call(&s->prof, SK_STORE, st, [&] {
-                             k_sweep_store<<<s->n_runs, 128, 0, st>>>(s->runs, s->n_runs, s->consts, s->mom, s->e, er, sr);
+                             k_sweep_store<<<s->n_runs, 128, 0, st>>>(s->runs, s->n_runs, s->consts, s->mom, s->e32, s->e, er, sr);
                              return cudaGetLastError();
                            }),
                            "sweep store"));
@@ -1124,6 +1150,7 @@ int vg_sweep_create(const vg_sweep_desc* d, vg_sweep** out) {
   s->vmax = d->vmax;
   s->dt = d->dt;
   std::memset(&s->consts_h, 0, sizeof(SweepConsts));
+  for (int m = 1; m <= 128; ++m) s->consts_h.inv_m[m] = split_f2(1.0 / m);
   std::map<int, int> cls_of;
   long long cells = 0, dp = 0;
   int xoff = 0;
@@ -1157,6 +1184,7 @@ int vg_sweep_create(const vg_sweep_desc* d, vg_sweep** out) {
     r.x_off = xoff;
     r.dp_off = dp;
     r.k = q.k;
+    r.inv_k = split_f2(1.0 / q.k);
     r.nudt = q.nu * d->dt;
     r.kdt = split_f2(-q.k * d->dt);
     r.nudt_f = (float)r.nudt;
