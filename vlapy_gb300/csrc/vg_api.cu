@@ -673,7 +673,7 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
   TRY(dev_copy<double>(p, &p->rho, nullptr, nx, "scratch"));
   TRY(dev_copy<double>(p, &p->etmp, nullptr, 4 * nx + 4, "scratch"));
   TRY(dev_copy<int>(p, &p->flags, nullptr, 1, "status"));
-  if (d->nx <= POISSON_FX_NX) {
+  if (d->nx <= POISSON_FX_NX && d->precision == VG_F64) {
     TRY(dev_copy<int2>(p, &p->green, nullptr, nx, "Green's function"));
     TRY(dev_copy<int>(p, &p->green_e, nullptr, 1, "Green's function"));
     TRY(cuda_status(build_poisson_fx(p->inv_kx, d->nx, 1, p->green, p->green_e, p->etmp, 0), "Green's function"));

@@ -2,11 +2,11 @@
 //
 // Per leapfrog step the state g[nx][nv] (FP32) crosses HBM twice:
 //   k_col_f32   x-drift (FFT along x per column pair) + density partials
-//   k_dens_f32  per-x reduction of the partials (double-float)
-//   k_field_f32 Poisson solve: 1 - n in FP64, FFT in FP32, + driver
+//   k_field_f32 per-x reduction of the partials (double-float; k_dens_f32 where
+//               those are many), Poisson solve: 1 - n in FP64, FFT in FP32, + driver
 //   k_row_f32   half kick(E_{n+1}) -> Fokker-Planck -> storage moments and
 //               x-mode partials -> half kick(E_{n+1}) of the next step
-//   k_store_f32 fields, series and stored modes of the step
+//   k_store_f32 fields, series and stored modes of the step (one launch)
 // The first half kick of a batch runs once as a row pass of its own; the
 // last step of a batch skips the trailing kick, so the state handed back is
 // the reference's f after its collision step.
@@ -40,69 +40,131 @@ __global__ void __launch_bounds__((NX / R) * col32_seqs(NX, R)) k_col_f32(
 // density reduction and field solve
 // ---------------------------------------------------------------------------
 
-__global__ void k_dens_f32(const float2* __restrict__ dpart, int npart, int nx, double dv, double c0,
-                           double* __restrict__ rho) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= nx) return;
+// the charge 1 - n = -(dv sum g) - (trapz(f0) - 1) in FP64
+__device__ __forceinline__ double charge_f32(df32 sum, double dv, double c0) { return -(dv * df_to_double(sum)) - c0; }
+
+// CTAs' density partials p0 .. p1 - 1 of point x added in their order, eight loads
+// in flight (one at a time, each waits out an L2 latency)
+__device__ __forceinline__ df32 sum_partials(const float2* __restrict__ dpart, int p0, int p1, int nx, int x) {
   df32 acc = {0.f, 0.f};
-  for (int p = 0; p < npart; ++p) {
-    const float2 v = dpart[(size_t)p * nx + x];
-    acc = df_add(acc, {v.x, v.y});
+  for (; p0 + 8 <= p1; p0 += 8) {
+    float2 q[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) q[u] = dpart[(size_t)(p0 + u) * nx + x];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) acc = df_add(acc, {q[u].x, q[u].y});
   }
-  // 1 - n = -(dv sum g) - (trapz(f0) - 1), in FP64
-  rho[x] = -(dv * df_to_double(acc)) - c0;
+  for (; p0 < p1; ++p0) {
+    const float2 q = dpart[(size_t)p0 * nx + x];
+    acc = df_add(acc, {q.x, q.y});
+  }
+  return acc;
+}
+
+// a CTA's DENS_SPLIT warps each add a share of the partials of 32 points, and the
+// shares are added in order (one thread a point: 24 us at nx = 4096 over 152
+// partials, now 6)
+constexpr int DENS_SPLIT = 8;
+__global__ void __launch_bounds__(32 * DENS_SPLIT) k_dens_f32(const float2* __restrict__ dpart, int npart, int nx, double dv,
+                                                              double c0, double* __restrict__ rho) {
+  __shared__ df32 part[DENS_SPLIT][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int x = blockIdx.x * 32 + lane;
+  const int per = (npart + DENS_SPLIT - 1) / DENS_SPLIT;
+  if (x < nx) part[w][lane] = sum_partials(dpart, min(npart, w * per), min(npart, (w + 1) * per), nx, x);
+  __syncthreads();
+  if (w != 0 || x >= nx) return;
+  df32 acc = part[0][lane];
+#pragma unroll
+  for (int q = 1; q < DENS_SPLIT; ++q) acc = df_add(acc, part[q][lane]);
+  rho[x] = charge_f32(acc, dv, c0);
 }
 
 // driver: scalar envelope in FP64, phase k x - w t reduced mod 2 pi in FP64,
 // sine in FP32 (the driver amplitude is small; this is the FP32 path)
-__device__ __forceinline__ float pulse_sum_f32(const vg_pulse* __restrict__ P, int np, double t, double x) {
-  float total = 0.f;
-  for (int i = 0; i < np; ++i) {
-    const vg_pulse q = P[i];
-    double amp;
-    if (q.envelope == VG_ENV_SIN2) {
-      if (t < 0.0 || t > q.t_R) continue;
-      const double sn = sin(3.141592653589793 * t / q.t_R);
-      amp = q.a0 * sn * sn;
-    } else {
-      amp = 0.5 * (tanh((t - q.t_L) / q.t_wL) - tanh((t - q.t_R) / q.t_wR)) * q.k0 * q.a0;
-    }
-    double arg = q.k0 * x - q.w0 * t;
-    arg -= 6.283185307179586 * rint(arg * 0.15915494309189535);
-    total += (float)amp * sinf((float)arg);
+__device__ __forceinline__ bool pulse_amplitude(const vg_pulse& q, double t, double* amp) {
+  if (q.envelope == VG_ENV_SIN2) {
+    if (t < 0.0 || t > q.t_R) return false;
+    const double sn = sin(3.141592653589793 * t / q.t_R);
+    *amp = q.a0 * sn * sn;
+  } else {
+    *amp = 0.5 * (tanh((t - q.t_L) / q.t_wL) - tanh((t - q.t_R) / q.t_wR)) * q.k0 * q.a0;
   }
-  return total;
+  return true;
 }
 
+// Field of one run.  Up to nx = 1024 the CTA has 256 threads, more than its
+// transforms use: the points' charges and the pulses' sines are spread over all of
+// them, and one warp evaluates the envelopes, a pulse a lane (FP64 instructions take
+// 64 cycles each whatever the number of lanes: eight threads with eight points each
+// spent 31 us at nx = 64 with one pulse; with the density launch that this kernel
+// takes over 35, now 9).
+constexpr int FIELD32_WIDE_NX = 1024;
+constexpr int FIELD32_PULSES = 32;  // pulses whose envelopes are held at a time
+__host__ __device__ constexpr int field32_block(int nx) {
+  return nx <= FIELD32_WIDE_NX ? 256 : fft_threads<float>(nx);
+}
 template <int NX>
-__global__ void __launch_bounds__(fft_threads<float>(NX)) k_field_f32(
-    const double* __restrict__ rho, const double* __restrict__ inv_kx, const double* __restrict__ driver,
-    int use_pulses, const vg_pulse* __restrict__ P, int np, const double* __restrict__ x, const double* t_ptr,
-    double t_host, int nadd, double a0, double a1, double a2, double a3, double a4,
-    const cx<float>* __restrict__ tw, double* __restrict__ e, float* __restrict__ e32, int* flags) {
+__global__ void __launch_bounds__(field32_block(NX)) k_field_f32(
+    const double* __restrict__ rho, const float2* __restrict__ dpart, int npart, double dv, double c0,
+    const double* __restrict__ inv_kx, const double* __restrict__ driver, int use_pulses,
+    const vg_pulse* __restrict__ P, int np, const double* __restrict__ x, const double* t_ptr, double t_host, int nadd,
+    double a0, double a1, double a2, double a3, double a4, const cx<float>* __restrict__ tw, double* __restrict__ e,
+    float* __restrict__ e32, int* flags) {
   constexpr int G = fft_threads<float>(NX);
+  constexpr int B = field32_block(NX);
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double amp[FIELD32_PULSES];
   cx<float>* s = reinterpret_cast<cx<float>*>(smem_raw);
+  float* drv = reinterpret_cast<float*>(s + sp_len<float>(NX));  // [NX]
   const int t = threadIdx.x;
-  for (int n = t; n < NX; n += G) s[sp<float>(n)] = {(float)rho[n], 0.f};
-  __syncthreads();
-  block_fft<float, NX, false>(s, t, tw);
-  const float sc = 1.f / NX;
-  for (int k = t; k < NX; k += G) {
-    const cx<float> z = s[sp<float>(k)];
-    const float ik = (float)inv_kx[k] * sc;
-    s[sp<float>(k)] = {-ik * z.y, ik * z.x};
-  }
-  __syncthreads();
-  block_fft<float, NX, true>(s, t, tw);
   double tt = t_ptr ? *t_ptr : t_host;
   const double adds[5] = {a0, a1, a2, a3, a4};
   for (int i = 0; i < nadd; ++i) tt += adds[i];
-  for (int n = t; n < NX; n += G) {
-    float drv = 0.f;
-    if (driver) drv = (float)driver[n];
-    else if (use_pulses) drv = pulse_sum_f32(P, np, tt, x[n]);
-    const float en = drv + s[sp<float>(n)].x;
+  const bool pulses = !driver && use_pulses;
+  for (int n = t; n < NX; n += B) {
+    s[sp<float>(n)] = {(float)(rho ? rho[n] : charge_f32(sum_partials(dpart, 0, npart, NX, n), dv, c0)), 0.f};
+    drv[n] = driver ? (float)driver[n] : 0.f;
+  }
+  if (pulses)
+    for (int p0 = 0; p0 < np; p0 += FIELD32_PULSES) {
+      const int n_here = min(FIELD32_PULSES, np - p0);
+      // (a silent pulse: its amplitude is NaN here and it adds nothing)
+      if (t >= B - 32 && t - (B - 32) < n_here) {
+        double a;
+        amp[t - (B - 32)] = pulse_amplitude(P[p0 + t - (B - 32)], tt, &a) ? a : __longlong_as_double(0x7ff8000000000000ll);
+      }
+      __syncthreads();
+      for (int n = t; n < NX; n += B) {
+        float total = drv[n];
+        for (int i = 0; i < n_here; ++i) {
+          const double a = amp[i];
+          if (isnan(a)) continue;
+          const vg_pulse& q = P[p0 + i];
+          double arg = q.k0 * x[n] - q.w0 * tt;
+          arg -= 6.283185307179586 * rint(arg * 0.15915494309189535);
+          total += (float)a * sinf((float)arg);
+        }
+        drv[n] = total;
+      }
+      __syncthreads();
+    }
+  __syncthreads();
+  if (t < G) {
+    const GroupSync sync = GroupSync::of(0, G);
+    block_fft<float, NX, false>(s, t, tw, sync);
+    const float sc = 1.f / NX;
+    for (int k = t; k < NX; k += G) {
+      const cx<float> z = s[sp<float>(k)];
+      const float ik = (float)inv_kx[k] * sc;
+      s[sp<float>(k)] = {-ik * z.y, ik * z.x};
+    }
+    sync();
+    block_fft<float, NX, true>(s, t, tw, sync);
+  }
+  __syncthreads();
+  for (int n = t; n < NX; n += B) {
+    const float en = drv[n] + s[sp<float>(n)].x;
     e[n] = (double)en;
     e32[n] = en;
     if (flags && !isfinite(en)) atomicOr(flags, VG_FLAG_NONFINITE);
@@ -146,36 +208,44 @@ __global__ void __launch_bounds__(row32_block(N, R), (KICK || R == 32) ? 2 : 1) 
 // storage of one step: fields, series and stored modes
 // ---------------------------------------------------------------------------
 
-// fields of one step and the series partial sums of this CTA's rows (rows
-// blockIdx.x * blockDim.x + threadIdx.x, stride the whole grid); spart[b][q]
-// is CTA b's double-float partial of series q
-__global__ void k_store_fields_f32(const double* __restrict__ mom, RowConsts rc, const double* __restrict__ e,
-                                   const double* __restrict__ de, int nx, int i, vg_history h,
-                                   float2* __restrict__ spart) {
-  __shared__ df32 red[32 * 7];
+// Storage of one step in one launch.  CTAs 0 .. nb - 1 write the fields of their
+// 256 rows and the series' partial sums spart[b][q] (a warp per moment: warps 0 ..
+// 7 the eight moments, warp 8 the field, warp 9 the driver; with one such CTA the
+// partial sums are the series).  The CTAs after them add up the stored modes.
+constexpr int STORE_BLOCK = 320;
+constexpr int STORE_ROWS = 256;
+constexpr int STORE_MODE_SPLIT = STORE_BLOCK / 32;
+__device__ __forceinline__ void store_fields_cta(const double* __restrict__ mom, const RowConsts& rc,
+                                                 const double* __restrict__ e, const double* __restrict__ de, int nx,
+                                                 int i, const vg_history& h, float2* __restrict__ spart, int b, int nb) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t off = (size_t)i * nx;
-  df32 acc[7];
-  for (int q = 0; q < 7; ++q) acc[q] = {0.f, 0.f};
-  for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nx; n += gridDim.x * blockDim.x) {
-    const double* slots = mom + (size_t)n * MOM_STRIDE;
-    double m[8];
-    for (int q = 0; q < 8; ++q) m[q] = row_moment(slots, q, rc);
-    if (h.fields[0]) h.fields[0][off + n] = e[n];
-    if (h.fields[1]) h.fields[1][off + n] = de ? de[n] : 0.0;
-    for (int q = 0; q < 6; ++q)
-      if (h.fields[2 + q]) h.fields[2 + q][off + n] = m[q];
-    const double src[7] = {m[0], m[1], m[2], e[n] * e[n], de ? de[n] * de[n] : 0.0, m[6], m[7]};
-    for (int q = 0; q < 7; ++q) {
-      const float hi = (float)src[q];
-      acc[q] = df_add(acc[q], {hi, (float)(src[q] - (double)hi)});
+  // the field and the series this warp writes (-1: none)
+  const int field = w < 6 ? 2 + w : w == 8 ? 0 : w == 9 ? 1 : -1;
+  const int ser = w < 3 ? w : w == 8 ? 3 : w == 9 ? 4 : w == 6 ? 5 : w == 7 ? 6 : -1;
+  df32 acc = {0.f, 0.f};
+  for (int n0 = b * STORE_ROWS; n0 < nx; n0 += nb * STORE_ROWS)
+    for (int n = n0 + lane; n < min(nx, n0 + STORE_ROWS); n += 32) {
+      const double v = w < 8 ? row_moment(mom + (size_t)n * MOM_STRIDE, w, rc) : w == 8 ? e[n] : de ? de[n] : 0.0;
+      if (field >= 0 && h.fields[field]) h.fields[field][off + n] = v;
+      if (ser >= 0) {
+        const double src = w >= 8 ? v * v : v;
+        const float hi = (float)src;
+        acc = df_add(acc, {hi, (float)(src - (double)hi)});
+      }
     }
+  if (ser < 0) return;
+  acc = df_warp_sum(acc);
+  if (lane != 0) return;
+  if (nb == 1) {
+    if (h.series[ser]) h.series[ser][i] = df_to_double(acc) / nx;
+  } else {
+    spart[b * 7 + ser] = make_float2(acc.hi, acc.lo);
   }
-  block_df_sum<7>(acc, red);
-  if (threadIdx.x < 7) spart[blockIdx.x * 7 + threadIdx.x] = make_float2(acc[threadIdx.x].hi, acc[threadIdx.x].lo);
 }
 
-// the series of one step: the CTAs' partials added in CTA order (one thread
-// per series, so the sum is the same on every run)
+// the series of one step where several CTAs hold partials: added in CTA order
+// (one thread per series, so the sum is the same on every run)
 __global__ void k_store_series_f32(const float2* __restrict__ spart, int nb, int nx, int i, vg_history h) {
   const int q = threadIdx.x;
   if (q >= 7 || !h.series[q]) return;
@@ -184,28 +254,24 @@ __global__ void k_store_series_f32(const float2* __restrict__ spart, int nb, int
   h.series[q][i] = df_to_double(acc) / nx;
 }
 
-// stored x-modes of one step: thread (j, m) adds mode m of velocity j over
-// the row kernel's per-CTA partials, in four interleaved double-float chains
-// (partials p = 0, 4, 8, ... in the first, and so on) joined in a fixed order
-// stored x modes of one step: the CTAs' mode partials summed in double-float.
-// A block is 32 bins x STORE_MODE_SPLIT slice ranges: thread (jx, gy) sums
-// the slices of range gy for bin j (consecutive jx, consecutive j: coalesced),
-// then the ranges are added in order (deterministic)
-constexpr int STORE_MODE_SPLIT = 8;
-__global__ void __launch_bounds__(32 * STORE_MODE_SPLIT) k_store_modes_f32(
-    const cx<float>* __restrict__ mpart, int npart, int nm, int nv, int nx, const double* __restrict__ f0,
-    int n_slots, int i, cx<float>* __restrict__ out) {
+// stored x modes of one step: the CTAs' mode partials summed in double-float.  A
+// block is 32 bins x STORE_MODE_SPLIT slice ranges: thread (jx, gy) sums the
+// slices of range gy for bin j (consecutive jx, consecutive j: coalesced), then
+// the ranges are added in order (deterministic)
+__device__ __forceinline__ void store_modes_cta(const cx<float>* __restrict__ mpart, int npart, int nm, int nv, int nx,
+                                                const double* __restrict__ f0, int n_slots, int i,
+                                                cx<float>* __restrict__ out, int jb, int m) {
   __shared__ df32 part_re[STORE_MODE_SPLIT][32], part_im[STORE_MODE_SPLIT][32];
   const int jx = threadIdx.x & 31, gy = threadIdx.x >> 5;
-  const int j = blockIdx.x * 32 + jx;
-  const int m = blockIdx.y;
+  const int j = jb * 32 + jx;
   const bool live = j < nv && m < nm && m < n_slots;
   df32 re[2] = {{0.f, 0.f}, {0.f, 0.f}}, im[2] = {{0.f, 0.f}, {0.f, 0.f}};
   if (live) {
     const int per = (npart + STORE_MODE_SPLIT - 1) / STORE_MODE_SPLIT;
     const int p0 = gy * per, p1 = min(npart, p0 + per);
-    int p = p0, u = 0;
-    for (; p < p1; ++p, u ^= 1) {
+    int u = 0;
+#pragma unroll 4
+    for (int p = p0; p < p1; ++p, u ^= 1) {
       const cx<float> z = mpart[((size_t)p * nm + m) * nv + j];
       re[u] = df_add(re[u], {z.x, 0.f});
       im[u] = df_add(im[u], {z.y, 0.f});
@@ -228,6 +294,19 @@ __global__ void __launch_bounds__(32 * STORE_MODE_SPLIT) k_store_modes_f32(
     for (int sl = 0; sl < n_slots; ++sl) dst[(size_t)sl * nv + j] = z;
   } else {
     dst[(size_t)m * nv + j] = z;
+  }
+}
+
+__global__ void __launch_bounds__(STORE_BLOCK) k_store_f32(const double* __restrict__ mom, const RowConsts* __restrict__ rc,
+                                                           const double* __restrict__ e, const double* __restrict__ de,
+                                                           int nx, int i, vg_history h, float2* __restrict__ spart, int nb,
+                                                           const cx<float>* __restrict__ mpart, int npart, int nm, int nv,
+                                                           const double* __restrict__ f0) {
+  if ((int)blockIdx.x < nb) {
+    store_fields_cta(mom, *rc, e, de, nx, i, h, spart, blockIdx.x, nb);
+  } else {
+    const int b = blockIdx.x - nb, tiles = (nv + 31) / 32;
+    store_modes_cta(mpart, npart, nm, nv, nx, f0, h.n_slots, i, static_cast<cx<float>*>(h.stored_f), b % tiles, b / tiles);
   }
 }
 
@@ -259,15 +338,17 @@ cudaError_t col_n(const vg_plan& p, float* g, double dt, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+// rho null: the density partials of the last x-drift
 template <int NX>
-cudaError_t field_n(const vg_plan& p, const double* driver, const FieldTime& ft, double* e, cudaStream_t s) {
-  constexpr int G = fft_threads<float>(NX);
-  const size_t smem = (size_t)sp_len<float>(NX) * sizeof(cx<float>);
+cudaError_t field_n(const vg_plan& p, const double* rho, const double* driver, const FieldTime& ft, double* e,
+                    cudaStream_t s) {
+  const size_t smem = (size_t)sp_len<float>(NX) * sizeof(cx<float>) + (size_t)NX * sizeof(float);
   cudaError_t err = ensure_smem((const void*)k_field_f32<NX>, smem);
   if (err != cudaSuccess) return err;
-  k_field_f32<NX><<<1, G, smem, s>>>(p.rho, p.inv_kx, driver, ft.use_pulses, p.pulses, p.n_pulses, p.x, ft.t_ptr,
-                                     ft.t_host, ft.nadd, ft.add[0], ft.add[1], ft.add[2], ft.add[3], ft.add[4],
-                                     p.tw32, e, p.f32->e32, p.flags);
+  k_field_f32<NX><<<1, field32_block(NX), smem, s>>>(rho, p.f32->dpart, p.f32->npart, p.dv, p.f32->c0, p.inv_kx, driver,
+                                                     ft.use_pulses, p.pulses, p.n_pulses, p.x, ft.t_ptr, ft.t_host,
+                                                     ft.nadd, ft.add[0], ft.add[1], ft.add[2], ft.add[3], ft.add[4],
+                                                     p.tw32, e, p.f32->e32, p.flags);
   return cudaGetLastError();
 }
 
@@ -313,26 +394,32 @@ cudaError_t launch_col_f32(const vg_plan& p, float* g, double dt, cudaStream_t s
   }
 }
 
-cudaError_t launch_poisson_only_f32(const vg_plan& p, const double* rho, const double* driver,
-                                    const FieldTime& ft, double* e, cudaStream_t s) {
-  if (rho != p.rho) {
-    cudaError_t err = cudaMemcpyAsync(p.rho, rho, (size_t)p.nx * sizeof(double), cudaMemcpyDeviceToDevice, s);
-    if (err != cudaSuccess) return err;
-  }
+static cudaError_t field_any(const vg_plan& p, const double* rho, const double* driver, const FieldTime& ft, double* e,
+                             cudaStream_t s) {
   switch (ilog2(p.nx)) {
-#define CASE(L) case L: return field_n<(1 << L)>(p, driver, ft, e, s);
+#define CASE(L) case L: return field_n<(1 << L)>(p, rho, driver, ft, e, s);
     VG_F32_POW2_CASES(CASE)
 #undef CASE
     default: return cudaErrorInvalidValue;
   }
 }
 
+cudaError_t launch_poisson_only_f32(const vg_plan& p, const double* rho, const double* driver,
+                                    const FieldTime& ft, double* e, cudaStream_t s) {
+  return field_any(p, rho, driver, ft, e, s);
+}
+
 cudaError_t launch_field_f32(const vg_plan& p, const double* driver, const FieldTime& ft, double* e,
                              cudaStream_t s) {
-  k_dens_f32<<<div_up(p.nx, 128), 128, 0, s>>>(p.f32->dpart, p.f32->npart, p.nx, p.dv, p.f32->c0, p.rho);
+  // The field kernel adds the density partials where that is at most 32 loads a
+  // thread, four waits: nx = 64 with 16 partials takes 9 us in all, against 4 + 9 in
+  // two launches.  Above, many CTAs read them faster than its one.
+  if (p.nx <= FIELD32_WIDE_NX && div_up(p.nx, field32_block(p.nx)) * p.f32->npart <= 32)
+    return field_any(p, nullptr, driver, ft, e, s);
+  k_dens_f32<<<div_up(p.nx, 32), 32 * DENS_SPLIT, 0, s>>>(p.f32->dpart, p.f32->npart, p.nx, p.dv, p.f32->c0, p.rho);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
-  return launch_poisson_only_f32(p, p.rho, driver, ft, e, s);
+  return field_any(p, p.rho, driver, ft, e, s);
 }
 
 // density of the current state by rows (stand-alone field solve / density):
@@ -410,23 +497,23 @@ cudaError_t launch_row_f32(const vg_plan& p, float* g, const double* e, double d
 
 cudaError_t launch_store_f32(const vg_plan& p, const float* g, const double* e, const double* de,
                              const vg_history& h, int i, int n_modes, cudaStream_t s) {
-  const int nb = std::min(F32_STORE_MAX_CTAS, (p.nx + 255) / 256);
-  k_store_fields_f32<<<nb, 256, 0, s>>>(p.mom, p.f32->rc, e, de, p.nx, i, h, p.f32->spart);
+  const int nb = std::min(F32_STORE_MAX_CTAS, div_up(p.nx, STORE_ROWS));
+  const bool modes = h.stored_f && !h.store_all && n_modes > 0;
+  const int mode_ctas = modes ? div_up(p.nv, 32) * n_modes : 0;
+  k_store_f32<<<nb + mode_ctas, STORE_BLOCK, 0, s>>>(p.mom, p.f32->rc_dev, e, de, p.nx, i, h, p.f32->spart, nb, p.f32->mpart,
+                                                     p.f32->mgrid, n_modes, p.nv, p.f_bg);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
-  k_store_series_f32<<<1, 32, 0, s>>>(p.f32->spart, nb, p.nx, i, h);
-  err = cudaGetLastError();
-  if (err != cudaSuccess) return err;
+  if (nb > 1) {
+    k_store_series_f32<<<1, 32, 0, s>>>(p.f32->spart, nb, p.nx, i, h);
+    err = cudaGetLastError();
+    if (err != cudaSuccess) return err;
+  }
   if (h.stored_f && h.store_all) {
     const size_t n = (size_t)p.nx * p.nv;
     const int blocks = (int)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096);
     k_store_all_f32<<<blocks, 256, 0, s>>>(g, p.f_bg, p.nx, p.nv, static_cast<double*>(h.stored_f) + (size_t)i * n);
     return cudaGetLastError();
-  }
-  if (h.stored_f && !h.store_all && n_modes > 0) {
-    k_store_modes_f32<<<dim3(div_up(p.nv, 32), n_modes), 32 * STORE_MODE_SPLIT, 0, s>>>(
-        p.f32->mpart, p.f32->mgrid, n_modes, p.nv, p.nx, p.f_bg, h.n_slots, i, static_cast<cx<float>*>(h.stored_f));
-    err = cudaGetLastError();
   }
   return err;
 }
