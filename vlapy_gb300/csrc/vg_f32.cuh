@@ -34,6 +34,9 @@ __device__ __forceinline__ df32 df_add(df32 a, df32 b) {
 __device__ __forceinline__ df32 df_shfl_xor(df32 a, int m) {
   return {__shfl_xor_sync(0xffffffffu, a.hi, m), __shfl_xor_sync(0xffffffffu, a.lo, m)};
 }
+__device__ __forceinline__ df32 df_shfl_down(df32 a, int m) {
+  return {__shfl_down_sync(0xffffffffu, a.hi, m), __shfl_down_sync(0xffffffffu, a.lo, m)};
+}
 __device__ __forceinline__ df32 df_warp_sum(df32 a) {
 #pragma unroll
   for (int m = 16; m > 0; m >>= 1) a = df_add(a, df_shfl_xor(a, m));
@@ -210,6 +213,28 @@ __device__ __forceinline__ void group_df_sum(df32 (&v)[NQ], df32* red, int G, in
   }
 }
 
+// The same sums where the group's thread q < NQ <= 32 alone needs the total of v[q]
+// (its return value): the warps' sums are added by NQ lanes side by side.  G a
+// multiple of 32; red holds G / 32 * NQ entries per group and may be written again
+// after the caller's next sync.
+template <int NQ, typename Sync>
+__device__ __forceinline__ df32 group_df_sum_lanes(const df32 (&v)[NQ], df32* red, int G, int t, const Sync& sync) {
+  static_assert(NQ <= 32, "one lane per value");
+  const int lane = t & 31, wid = t >> 5, nw = G >> 5;
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    float x = v[q].hi + v[q].lo;
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) x += __shfl_xor_sync(0xffffffffu, x, m);
+    if (lane == q) red[wid * NQ + q] = {x, 0.f};
+  }
+  sync();
+  df32 tot = {0.f, 0.f};
+  if (t < NQ)
+    for (int w = 0; w < nw; ++w) tot = df_add(tot, red[w * NQ + t]);
+  return tot;
+}
+
 // ---- tridiagonal solve: partition (interior Thomas) + reduced system -----
 // Solves rows j = 0..N-1: l(j) x[j-1] + b x[j] + u(j) x[j+1] = x_in[j]
 // (l(0) and u(N-1) ignored).  x is one component of a padded complex-float
@@ -340,7 +365,7 @@ __device__ __forceinline__ void partition_solve(float* x, int t, float b, LFn lf
     D = RD1 - RD0 * k1 - (up ? n0.w * k2 : 0.f);
   }
   // PCR on the G rows in x_e(t)
-#pragma unroll
+#pragma unroll 1
   for (int st = 1; st < G; st <<= 1) {
     const float4 me = make_float4(A, B, C, D);
     publish(me);

@@ -131,7 +131,8 @@ __device__ __forceinline__ df32 row_moment_df(const double* __restrict__ slots, 
 }
 
 // rotation of one packed row pair with the delta-f background term; the 1/N of
-// the inverse transform is folded in.  ha/hb: half-angle per kv index.
+// the inverse transform is folded in.  ha/hb: half-angle per kv index.  The
+// result is left with real and imaginary parts exchanged, for kick_io.
 template <int N, int PS = pad_shift<float>()>
 __device__ __forceinline__ void kick_rotate(cx<float>* s, int t, int G, Ang ha, Ang hb,
                                             const cx<float>* __restrict__ F0) {
@@ -151,7 +152,7 @@ __device__ __forceinline__ void kick_rotate(cx<float>* s, int t, int G, Ang ha, 
     if (k == 0 || 2 * k == N) {
       const cx<float> z = s[sp<float, PS>(k)];
       // real bins: only Re(P) survives
-      s[sp<float, PS>(k)] = {(pa_r * z.x + pa_m1r * f0.x) * sc, (pb_r * z.y + pb_m1r * f0.x) * sc};
+      s[sp<float, PS>(k)] = {(pb_r * z.y + pb_m1r * f0.x) * sc, (pa_r * z.x + pa_m1r * f0.x) * sc};
     } else {
       const cx<float> zk = s[sp<float, PS>(k)], zm = s[sp<float, PS>(N - k)];
       const cx<float> fa = {(zk.x + zm.x) * 0.5f, (zk.y - zm.y) * 0.5f};
@@ -160,8 +161,8 @@ __device__ __forceinline__ void kick_rotate(cx<float>* s, int t, int G, Ang ha, 
                             (pa_r * fa.y + pa_i * fa.x + pa_m1r * f0.y + pa_i * f0.x) * sc};
       const cx<float> gb = {(pb_r * fb.x - pb_i * fb.y + pb_m1r * f0.x - pb_i * f0.y) * sc,
                             (pb_r * fb.y + pb_i * fb.x + pb_m1r * f0.y + pb_i * f0.x) * sc};
-      s[sp<float, PS>(k)] = {ga.x - gb.y, ga.y + gb.x};
-      s[sp<float, PS>(N - k)] = {ga.x + gb.y, gb.x - ga.y};
+      s[sp<float, PS>(k)] = {ga.y + gb.x, ga.x - gb.y};
+      s[sp<float, PS>(N - k)] = {gb.x - ga.y, ga.x + gb.y};
     }
     const float na = sa * cga + ca * sga, nca = ca * cga - sa * sga;
     const float nb = sb * cgb + cb * sgb, ncb = cb * cgb - sb * sgb;
@@ -172,24 +173,33 @@ __device__ __forceinline__ void kick_rotate(cx<float>* s, int t, int G, Ang ha, 
   }
 }
 
-// the kick with the row pair in registers at either end (IO bit 0: io holds
-// the pair's elements t + i G on entry and s need not; bit 1: they end in io;
-// the row pass uses IO = 3, both)
-template <int N, int R, int IO, typename Sync>
+// The kick of a row pair whose elements t + i G are in registers, before and after.
+// Both transforms run the same code: with real and imaginary parts exchanged at
+// either end, the forward transform is the inverse one.
+template <int N, int R, typename Sync>
 __device__ __forceinline__ void kick_io(cx<float>* s, int t, float hk, float ea, float eb,
                                         const cx<float>* __restrict__ F0, const cx<float>* __restrict__ tw,
                                         const Sync& sync, cx<float> (&io)[R]) {
   constexpr int G = N / R;
   constexpr int PS = row_pad_shift(R);
-  block_fft_io<float, N, false, R, IO & 1, Sync, PS>(s, t, tw, sync, io);
-  // theta(k) = -kv_k dt e = k * (-dkv dt e); hk = -dkv dt / 2 gives the half
-  // angle for P - 1.  The kick angle stays O(10) rad, so an FP32 product is
-  // accurate to ~1e-6 rad here
-  const Ang ha = {hk * ea, 0.f};
-  const Ang hb = {hk * eb, 0.f};
-  kick_rotate<N, PS>(s, t, G, ha, hb, F0);
-  sync();
-  block_fft_io<float, N, true, R, IO & 2, Sync, PS>(s, t, tw, sync, io);
+#pragma unroll 1
+  for (int inverse = 0; inverse < 2; ++inverse) {
+    block_fft_io<float, N, false, R, 3, Sync, PS>(s, t, tw, sync, io);
+    if (inverse) break;
+    sync();
+#pragma unroll
+    for (int i = 0; i < R; ++i) s[sp<float, PS>(t + i * G)] = io[i];
+    sync();
+    // theta(k) = -kv_k dt e = k * (-dkv dt e); hk = -dkv dt / 2 gives the half
+    // angle for P - 1.  The kick angle stays O(10) rad, so an FP32 product is
+    // accurate to ~1e-6 rad here
+    kick_rotate<N, PS>(s, t, G, {hk * ea, 0.f}, {hk * eb, 0.f}, F0);
+    sync();
+#pragma unroll
+    for (int i = 0; i < R; ++i) io[i] = s[sp<float, PS>(t + i * G)];
+  }
+#pragma unroll
+  for (int i = 0; i < R; ++i) io[i] = {io[i].y, io[i].x};
 }
 
 // Per-row collision scalars from the row's raw moment sums (sum w g v^p,
@@ -219,7 +229,18 @@ __device__ __forceinline__ void collision_scalars(const RowConsts& rc, float2 nu
 // in the real parts of s, row b in the imaginary parts).  The moments and the
 // right-hand sides of the two rows share one pass over the pair (one 8-byte
 // access per element, one load of each constant) and one reduction; the two
-// tridiagonal solves run one after the other.
+// tridiagonal solves run one after the other, in one copy of the code.
+//
+// What bounds the row pass is the instruction cache, before FP32 issue: a row pair
+// walks through all of its code once, and two CTAs do so at different places.  With
+// the transforms of a kick, the two solves and the loops over a thread's R elements
+// all written out, a third to a half of the stalls were for instructions (nv = 8192:
+// 555 us a pass over 4096 rows, now 430) and the time changed by 15 % with whatever
+// else the library held.  So each of them is there once, in loops that stay rolled,
+// and the passes over shared memory are unrolled by ROW_UNROLL (2: 8 % slower over
+// the whole step at 4096 x 8192, 4: 2 %, 16: as fast; a sweep of 64 runs 7 %, 2 %,
+// 0 %).
+constexpr int ROW_UNROLL = 8;
 template <int N, int R, typename Sync = CtaSync>
 __device__ __forceinline__ void collide_pair(cx<float>* s, int t, const RowConsts& rc, float2 nudt2, float nudt_f,
                                              int dougherty, df32* red, float* pcr, const Sync& sync = Sync()) {
@@ -230,7 +251,7 @@ __device__ __forceinline__ void collide_pair(cx<float>* s, int t, const RowConst
   df32 mv[6];
   {
     float m[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
+#pragma unroll ROW_UNROLL
     for (int i = 0; i < R; ++i) {
       const int j = t + i * G;
       const float w = (j == 0 || j == N - 1) ? 0.5f : 1.f;
@@ -247,12 +268,18 @@ __device__ __forceinline__ void collide_pair(cx<float>* s, int t, const RowConst
 #pragma unroll
     for (int q = 0; q < 6; ++q) mv[q] = {m[q], 0.f};
   }
-  group_df_sum<6, true>(mv, red, G, t, sync);
-  // per-row scalars in double-float by one thread; the group reads them back
+  // per-row scalars in double-float, each row's by one thread; the group reads them back
   float* sc = reinterpret_cast<float*>(red);
-  if (t == 0) {
-    collision_scalars(rc, nudt2, dougherty, mv[0], mv[1], mv[2], sc);
-    collision_scalars(rc, nudt2, dougherty, mv[3], mv[4], mv[5], sc + 5);
+  if constexpr (G >= 32) {
+    df32 s0 = group_df_sum_lanes<6>(mv, reinterpret_cast<df32*>(pcr), G, t, sync);
+    if (t < 32) {
+      const df32 s1 = df_shfl_down(s0, 1), s2 = df_shfl_down(s0, 2);
+      if (t == 0 || t == 3) collision_scalars(rc, nudt2, dougherty, s0, s1, s2, sc + (t ? 5 : 0));
+    }
+  } else {
+    group_df_sum<6, true>(mv, red, G, t, sync);
+    for (int q = t; q < 2; q += G)
+      collision_scalars(rc, nudt2, dougherty, q ? mv[3] : mv[0], q ? mv[4] : mv[1], q ? mv[5] : mv[2], sc + 5 * q);
   }
   sync();
   float sa[5], sb[5];
@@ -266,7 +293,7 @@ __device__ __forceinline__ void collide_pair(cx<float>* s, int t, const RowConst
   const float i2dv = rc.i2dv;
   sync();
   // right-hand sides: g - (A - I) f0 with (A - I) f0 = nudt (-vth S + Mv - vbar D)
-#pragma unroll
+#pragma unroll ROW_UNROLL
   for (int i = 0; i < R; ++i) {
     const int j = t + i * G;
     const float S = rc.S[j], Mv = rc.Mv[j], D = rc.D[j];
@@ -279,18 +306,12 @@ __device__ __forceinline__ void collide_pair(cx<float>* s, int t, const RowConst
   // off-diagonals at v[j -+ 1] of the uniform grid v[j] = v[0] + j dv,
   // formed in registers (within an FP32 ulp of the tabulated grid)
   const float v0 = rc.v0f, dvf = rc.dvf;
-  float* x = reinterpret_cast<float*>(s);
-  {
-    const float Af = sa[0], vb = sa[2];
+#pragma unroll 1
+  for (int row = 0; row < 2; ++row) {
+    const float Af = row ? sb[0] : sa[0], diag = row ? sb[1] : sa[1], vb = row ? sb[2] : sa[2];
     auto lf = [&](int j) { return nu * (Af + (fmaf((float)(j - 1), dvf, v0) - vb) * i2dv); };
     auto uf = [&](int j) { return nu * (Af - (fmaf((float)(j + 1), dvf, v0) - vb) * i2dv); };
-    partition_solve<R, G>(x, t, sa[1], lf, uf, pcr, sync);
-  }
-  {
-    const float Af = sb[0], vb = sb[2];
-    auto lf = [&](int j) { return nu * (Af + (fmaf((float)(j - 1), dvf, v0) - vb) * i2dv); };
-    auto uf = [&](int j) { return nu * (Af - (fmaf((float)(j + 1), dvf, v0) - vb) * i2dv); };
-    partition_solve<R, G>(x + 1, t, sb[1], lf, uf, pcr, sync);
+    partition_solve<R, G>(reinterpret_cast<float*>(s) + row, t, diag, lf, uf, pcr, sync);
   }
 }
 
@@ -327,7 +348,7 @@ __device__ __forceinline__ void row_pair(const RowArgs& a, int pair, unsigned ch
       const int n = t + i * G;
       io[i] = {va ? ga[n] : 0.f, vb ? gbp[n] : 0.f};
     }
-    if (a.hk1 != 0.f) kick_io<N, R, 3>(s, t, a.hk1, ea, eb, a.F0, a.tw, sync, io);
+    if (a.hk1 != 0.f) kick_io<N, R>(s, t, a.hk1, ea, eb, a.F0, a.tw, sync, io);
 #pragma unroll
     for (int i = 0; i < R; ++i) {
       const int n = t + i * G;
@@ -358,7 +379,7 @@ __device__ __forceinline__ void row_pair(const RowArgs& a, int pair, unsigned ch
       for (int i = 0; i < R; ++i) io[i] = s[sp<float, row_pad_shift(R)>(t + i * G)];
     }
     if (hk != 0.f) {
-      kick_io<N, R, 3>(s, t, hk, ea, eb, a.F0, a.tw, sync, io);
+      kick_io<N, R>(s, t, hk, ea, eb, a.F0, a.tw, sync, io);
     }
     if (kpass == 1) {
       // the last FFT pass left elements t + i G in registers: the store
@@ -386,7 +407,7 @@ __device__ __forceinline__ void row_pair(const RowArgs& a, int pair, unsigned ch
       static_assert(NPOW >= 1 && NPOW <= 6, "power moments");
       constexpr int NQ = NPOW + 3;
       float sa[NQ] = {0}, sb[NQ] = {0};
-  #pragma unroll
+  #pragma unroll ROW_UNROLL
       for (int i = 0; i < R; ++i) {
         const int j = t + i * G;  // consecutive threads, consecutive j: coalesced loads
         const float w = (j == 0 || j == N - 1) ? 0.5f : 1.f;
@@ -417,40 +438,34 @@ __device__ __forceinline__ void row_pair(const RowArgs& a, int pair, unsigned ch
         m2[q] = {sa[q], 0.f};
         m2[NQ + q] = {sb[q], 0.f};
       }
-      // one reduction of both rows where red has the room (9 slots per warp
-      // and one more warp's worth; a group inside one warp needs none), else
-      // one per row
-      constexpr int NW = G >= 32 ? G / 32 : 1;
-      if constexpr (G < 32 || 2 * NQ * NW <= 9 * (G / 32 + 1)) {
-        group_df_sum<2 * NQ, true>(m2, red, G, t, sync);
+      // raw sums; the storage kernels form dv * sum + trapz(f0 ...) in FP64: slots
+      // 0 .. NPOW - 1 the powers, 6 sum w (g^2 + 2 g f0), 7 sum w f log f
+      if constexpr (G >= 32) {
+        const df32 tot = group_df_sum_lanes<2 * NQ>(m2, reinterpret_cast<df32*>(pcr), G, t, sync);
+        if (t < 32) {
+          const df32 nx1 = df_shfl_down(tot, 1);
+          const int q = t < NQ ? t : t - NQ, row = t < NQ ? ra : rb;
+          if (t < 2 * NQ && row < a.nx && q != NPOW + 1) {
+            df32* out = reinterpret_cast<df32*>(a.mom + (size_t)row * MOM_STRIDE);
+            if (q < NPOW) out[q] = tot;
+            else if (q == NPOW) out[6] = df_add(tot, {2.f * nx1.hi, 2.f * nx1.lo});
+            else out[7] = tot;
+          }
+        }
       } else {
-        df32 ma[NQ], mb[NQ];
+        group_df_sum<2 * NQ, true>(m2, red, G, t, sync);
+        if (t == 0) {
+          // each array is indexed by constants only, so it stays in registers
+          auto put = [&](int o, int row) {
+            df32* out = reinterpret_cast<df32*>(a.mom + (size_t)row * MOM_STRIDE);
   #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-          ma[q] = m2[q];
-          mb[q] = m2[NQ + q];
+            for (int p = 0; p < NPOW; ++p) out[p] = m2[o + p];
+            out[6] = df_add(m2[o + NPOW], {2.f * m2[o + NPOW + 1].hi, 2.f * m2[o + NPOW + 1].lo});
+            out[7] = m2[o + NPOW + 2];
+          };
+          if (va) put(0, ra);
+          if (vb) put(NQ, rb);
         }
-        group_df_sum<NQ, true>(ma, red, G, t, sync);
-        group_df_sum<NQ, true>(mb, red, G, t, sync);
-  #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-          m2[q] = ma[q];
-          m2[NQ + q] = mb[q];
-        }
-      }
-      if (t == 0) {
-        // raw sums; the storage kernels form dv * sum + trapz(f0 ...) in FP64.
-        // Each array is indexed by constants only, so it stays in registers.
-        auto put = [&](int o, int row) {
-          df32* out = reinterpret_cast<df32*>(a.mom + (size_t)row * MOM_STRIDE);
-  #pragma unroll
-          for (int p = 0; p < NPOW; ++p) out[p] = m2[o + p];
-          // sum w (g^2 + 2 g f0)
-          out[6] = df_add(m2[o + NPOW], {2.f * m2[o + NPOW + 1].hi, 2.f * m2[o + NPOW + 1].lo});
-          out[7] = m2[o + NPOW + 2];
-        };
-        if (va) put(0, ra);
-        if (vb) put(NQ, rb);
       }
       // x-Fourier modes of f (the f0 part of mode 0 is added in the reduction);
       // the groups of a CTA hold different rows but add into the same bins,
@@ -463,6 +478,7 @@ __device__ __forceinline__ void row_pair(const RowArgs& a, int pair, unsigned ch
               float swa = 0.f, cwa = 0.f, swb = 0.f, cwb = 0.f;
               if (va) sincospif(-2.f * (float)((mq * ra) % a.nx) / (float)a.nx, &swa, &cwa);
               if (vb) sincospif(-2.f * (float)((mq * rb) % a.nx) / (float)a.nx, &swb, &cwb);
+  #pragma unroll ROW_UNROLL
               for (int i = 0; i < R; ++i) {
                 const int n = t + i * G;
                 const cx<float> z = s[sp<float, row_pad_shift(R)>(n)];
