@@ -478,13 +478,29 @@ __device__ __forceinline__ void row_pair(const RowArgs& a, int pair, unsigned ch
               float swa = 0.f, cwa = 0.f, swb = 0.f, cwb = 0.f;
               if (va) sincospif(-2.f * (float)((mq * ra) % a.nx) / (float)a.nx, &swa, &cwa);
               if (vb) sincospif(-2.f * (float)((mq * rb) % a.nx) / (float)a.nx, &swb, &cwb);
-  #pragma unroll ROW_UNROLL
-              for (int i = 0; i < R; ++i) {
-                const int n = t + i * G;
-                const cx<float> z = s[sp<float, row_pad_shift(R)>(n)];
-                cx<float>& acc = macc[(size_t)mq * N + n];
-                acc.x += z.x * cwa + z.y * cwb;
-                acc.y += z.x * swa + z.y * swb;
+              // in batches: reads first, so that a batch waits once.  Accumulators in
+              // global memory are added to in L2, whence nothing returns to wait for
+              // (a bin is one thread's at a time, so the order is fixed)
+              constexpr int U = R < ROW_UNROLL ? R : ROW_UNROLL;
+              cx<float>* m0 = macc + (size_t)mq * N + t;
+              for (int i0 = 0; i0 < R; i0 += U) {
+                cx<float> z[U];
+  #pragma unroll
+                for (int u = 0; u < U; ++u) {
+                  const cx<float> q = s[sp<float, row_pad_shift(R)>(t + (i0 + u) * G)];
+                  z[u] = {q.x * cwa + q.y * cwb, q.x * swa + q.y * swb};
+                }
+                if (a.macc_global) {
+  #pragma unroll
+                  for (int u = 0; u < U; ++u)
+                    atomicAdd(reinterpret_cast<float2*>(m0 + (i0 + u) * G), make_float2(z[u].x, z[u].y));
+                } else {
+                  cx<float> acc[U];
+  #pragma unroll
+                  for (int u = 0; u < U; ++u) acc[u] = m0[(i0 + u) * G];
+  #pragma unroll
+                  for (int u = 0; u < U; ++u) m0[(i0 + u) * G] = {acc[u].x + z[u].x, acc[u].y + z[u].y};
+                }
               }
             }
           }
