@@ -10,46 +10,65 @@
 
 namespace vg {
 
-constexpr int COL32_PAD = 1;
-
-// One column tile [NX x W] at column c0: x-drift by exp(i m (-dkx dt) v_col)
-// and the tile's trapz-weighted density partials added into dacc[x].
-// smem: W/2 padded sequences of NX complex floats.
+// Shape of a column tile of the single-run x-drift: S column pairs by G threads
+// each, laid out so that L neighbouring lanes hold neighbouring pairs of one row
+// (8 L contiguous bytes), the rows following.  The sequences start 16 / L elements
+// apart modulo the banks (a row of 16 lanes then covers all of them), at least one.
 template <int NX, int R>
-__device__ __forceinline__ void col_tile(float* __restrict__ g, int nv, int c0, int W, float2 kdt,
+struct Col32 {
+  static constexpr int G = NX / R;
+  static constexpr int S = col32_seqs(NX, R);
+  static constexpr int L = S < 32 ? S : 32;
+  static constexpr int SETS = S / L;
+  static constexpr int LD = (sp_len<float>(NX) + 15) / 16 * 16 + (L < 16 ? 16 / L : 1);
+  static constexpr size_t smem =
+      (size_t)S * LD * sizeof(cx<float>) + (size_t)NX * sizeof(df32) + (SETS > 1 ? (size_t)SETS * NX * sizeof(float) : 0);
+};
+
+// One column tile at column c0: x-drift by exp(i m (-dkx dt) v_col) and the tile's
+// trapz-weighted density partials added into dacc[x].  Columns past nv (the tile is
+// wider than a short row) are zeros that nothing reads.  vec: g is 8-byte aligned.
+//
+// The elements t + i G of a pair go from global memory into the first pass's
+// registers and from the last pass's back; both transforms run the same code
+// (exchanged parts, as in kick_io).  A pass over 4096 x 8192 took 229 us by way of
+// shared memory at either end, with each transform written out; now 155.
+template <int NX, int R>
+__device__ __forceinline__ void col_tile(float* __restrict__ g, int nv, int c0, bool vec, float2 kdt,
                                          const float2* __restrict__ vhl, const cx<float>* __restrict__ tw,
-                                         unsigned char* smem, df32* dacc) {
-  constexpr int G = NX / R;
-  constexpr int LD = sp_len<float>(NX) + COL32_PAD;
-  cx<float>* s = reinterpret_cast<cx<float>*>(smem);
-  float* sf = reinterpret_cast<float*>(smem);
-  const int grp = threadIdx.x / G, t = threadIdx.x - grp * G;
-  cx<float>* sg = s + (size_t)grp * LD;
-  const float scale = 1.f / NX;
-  // the tile in 16-byte vectors when W and nv are multiples of 4 floats
-  // (then so are c0 and every row start), else float by float
-  const bool vec = ((W | nv) & 3) == 0;
-  const int total = NX * W, total4 = vec ? total / 4 : 0;
-  for (int q = threadIdx.x; q < total4; q += blockDim.x) {
-    const int x = q / (W / 4), c = 4 * (q - x * (W / 4));
-    const float4 v = *reinterpret_cast<const float4*>(g + (size_t)x * nv + c0 + c);
-    sf[2 * ((c >> 1) * LD + sp<float>(x))] = v.x;
-    sf[2 * ((c >> 1) * LD + sp<float>(x)) + 1] = v.y;
-    sf[2 * (((c >> 1) + 1) * LD + sp<float>(x))] = v.z;
-    sf[2 * (((c >> 1) + 1) * LD + sp<float>(x)) + 1] = v.w;
+                                         cx<float>* smem, float* dset, df32* dacc) {
+  using C = Col32<NX, R>;
+  constexpr int G = C::G, L = C::L;
+  const int lane = threadIdx.x & 31;
+  const int slot = threadIdx.x / L;
+  const int t = slot & (G - 1), set = slot / G;
+  const int grp = (threadIdx.x & (L - 1)) + L * set;
+  cx<float>* sg = smem + (size_t)grp * C::LD;
+  const int c = c0 + 2 * grp;
+  const bool valid = c < nv;
+  float* gc = g + c;
+  const CtaSync sync;
+  cx<float> io[R];
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const float* q = gc + (size_t)(t + i * G) * nv;
+    if (!valid) io[i] = {0.f, 0.f};
+    else if (vec) io[i] = *reinterpret_cast<const cx<float>*>(q);
+    else io[i] = {q[0], q[1]};
   }
-  if (!vec)
-    for (int q = threadIdx.x; q < total; q += blockDim.x) {
-      const int x = q / W, c = q - x * W;
-      sf[2 * ((c >> 1) * LD + sp<float>(x)) + (c & 1)] = g[(size_t)x * nv + c0 + c];
-    }
-  __syncthreads();
-  block_fft<float, NX, false, R>(sg, t, tw);
-  // theta(m) = m * (-dkx dt) v_col (kx = m dkx on the bins m <= NX/2); the angle
-  // per unit m is the double-float product of kdt = -dkx dt and v (both split)
-  const Ang aa = mul_angle(kdt, vhl[c0 + 2 * grp]);
-  const Ang ab = mul_angle(kdt, vhl[c0 + 2 * grp + 1]);
-  {
+#pragma unroll 1
+  for (int inverse = 0; inverse < 2; ++inverse) {
+    block_fft_io<float, NX, false, R, 3>(sg, t, tw, sync, io);
+    if (inverse) break;
+    sync();
+#pragma unroll
+    for (int i = 0; i < R; ++i) sg[sp<float>(t + i * G)] = io[i];
+    sync();
+    // theta(m) = m * (-dkx dt) v_col (kx = m dkx on the bins m <= NX/2); the angle
+    // per unit m is the double-float product of kdt = -dkx dt and v (both split)
+    const Ang aa = mul_angle(kdt, vhl[valid ? c : 0]);
+    const Ang ab = mul_angle(kdt, vhl[valid ? c + 1 : 0]);
+    const float scale = 1.f / NX;
     // phases exp(i m a) for this thread's bins m = t, t+G, ...: one sincos for
     // the start, one for the step, complex products in between
     float sa, ca, sb, cb, sga, cga, sgb, cgb;
@@ -57,7 +76,7 @@ __device__ __forceinline__ void col_tile(float* __restrict__ g, int nv, int c0, 
     sincos_m((float)t, ab, sb, cb);
     sincos_m((float)G, aa, sga, cga);
     sincos_m((float)G, ab, sgb, cgb);
-    two_real_rotate<float>(sg, NX, t, G, [&](int, float& pca, float& psa, float& pcb, float& psb) {
+    two_real_rotate<float, true>(sg, NX, t, G, [&](int, float& pca, float& psa, float& pcb, float& psb) {
       pca = ca * scale;
       psa = sa * scale;
       pcb = cb * scale;
@@ -69,51 +88,45 @@ __device__ __forceinline__ void col_tile(float* __restrict__ g, int nv, int c0, 
       sb = nb;
       cb = ncb;
     });
+    sync();
+#pragma unroll
+    for (int i = 0; i < R; ++i) io[i] = sg[sp<float>(t + i * G)];
   }
-  __syncthreads();
-  block_fft<float, NX, true, R>(sg, t, tw);
-  // density partial sums (trapz weights: 1/2 at the two v end points): the
-  // tpx threads of an x point (consecutive lanes) share its W columns and
-  // add their sums by shuffles
-  const int tpx = (int)blockDim.x >= NX ? (int)blockDim.x / NX : 1;
-  if (tpx > 1 && tpx <= 32) {
-    const int x = threadIdx.x / tpx, part = threadIdx.x - x * tpx;
-    float acc = 0.f;
-    for (int c = part; c < W; c += tpx) {
-      const int col = c0 + c;
-      const float w = (col == 0 || col == nv - 1) ? 0.5f : 1.f;
-      acc = fmaf(w, sf[2 * ((c >> 1) * LD + sp<float>(x)) + (c & 1)], acc);
+  // column c is in the imaginary parts now, c + 1 in the real ones.  Density
+  // partials with trapz weights: 1/2 at the two v end points
+  float d[R];
+  const float wa = c == 0 ? 0.5f : 1.f, wb = c + 1 == nv - 1 ? 0.5f : 1.f;
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    float* q = gc + (size_t)(t + i * G) * nv;
+    if (valid && vec) {
+      *reinterpret_cast<cx<float>*>(q) = {io[i].y, io[i].x};
+    } else if (valid) {
+      q[0] = io[i].y;
+      q[1] = io[i].x;
     }
-    for (int m = tpx >> 1; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
-    if (part == 0) dacc[x] = df_add(dacc[x], {acc, 0.f});
-  } else {
-    for (int x = threadIdx.x; x < NX; x += blockDim.x) {
+    d[i] = fmaf(wb, io[i].x, wa * io[i].y);
+  }
+  int idx;
+  bool writer;
+  lane_transpose_sum<R, L>(d, lane, idx, writer);
+  if (writer) {
+#pragma unroll
+    for (int q = 0; q < (R > L ? R / L : 1); ++q) {
+      const int x = t + (idx + q) * G;
+      if constexpr (C::SETS == 1) dacc[x] = df_add(dacc[x], {d[q], 0.f});
+      else dset[set * NX + x] = d[q];
+    }
+  }
+  if constexpr (C::SETS > 1) {
+    sync();
+    for (int x = threadIdx.x; x < NX; x += C::S * G) {
       float acc = 0.f;
-      for (int c = 0; c < W; ++c) {
-        const int col = c0 + c;
-        const float w = (col == 0 || col == nv - 1) ? 0.5f : 1.f;
-        acc = fmaf(w, sf[2 * ((c >> 1) * LD + sp<float>(x)) + (c & 1)], acc);
-      }
+      for (int q = 0; q < C::SETS; ++q) acc += dset[q * NX + x];
       dacc[x] = df_add(dacc[x], {acc, 0.f});
     }
   }
-  for (int q = threadIdx.x; q < total4; q += blockDim.x) {
-    const int x = q / (W / 4), c = 4 * (q - x * (W / 4));
-    float4 v;
-    v.x = sf[2 * ((c >> 1) * LD + sp<float>(x))];
-    v.y = sf[2 * ((c >> 1) * LD + sp<float>(x)) + 1];
-    v.z = sf[2 * (((c >> 1) + 1) * LD + sp<float>(x))];
-    v.w = sf[2 * (((c >> 1) + 1) * LD + sp<float>(x)) + 1];
-    *reinterpret_cast<float4*>(g + (size_t)x * nv + c0 + c) = v;
-  }
-  if (!vec)
-    for (int q = threadIdx.x; q < total; q += blockDim.x) {
-      const int x = q / W, c = q - x * W;
-      g[(size_t)x * nv + c0 + c] = sf[2 * ((c >> 1) * LD + sp<float>(x)) + (c & 1)];
-    }
-  __syncthreads();
 }
-
 
 // Moment slot q of one row (0..5: n, j, T, q, fv4, vN; 6: trapz(f^2);
 // 7: trapz(f log f)) from the raw double-float sums the row pass leaves in

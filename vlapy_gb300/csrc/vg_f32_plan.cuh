@@ -69,15 +69,17 @@ struct F32Plan {
 
 // launch shapes of the single-run kernels (shared by their __launch_bounds__
 // and the launchers; the batched sweep chooses its own)
-// column tiles: radix 8 up to nx = 1024, radix 16 above; S column pairs per
-// CTA, at least 4 (32-byte row segments) but at most 512 threads, so that a
-// thread keeps up to 128 registers
-__host__ __device__ constexpr int col32_radix(int nx) { return nx <= 8 ? nx : (nx <= 1024 ? 8 : 16); }
-__host__ __device__ constexpr int col32_seqs_raw(int g) { return (256 / g) > 4 ? (256 / g) : 4; }
-__host__ __device__ constexpr int col32_seqs(int nx, int r) {
-  return (nx / r) * col32_seqs_raw(nx / r) <= 512 ? col32_seqs_raw(nx / r)
-                                                   : (512 / (nx / r) > 1 ? 512 / (nx / r) : 1);
-}
+// Column tiles: as few passes as the threads' registers allow.  From nx = 1024 on
+// radix 32 by 512 threads (two passes at 1024, three to 8192), one CTA per SM: at
+// nx = 4096 that is four column pairs, whole 32-byte sectors of a row, and a pass
+// over 4096 x 8192 takes 155 us; with radix 16 and two pairs 181, with radix 32 in
+// two CTAs of two pairs 216.  Below, 256 threads: radix 16 at 256 and 512 (282 ->
+// 276 and 404 -> 390 us for four steps by 4096, against radix 8), radix 8 up to 128
+// (256 us; 259 with radix 16).
+__host__ __device__ constexpr int col32_radix(int nx) { return nx <= 8 ? nx : nx <= 128 ? 8 : nx <= 512 ? 16 : 32; }
+__host__ __device__ constexpr int col32_threads(int nx) { return nx < 1024 ? 256 : 512; }
+__host__ __device__ constexpr int col32_seqs(int nx, int r) { return col32_threads(nx) / (nx / r); }
+__host__ __device__ constexpr int col32_min_blocks(int nx, int r) { return col32_threads(nx) == 256 && r == 16 ? 2 : 1; }
 // row radix of the single-run kernels: radix 8 up to 4096; radix 32 above
 // (8192 = 32 x 32 x 8: three passes, and a 256-thread row-pair group that
 // leaves room for a second CTA on the SM to hide the passes' barriers)

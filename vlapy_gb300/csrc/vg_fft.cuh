@@ -271,8 +271,9 @@ __device__ __forceinline__ void block_fft_io(cx<T>* s, int t, const cx<T>* __res
 // P(k) = cos(th(k)) + i sin(th(k)).  At the Nyquist bin only Re(P) acts,
 // which is what taking the real part of the inverse transform does to the
 // reference's full complex product.  phase(k, &ca, &sa, &cb, &sb) returns the
-// two rotations for bin k.
-template <typename T, typename PhaseFn>
+// two rotations for bin k.  SWAP: the result with real and imaginary parts
+// exchanged, whose forward transform is the inverse transform, exchanged.
+template <typename T, bool SWAP = false, typename PhaseFn>
 __device__ __forceinline__ void two_real_rotate(cx<T>* s, int N, int t, int G, PhaseFn phase) {
   for (int k = t; k <= N / 2; k += G) {
     T ca, sa, cb, sb;
@@ -282,12 +283,12 @@ __device__ __forceinline__ void two_real_rotate(cx<T>* s, int N, int t, int G, P
     if (k == 0) {
       const cx<T> z = s[0];
       // DC bins of both real sequences are real: only Re(P) survives
-      s[0] = {z.x * ca, z.y * cb};
+      s[0] = SWAP ? cx<T>{z.y * cb, z.x * ca} : cx<T>{z.x * ca, z.y * cb};
       continue;
     }
     if (2 * k == N) {
       const cx<T> z = s[sp<T>(k)];
-      s[sp<T>(k)] = {z.x * ca, z.y * cb};
+      s[sp<T>(k)] = SWAP ? cx<T>{z.y * cb, z.x * ca} : cx<T>{z.x * ca, z.y * cb};
       continue;
     }
     const cx<T> zk = s[sp<T>(k)], zm = s[sp<T>(N - k)];
@@ -295,8 +296,8 @@ __device__ __forceinline__ void two_real_rotate(cx<T>* s, int N, int t, int G, P
     const cx<T> fb = {(zk.y + zm.y) * T(0.5), (zm.x - zk.x) * T(0.5)};
     const cx<T> ga = {ca * fa.x - sa * fa.y, ca * fa.y + sa * fa.x};
     const cx<T> gb = {cb * fb.x - sb * fb.y, cb * fb.y + sb * fb.x};
-    s[sp<T>(k)] = {ga.x - gb.y, ga.y + gb.x};
-    s[sp<T>(N - k)] = {ga.x + gb.y, gb.x - ga.y};
+    s[sp<T>(k)] = SWAP ? cx<T>{ga.y + gb.x, ga.x - gb.y} : cx<T>{ga.x - gb.y, ga.y + gb.x};
+    s[sp<T>(N - k)] = SWAP ? cx<T>{gb.x - ga.y, ga.x + gb.y} : cx<T>{ga.x + gb.y, gb.x - ga.y};
   }
 }
 

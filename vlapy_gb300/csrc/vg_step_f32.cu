@@ -22,16 +22,22 @@ namespace vg {
 // ---------------------------------------------------------------------------
 
 template <int NX, int R>
-__global__ void __launch_bounds__((NX / R) * col32_seqs(NX, R)) k_col_f32(
-    float* __restrict__ g, int nv, int ntiles, int W, float2 kdt,
-    const float2* __restrict__ vhl, const cx<float>* __restrict__ tw, float2* __restrict__ dpart) {
-  constexpr int LD = sp_len<float>(NX) + COL32_PAD;
+__global__ void __launch_bounds__(Col32<NX, R>::S* Col32<NX, R>::G, col32_min_blocks(NX, R)) k_col_f32(
+    float* __restrict__ g, int nv, int ntiles, float2 kdt, const float2* __restrict__ vhl,
+    const cx<float>* __restrict__ tw, float2* __restrict__ dpart) {
+  using C = Col32<NX, R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int S = W / 2;
-  df32* dacc = reinterpret_cast<df32*>(smem_raw + (size_t)S * LD * sizeof(cx<float>));
+  cx<float>* s = reinterpret_cast<cx<float>*>(smem_raw);
+  df32* dacc = reinterpret_cast<df32*>(s + (size_t)C::S * C::LD);
+  float* dset = reinterpret_cast<float*>(dacc + NX);
   for (int x = threadIdx.x; x < NX; x += blockDim.x) dacc[x] = {0.f, 0.f};
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-    col_tile<NX, R>(g, nv, tile * W, W, kdt, vhl, tw, smem_raw, dacc);
+  const bool vec = (reinterpret_cast<uintptr_t>(g) & 7) == 0;  // (nv and the tiles' starts are even)
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    // (every thread has written dacc's zeros, or done with the last tile's sequences)
+    __syncthreads();
+    col_tile<NX, R>(g, nv, tile * 2 * C::S, vec, kdt, vhl, tw, s, dset, dacc);
+  }
+  __syncthreads();
   for (int x = threadIdx.x; x < NX; x += blockDim.x)
     dpart[(size_t)blockIdx.x * NX + x] = make_float2(dacc[x].hi, dacc[x].lo);
 }
@@ -319,21 +325,17 @@ namespace {
 template <int NX>
 cudaError_t col_n(const vg_plan& p, float* g, double dt, cudaStream_t s) {
   constexpr int R = col32_radix(NX);
-  constexpr int G = NX / R;
-  int S = col32_seqs(NX, R);
-  if (2 * S > p.nv) S = p.nv / 2;
-  const int W = 2 * S;
-  const int ntiles = p.nv / W;
-  const size_t smem = (size_t)S * (sp_len<float>(NX) + COL32_PAD) * sizeof(cx<float>) + (size_t)NX * sizeof(df32);
-  cudaError_t err = ensure_smem((const void*)k_col_f32<NX, R>, smem);
+  using C = Col32<NX, R>;
+  const int ntiles = div_up(p.nv, 2 * C::S);
+  cudaError_t err = ensure_smem((const void*)k_col_f32<NX, R>, C::smem);
   if (err != cudaSuccess) return err;
   int occ = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_col_f32<NX, R>, S * G, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_col_f32<NX, R>, C::S * C::G, C::smem);
   int grid = (occ > 0 ? occ : 1) * p.f32->n_sm;
   if (grid > p.f32->col_grid_max) grid = p.f32->col_grid_max;
   if (grid > ntiles) grid = ntiles;
-  k_col_f32<NX, R><<<grid, S * G, smem, s>>>(g, p.nv, ntiles, W, split_f2(-p.f32->dkx * dt), p.f32->vhl, p.tw32,
-                                             p.f32->dpart);
+  k_col_f32<NX, R><<<grid, C::S * C::G, C::smem, s>>>(g, p.nv, ntiles, split_f2(-p.f32->dkx * dt), p.f32->vhl, p.tw32,
+                                                     p.f32->dpart);
   p.f32->npart = grid;
   return cudaGetLastError();
 }

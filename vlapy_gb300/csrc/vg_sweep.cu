@@ -90,7 +90,7 @@ constexpr int SWEEP_MAX_CLASSES = 6;  // nv in {64, ..., 2048}
 __host__ __device__ constexpr int sweep_col_radix(int nx) {
   return (nx >= 64 && nx <= 256 && ((VG_SWEEP_COL_R32_MASK >> ilog2(nx)) & 1))   ? 32
          : (nx >= 32 && nx <= 256 && ((VG_SWEEP_COL_R16_MASK >> ilog2(nx)) & 1)) ? 16
-                                                                                 : col32_radix(nx);
+                                                                                 : (nx <= 8 ? nx : 8);
 }
 __host__ __device__ constexpr int sweep_col_min_blocks(int nx) {
   return sweep_col_radix(nx) == 32   ? VG_COL_MIN_BLOCKS_R32
