@@ -21,10 +21,10 @@
 // is the reference's own operation on the reference's own operands: by
 // induction over the lanes from the first, whose start is exact, the result is
 // the serial one bit for bit.  The k-th sweep leaves at least k lanes exact,
-// so there are never more sweeps than lanes; contraction makes it two to five
+// so there are never more sweeps than lanes; contraction makes it two
 // (the pivots forget their start by a factor a c / p^2 per element, below 0.6
-// for c = nu dt vth / dv^2 up to 13).  Measured: 64 x 1024 from 1.59 to 0.09 ms,
-// 2048 x 4096 from 6.4 to 1.2 ms, against one thread per row.
+// for c = nu dt vth / dv^2 up to 13).  Measured: 64 x 1024 from 1.59 to 0.03 ms,
+// 2048 x 4096 from 6.4 to 1.07 ms, against one thread per row.
 //
 // Divisions that share a divisor (by 2 dv, by a pivot) go through its
 // correctly rounded reciprocal y and remainder term yl: q = n y + n yl is
@@ -33,7 +33,16 @@
 // System/6000 processor, IBM J. Res. Dev. 34, 1990): four FP64 instructions
 // instead of about eight.  Operands near the ends of the exponent range take
 // the IEEE division itself.
+//
+// The guesses.  What a guess is off by costs sweeps: the values forget it by a factor
+// m = a / p an element, 0.58 at c = 3, so from three digits a double takes 55 elements
+// to come out the same, seven chunks of eight.  So each lane first runs the recurrence
+// over the elements before its chunk (K of them, WARM_BITS / -log2 m) in double-float:
+// that is some 90 cycles an element on the FP32 and integer pipes, where the FP64
+// sweep takes 130 to 600, and leaves about nine elements to sweep again: two sweeps
+// instead of two to eight, 2048 x 4096 from 1.31 to 1.07 ms, 64 x 1024 from 45 to 33 us.
 #include "vg_internal.cuh"
+#include "vg_f32.cuh"
 #include "vg_f64_body.cuh"
 
 namespace vg {
@@ -71,6 +80,38 @@ __device__ __forceinline__ bool same_bits(double a, double b) {
   return __double_as_longlong(a) == __double_as_longlong(b);
 }
 
+// The double v 2^k as double-float, by integer arithmetic (conversions between the
+// two run on the FP64 pipe); 0 outside FP32's range, and for infinities and NaN.
+__device__ __forceinline__ df32 df_of(double v, int k) {
+  const int h = __double2hiint(v);
+  const unsigned l = (unsigned)__double2loint(v);
+  const int e = ((h >> 20) & 0x7ff) + k - 896;
+  const bool ok = (unsigned)(e - 53) < 202u;  // (lo's exponent is 52 below)
+  const unsigned sign = (unsigned)h & 0x80000000u;
+  const float hi = __uint_as_float(sign | (unsigned)e << 23 | (__funnelshift_l(l, (unsigned)h, 3) & 0x7fffffu));
+  const float lo = __uint2float_rn(l & 0x1fffffffu) * __uint_as_float(sign | (unsigned)(e - 52) << 23);
+  return {ok ? hi : 0.f, ok ? lo : 0.f};
+}
+// and back: a 2^-k, or `other` where that is not an ordinary number
+__device__ __forceinline__ double df_back(df32 a, int k, double other) {
+  const double d = __dadd_rn((double)a.hi, (double)a.lo);
+  const int e = (__double2hiint(d) >> 20) & 0x7ff;
+  if (!(fabsf(a.hi) > 0.f && fabsf(a.hi) <= 3e38f) || e - k < 1 || e - k > 2046) return other;
+  return __hiloint2double(__double2hiint(d) - (k << 20), __double2loint(d));
+}
+__device__ __forceinline__ df32 df_neg(df32 a) { return {-a.hi, -a.lo}; }
+// a / b, |error| some 2^-45
+__device__ __forceinline__ df32 df_div(df32 a, df32 b) {
+  const float r = __frcp_rn(b.hi);
+  const float q = a.hi * r;
+  const float rem = fmaf(-q, b.hi, a.hi) + fmaf(-q, b.lo, a.lo);
+  const float q1 = rem * r;
+  const float hi = q + q1;
+  return {hi, q1 - (hi - q)};
+}
+constexpr float WARM_BITS = 36.f;  // a 2^-44 or so from a guess good to two digits (28, 34, 40: within 1 %)
+constexpr int WARM_MAX = 96;
+
 }  // namespace
 
 struct ThomasArgs {
@@ -101,7 +142,8 @@ __global__ void k_thomas_serial(ThomasArgs a) {
 // arrays indexed [i][lane] (element i of the lane's chunk: consecutive lanes,
 // consecutive words; the row stride S is odd, so the copy out, which walks i
 // first, is free of bank conflicts too): a (then the solution x), c, the
-// pivots p, m (then the pivots' reciprocals), d.  GLOBAL_AC: a and c in the
+// pivots p, m (then the pivots' reciprocals), d (at
+// first f).  GLOBAL_AC: a and c in the
 // scratch instead of shared memory (rows of more than 4096).
 template <int L, bool WIDE, bool GLOBAL_AC>
 __global__ void __launch_bounds__(WIDE ? 512 : 32) k_thomas_chunks(ThomasArgs g, int T) {
@@ -156,7 +198,30 @@ __global__ void __launch_bounds__(WIDE ? 512 : 32) k_thomas_chunks(ThomasArgs g,
   const double b = add_rn(1.0, mul_rn(nudt, __ddiv_rn(mul_rn(2.0, vth), g.dv_sq)));
   // drift(j) = ((v_j - vbar) 0.5) / dv = (v_j - vbar) / (2 dv): the factor 2 is exact
   const Recip two_dv = recip_of(2.0 * g.dv);
-  auto drift = [&](int j) { return div_recip(g.dougherty ? sub_rn(g.v[j], vbar) : g.v[j], two_dv); };
+  // element j's place in an array of row stride st
+  auto at = [&](int j, int st) { return (int)((unsigned)j % L) * st + (lane - t) + (int)((unsigned)j / L); };
+  // v waits in the pivots' place and f in the forward values' (a lane's walk along its
+  // chunk in global memory touches 32 lines a load)
+  if constexpr (WIDE) {
+    for (int j = lane; j < N; j += T) {
+      sp[at(j, S)] = g.v[j];
+      sd[at(j, S)] = fr[j];
+    }
+  } else {
+    for (int r = 0; r < rows_per; ++r) {
+      const int rr = min(blockIdx.x * rows_per + r, g.nrows - 1);
+      for (int j = lane; j < N; j += 32) {
+        const int q = (int)((unsigned)j % L) * S + r * T + (int)((unsigned)j / L);
+        sp[q] = g.v[j];
+        sd[q] = g.f[(size_t)rr * N + j];
+      }
+    }
+  }
+  sync();
+  auto drift = [&](int j) {
+    const double vj = sp[at(j, S)];
+    return div_recip(g.dougherty ? sub_rn(vj, vbar) : vj, two_dv);
+  };
 
   // the diagonals: a[j] of row j + 1, c[j] of row j (a is stored at j + 1's place)
   double c_in = 0.0;  // c[j0 - 1]
@@ -174,13 +239,42 @@ __global__ void __launch_bounds__(WIDE ? 512 : 32) k_thomas_chunks(ThomasArgs g,
   }
   sync();
 
-  // ---- pivots: p_0 = b, m_j = a[j-1] / p_{j-1}, p_j = b - m_j c[j-1] ----------
-  double in;
+  // elements of the warm-ups
+  int K;
   {
-    // the map's fixed point with this chunk's coefficients, in FP32
-    const float af = n > 0 ? (float)sa[lane] : 0.f, cf = (float)c_in, bf = (float)b;
-    in = (double)(0.5f * (bf + sqrtf(fmaxf(bf * bf - 4.f * af * cf, 0.f))));
+    const float c = (float)nudt * (float)vth / (float)g.dv_sq, bf = 1.f + 2.f * c;
+    const float m = 2.f * c / (bf + sqrtf(fmaxf(bf * bf - 4.f * c * c, 0.f)));
+    K = (int)fminf(WARM_BITS / fmaxf(-__log2f(m), 0.1f), (float)WARM_MAX) + 2;
   }
+
+  // ---- pivots: p_0 = b, m_j = a[j-1] / p_{j-1}, p_j = b - m_j c[j-1] ----------
+  double in = b;
+  if (n > 0 && t > 0) {
+    // the map's fixed point with the coefficients there, in FP32; then the map (the
+    // pivots forget twice as fast as the values)
+    const int js = max(j0 - 1 - (K + 1) / 2, 0);
+    const df32 bd = df_of(b, 0);
+    df32 P = bd;
+    if (js > 0) {
+      const float ac = df_of(sa[at(js, SG)], 0).hi * df_of(sc[at(js - 1, SG)], 0).hi;
+      P = {0.5f * (bd.hi + sqrtf(fmaxf(bd.hi * bd.hi - 4.f * ac, 0.f))), 0.f};
+    }
+    // (in batches: the conversions of four elements, which do not wait for one
+    // another, then the chain)
+    for (int j = js + 1; j < j0; j += 4) {
+      df32 ac[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int q = min(j + u, j0 - 1);
+        ac[u] = df_mul(df_of(sa[at(q, SG)], 0), df_of(sc[at(q - 1, SG)], 0));
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (j + u < j0) P = df_add(bd, df_neg(df_div(ac[u], P)));
+    }
+    in = df_back(P, 0, b);
+  }
+  sync();  // (the pivots go where v waits)
   double out = in;
   bool act = n > 0, first = true;
   for (int sweep = 0; sweep <= T; ++sweep) {
@@ -216,8 +310,29 @@ __global__ void __launch_bounds__(WIDE ? 512 : 32) k_thomas_chunks(ThomasArgs g,
   }
 
   // ---- forward values: d_0 = f_0, d_j = f_j - m_j d_{j-1} ----------------------
+  sync();
   in = 0.0;
-  if (n > 0 && t > 0) in = (double)((float)fr[j0 - 1] / (1.f + (float)smm[lane]));
+  int sh = 0;  // the warm-ups' scale: f is about 1 there
+  if (n > 0) sh = 1023 - ((__double2hiint(sd[at(j0, S)]) >> 20) & 0x7ff);
+  if (n > 0 && t > 0) {
+    const int js = max(j0 - 1 - K, 0);
+    df32 D = df_of(sd[at(js, S)], sh);
+    if (js > 0) D = {__fdividef(D.hi, 1.f + df_of(smm[at(js, S)], 0).hi), 0.f};
+    for (int j = js + 1; j < j0; j += 4) {
+      df32 f4[4], m4[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int q = min(j + u, j0 - 1);
+        f4[u] = df_of(sd[at(q, S)], sh);
+        m4[u] = df_neg(df_of(smm[at(q, S)], 0));
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (j + u < j0) D = df_add(f4[u], df_mul(m4[u], D));
+    }
+    in = df_back(D, sh, sd[at(j0 - 1, S)]);
+  }
+  sync();  // (the forward values go where f waits)
   out = in;
   act = n > 0;
   first = true;
@@ -228,11 +343,11 @@ __global__ void __launch_bounds__(WIDE ? 512 : 32) k_thomas_chunks(ThomasArgs g,
       if (t == 0) {
         dp = fr[0];
         sd[lane] = dp;
-        i = 1;
+        i = 1;  // (sd holds f_j the first time, the last sweep's d_j afterwards)
       }
       bool merged = false;
       for (; i < n; ++i) {
-        dp = sub_rn(fr[j0 + i], mul_rn(smm[i * S + lane], dp));
+        dp = sub_rn(first ? sd[i * S + lane] : fr[j0 + i], mul_rn(smm[i * S + lane], dp));
         if (!first && same_bits(dp, sd[i * S + lane])) {
           merged = true;
           break;
@@ -250,7 +365,27 @@ __global__ void __launch_bounds__(WIDE ? 512 : 32) k_thomas_chunks(ThomasArgs g,
 
   // ---- back substitution: x_{N-1} = d / p, x_j = (d_j - c_j x_{j+1}) / p_j -----
   for (int i = 0; i < n; ++i) smm[i * S + lane] = __drcp_rn(sp[i * S + lane]);
-  in = j1 < N && n > 0 ? fr[j1] : 0.0;  // the step moves f little: its old value next door
+  sync();
+  in = 0.0;
+  if (n > 0 && j1 < N) {
+    // from the old value there: the step moves f little
+    const int js = min(j1 + K, N - 1);
+    df32 X = js == N - 1 ? df_mul(df_of(sd[at(js, S)], sh), df_of(smm[at(js, S)], 0)) : df_of(fr[js], sh);
+    for (int j = js - 1; j >= j1; j -= 4) {
+      df32 d4[4], c4[4], y4[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int q = max(j - u, j1);
+        d4[u] = df_of(sd[at(q, S)], sh);
+        c4[u] = df_neg(df_of(sc[at(q, SG)], 0));
+        y4[u] = df_of(smm[at(q, S)], 0);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (j - u >= j1) X = df_mul(df_add(d4[u], df_mul(c4[u], X)), y4[u]);
+    }
+    in = df_back(X, sh, fr[j1]);
+  }
   out = in;
   act = n > 0;
   first = true;
