@@ -155,8 +155,39 @@ struct DevArena {
   std::vector<void*> blocks;
   char* cur = nullptr;
   size_t left = 0;
+  // what is copied in waits in `stage` and goes in one copy: every copy from
+  // pageable memory is a wait of some 6 us (plans hold ten to twenty of them)
+  static constexpr size_t STAGE = (size_t)256 << 10;
+  std::vector<char> stage;
+  char* stage_dst = nullptr;
   ~DevArena() {
     for (void* b : blocks) cudaFree(b);
+  }
+  cudaError_t flush() {
+    if (stage.empty()) return cudaSuccess;
+    const cudaError_t err = cudaMemcpy(stage_dst, stage.data(), stage.size(), cudaMemcpyHostToDevice);
+    stage.clear();
+    stage_dst = nullptr;
+    return err;
+  }
+  // a copy of src, there after the next flush (at once where it is long)
+  void* take_copy(const void* src, size_t bytes, cudaError_t* err) {
+    const size_t room = (bytes + ALIGN - 1) / ALIGN * ALIGN;
+    if (room > STAGE / 2) {
+      void* p = take(bytes, true, err);
+      if (p) *err = cudaMemcpy(p, src, bytes, cudaMemcpyHostToDevice);
+      return p;
+    }
+    if (stage_dst && stage.size() + room > STAGE) *err = flush();  // (the next copies take a new stage)
+    if (*err == cudaSuccess && !stage_dst) {
+      stage_dst = static_cast<char*>(take(STAGE, true, err));
+      stage.reserve(STAGE);
+    }
+    if (*err != cudaSuccess) return nullptr;
+    void* p = stage_dst + stage.size();
+    stage.insert(stage.end(), static_cast<const char*>(src), static_cast<const char*>(src) + bytes);
+    stage.resize((stage.size() + ALIGN - 1) / ALIGN * ALIGN);
+    return p;
   }
   // bytes (zeroed unless scratch), or null with the error in *err
   void* take(size_t bytes, bool scratch, cudaError_t* err) {
@@ -185,16 +216,16 @@ struct DevArena {
   }
 };
 
-// n elements of the plan's memory, copied from src, or zero where src is null
+// n elements of the plan's memory, copied from src (with the arena's next flush),
+// or zero where src is null
 // (left as they are when scratch)
 template <typename T>
 int dev_copy(vg_plan* p, T** dst, const T* src, size_t n, const char* what, bool scratch = false) {
   *dst = nullptr;
   if (n == 0) return VG_OK;
   cudaError_t err = cudaSuccess;
-  *dst = static_cast<T*>(static_cast<DevArena*>(p->arena)->take(n * sizeof(T), scratch || src, &err));
-  if (err != cudaSuccess) return cuda_status(err, what);
-  if (src) err = cudaMemcpy(*dst, src, n * sizeof(T), cudaMemcpyHostToDevice);
+  DevArena* a = static_cast<DevArena*>(p->arena);
+  *dst = static_cast<T*>(src ? a->take_copy(src, n * sizeof(T), &err) : a->take(n * sizeof(T), scratch, &err));
   return cuda_status(err, what);
 }
 
@@ -676,11 +707,13 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
   if (d->nx <= POISSON_FX_NX && d->precision == VG_F64) {
     TRY(dev_copy<int2>(p, &p->green, nullptr, nx, "Green's function"));
     TRY(dev_copy<int>(p, &p->green_e, nullptr, 1, "Green's function"));
+    TRY(cuda_status(static_cast<DevArena*>(p->arena)->flush(), "plan setup"));
     TRY(cuda_status(build_poisson_fx(p->inv_kx, d->nx, 1, p->green, p->green_e, p->etmp, 0), "Green's function"));
   }
   if (d->precision == VG_F64 && d->collision != VG_COLL_NONE)
     TRY(dev_copy<double>(p, &p->bb, nullptr, 2 * nx * thomas_pad(d->nv), "thomas scratch", true));
   if (d->precision == VG_F32_DELTA_F) TRY(setup_f32(p, d));
+  TRY(cuda_status(static_cast<DevArena*>(p->arena)->flush(), "plan setup"));
   TRY(cuda_status(launch_twiddles(*p, 0), "twiddles"));
   TRY(cuda_status(cudaDeviceSynchronize(), "plan setup"));
   p->graph_cache = new GraphCache();
