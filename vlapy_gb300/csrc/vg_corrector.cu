@@ -207,6 +207,35 @@ __global__ void __launch_bounds__(CORR_THREADS) k_conv(const __nv_bfloat16* __re
   }
 }
 
+// Bias gradients of a row of dy by 128 threads, in the order both engines share:
+// piece q = i 128 + p of thread p is 16 bytes (8 channels) of position q / (COUTP / 8),
+// so a thread's pieces are the same channels of every G-th position, which it adds up
+// over i and the rows; bias_total adds the G threads' sums of a channel in order.
+// (One thread a channel walking the 128 positions took 2900 cycles a row, a third of
+// k_wgrad_tc's time.)
+__device__ __forceinline__ void bias_add(const uint4& v, float (&sum)[8]) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    sum[2 * u] += __uint_as_float(w[u] << 16);  // bf16 is the upper half of an FP32
+    sum[2 * u + 1] += __uint_as_float(w[u] & 0xffff0000u);
+  }
+}
+// scratch: CP / (COUTP / 8) x COUTP floats that nothing else uses; all threads call it
+template <int COUTP>
+__device__ __forceinline__ void bias_total(const float (&sum)[8], float* scratch, float* __restrict__ out) {
+  constexpr int PIECES = COUTP / 8, G = 128 / PIECES;
+  const int g = threadIdx.x / PIECES, j = threadIdx.x % PIECES;
+#pragma unroll
+  for (int u = 0; u < 8; ++u) scratch[g * COUTP + 8 * j + u] = sum[u];
+  __syncthreads();
+  if (threadIdx.x < COUTP) {
+    float t = 0.f;
+    for (int q = 0; q < G; ++q) t += scratch[q * COUTP + threadIdx.x];
+    out[threadIdx.x] = t;
+  }
+}
+
 // Weight gradients of one tap t (grid.y) over a chunk of rows (grid.x):
 // part[chunk][t][o][c] = sum_rows sum_p dy[row][p][o] * x[row][p + t - 2][c].
 // dy has COUTP >= 16 channels (zero beyond the layer's real outputs).  The
@@ -234,18 +263,19 @@ __global__ void __launch_bounds__(CORR_THREADS) k_wgrad(const __nv_bfloat16* __r
   zero_rows<CIN>(xt, CHALO + CP, CHALO);
   const int r_begin = blockIdx.x * rows_per_chunk;
   const int r_end = min(rows, r_begin + rows_per_chunk);
-  const bool bias_sum = (t == 2) && (int)threadIdx.x < COUTP;
-  float bsum = 0.f;
+  const bool bias_sum = t == 2;
+  float bsum[8] = {};
   for (int row = r_begin; row < r_end; ++row) {
     __syncthreads();
     load_tile<COUTP>(yt, 0, dy + (size_t)row * CP * COUTP, CP);
     load_tile<CIN>(xt, CHALO, x + (size_t)row * CP * CIN, CP);
     __syncthreads();
     if (bias_sum) {
-      float rs = 0.f;
-      for (int p = 0; p < CP; ++p)
-        rs += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(yt + swz<COUTP>(p, threadIdx.x)));
-      bsum += rs;
+#pragma unroll
+      for (int i = 0; i < COUTP / 8; ++i) {
+        const int q = i * CORR_THREADS + threadIdx.x;
+        bias_add(*reinterpret_cast<const uint4*>(yt + swz<COUTP>(q / (COUTP / 8), 8 * (q % (COUTP / 8)))), bsum);
+      }
     }
     if (active) {
 #pragma unroll 2
@@ -271,7 +301,10 @@ __global__ void __launch_bounds__(CORR_THREADS) k_wgrad(const __nv_bfloat16* __r
       }
     }
   }
-  if (bias_sum) bpart[(size_t)blockIdx.x * COUTP + threadIdx.x] = bsum;
+  if (bias_sum) {
+    __syncthreads();  // (every thread is done with the tiles)
+    bias_total<COUTP>(bsum, reinterpret_cast<float*>(smem), bpart + (size_t)blockIdx.x * COUTP);
+  }
   if (active) {
     float* dst = part + ((size_t)blockIdx.x * 5 + t) * COUTP * CIN;
 #pragma unroll
@@ -287,21 +320,42 @@ __global__ void __launch_bounds__(CORR_THREADS) k_wgrad(const __nv_bfloat16* __r
 
 // dW[o][c][t] (PyTorch order, FP32) and db[o]: sums over the chunks in a
 // fixed order (deterministic)
-__global__ void k_wgrad_reduce(const float* __restrict__ part, const float* __restrict__ bpart, int nchunks,
-                               int coutp, int cin, int cout, float* __restrict__ dw, float* __restrict__ db) {
+// A CTA's WRED_SPLIT warps each add a share of the chunks of 32 consecutive entries,
+// eight loads in flight, and the shares are added in order.  (One thread an entry, one
+// load after another: 148 us for 64 x 64 x 5 over 296 chunks, now 8.)
+constexpr int WRED_SPLIT = 8;
+__global__ void __launch_bounds__(32 * WRED_SPLIT) k_wgrad_reduce(const float* __restrict__ part,
+                                                                  const float* __restrict__ bpart, int nchunks, int coutp,
+                                                                  int cin, int cout, float* __restrict__ dw,
+                                                                  float* __restrict__ db) {
+  __shared__ float share[WRED_SPLIT][32];
   const int n = cout * cin * 5;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n + cout; q += gridDim.x * blockDim.x) {
-    float s = 0.f;
-    if (q < n) {
-      const int t = q % 5, c = (q / 5) % cin, o = q / (5 * cin);
-      for (int k = 0; k < nchunks; ++k) s += part[(((size_t)k * 5 + t) * coutp + o) * cin + c];
-      dw[q] = s;
-    } else {
-      const int o = q - n;
-      for (int k = 0; k < nchunks; ++k) s += bpart[(size_t)k * coutp + o];
-      db[o] = s;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int q = blockIdx.x * 32 + lane;  // (tap, output, input channel), then the biases
+  const int c = q % cin, o = (q / cin) % cout, t = q / (cin * cout);
+  const float* src = q < n ? part + ((size_t)t * coutp + o) * cin + c : bpart + (q - n);
+  const size_t step = q < n ? (size_t)5 * coutp * cin : (size_t)coutp;
+  const int per = (nchunks + WRED_SPLIT - 1) / WRED_SPLIT;
+  int k = min(nchunks, w * per);
+  const int k1 = min(nchunks, k + per);
+  float s = 0.f;
+  if (q < n + cout) {
+    for (; k + 8 <= k1; k += 8) {
+      float x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) x[u] = src[(size_t)(k + u) * step];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s += x[u];
     }
+    for (; k < k1; ++k) s += src[(size_t)k * step];
   }
+  share[w][lane] = s;
+  __syncthreads();
+  if (w != 0 || q >= n + cout) return;
+#pragma unroll
+  for (int u = 1; u < WRED_SPLIT; ++u) s += share[u][lane];
+  if (q < n) dw[(o * cin + c) * 5 + t] = s;
+  else db[q - n] = s;
 }
 
 // mean over each group of `group_rows` consecutive rows (the x-mean of a
@@ -345,6 +399,11 @@ __device__ __forceinline__ float with_mean(float dn, const float2* __restrict__ 
   return __fadd_rn(m.x, __fadd_rn(m.y, dn));
 }
 
+__device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
+  const __nv_bfloat162 pr = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&pr);
+}
+
 // features [row][p][16]: d / s, v / vmax, the row's scalar feature (the
 // collision-rate channel), d_prev / s, zeros; d = g minus its group mean
 // (or g itself without groups), d_prev the same of the row before the
@@ -361,117 +420,124 @@ __global__ void k_features(const float* __restrict__ g, const float2* __restrict
   const float prev = gp ? deviation(gp[q], pmean, group_rows, row, p) : 0.f;
   red[p] = val * val;
   __syncthreads();
-  for (int m = CP / 2; m > 0; m >>= 1) {
-    if (p < m) red[p] += red[p + m];
-    __syncthreads();
+  // the tree of partners 64, 32, ..., 1, by the first warp
+  if (p < 32) {
+    float t = (red[p] + red[p + 64]) + (red[p + 32] + red[p + 96]);
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) t += __shfl_down_sync(0xffffffffu, t, m);
+    if (p == 0) red[0] = t;
   }
+  __syncthreads();
   const float s = sqrtf(red[0] / CP) + 1e-30f;
   if (p == 0) scale[row] = s;
   const float dv = 2.f * vmax / CP;
   const float v = __fadd_rn(-vmax, __fmul_rn(dv, (float)p + 0.5f));
-  __nv_bfloat16* dst = x0 + q * L1_IN;
-  dst[0] = __float2bfloat16(val / s);
-  dst[1] = __float2bfloat16(v / vmax);
-  dst[2] = __float2bfloat16(row_feat ? row_feat[row] : 0.f);
-  dst[3] = __float2bfloat16(prev / s);
-#pragma unroll
-  for (int c = 4; c < L1_IN; ++c) dst[c] = __float2bfloat16(0.f);
-}
-
-// Orthogonal projection of one row (one value per thread, blockDim = CP)
-// onto the complement of the v-Fourier modes |m| < M of the 128-point row:
-// v - sum_q <v, b_q> b_q over the orthonormal basis b_q (1, cos, sin of
-// 2 pi m j / 128 for 0 < m < M).  basis [nq][CP], basis_t [CP][nq_pad].
-// All threads of the CTA must call it; sh and coef are [CP] shared arrays.
-__device__ __forceinline__ float high_pass(float v, const float* __restrict__ basis,
-                                           const float* __restrict__ basis_t, int nq, float* sh, float* coef) {
-  const int p = threadIdx.x;
-  if (nq == 0) return v;
-  sh[p] = v;
-  __syncthreads();
-  if (p < nq) {
-    float a = 0.f;
-    for (int j = 0; j < CP; ++j) a = fmaf(sh[j], basis_t[j * CP + p], a);
-    coef[p] = a;
-  }
-  __syncthreads();
-  float r = v;
-  for (int q = 0; q < nq; ++q) r = fmaf(-coef[q], basis[q * CP + p], r);
-  __syncthreads();
-  return r;
-}
-
-// high_pass for two rows' values at once (one pass over the basis)
-__device__ __forceinline__ void high_pass2(float a, float b, const float* __restrict__ basis,
-                                           const float* __restrict__ basis_t, int nq, float* sh, float* coef,
-                                           float& ha, float& hb) {
-  const int p = threadIdx.x;
-  if (nq == 0) {
-    ha = a;
-    hb = b;
-    return;
-  }
-  sh[p] = a;
-  sh[CP + p] = b;
-  __syncthreads();
-  if (p < nq) {
-    float ca0 = 0.f, ca1 = 0.f, cb0 = 0.f, cb1 = 0.f;
-#pragma unroll 8
-    for (int j = 0; j < CP; j += 2) {
-      const float w0 = basis_t[j * CP + p], w1 = basis_t[(j + 1) * CP + p];
-      ca0 = fmaf(sh[j], w0, ca0);
-      cb0 = fmaf(sh[CP + j], w0, cb0);
-      ca1 = fmaf(sh[j + 1], w1, ca1);
-      cb1 = fmaf(sh[CP + j + 1], w1, cb1);
-    }
-    coef[p] = ca0 + ca1;
-    coef[CP + p] = cb0 + cb1;
-  }
-  __syncthreads();
-  float ra = a, rb = b;
-#pragma unroll 4
-  for (int q = 0; q < nq; ++q) {
-    const float w = basis[q * CP + p];
-    ra = fmaf(-coef[q], w, ra);
-    rb = fmaf(-coef[CP + q], w, rb);
-  }
-  __syncthreads();
-  ha = ra;
-  hb = rb;
+  // a position's 32 bytes in two stores (sixteen of two bytes took 88 us for 8192
+  // rows, now 14)
+  uint4* dst = reinterpret_cast<uint4*>(x0 + q * L1_IN);
+  dst[0] = make_uint4(bf16_pair(val / s, v / vmax), bf16_pair(row_feat ? row_feat[row] : 0.f, prev / s), 0u, 0u);
+  dst[1] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 // loss = mean((P (pred - want))^2) over rows x positions, P the projection
 // onto the corrected modes (|m| >= M) and want = ((target - tmean) - (g -
 // gmean)) / (s tau) the correction in units of the row RMS s times a global
 // scale tau (means only with groups); dy4 channel 0 = d loss / d pred =
-// 2 P (pred - want) / n.  One row at a time per CTA, blockDim = CP.
-__global__ void k_loss(const float* __restrict__ pred, const float* __restrict__ g, const float* __restrict__ target,
-                       const float2* __restrict__ gmean, const float2* __restrict__ tmean, int group_rows,
-                       const float* __restrict__ scale, float tau, const float* __restrict__ basis,
-                       const float* __restrict__ basis_t, int nq, int rows, __nv_bfloat16* __restrict__ dy4,
-                       float* __restrict__ loss_part) {
-  __shared__ float sh[CP], coef[CP];
+// 2 P (pred - want) / n.  P removes the v-Fourier modes |m| < M of the 128-point row:
+// v - sum_q <v, b_q> b_q over the orthonormal basis b_q (1, cos, sin of 2 pi m j / 128
+// for 0 < m < M); basis [nq][CP], basis_t [CP][nq padded].  blockDim = CP, LOSS_ROWS rows at a time per CTA: the
+// projections' coefficients are (basis function, row) pairs spread over all threads,
+// and a basis value serves all the rows.  (A row at a time, nq threads on its
+// coefficients, and a position's 32 bytes in sixteen stores: 146 us for 8192 rows,
+// now 50.)
+constexpr int LOSS_ROWS = 8;
+__global__ void __launch_bounds__(CP) k_loss(const float* __restrict__ pred, const float* __restrict__ g,
+                                             const float* __restrict__ target, const float2* __restrict__ gmean,
+                                             const float2* __restrict__ tmean, int group_rows,
+                                             const float* __restrict__ scale, float tau, const float* __restrict__ basis,
+                                             const float* __restrict__ basis_t, int nq, int rows,
+                                             __nv_bfloat16* __restrict__ dy4, float* __restrict__ loss_part) {
+  static_assert(LOSS_ROWS == 8, "two quads of rows");
+  __shared__ float4 sh[CP][2], coef[CP][2];  // [position or basis function][quad of rows]
+  __shared__ float red[CP];
   const int p = threadIdx.x;
   const float inv_n = 1.f / ((float)rows * CP);
   float acc = 0.f;
-  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    const size_t q = (size_t)row * CP + p;
-    const float diff = deviation(target[q], tmean, group_rows, row, p) - deviation(g[q], gmean, group_rows, row, p);
-    const float want = diff / (scale[row] * tau);
-    const float d = high_pass(pred[q] - want, basis, basis_t, nq, sh, coef);
-    acc += d * d;
-    __nv_bfloat16* dst = dy4 + q * 16;
-    dst[0] = __float2bfloat16(2.f * d * inv_n);
+  for (int row0 = blockIdx.x; row0 < rows; row0 += LOSS_ROWS * gridDim.x) {
+    float d[LOSS_ROWS];
 #pragma unroll
-    for (int c = 1; c < 16; ++c) dst[c] = __float2bfloat16(0.f);
+    for (int u = 0; u < LOSS_ROWS; ++u) {
+      const int row = row0 + u * gridDim.x;
+      d[u] = 0.f;
+      if (row < rows) {
+        const size_t q = (size_t)row * CP + p;
+        const float diff =
+            deviation(target[q], tmean, group_rows, row, p) - deviation(g[q], gmean, group_rows, row, p);
+        d[u] = pred[q] - diff / (scale[row] * tau);
+      }
+    }
+    if (nq > 0) {
+      sh[p][0] = make_float4(d[0], d[1], d[2], d[3]);
+      sh[p][1] = make_float4(d[4], d[5], d[6], d[7]);
+      __syncthreads();
+      // thread (q, quad): the coefficients of q for four rows
+      const int quad = p >> 6;
+      for (int q = p & 63; q < nq; q += 64) {
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int j0 = 0; j0 < CP; j0 += 16) {
+          float w[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) w[j] = basis_t[(j0 + j) * CP + q];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const float4 x = sh[j0 + j][quad];
+            a.x = fmaf(x.x, w[j], a.x);
+            a.y = fmaf(x.y, w[j], a.y);
+            a.z = fmaf(x.z, w[j], a.z);
+            a.w = fmaf(x.w, w[j], a.w);
+          }
+        }
+        coef[q][quad] = a;
+      }
+      __syncthreads();
+      for (int q0 = 0; q0 < nq; q0 += 16) {
+        float w[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) w[j] = q0 + j < nq ? basis[(q0 + j) * CP + p] : 0.f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          if (q0 + j >= nq) break;
+          const float4 a = coef[q0 + j][0], b = coef[q0 + j][1];
+          d[0] = fmaf(-a.x, w[j], d[0]);
+          d[1] = fmaf(-a.y, w[j], d[1]);
+          d[2] = fmaf(-a.z, w[j], d[2]);
+          d[3] = fmaf(-a.w, w[j], d[3]);
+          d[4] = fmaf(-b.x, w[j], d[4]);
+          d[5] = fmaf(-b.y, w[j], d[5]);
+          d[6] = fmaf(-b.z, w[j], d[6]);
+          d[7] = fmaf(-b.w, w[j], d[7]);
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < LOSS_ROWS; ++u) {
+      const int row = row0 + u * gridDim.x;
+      if (row >= rows) break;
+      acc += d[u] * d[u];
+      uint4* dst = reinterpret_cast<uint4*>(dy4 + ((size_t)row * CP + p) * 16);
+      dst[0] = make_uint4(bf16_pair(2.f * d[u] * inv_n, 0.f), 0u, 0u, 0u);
+      dst[1] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    // (a thread reaches the next rows' first barrier only after every thread has read
+    // these coefficients' values; the coefficients are written after that barrier)
   }
-  sh[p] = acc;
+  red[p] = acc;
   __syncthreads();
   for (int m = CP / 2; m > 0; m >>= 1) {
-    if (p < m) sh[p] += sh[p + m];
+    if (p < m) red[p] += red[p + m];
     __syncthreads();
   }
-  if (p == 0) loss_part[blockIdx.x] = sh[0];
+  if (p == 0) loss_part[blockIdx.x] = red[0];
 }
 
 // g_out = m + P'd + (Pd + c) * min(1, |Pd| / |Pd + c|) per row, with m the
@@ -1108,6 +1174,18 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
+// the 32 bytes at a 32-byte aligned address
+__device__ __forceinline__ void load_sector(const void* src, uint32_t (&r)[8]) {
+  asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "l"(src));
+}
+__device__ __forceinline__ void store_sector(void* dst, const uint32_t (&r)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(dst), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+
 __host__ __device__ constexpr int tmem_cols_for(int n) { return n <= 32 ? 32 : (n <= 64 ? 64 : (n <= 128 ? 128 : (n <= 256 ? 256 : 512))); }
 
 template <int CIN, int COUT>
@@ -1148,6 +1226,8 @@ __global__ void __launch_bounds__(TRN_THREADS, 1)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar0 + 8 * q) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
+  __shared__ __align__(16) float sbias[COUT];
+  if (MODE != 2 && threadIdx.x < (MODE == 1 ? 1 : COUT)) sbias[threadIdx.x] = bias[threadIdx.x];
   // weights: tap t, output row n, input chunk j -> t WTAP + tc_off(n, 8 j, 16 COUT)
   for (int i = threadIdx.x; i < 5 * COUT * (CIN / 8); i += TRN_THREADS) {
     const int j = i % (CIN / 8), n = (i / (CIN / 8)) % COUT, t = i / ((CIN / 8) * COUT);
@@ -1175,12 +1255,17 @@ __global__ void __launch_bounds__(TRN_THREADS, 1)
   uint32_t phase = 0;
   int commits = 0;
   bool ok = true;
-  // this thread's position of a row into row p + 2 of tile b, asynchronously
+  // a row into tile b (position n to its row n + 2), asynchronously.  The slot's
+  // threads take consecutive 16 bytes: a warp's request is four whole lines (with a
+  // position a thread it was a piece of 32).
   auto fetch = [&](int row, int b) {
-    const uint4* src = reinterpret_cast<const uint4*>(x + ((size_t)row * CP + p) * CIN);
+    const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)row * CP * CIN) + p;
     unsigned char* tile = smem + W_BYTES + (2 * slot + b) * TILE;
 #pragma unroll
-    for (int j = 0; j < CIN / 8; ++j) cp_async16(tile + tc_off(p + CHALO, 8 * j, TC_LBO_ACT), src + j);
+    for (int i = 0; i < CIN / 8; ++i) {
+      const int q = i * 128 + p;
+      cp_async16(tile + tc_off(q / (CIN / 8) + CHALO, 8 * (q % (CIN / 8)), TC_LBO_ACT), src + i * 128);
+    }
     cp_async_commit();
   };
   const int stride = gridDim.x * TRN_SLOTS;
@@ -1199,7 +1284,8 @@ __global__ void __launch_bounds__(TRN_THREADS, 1)
     }
     ++commits;
     // the next row into the other tile (its last reader, the previous row's
-    // MMAs, completed before that row's epilogue)
+    // MMAs, completed before that row's epilogue).  Two rows ahead, after these MMAs,
+    // was slower: 83 -> 84 us for 64 to 64 channels, 40 -> 58 for 64 to 1.
     if (row + stride < rows) fetch(row + stride, b ^ 1);
     const bool done = mbar_wait(bar, phase);
     phase ^= 1u;
@@ -1213,31 +1299,29 @@ __global__ void __launch_bounds__(TRN_THREADS, 1)
       float v[16];
       tc_ld16(td + lane_base + c0, v);
       if (MODE == 1) {
-        static_cast<float*>(out)[q] = v[0] + bias[0];
+        static_cast<float*>(out)[q] = v[0] + sbias[0];
       } else {
+        // 16 channels, a whole sector, in one load and one store
+        uint32_t wv[8], mk[8];
+        if (MODE == 2) load_sector(mask + q * COUT + c0, mk);
+        float4 b4[4];
+        if (MODE == 0)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          uint32_t wv[4];
-          uint4 mk = make_uint4(0u, 0u, 0u, 0u);
-          if (MODE == 2) mk = reinterpret_cast<const uint4*>(mask + q * COUT + c0 + 8 * h)[0];
-          const __nv_bfloat162* m2 = reinterpret_cast<const __nv_bfloat162*>(&mk);
+          for (int j = 0; j < 4; ++j) b4[j] = *reinterpret_cast<const float4*>(sbias + c0 + 4 * j);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int c = c0 + 8 * h + 2 * j;
-            float a = v[8 * h + 2 * j], b = v[8 * h + 2 * j + 1];
-            if (MODE == 0) {
-              a = fmaxf(a + bias[c], 0.f);
-              b = fmaxf(b + bias[c + 1], 0.f);
-            } else {
-              if (!(__bfloat162float(m2[j].x) > 0.f)) a = 0.f;
-              if (!(__bfloat162float(m2[j].y) > 0.f)) b = 0.f;
-            }
-            const __nv_bfloat162 pr = __floats2bfloat162_rn(a, b);
-            wv[j] = *reinterpret_cast<const uint32_t*>(&pr);
+        for (int j = 0; j < 8; ++j) {
+          float a = v[2 * j], b = v[2 * j + 1];
+          if (MODE == 0) {
+            a = fmaxf(a + (j & 1 ? b4[j >> 1].z : b4[j >> 1].x), 0.f);
+            b = fmaxf(b + (j & 1 ? b4[j >> 1].w : b4[j >> 1].y), 0.f);
+          } else {
+            const __nv_bfloat162 m2 = *reinterpret_cast<const __nv_bfloat162*>(&mk[j]);
+            if (!(__bfloat162float(m2.x) > 0.f)) a = 0.f;
+            if (!(__bfloat162float(m2.y) > 0.f)) b = 0.f;
           }
-          reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(out) + q * COUT + c0 + 8 * h)[0] =
-              make_uint4(wv[0], wv[1], wv[2], wv[3]);
+          wv[j] = bf16_pair(a, b);
         }
+        store_sector(static_cast<__nv_bfloat16*>(out) + q * COUT + c0, wv);
       }
     }
     // every thread of the slot has read its TMEM lanes before the next row's
@@ -1269,9 +1353,12 @@ struct WgradShape {
   static constexpr int R = CP + (NGROUP - 1) * NCOPY;
   static constexpr int A_BYTES = 16 * R * 16;  // 16 chunks of 8 (copy, channel) rows
 };
+// bytes between dy's groups of 8 channels: 132 positions, so that eight lanes with a
+// position's eight pieces and four positions meet every bank alike
+constexpr int WGRAD_MN_B = (CP + 4) * 16;
 template <int CIN, int COUTP>
 __host__ __device__ constexpr int trn_wgrad_stage() {
-  return WgradShape<CIN>::A_BYTES + (COUTP / 8) * CP * 16;
+  return WgradShape<CIN>::A_BYTES + (COUTP / 8) * WGRAD_MN_B;
 }
 template <int CIN, int COUTP>
 __host__ __device__ constexpr int trn_wgrad_smem() {
@@ -1290,7 +1377,7 @@ __global__ void __launch_bounds__(128, 1)
   static_assert(COUTP % 16 == 0 && COUTP <= 64, "output channels");
   constexpr int STAGE = trn_wgrad_stage<CIN, COUTP>();
   constexpr int TMEM_COLS = tmem_cols_for(S::NGROUP * COUTP);
-  constexpr uint32_t MN_A = (uint32_t)S::R * 16, MN_B = (uint32_t)CP * 16;
+  constexpr uint32_t MN_A = (uint32_t)S::R * 16, MN_B = (uint32_t)WGRAD_MN_B;
   constexpr uint32_t idesc = tc_idesc(128, COUTP) | (1u << 15) | (1u << 16);  // A and B MN-major
   extern __shared__ __align__(128) unsigned char smem[];
   const uint32_t s_base = (uint32_t)__cvta_generic_to_shared(smem);
@@ -1318,38 +1405,62 @@ __global__ void __launch_bounds__(128, 1)
   const uint32_t tmem = *tmem_slot;
   const int r_begin = blockIdx.x * rows_per_chunk;
   const int r_end = min(rows, r_begin + rows_per_chunk);
-  float bsum = 0.f;
+  float bsum[8] = {};
   uint32_t phase[2] = {0u, 0u};
   bool pending[2] = {false, false};
   bool ok = true;
   int n = 0;
-  // row `row`'s input copies and dy into stage st, asynchronously (copy c
-  // holds x[r + c - 2] at row r)
-  auto fetch = [&](int row, int st) {
-    unsigned char* A = smem + st * STAGE;
-    unsigned char* B = A + S::A_BYTES;
-    const size_t q = (size_t)row * CP + p;
-    const uint4* xs = reinterpret_cast<const uint4*>(x + q * CIN);
-    const uint4* ys = reinterpret_cast<const uint4*>(dy + q * COUTP);
+  // The next row waits in registers while this one is stored and its MMAs run:
+  // consecutive threads, consecutive 16 bytes.  (By 24 cp.async a thread, straight
+  // into the other stage, the issue alone took 4500 of 9300 cycles a row.)
+  uint4 xr[CIN / 8], yr[COUTP / 8];
+  auto load = [&](int row) {
+    const uint4* xs = reinterpret_cast<const uint4*>(x + (size_t)row * CP * CIN) + p;
+    const uint4* ys = reinterpret_cast<const uint4*>(dy + (size_t)row * CP * COUTP) + p;
 #pragma unroll
-    for (int j = 0; j < CIN / 8; ++j)
+    for (int i = 0; i < CIN / 8; ++i) xr[i] = __ldg(xs + i * 128);
 #pragma unroll
-      for (int c = 0; c < S::NCOPY; ++c) {
-        const int r = p + CHALO - c;
-        if (r >= 0 && r < S::R) cp_async16(A + (c * (CIN / 8) + j) * MN_A + r * 16, xs + j);
-      }
-#pragma unroll
-    for (int j = 0; j < COUTP / 8; ++j) cp_async16(B + j * MN_B + p * 16, ys + j);
-    cp_async_commit();
+    for (int i = 0; i < COUTP / 8; ++i) yr[i] = __ldg(ys + i * 128);
   };
-  if (r_begin < r_end) fetch(r_begin, 0);
+  if (r_begin < r_end) load(r_begin);
   for (int row = r_begin; row < r_end; ++row, ++n) {
     const int st = n & 1;
-    unsigned char* B = smem + st * STAGE + S::A_BYTES;
-    cp_async_wait_all();
+    // this stage once more, when the MMAs of the row before the last are done with it
+    bool done = true;
+    if (pending[st]) {
+      done = mbar_wait(bar0 + 8 * st, phase[st]);
+      if (done) {
+        phase[st] ^= 1u;
+        pending[st] = false;
+      }
+    }
+    if (done) {
+      unsigned char* A = smem + st * STAGE;
+      unsigned char* B = A + S::A_BYTES;
+      // copy c holds x[r + c - 2] at row r
+#pragma unroll
+      for (int i = 0; i < CIN / 8; ++i) {
+        const int q = i * 128 + p, pos = q / (CIN / 8), j = q % (CIN / 8);
+#pragma unroll
+        for (int c = 0; c < S::NCOPY; ++c) {
+          const int r = pos + CHALO - c;
+          if (r >= 0 && r < S::R) *reinterpret_cast<uint4*>(A + (c * (CIN / 8) + j) * MN_A + r * 16) = xr[i];
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < COUTP / 8; ++i) {
+        const int q = i * 128 + p, pos = q / (COUTP / 8), j = q % (COUTP / 8);
+        *reinterpret_cast<uint4*>(B + j * MN_B + pos * 16) = yr[i];
+        bias_add(yr[i], bsum);
+      }
+    }
+    if (row + 1 < r_end) load(row + 1);
     fence_async_smem();
     tc_fence_before();
-    __syncthreads();
+    if (__syncthreads_or(!done)) {
+      ok = false;
+      break;
+    }
     if (threadIdx.x == 0) {
       tc_fence_after();
       const uint32_t a_s = s_base + st * STAGE, b_s = a_s + S::A_BYTES;
@@ -1365,30 +1476,7 @@ __global__ void __launch_bounds__(128, 1)
       tc_commit(bar0 + 8 * st);
     }
     pending[st] = true;
-    // the next row into the other stage, once the MMAs that read it are done
-    if (row + 1 < r_end) {
-      const int so = st ^ 1;
-      if (pending[so]) {
-        const bool done = mbar_wait(bar0 + 8 * so, phase[so]);
-        phase[so] ^= 1u;
-        pending[so] = false;
-        if (__syncthreads_or(!done)) {
-          ok = false;
-          break;
-        }
-      }
-      fetch(row + 1, so);
-    }
-    // bias gradient: column sums of dy over the row's positions
-    if (threadIdx.x < COUTP) {
-      const int o = threadIdx.x;
-      const unsigned char* col = B + (o >> 3) * MN_B + (o & 7) * 2;
-      float rs = 0.f;
-      for (int pp = 0; pp < CP; ++pp) rs += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(col + pp * 16));
-      bsum += rs;
-    }
   }
-  cp_async_wait_all();
   // the outstanding commits of both stages
   for (int st = 0; st < 2; ++st)
     if (pending[st]) {
@@ -1414,7 +1502,8 @@ __global__ void __launch_bounds__(128, 1)
         }
       }
     }
-    if (threadIdx.x < COUTP) bpart[(size_t)blockIdx.x * COUTP + threadIdx.x] = bsum;
+    // (the stages: nothing reads them any more)
+    bias_total<COUTP>(bsum, reinterpret_cast<float*>(smem), bpart + (size_t)blockIdx.x * COUTP);
   } else if (r_end > r_begin) {
     if (threadIdx.x == 0) atomicOr(err, 1);
   } else {
@@ -1504,7 +1593,7 @@ cudaError_t wgrad(vg_corrector* c, const __nv_bfloat16* x, const __nv_bfloat16* 
   k_wgrad<CIN, COUTP><<<dim3(chunks, 5), CORR_THREADS, smem, s>>>(x, dy, rows, per, c->part, c->bpart);
   err = cudaGetLastError();
   if (err != cudaSuccess) return err;
-  k_wgrad_reduce<<<div_up(cout * CIN * 5 + cout, 256), 256, 0, s>>>(c->part, c->bpart, chunks, COUTP, CIN, cout, dw,
+  k_wgrad_reduce<<<div_up(cout * CIN * 5 + cout, 32), 32 * WRED_SPLIT, 0, s>>>(c->part, c->bpart, chunks, COUTP, CIN, cout, dw,
                                                                    db);
   return cudaGetLastError();
 }
@@ -1532,7 +1621,7 @@ cudaError_t wgrad_tc(vg_corrector* c, const __nv_bfloat16* x, const __nv_bfloat1
   k_wgrad_tc<CIN, COUTP><<<chunks, 128, smem, s>>>(x, dy, rows, per, c->part, c->bpart, c->err);
   err = cudaGetLastError();
   if (err != cudaSuccess) return err;
-  k_wgrad_reduce<<<div_up(cout * CIN * 5 + cout, 256), 256, 0, s>>>(c->part, c->bpart, chunks, COUTP, CIN, cout, dw,
+  k_wgrad_reduce<<<div_up(cout * CIN * 5 + cout, 32), 32 * WRED_SPLIT, 0, s>>>(c->part, c->bpart, chunks, COUTP, CIN, cout, dw,
                                                                    db);
   return cudaGetLastError();
 }
