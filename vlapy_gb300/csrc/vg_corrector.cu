@@ -99,6 +99,14 @@ __device__ __forceinline__ void zero_rows(unsigned char* tile, int r0, int rows)
   }
 }
 
+// The 64-channel tensors of this engine lie as [row][group of 8 channels][position]
+// [8]: a group is the 2 KB run that a tile's group is, so a row comes by eight bulk
+// copies that one thread issues, and the epilogue's store of a group is 512 contiguous
+// bytes a warp.  (With a position's channels together, every load and store of a warp
+// touched 32 lines: 97 us for 64 to 64 channels over 8192 rows and 113 for their
+// gradient, now 50 and 65.)  The 16-channel ones (features, the loss's gradient) are
+// [row][position][16], as the mma.sync engine has all of them.
+//
 // MODE 0: out = relu(conv + b) (bf16); MODE 1: out[p] = conv + b, channel 0
 // only (fp32); MODE 2: out = conv * (mask > 0) (bf16, no bias).
 // Weights W: bf16 [5][COUT][CIN] (for MODE 2: transposed, tap-flipped).
@@ -1174,27 +1182,23 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-// the 32 bytes at a 32-byte aligned address
-__device__ __forceinline__ void load_sector(const void* src, uint32_t (&r)[8]) {
-  asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "l"(src));
-}
-__device__ __forceinline__ void store_sector(void* dst, const uint32_t (&r)[8]) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(dst), "r"(r[0]), "r"(r[1]), "r"(r[2]),
-               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
-}
-
 __host__ __device__ constexpr int tmem_cols_for(int n) { return n <= 32 ? 32 : (n <= 64 ? 64 : (n <= 128 ? 128 : (n <= 256 ? 256 : 512))); }
 
 template <int CIN, int COUT>
 __host__ __device__ constexpr int trn_conv_wbytes() { return 5 * COUT * CIN * 2; }
 template <int CIN, int COUT>
 __host__ __device__ constexpr int trn_conv_smem() {
-  return trn_conv_wbytes<CIN, COUT>() + 2 * TRN_SLOTS * (CIN / 8) * TC_LBO_ACT + 8 * TRN_SLOTS + 16;
+  return trn_conv_wbytes<CIN, COUT>() + 2 * TRN_SLOTS * (CIN / 8) * TC_LBO_ACT + 24 * TRN_SLOTS + 16;
 }
 
+// The 64-channel tensors of this engine lie as [row][group of 8 channels][position]
+// [8]: a group is the 2 KB run that a tile's group is, so a row comes by eight bulk
+// copies that one thread issues, and the epilogue's store of a group is 512 contiguous
+// bytes a warp.  (With a position's channels together, every load and store of a warp
+// touched 32 lines: 97 us for 64 to 64 channels over 8192 rows and 113 for their
+// gradient, now 50 and 65.)  The 16-channel ones (features, the loss's gradient) are
+// [row][position][16], as the mma.sync engine has all of them.
+//
 // MODE 0: out = relu(conv + b) (bf16); MODE 1: out[p] = conv + b, channel 0
 // only (fp32); MODE 2: out = conv * (mask > 0) (bf16, no bias).
 // w: bf16 [5][WROWS][CIN] (rows WROWS..COUT - 1 are zero)
@@ -1212,17 +1216,17 @@ __global__ void __launch_bounds__(TRN_THREADS, 1)
   extern __shared__ __align__(128) unsigned char smem[];
   const uint32_t s_base = (uint32_t)__cvta_generic_to_shared(smem);
   const uint32_t bar0 = s_base + W_BYTES + TILES * TILE;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + W_BYTES + TILES * TILE + 8 * TRN_SLOTS);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + W_BYTES + TILES * TILE + 24 * TRN_SLOTS);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
-                     bar0 + 8 * TRN_SLOTS),
+                     bar0 + 24 * TRN_SLOTS),
                  "r"(TMEM_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
   if (threadIdx.x == 0) {
-    for (int q = 0; q < TRN_SLOTS; ++q)
+    for (int q = 0; q < 3 * TRN_SLOTS; ++q)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar0 + 8 * q) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
@@ -1255,9 +1259,30 @@ __global__ void __launch_bounds__(TRN_THREADS, 1)
   uint32_t phase = 0;
   int commits = 0;
   bool ok = true;
-  // a row into tile b (position n to its row n + 2), asynchronously.  The slot's
-  // threads take consecutive 16 bytes: a warp's request is four whole lines (with a
-  // position a thread it was a piece of 32).
+  // (barriers: the slots' finished MMAs, then the slots' filled tiles, two each)
+  constexpr bool BULK = CIN == 64;
+  const uint32_t full = bar0 + 8 * TRN_SLOTS + 16 * slot;
+  uint32_t full_phase = 0;  // bit b: the phase tile b fills next
+  bool in_flight = false;   // a bulk copy that nothing has waited for yet (the issuer's),
+  uint32_t flight_bar = full, flight_phase = 0;  // and what it completes
+  // a row into tile b (position n to its row n + 2), asynchronously: by the issuer's
+  // bulk copies, or by all of the slot's threads, consecutive 16 bytes each
+  auto fetch_bulk = [&](int row, int b) {
+    const unsigned char* src = reinterpret_cast<const unsigned char*>(x + (size_t)row * CP * CIN);
+    const uint32_t dst = s_base + W_BYTES + (2 * slot + b) * TILE + CHALO * 16;
+    in_flight = true;
+    flight_bar = full + 8 * b;
+    flight_phase = (full_phase >> b) & 1u;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(full + 8 * b), "r"(CP * CIN * 2)
+                 : "memory");
+#pragma unroll
+    for (int j = 0; j < CIN / 8; ++j)
+      asm volatile(
+          "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+              dst + j * TC_LBO_ACT),
+          "l"(src + j * CP * 16), "r"(CP * 16), "r"(full + 8 * b)
+          : "memory");
+  };
   auto fetch = [&](int row, int b) {
     const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)row * CP * CIN) + p;
     unsigned char* tile = smem + W_BYTES + (2 * slot + b) * TILE;
@@ -1270,23 +1295,58 @@ __global__ void __launch_bounds__(TRN_THREADS, 1)
   };
   const int stride = gridDim.x * TRN_SLOTS;
   int b = 0;
-  if (blockIdx.x * TRN_SLOTS + slot < rows) fetch(blockIdx.x * TRN_SLOTS + slot, 0);
-  for (int row = blockIdx.x * TRN_SLOTS + slot; row < rows; row += stride, b ^= 1) {
+  const int row_first = blockIdx.x * TRN_SLOTS + slot;
+  if (row_first < rows) {
+    if (!BULK) {
+      fetch(row_first, 0);
+    } else if (issuer) {
+      fetch_bulk(row_first, 0);
+    }
+  }
+  for (int row = row_first; row < rows; row += stride, b ^= 1) {
     const size_t q = (size_t)row * CP + p;
-    cp_async_wait_all();
-    fence_async_smem();
-    tc_fence_before();
-    slot_sync(slot);
-    if (issuer) {
+    if (!BULK) {
+      cp_async_wait_all();
+      fence_async_smem();
+      tc_fence_before();
+      slot_sync(slot);
+    }
+    // (a tile that never fills: the slot's wait for these MMAs runs out as well)
+    if (issuer && (!BULK || mbar_wait(full + 8 * b, (full_phase >> b) & 1u))) {
+      in_flight = false;
       tc_fence_after();
       tc_layer_issue<CIN, COUT>(td, s_base + W_BYTES + (2 * slot + b) * TILE, s_base);
       tc_commit(bar);
     }
+    full_phase ^= 1u << b;
     ++commits;
     // the next row into the other tile (its last reader, the previous row's
-    // MMAs, completed before that row's epilogue).  Two rows ahead, after these MMAs,
-    // was slower: 83 -> 84 us for 64 to 64 channels, 40 -> 58 for 64 to 1.
-    if (row + stride < rows) fetch(row + stride, b ^ 1);
+    // MMAs, completed before that row's epilogue)
+    if (row + stride < rows) {
+      if (!BULK) {
+        fetch(row + stride, b ^ 1);
+      } else if (issuer && !in_flight) {
+        fetch_bulk(row + stride, b ^ 1);
+      }
+    }
+    // the mask of the 64 channels, a bit each, while the MMAs run
+    uint32_t keep[2] = {0u, 0u};
+    if (MODE == 2) {
+      const uint4* m = reinterpret_cast<const uint4*>(mask + (size_t)row * CP * COUT) + p;
+      uint4 mk[COUT / 8];
+#pragma unroll
+      for (int j = 0; j < COUT / 8; ++j) mk[j] = __ldg(m + j * CP);
+#pragma unroll
+      for (int j = 0; j < COUT / 8; ++j) {
+        const uint32_t w[4] = {mk[j].x, mk[j].y, mk[j].z, mk[j].w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int c = 8 * j + 2 * u;
+          if (__uint_as_float(w[u] << 16) > 0.f) keep[c >> 5] |= 1u << (c & 31);
+          if (__uint_as_float(w[u] & 0xffff0000u) > 0.f) keep[c >> 5] |= 2u << (c & 31);
+        }
+      }
+    }
     const bool done = mbar_wait(bar, phase);
     phase ^= 1u;
     if (slot_any(slot, !done)) {
@@ -1301,13 +1361,11 @@ __global__ void __launch_bounds__(TRN_THREADS, 1)
       if (MODE == 1) {
         static_cast<float*>(out)[q] = v[0] + sbias[0];
       } else {
-        // 16 channels, a whole sector, in one load and one store
-        uint32_t wv[8], mk[8];
-        if (MODE == 2) load_sector(mask + q * COUT + c0, mk);
         float4 b4[4];
         if (MODE == 0)
 #pragma unroll
           for (int j = 0; j < 4; ++j) b4[j] = *reinterpret_cast<const float4*>(sbias + c0 + 4 * j);
+        uint32_t wv[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           float a = v[2 * j], b = v[2 * j + 1];
@@ -1315,13 +1373,16 @@ __global__ void __launch_bounds__(TRN_THREADS, 1)
             a = fmaxf(a + (j & 1 ? b4[j >> 1].z : b4[j >> 1].x), 0.f);
             b = fmaxf(b + (j & 1 ? b4[j >> 1].w : b4[j >> 1].y), 0.f);
           } else {
-            const __nv_bfloat162 m2 = *reinterpret_cast<const __nv_bfloat162*>(&mk[j]);
-            if (!(__bfloat162float(m2.x) > 0.f)) a = 0.f;
-            if (!(__bfloat162float(m2.y) > 0.f)) b = 0.f;
+            const int c = c0 + 2 * j;
+            if (!(keep[c >> 5] & (1u << (c & 31)))) a = 0.f;
+            if (!(keep[c >> 5] & (2u << (c & 31)))) b = 0.f;
           }
           wv[j] = bf16_pair(a, b);
         }
-        store_sector(static_cast<__nv_bfloat16*>(out) + q * COUT + c0, wv);
+        uint4* o = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(out) + (size_t)row * CP * COUT) +
+                   (c0 / 8) * CP + p;
+        o[0] = make_uint4(wv[0], wv[1], wv[2], wv[3]);
+        o[CP] = make_uint4(wv[4], wv[5], wv[6], wv[7]);
       }
     }
     // every thread of the slot has read its TMEM lanes before the next row's
@@ -1331,6 +1392,7 @@ __global__ void __launch_bounds__(TRN_THREADS, 1)
   }
   cp_async_wait_all();  // no copy may land after the CTA is gone
   if (!ok) {
+    if (in_flight) mbar_wait(flight_bar, flight_phase);
     if (p == 0) atomicOr(err, 1);
     // no MMA of this slot may still write TMEM when it is freed
     if (commits > 0) mbar_wait(bar, (uint32_t)((commits - 1) & 1));
@@ -1440,7 +1502,8 @@ __global__ void __launch_bounds__(128, 1)
       // copy c holds x[r + c - 2] at row r
 #pragma unroll
       for (int i = 0; i < CIN / 8; ++i) {
-        const int q = i * 128 + p, pos = q / (CIN / 8), j = q % (CIN / 8);
+        // (64 channels lie by groups of 8, 16 by positions)
+        const int q = i * 128 + p, pos = CIN == 64 ? p : q / (CIN / 8), j = CIN == 64 ? i : q % (CIN / 8);
 #pragma unroll
         for (int c = 0; c < S::NCOPY; ++c) {
           const int r = pos + CHALO - c;
@@ -1449,9 +1512,8 @@ __global__ void __launch_bounds__(128, 1)
       }
 #pragma unroll
       for (int i = 0; i < COUTP / 8; ++i) {
-        const int q = i * 128 + p, pos = q / (COUTP / 8), j = q % (COUTP / 8);
+        const int q = i * 128 + p, pos = COUTP == 64 ? p : q / (COUTP / 8), j = COUTP == 64 ? i : q % (COUTP / 8);
         *reinterpret_cast<uint4*>(B + j * MN_B + pos * 16) = yr[i];
-        bias_add(yr[i], bsum);
       }
     }
     if (row + 1 < r_end) load(row + 1);
@@ -1476,6 +1538,14 @@ __global__ void __launch_bounds__(128, 1)
       tc_commit(bar0 + 8 * st);
     }
     pending[st] = true;
+    // the bias sums, while the MMAs run (this stage is written again after the next
+    // row's barrier)
+    const unsigned char* B = smem + st * STAGE + S::A_BYTES;
+#pragma unroll
+    for (int i = 0; i < COUTP / 8; ++i) {
+      const int q = i * 128 + p;
+      bias_add(*reinterpret_cast<const uint4*>(B + (q % (COUTP / 8)) * MN_B + (q / (COUTP / 8)) * 16), bsum);
+    }
   }
   // the outstanding commits of both stages
   for (int st = 0; st < 2; ++st)
