@@ -22,6 +22,7 @@
 #include <cstring>
 #include <vector>
 
+#include "vg_f32.cuh"
 #include "vg_internal.cuh"
 
 namespace vg {
@@ -376,13 +377,21 @@ __global__ void k_group_mean(const float* __restrict__ g, int group_rows, float2
   const float* src = g + (size_t)grp * group_rows * CP + p;
   // double-float (TwoSum) accumulation: FP64-grade, on the FP32 pipes
   float hi = 0.f, lo = 0.f;
-  for (int r = 0; r < group_rows; ++r) {
-    const float x = src[(size_t)r * CP];
+  auto add = [&](float x) {
     const float t = hi + x;
     const float bb = t - hi;
     lo += (hi - (t - bb)) + (x - bb);
     hi = t;
+  };
+  int r = 0;
+  for (; r + 16 <= group_rows; r += 16) {  // 16 loads in flight
+    float x[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) x[u] = src[(size_t)(r + u) * CP];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) add(x[u]);
   }
+  for (; r < group_rows; ++r) add(src[(size_t)r * CP]);
   // the mean as a double-float pair (hi, lo), so that the kernels that take
   // it out of a row stay on the FP32 pipes
   const double m = ((double)hi + (double)lo) / (double)group_rows;
@@ -399,14 +408,6 @@ __device__ __forceinline__ float deviation(float gq, const float2* __restrict__ 
   const float2 m = gmean[(size_t)(row / group_rows) * CP + p];
   return __fsub_rn(__fsub_rn(gq, m.x), m.y);
 }
-// the group mean plus a deviation, rounded once more (inverse of deviation)
-__device__ __forceinline__ float with_mean(float dn, const float2* __restrict__ gmean, int group_rows, int row,
-                                           int p) {
-  if (group_rows <= 0) return dn;
-  const float2 m = gmean[(size_t)(row / group_rows) * CP + p];
-  return __fadd_rn(m.x, __fadd_rn(m.y, dn));
-}
-
 __device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
   const __nv_bfloat162 pr = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&pr);
@@ -573,11 +574,22 @@ __global__ void __launch_bounds__(CP) k_apply(const float* __restrict__ g, const
   __shared__ float wsum[2][APPLY_ROWS][CP / 32];
   const int p = threadIdx.x, row0 = blockIdx.x * APPLY_ROWS;
   float d[APPLY_ROWS], c[APPLY_ROWS];
+  float2 mean[APPLY_ROWS];  // the rows' group means, read once (with one division)
+  int grp = group_rows > 0 ? row0 / group_rows : 0, left = group_rows > 0 ? (grp + 1) * group_rows - row0 : 0;
 #pragma unroll
   for (int r = 0; r < APPLY_ROWS; ++r) {
     const int row = row0 + r < rows ? row0 + r : rows - 1;  // a short last block repeats its last row
     const size_t q = (size_t)row * CP + p;
-    d[r] = deviation(g[q], gmean, group_rows, row, p);
+    if (group_rows > 0) {
+      mean[r] = gmean[(size_t)grp * CP + p];
+      if (--left == 0 && row0 + r + 1 < rows) {
+        ++grp;
+        left = group_rows;
+      }
+      d[r] = __fsub_rn(__fsub_rn(g[q], mean[r].x), mean[r].y);
+    } else {
+      d[r] = g[q];
+    }
     c[r] = (scale[row] * tau) * pred[q];
   }
   float dh[APPLY_ROWS], ch[APPLY_ROWS];
@@ -616,22 +628,19 @@ __global__ void __launch_bounds__(CP) k_apply(const float* __restrict__ g, const
       ch[r] = c[r];
     }
   }
-  // hn = Pd + Pc; row sums of (Pd)^2 and hn^2 by warp shuffles, then the warps
-  float hn[APPLY_ROWS];
+  // hn = Pd + Pc; row sums of (Pd)^2 and hn^2: 16 sums of a warp by transposition,
+  // then the warps
+  float hn[APPLY_ROWS], sums[2 * APPLY_ROWS];
 #pragma unroll
   for (int r = 0; r < APPLY_ROWS; ++r) {
     hn[r] = dh[r] + ch[r];
-    float so = dh[r] * dh[r], sn = hn[r] * hn[r];
-#pragma unroll
-    for (int m = 16; m > 0; m >>= 1) {
-      so += __shfl_xor_sync(0xffffffffu, so, m);
-      sn += __shfl_xor_sync(0xffffffffu, sn, m);
-    }
-    if ((p & 31) == 0) {
-      wsum[0][r][p >> 5] = so;
-      wsum[1][r][p >> 5] = sn;
-    }
+    sums[r] = dh[r] * dh[r];
+    sums[APPLY_ROWS + r] = hn[r] * hn[r];
   }
+  int idx;
+  bool writer;
+  lane_transpose_sum<2 * APPLY_ROWS, 32>(sums, p & 31, idx, writer);
+  if (writer) wsum[idx / APPLY_ROWS][idx % APPLY_ROWS][p >> 5] = sums[0];
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < APPLY_ROWS; ++r) {
@@ -641,7 +650,7 @@ __global__ void __launch_bounds__(CP) k_apply(const float* __restrict__ g, const
     const float r_new = (wsum[1][r][0] + wsum[1][r][1]) + (wsum[1][r][2] + wsum[1][r][3]);
     const float factor = r_new > r_old ? sqrtf(r_old / r_new) : 1.f;
     const float dn = (d[r] - dh[r]) + hn[r] * factor;
-    out[(size_t)row * CP + p] = with_mean(dn, gmean, group_rows, row, p);
+    out[(size_t)row * CP + p] = group_rows > 0 ? __fadd_rn(mean[r].x, __fadd_rn(mean[r].y, dn)) : dn;
   }
 }
 
