@@ -16,6 +16,33 @@ template <typename T>
 __device__ __forceinline__ cx<T> operator+(cx<T> a, cx<T> b) { return {a.x + b.x, a.y + b.y}; }
 template <typename T>
 __device__ __forceinline__ cx<T> operator-(cx<T> a, cx<T> b) { return {a.x - b.x, a.y - b.y}; }
+// Two FP32 operations in one instruction (Blackwell's packed FP32; each half rounds as
+// the plain operation does).  The FP32 pipe takes two cycles for it, so its rate is the
+// same, but the FP32 transforms are bound by instruction issue: with complex sums and
+// differences packed, and a row pair's moments, a 4096-run sweep step takes 1.61 ms
+// instead of 1.68, a 64-run one 61 us instead of 65.
+#ifdef __CUDA_ARCH__
+__device__ __forceinline__ cx<float> add2(cx<float> a, cx<float> b) {
+  const float2 r = __fadd2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y));
+  return {r.x, r.y};
+}
+__device__ __forceinline__ cx<float> mul2(cx<float> a, cx<float> b) {
+  const float2 r = __fmul2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y));
+  return {r.x, r.y};
+}
+__device__ __forceinline__ cx<float> fma2(cx<float> a, cx<float> b, cx<float> c) {
+  const float2 r = __ffma2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y), make_float2(c.x, c.y));
+  return {r.x, r.y};
+}
+template <>
+__device__ __forceinline__ cx<float> operator+<float>(cx<float> a, cx<float> b) { return add2(a, b); }
+template <>
+__device__ __forceinline__ cx<float> operator-<float>(cx<float> a, cx<float> b) { return add2(a, {-b.x, -b.y}); }
+#else
+__device__ cx<float> add2(cx<float> a, cx<float> b);
+__device__ cx<float> mul2(cx<float> a, cx<float> b);
+__device__ cx<float> fma2(cx<float> a, cx<float> b, cx<float> c);
+#endif
 template <typename T>
 __device__ __forceinline__ cx<T> cmul(cx<T> a, cx<T> b) {
   return {a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x};

@@ -168,8 +168,8 @@ __device__ __forceinline__ void kick_rotate(cx<float>* s, int t, int G, Ang ha, 
       s[sp<float, PS>(k)] = {(pb_r * z.y + pb_m1r * f0.x) * sc, (pa_r * z.x + pa_m1r * f0.x) * sc};
     } else {
       const cx<float> zk = s[sp<float, PS>(k)], zm = s[sp<float, PS>(N - k)];
-      const cx<float> fa = {(zk.x + zm.x) * 0.5f, (zk.y - zm.y) * 0.5f};
-      const cx<float> fb = {(zk.y + zm.y) * 0.5f, (zm.x - zk.x) * 0.5f};
+      const cx<float> hs = mul2({0.5f, 0.5f}, zk + zm), hd = mul2({0.5f, 0.5f}, zk - zm);
+      const cx<float> fa = {hs.x, hd.y}, fb = {hs.y, -hd.x};
       const cx<float> ga = {(pa_r * fa.x - pa_i * fa.y + pa_m1r * f0.x - pa_i * f0.y) * sc,
                             (pa_r * fa.y + pa_i * fa.x + pa_m1r * f0.y + pa_i * f0.x) * sc};
       const cx<float> gb = {(pb_r * fb.x - pb_i * fb.y + pb_m1r * f0.x - pb_i * f0.y) * sc,
@@ -263,23 +263,24 @@ __device__ __forceinline__ void collide_pair(cx<float>* s, int t, const RowConst
   // vectors load coalesced; only the tridiagonal solves work on chunks
   df32 mv[6];
   {
-    float m[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    // (both rows in one packed operation)
+    cx<float> m[3] = {};
 #pragma unroll ROW_UNROLL
     for (int i = 0; i < R; ++i) {
       const int j = t + i * G;
       const float w = (j == 0 || j == N - 1) ? 0.5f : 1.f;
-      const cx<float> z = s[sp<float, row_pad_shift(R)>(j)];
       const float vj = rc.v[j];
-      const float ga = w * z.x, gb = w * z.y;
-      m[0] += ga;
-      m[1] = fmaf(ga, vj, m[1]);
-      m[2] = fmaf(ga * vj, vj, m[2]);
-      m[3] += gb;
-      m[4] = fmaf(gb, vj, m[4]);
-      m[5] = fmaf(gb * vj, vj, m[5]);
+      const cx<float> vv = {vj, vj};
+      const cx<float> z = mul2({w, w}, s[sp<float, row_pad_shift(R)>(j)]);
+      m[0] = add2(m[0], z);
+      m[1] = fma2(z, vv, m[1]);
+      m[2] = fma2(mul2(z, vv), vv, m[2]);
     }
 #pragma unroll
-    for (int q = 0; q < 6; ++q) mv[q] = {m[q], 0.f};
+    for (int q = 0; q < 3; ++q) {
+      mv[q] = {m[q].x, 0.f};
+      mv[3 + q] = {m[q].y, 0.f};
+    }
   }
   // per-row scalars in double-float, each row's by one thread; the group reads them back
   float* sc = reinterpret_cast<float*>(red);
@@ -310,10 +311,11 @@ __device__ __forceinline__ void collide_pair(cx<float>* s, int t, const RowConst
   for (int i = 0; i < R; ++i) {
     const int j = t + i * G;
     const float S = rc.S[j], Mv = rc.Mv[j], D = rc.D[j];
-    cx<float> z = s[sp<float, row_pad_shift(R)>(j)];
-    z.x -= -sa[3] * S + cm * Mv - sa[4] * D;
-    z.y -= -sb[3] * S + cm * Mv - sb[4] * D;
-    s[sp<float, row_pad_shift(R)>(j)] = z;
+    const cx<float> z = s[sp<float, row_pad_shift(R)>(j)];
+    // (the three terms nearly cancel: their sum first)
+    const float cM = -cm * Mv;
+    const cx<float> u = fma2({sa[4], sb[4]}, {D, D}, fma2({sa[3], sb[3]}, {S, S}, {cM, cM}));
+    s[sp<float, row_pad_shift(R)>(j)] = add2(z, u);
   }
   sync();
   // off-diagonals at v[j -+ 1] of the uniform grid v[j] = v[0] + j dv,
@@ -419,37 +421,31 @@ __device__ __forceinline__ void row_pair(const RowArgs& a, int pair, unsigned ch
       // both rows: [0, NQ) row a, [NQ, 2 NQ) row b
       static_assert(NPOW >= 1 && NPOW <= 6, "power moments");
       constexpr int NQ = NPOW + 3;
-      float sa[NQ] = {0}, sb[NQ] = {0};
+      cx<float> sum[NQ] = {};  // (row a, row b), packed
   #pragma unroll ROW_UNROLL
       for (int i = 0; i < R; ++i) {
         const int j = t + i * G;  // consecutive threads, consecutive j: coalesced loads
         const float w = (j == 0 || j == N - 1) ? 0.5f : 1.f;
         const float vj = a.rc->v[j], f0j = a.rc->f0[j];
-        const cx<float> z = s[sp<float, row_pad_shift(R)>(j)];
-        float pa = w * z.x, pb = w * z.y;
+        const cx<float> z = s[sp<float, row_pad_shift(R)>(j)], vv = {vj, vj}, f0 = {f0j, f0j}, ww = {w, w};
+        const cx<float> wz = mul2(ww, z);
+        cx<float> pw = wz;
   #pragma unroll
         for (int p = 0; p < NPOW; ++p) {
-          sa[p] += pa;
-          sb[p] += pb;
-          if (p + 1 < NPOW) {
-            pa *= vj;
-            pb *= vj;
-          }
+          sum[p] = add2(sum[p], pw);
+          if (p + 1 < NPOW) pw = mul2(pw, vv);
         }
-        sa[NPOW] = fmaf(w * z.x, z.x, sa[NPOW]);
-        sb[NPOW] = fmaf(w * z.y, z.y, sb[NPOW]);
-        sa[NPOW + 1] = fmaf(w * z.x, f0j, sa[NPOW + 1]);
-        sb[NPOW + 1] = fmaf(w * z.y, f0j, sb[NPOW + 1]);
+        sum[NPOW] = fma2(wz, z, sum[NPOW]);
+        sum[NPOW + 1] = fma2(wz, f0, sum[NPOW + 1]);
         // f log f by the fast logarithm (3 ulp; NaN for f < 0 as in FP64)
-        const float fa = z.x + f0j, fb = z.y + f0j;
-        sa[NPOW + 2] = fmaf(w * fa, __logf(fa), sa[NPOW + 2]);
-        sb[NPOW + 2] = fmaf(w * fb, __logf(fb), sb[NPOW + 2]);
+        const cx<float> f = add2(z, f0);
+        sum[NPOW + 2] = fma2(mul2(ww, f), {__logf(f.x), __logf(f.y)}, sum[NPOW + 2]);
       }
       df32 m2[2 * NQ];
   #pragma unroll
       for (int q = 0; q < NQ; ++q) {
-        m2[q] = {sa[q], 0.f};
-        m2[NQ + q] = {sb[q], 0.f};
+        m2[q] = {sum[q].x, 0.f};
+        m2[NQ + q] = {sum[q].y, 0.f};
       }
       // raw sums; the storage kernels form dv * sum + trapz(f0 ...) in FP64: slots
       // 0 .. NPOW - 1 the powers, 6 sum w (g^2 + 2 g f0), 7 sum w f log f
