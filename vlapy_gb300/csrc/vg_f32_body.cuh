@@ -318,15 +318,17 @@ __device__ __forceinline__ void collide_pair(cx<float>* s, int t, const RowConst
     s[sp<float, row_pad_shift(R)>(j)] = add2(z, u);
   }
   sync();
-  // off-diagonals at v[j -+ 1] of the uniform grid v[j] = v[0] + j dv,
-  // formed in registers (within an FP32 ulp of the tabulated grid)
+  // off-diagonals at v[j -+ 1] of the uniform grid v[j] = v[0] + j dv, formed in
+  // registers
   const float v0 = rc.v0f, dvf = rc.dvf;
 #pragma unroll 1
   for (int row = 0; row < 2; ++row) {
     const float Af = row ? sb[0] : sa[0], diag = row ? sb[1] : sa[1], vb = row ? sb[2] : sa[2];
-    auto lf = [&](int j) { return nu * (Af + (fmaf((float)(j - 1), dvf, v0) - vb) * i2dv); };
-    auto uf = [&](int j) { return nu * (Af - (fmaf((float)(j + 1), dvf, v0) - vb) * i2dv); };
-    partition_solve<R, G>(reinterpret_cast<float*>(s) + row, t, diag, lf, uf, pcr, sync);
+    // l(j) = nu (Af + (v[j - 1] - vb) / 2 dv), u(j) = nu (Af - (v[j + 1] - vb) / 2 dv)
+    const float ls = nu * (Af + (fmaf((float)(t * R - 1), dvf, v0) - vb) * i2dv);
+    const float us = nu * (Af - (fmaf((float)(t * R + 1), dvf, v0) - vb) * i2dv);
+    const float dl = nu * (dvf * i2dv);
+    partition_solve<R, G>(reinterpret_cast<float*>(s) + row, t, diag, ls, dl, us, -dl, pcr, sync);
   }
 }
 
