@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(fx_row_block(N), fx_row_block(N) > 256 ? 1 : 2
     for (int i = 0; i < R; ++i)
       io[i] = {bad_a ? 0 : fx_from_double(da[i], Ea), bad_b ? 0 : fx_from_double(db[i], Eb)};
   }
-  FxPass<N, false, 1, true, false>::run(s, t, tw, sync, io);
+  fx_fft<N, false, true, false>(s, t, tw, sync, io);
   FxNorms n = fx_rotate<N, DOWN>(s, t, fx_turn(turn, bad_a ? 0.0 : ea), fx_turn(turn, bad_b ? 0.0 : eb), tw);
   n.l1 = __reduce_add_sync(mask, n.l1);
   n.a2 = __reduce_add_sync(mask, n.a2);
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(fx_row_block(N), fx_row_block(N) > 256 ? 1 : 2
                    tw64, sync);
     return;
   }
-  FxPass<N, true, 1, false, true>::run(s, t, tw, sync, io, h);
+  fx_fft<N, true, false, true>(s, t, tw, sync, io, h);
   // lines of zeros stay so: the partner's rounding does not reach them
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
   const bool set_a = bad_a || zero_a, set_b = bad_b || zero_b;

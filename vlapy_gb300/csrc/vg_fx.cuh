@@ -272,65 +272,100 @@ __device__ __forceinline__ fxw fx_tw(const fxw* __restrict__ p) {
   return w;
 }
 
-// One Stockham pass and the ones after it, as StockhamPass of vg_fft.cuh: input
-// in io for the first pass, output in io after the last when OUT_REGS, else the
-// result ends in s.  Element i of thread t is t + i N / R.  The transform back
-// first divides its bins by 2^h.
-template <int N, bool INV, int NS, bool IN_REGS, bool OUT_REGS>
-struct FxPass {
-  static constexpr int R = fx_radix(N);
-  template <typename Sync>
-  static __device__ __forceinline__ void run(fx* s, int t, const fxw* __restrict__ tw, const Sync& sync, fx (&io)[R],
-                                             int h = 0) {
-    constexpr int r = (N / NS < R) ? (N / NS) : R;
-    constexpr int NB = N / r, G = N / R, BPT = NB / G;
-    constexpr bool last = NS * r == N;
-    fx a[BPT][r];
+// One Stockham pass (vg_fft.cuh) at span ns on r elements a butterfly: loads from s
+// (FIRST: from io), twiddles, butterflies, results in a.  The transform back first
+// divides its bins by 2^h.
+template <int N, bool INV, int r, bool FIRST>
+__device__ __forceinline__ void fx_pass(const fx* s, int t, const fxw* __restrict__ tw, int ns, int h,
+                                        const fx (&io)[fx_radix(N)], fx (&a)[fx_radix(N)]) {
+  constexpr int R = fx_radix(N), G = N / R, BPT = R / r;
 #pragma unroll
-    for (int b = 0; b < BPT; ++b) {
-      const int j = t + b * G;
-      const int k = j & (NS - 1);
+  for (int b = 0; b < BPT; ++b) {
+    const int j = t + b * G;
+    fx v[r];
 #pragma unroll
-      for (int m = 0; m < r; ++m) {
-        if constexpr (NS == 1 && IN_REGS) a[b][m] = io[m];
-        else a[b][m] = s[fx_sp(j + m * NB)];
-      }
-      if constexpr (NS > 1) {
-        const fxw* span = tw + (NS * r - 2);
-        if constexpr (!INV) a[b][0] = fx_down<2>(a[b][0]);
+    for (int m = 0; m < r; ++m) {
+      if constexpr (FIRST) v[m] = io[m];
+      else v[m] = s[fx_sp(j + m * (N / r))];
+    }
+    if constexpr (!FIRST) {
+      const int k = j & (ns - 1);
+      const fxw* span = tw + (ns * r - 2);
+      if constexpr (!INV) v[0] = fx_down<2>(v[0]);
 #pragma unroll
-        for (int m = 1; m < r; ++m) a[b][m] = fx_cmul<INV ? 2 : 0, INV>(a[b][m], fx_tw(span + m * k));
-      } else if constexpr (INV) {
-        if (h > 0) {
+      for (int m = 1; m < r; ++m) v[m] = fx_cmul<INV ? 2 : 0, INV>(v[m], fx_tw(span + m * k));
+    } else if constexpr (INV) {
+      if (h > 0) {
 #pragma unroll
-          for (int m = 0; m < r; ++m) {
-            a[b][m].x = (a[b][m].x + (1ll << (h - 1))) >> h;
-            a[b][m].y = (a[b][m].y + (1ll << (h - 1))) >> h;
-          }
+        for (int m = 0; m < r; ++m) {
+          v[m].x = (v[m].x + (1ll << (h - 1))) >> h;
+          v[m].y = (v[m].y + (1ll << (h - 1))) >> h;
         }
       }
-      FxDft<r, INV>::run(a[b]);
     }
-    if constexpr (last && OUT_REGS) {
+    FxDft<r, INV>::run(v);
 #pragma unroll
-      for (int b = 0; b < BPT; ++b)
-#pragma unroll
-        for (int m = 0; m < r; ++m) io[b + m * BPT] = a[b][m];
-    } else {
-      sync();
-#pragma unroll
-      for (int b = 0; b < BPT; ++b) {
-        const int j = t + b * G;
-        const int k = j & (NS - 1);
-        const int base = (j - k) * r + k;
-#pragma unroll
-        for (int m = 0; m < r; ++m) s[fx_sp(base + m * NS)] = a[b][m];
-      }
-      sync();
-      if constexpr (!last) FxPass<N, INV, NS * r, IN_REGS, OUT_REGS>::run(s, t, tw, sync, io);
-    }
+    for (int m = 0; m < r; ++m) a[b * r + m] = v[m];
   }
-};
+}
+template <int N, int r>
+__device__ __forceinline__ void fx_scatter(fx* s, int t, int ns, const fx (&a)[fx_radix(N)]) {
+  constexpr int R = fx_radix(N), G = N / R;
+#pragma unroll
+  for (int b = 0; b < R / r; ++b) {
+    const int j = t + b * G;
+    const int k = j & (ns - 1);
+    const int base = (j - k) * r + k;
+#pragma unroll
+    for (int m = 0; m < r; ++m) s[fx_sp(base + m * ns)] = a[b * r + m];
+  }
+}
+
+// The transform of a sequence: element i of thread t is t + i N / R.  IN_REGS: the
+// input is in io, else in s; OUT_REGS: the output ends in io, else in s.  The passes
+// of full radix after the first share their code, in a loop that stays rolled: a
+// small run is bound by instruction fetches (five of eight stall cycles at 64 x 1024
+// with every pass written out, 37 us a launch with cold caches, now 24).
+template <int N, bool INV, bool IN_REGS, bool OUT_REGS, typename Sync>
+__device__ __forceinline__ void fx_fft(fx* s, int t, const fxw* __restrict__ tw, const Sync& sync,
+                                       fx (&io)[fx_radix(N)], int h = 0) {
+  constexpr int R = fx_radix(N), G = N / R;
+  constexpr int FULL = ilog2(N) / ilog2(R);          // passes of radix R
+  constexpr int REST = N >> (FULL * ilog2(R));       // radix of the last one, or 1
+  fx a[R];
+  if constexpr (!IN_REGS) {
+#pragma unroll
+    for (int i = 0; i < R; ++i) io[i] = s[fx_sp(t + i * G)];
+  }
+  fx_pass<N, INV, R, true>(s, t, tw, 1, h, io, a);
+  int ns = 1;
+#pragma unroll 1
+  for (int q = 1; q < FULL; ++q) {
+    sync();
+    fx_scatter<N, R>(s, t, ns, a);
+    sync();
+    ns *= R;
+    fx_pass<N, INV, R, false>(s, t, tw, ns, h, io, a);
+  }
+  if constexpr (REST > 1) {
+    sync();
+    fx_scatter<N, R>(s, t, ns, a);
+    sync();
+    fx_pass<N, INV, REST, false>(s, t, tw, N / REST, h, io, a);
+  }
+  constexpr int r = REST > 1 ? REST : R;
+  if constexpr (OUT_REGS) {
+    // butterfly b of thread t holds elements t + G (b + m R / r)
+#pragma unroll
+    for (int b = 0; b < R / r; ++b)
+#pragma unroll
+      for (int m = 0; m < r; ++m) io[b + m * (R / r)] = a[b * r + m];
+  } else {
+    sync();
+    fx_scatter<N, r>(s, t, N / r, a);
+    sync();
+  }
+}
 
 // ---- doubles to fixed point and back ------------------------------------------
 // The largest element of a line decides its scale: element f -> f 2^(1081 - E)
@@ -363,6 +398,9 @@ __device__ __forceinline__ long long fx_from_double(double f, int E) {
   return (long long)u < 0 ? -m : m;
 }
 
+// (out of line, as are the other rare or repeated pieces: instruction fetches are what
+// a small run waits for)
+inline __device__ __noinline__ double fx_to_double_far(long long v, int k) { return ldexp(__ll2double_rn(v), k); }
 // v 2^k as a double, rounded to nearest even
 __device__ __forceinline__ double fx_to_double(long long v, int k) {
   if (v == 0) return 0.0;
@@ -373,7 +411,7 @@ __device__ __forceinline__ double fx_to_double(long long v, int k) {
   const unsigned long long m = n >> 11;              // 53 bits
   const unsigned long long rem = n & 0x7ff;
   const int e = 63 - z + k + 1023;                   // exponent field
-  if (e < 1 || e > 2045) return ldexp(__ll2double_rn(v), k);
+  if (e < 1 || e > 2045) return fx_to_double_far(v, k);
   // the implicit bit of m adds one to the exponent field; a carry of the rounding runs into it
   unsigned long long r = ((unsigned long long)(e - 1) << 52) + m;
   r += (rem > 0x400 || (rem == 0x400 && (m & 1))) ? 1 : 0;
@@ -431,6 +469,7 @@ __device__ __forceinline__ fxc fx_sincos(unsigned long long tau, const fxw* __re
   const long long c0 = ((long long)w.xh << 32) + w.xl, n0 = ((long long)w.yh << 32) + w.yl;
   return {c0 + p.x, p.y - n0};
 }
+inline __device__ __noinline__ fxc fx_sincos_call(unsigned long long tau, const fxw* tw) { return fx_sincos(tau, tw); }
 // the product of two unit rotations
 __device__ __forceinline__ fxc fx_turn_by(fxc a, const fxw& w) {
   const fx p = fx_cmul<0, false>({a.c, a.s}, w);
@@ -464,9 +503,9 @@ __device__ __forceinline__ FxNorms fx_rotate(fx* s, int t, unsigned long long fa
                                              const fxw* __restrict__ tw) {
   constexpr int G = fx_threads(N);
   FxNorms n = {0, 0, 0};
-  fxc pa = fx_sincos((unsigned long long)t * fa, tw), pb = fx_sincos((unsigned long long)t * fb, tw);
-  const fxw ga = fx_mult(fx_sincos((unsigned long long)G * fa, tw));
-  const fxw gb = fx_mult(fx_sincos((unsigned long long)G * fb, tw));
+  fxc pa = fx_sincos_call((unsigned long long)t * fa, tw), pb = fx_sincos_call((unsigned long long)t * fb, tw);
+  const fxw ga = fx_mult(fx_sincos_call((unsigned long long)G * fa, tw));
+  const fxw gb = fx_mult(fx_sincos_call((unsigned long long)G * fb, tw));
   for (int k = t; k <= N / 2; k += G) {
     const fxw wa = fx_mult(pa), wb = fx_mult(pb);
     const fx zk = fx_down<DOWN>(s[fx_sp(k)]);

@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(fx_col_block(NX), fx_col_block(NX) > 256 ? 1 :
       io[i] = {bad_a ? 0 : fx_from_double(da[i], Ea), bad_b ? 0 : fx_from_double(db[i], Eb)};
   }
   const CtaSync sync;
-  FxPass<NX, false, 1, true, false>::run(s, t, tw, sync, io);
+  fx_fft<NX, false, true, false>(s, t, tw, sync, io);
   FxNorms n = fx_rotate<NX, DOWN>(s, t, fx_turn(r.turn, bad_a ? 0.0 : ca), fx_turn(r.turn, bad_b ? 0.0 : cb), tw);
   if constexpr (G > 1) {
     atomicAdd(&red[5 * p + 2], n.l1);
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(fx_col_block(NX), fx_col_block(NX) > 256 ? 1 :
     fx_pair_f64<NX>({fc, ca, Ea, va, bad_a}, {fc + 1, cb, Eb, vb, bad_b}, nv, sd, t, r.kx, dt, tw64, sync);
     return;
   }
-  FxPass<NX, true, 1, false, true>::run(s, t, tw, sync, io, h);
+  fx_fft<NX, true, false, true>(s, t, tw, sync, io, h);
   // lines of zeros stay so: the partner's rounding does not reach them
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
   const bool set_a = bad_a || zero_a, set_b = bad_b || zero_b;
