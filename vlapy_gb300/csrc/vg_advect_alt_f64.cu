@@ -21,9 +21,8 @@
 //      elimination with a pivot table shared by all lines;
 //   2. evaluated on the cubic piece that holds each departure point, clamped
 //      to the padded range as FITPACK's evaluator (fpbisp) clamps it.
-// Step 1 runs one thread per v column for the x step (a serial recurrence over
-// nx; the columns are many) and one warp per x row for the v step (the rows are
-// few and long: a warp-parallel scan of the recurrence).  Step 2 runs one thread
+// Step 1 splits each line's recurrence over the threads of one to eight warps (one
+// thread per v column for the x step where the columns alone fill the chip).  Step 2 runs one thread
 // per cell, coalesced along v.  FITPACK solves for B-spline coefficients by Givens
 // rotations instead, so the two agree to rounding, not bit for bit.
 //
@@ -103,20 +102,103 @@ __global__ void k_sl_solve_x(const double* __restrict__ f, double* __restrict__ 
   sl_solve_line(f, (size_t)j, (size_t)nv, M, (size_t)j, (size_t)nv, nx, x[2] - x[1], w);
 }
 
-// v step: one WARP per x row; M[nx][nv + 2].  The rows are few (nx) and long
-// (nv), so the serial recurrences are split: lane l owns the unknowns
-// q in [l L, (l + 1) L), L = ceil(m / 32).  Each Thomas sweep is a chain of
-// affine maps (forward d_q = -w_q d_{q-1} + w_q r_q; backward
-// x_q = -w_q x_{q+1} + d_q), so a lane composes its chunk's map, a 5-step
-// shuffle scan composes the maps of the lanes before it (after it, for the
-// backward sweep), and the lane replays its chunk from the value that gives.
-// The maps contract (|w_q| < 0.27), so the reassociation changes only rounding.
-__global__ void k_sl_solve_v(const double* __restrict__ f, double* __restrict__ M, int nx, int nv,
-                             const double* __restrict__ v, const double* __restrict__ w) {
+// The split of a line's two recurrences.  Each Thomas sweep is a chain of affine maps
+// (forward d_q = -w_q d_{q-1} + w_q r_q; backward x_q = -w_q x_{q+1} + d_q), so a
+// thread composes the map of its chunk of the unknowns, the maps before it (after it,
+// backward) are composed for it, and it replays its chunk from the value that gives.
+// The maps contract (|w_q| < 0.27), so the reassociation changes only rounding.  It is
+// twice the FP64 instructions of one thread a line, each 64 cycles a warp whatever the
+// number of warps, so it pays as long as schedulers are idle.
+
+// x step, SL_X_SPLIT warps per 32 columns, each with a chunk of the nx unknowns.  One
+// thread a column took 33 us at 64 x 1024 (32 warps on the whole chip), now 14.
+constexpr int SL_X_SPLIT = 8;
+__global__ void __launch_bounds__(32 * SL_X_SPLIT) k_sl_solve_x_split(const double* __restrict__ f, double* __restrict__ M,
+                                                                      int nx, int nv, const double* __restrict__ x,
+                                                                      const double* __restrict__ w) {
+  __shared__ double ca[SL_X_SPLIT][32], cb[SL_X_SPLIT][32];
+  const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
+  const int col = blockIdx.x * 32 + lane, j = min(col, nv - 1);
+  const bool on = col < nv;  // (the lanes past the last column read it and write nothing)
+  const int N = nx, m = N - 2;
+  auto y = [&](int q) { return f[(size_t)q * nv + j]; };
+  auto Mr = [&](int k) -> double& { return M[(size_t)k * nv + j]; };
+  const double h = x[2] - x[1];
+  const double inv_h2 = 1.0 / (h * h);
+  const double c6 = 6.0 * inv_h2;
+  const double m1 = ((y(N - 1) + y(1)) - 2.0 * y(0)) * inv_h2;
+  const double mn = ((y(N - 2) + y(0)) - 2.0 * y(N - 1)) * inv_h2;
+  const int L = (m + SL_X_SPLIT - 1) / SL_X_SPLIT;
+  const int q0 = min(c * L, m), q1 = min(q0 + L, m);
+  auto rhs = [&](int q, double ym, double y0, double yp) {
+    double r = ((ym + yp) - 2.0 * y0) * c6;
+    if (q == 0) r -= m1;
+    if (q == m - 1) r -= mn;
+    return r;
+  };
+  // forward; the right-hand sides wait in M
+  double A = 1.0, B = 0.0;
+  {
+    double ym = y(q0), y0 = y(min(q0 + 1, N - 1));
+#pragma unroll 4
+    for (int q = q0; q < q1; ++q) {
+      const double yp = y(q + 2), wq = w[q];
+      const double r = rhs(q, ym, y0, yp) * wq;
+      if (on) Mr(q + 2) = r;
+      A = -wq * A;
+      B = r - wq * B;
+      ym = y0;
+      y0 = yp;
+    }
+  }
+  ca[c][lane] = A;
+  cb[c][lane] = B;
+  __syncthreads();
+  double d = 0.0;
+  for (int q = 0; q < c; ++q) d = ca[q][lane] * d + cb[q][lane];
+  __syncthreads();
+  for (int q = q0; q < q1; ++q) {
+    d = Mr(q + 2) - w[q] * d;
+    if (on) Mr(q + 2) = d;
+  }
+  // backward, from x_m = 0
+  A = 1.0;
+  B = 0.0;
+#pragma unroll 4
+  for (int q = q1 - 1; q >= q0; --q) {
+    const double wq = w[q];
+    A = -wq * A;
+    B = Mr(q + 2) - wq * B;
+  }
+  ca[c][lane] = A;
+  cb[c][lane] = B;
+  __syncthreads();
+  double v = 0.0;
+  for (int q = SL_X_SPLIT - 1; q > c; --q) v = ca[q][lane] * v + cb[q][lane];
+  for (int q = q1 - 1; q >= q0; --q) {
+    v = Mr(q + 2) - w[q] * v;
+    if (on) Mr(q + 2) = v;
+  }
+  __syncthreads();
+  if (c == 0 && on) {
+    Mr(1) = m1;
+    Mr(N) = mn;
+    Mr(0) = 2.0 * m1 - Mr(2);
+    Mr(N + 1) = 2.0 * mn - Mr(N - 1);
+  }
+}
+
+// v step: W warps per x row; M[nx][nv + 2].  The rows are few (nx) and long (nv): lane l
+// of the row owns the unknowns q in [l L, (l + 1) L), L = ceil(m / 32 W); a warp's maps
+// are composed by a 5-step shuffle scan, the warps' through shared memory.  One warp a
+// row, 32 unknowns a lane, took 45 us at 64 x 1024, now 15.
+template <int W>
+__global__ void __launch_bounds__(32 * W) k_sl_solve_v(const double* __restrict__ f, double* __restrict__ M, int nx, int nv,
+                                                       const double* __restrict__ v, const double* __restrict__ w) {
   constexpr unsigned FULL = 0xffffffffu;
-  const int row = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= nx) return;  // uniform per warp
+  __shared__ double ca[W], cb[W];
+  const int row = blockIdx.x;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int N = nv, m = N - 2;
   const double* y = f + (size_t)row * nv;   // y(k) = y[pad_src(k, N)]
   double* Mr = M + (size_t)row * (nv + 2);
@@ -125,8 +207,8 @@ __global__ void k_sl_solve_v(const double* __restrict__ f, double* __restrict__ 
   const double c6 = 6.0 * inv_h2;
   const double m1 = ((y[N - 1] + y[1]) - 2.0 * y[0]) * inv_h2;            // M_1
   const double mn = ((y[N - 2] + y[0]) - 2.0 * y[N - 1]) * inv_h2;        // M_{n-2}
-  const int L = (m + 31) >> 5;
-  const int q0 = min(lane * L, m), q1 = min(q0 + L, m);
+  const int L = (m + 32 * W - 1) / (32 * W);
+  const int q0 = min((int)threadIdx.x * L, m), q1 = min(q0 + L, m);
   // right-hand side of unknown q (padded node k = q + 2, line values k - 2 .. k)
   auto rhs = [&](int q) {
     double r = ((y[q] + y[q + 2]) - 2.0 * y[q + 1]) * c6;
@@ -134,12 +216,14 @@ __global__ void k_sl_solve_v(const double* __restrict__ f, double* __restrict__ 
     if (q == m - 1) r -= mn;
     return r;
   };
-  // forward sweep
+  // forward sweep; the right-hand sides wait in M
   double A = 1.0, B = 0.0;
+#pragma unroll 4
   for (int q = q0; q < q1; ++q) {
-    const double wq = w[q];
+    const double wq = w[q], r = rhs(q) * wq;
+    Mr[q + 2] = r;
     A = -wq * A;
-    B = (rhs(q) - B) * wq;
+    B = r - wq * B;
   }
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
@@ -149,15 +233,28 @@ __global__ void k_sl_solve_v(const double* __restrict__ f, double* __restrict__ 
       A = A * Ap;
     }
   }
-  double d = __shfl_up_sync(FULL, B, 1);
-  if (lane == 0) d = 0.0;
+  double d = 0.0;  // the value entering the warp
+  if constexpr (W > 1) {
+    if (lane == 31) {
+      ca[wid] = A;
+      cb[wid] = B;
+    }
+    __syncthreads();
+    for (int q = 0; q < wid; ++q) d = ca[q] * d + cb[q];
+    __syncthreads();
+  }
+  {
+    const double Ae = __shfl_up_sync(FULL, A, 1), Be = __shfl_up_sync(FULL, B, 1);
+    if (lane > 0) d = Ae * d + Be;
+  }
   for (int q = q0; q < q1; ++q) {
-    d = (rhs(q) - d) * w[q];
+    d = Mr[q + 2] - w[q] * d;
     Mr[q + 2] = d;
   }
   // backward sweep, from x_m = 0; each lane reads back only its own chunk
   A = 1.0;
   B = 0.0;
+#pragma unroll 4
   for (int q = q1 - 1; q >= q0; --q) {
     const double wq = w[q];
     A = -wq * A;
@@ -171,14 +268,25 @@ __global__ void k_sl_solve_v(const double* __restrict__ f, double* __restrict__ 
       A = A * Ap;
     }
   }
-  double x = __shfl_down_sync(FULL, B, 1);
-  if (lane == 31) x = 0.0;
+  double x = 0.0;
+  if constexpr (W > 1) {
+    if (lane == 0) {
+      ca[wid] = A;
+      cb[wid] = B;
+    }
+    __syncthreads();
+    for (int q = W - 1; q > wid; --q) x = ca[q] * x + cb[q];
+  }
+  {
+    const double Ae = __shfl_down_sync(FULL, A, 1), Be = __shfl_down_sync(FULL, B, 1);
+    if (lane < 31) x = Ae * x + Be;
+  }
   for (int q = q1 - 1; q >= q0; --q) {
     x = Mr[q + 2] - w[q] * x;
     Mr[q + 2] = x;
   }
-  __syncwarp();  // M_2 and M_{N-1} come from other lanes' chunks
-  if (lane == 0) {
+  __syncthreads();  // M_2 and M_{N-1} come from other lanes' chunks
+  if (threadIdx.x == 0) {
     Mr[1] = m1;
     Mr[N] = mn;
     Mr[0] = 2.0 * m1 - Mr[2];
@@ -279,7 +387,11 @@ cudaError_t ensure_sl_scratch(vg_plan& p) {
 
 cudaError_t launch_vdfdx_sl_f64(const vg_plan& p, const double* fin, double* fout, double dt, cudaStream_t s) {
   // one-warp CTAs (each column's chain is bound by its warp's FP64 issue, not by the CTA shape)
-  k_sl_solve_x<<<div_up(p.nv, 32), 32, 0, s>>>(fin, p.sl_m, p.nx, p.nv, p.x, p.sl_w);
+  // split while its warps are no more than two a scheduler (152 x 8)
+  if (p.nx >= 4 * SL_X_SPLIT && div_up(p.nv, 32) * SL_X_SPLIT <= 1216)
+    k_sl_solve_x_split<<<div_up(p.nv, 32), 32 * SL_X_SPLIT, 0, s>>>(fin, p.sl_m, p.nx, p.nv, p.x, p.sl_w);
+  else
+    k_sl_solve_x<<<div_up(p.nv, 32), 32, 0, s>>>(fin, p.sl_m, p.nx, p.nv, p.x, p.sl_w);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
   k_sl_eval<true><<<cell_blocks((size_t)p.nx * p.nv), 256, 0, s>>>(fin, fout, p.sl_m, p.nx, p.nv, p.x, p.v,
@@ -289,7 +401,10 @@ cudaError_t launch_vdfdx_sl_f64(const vg_plan& p, const double* fin, double* fou
 
 cudaError_t launch_edfdv_sl_f64(const vg_plan& p, const double* fin, const double* e, double* fout, double dt,
                                 cudaStream_t s) {
-  k_sl_solve_v<<<div_up(p.nx, 4), 128, 0, s>>>(fin, p.sl_m, p.nx, p.nv, p.v, p.sl_w);  // a warp per row
+  // warps per row: at least four unknowns a lane (the scan costs some five)
+  if (p.nv >= 512) k_sl_solve_v<4><<<p.nx, 128, 0, s>>>(fin, p.sl_m, p.nx, p.nv, p.v, p.sl_w);
+  else if (p.nv >= 256) k_sl_solve_v<2><<<p.nx, 64, 0, s>>>(fin, p.sl_m, p.nx, p.nv, p.v, p.sl_w);
+  else k_sl_solve_v<1><<<p.nx, 32, 0, s>>>(fin, p.sl_m, p.nx, p.nv, p.v, p.sl_w);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
   k_sl_eval<false><<<cell_blocks((size_t)p.nx * p.nv), 256, 0, s>>>(fin, fout, p.sl_m, p.nx, p.nv, p.x, p.v,
