@@ -90,6 +90,28 @@ std::vector<int> pairwise_table(int n) {
   out.push_back((int)prog.size());
   out.insert(out.end(), leaves.begin(), leaves.end());
   out.insert(out.end(), prog.begin(), prog.end());
+  // the additions by height in the tree, each of leaf slot `src` into slot `dst`:
+  // [levels, (count, (dst, src) per addition) per level]
+  std::vector<std::pair<int, int>> stack;  // (slot, height)
+  std::vector<std::vector<int>> levels;
+  for (int op : prog) {
+    if (op >= 0) {
+      stack.push_back({op, 0});
+      continue;
+    }
+    const std::pair<int, int> r = stack.back();
+    stack.pop_back();
+    const int h = std::max(stack.back().second, r.second);
+    if ((int)levels.size() <= h) levels.resize(h + 1);
+    levels[h].push_back(stack.back().first);
+    levels[h].push_back(r.first);
+    stack.back().second = h + 1;
+  }
+  out.push_back((int)levels.size());
+  for (const std::vector<int>& l : levels) {
+    out.push_back((int)l.size() / 2);
+    out.insert(out.end(), l.begin(), l.end());
+  }
   return out;
 }
 
@@ -694,6 +716,7 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
   }
   std::vector<int> tv = pairwise_table(d->nv - 1), tx = pairwise_table(d->nx);
   p->pw_v_leaves = tv[0];
+  p->pw_v_levels = 1;
   p->pw_x_leaves = tx[0];
   p->pw_v_words = (int)tv.size();
   p->pw_x_words = (int)tx.size();

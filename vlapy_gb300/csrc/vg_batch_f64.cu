@@ -189,6 +189,7 @@ vg_plan class_view(const vg_batch* b, const vg_batch::Cls& c) {
   v.v_pow = c.v_pow;
   v.pw_v = c.pw_v;
   v.pw_v_leaves = c.pw_v_leaves;
+  v.pw_v_levels = 1;
   v.tw64 = b->tw64;
   v.tw32 = b->tw32;
   v.tw_fx = b->fx_tables->tw;

@@ -14,7 +14,8 @@
 // transposed, tap-flipped weights for the data gradient (ReLU mask fused) and
 // a third one, reducing over positions, for the weight gradients.  Weights
 // are kept in FP32 (Adam state too) and copied to BF16 for the GEMMs.
-// Activations are channels-last BF16 [row][128][C].
+// Activations are BF16, channels-last [row][128][C] or, the 64-channel ones of
+// the tcgen05 engine, by channel groups [row][8][128][8].
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -1160,10 +1161,9 @@ __global__ void k_pack_tc(const float* __restrict__ w, __nv_bfloat16* __restrict
 //
 // The weight gradients reduce over positions:
 // dW[o][c][t] = sum_rows sum_p dy[p][o] x[p + t - 2][c].  k_wgrad_tc makes
-// the position the MMA's K and keeps both operands in the MN-major layout,
-// which is the channels-last tile itself: 8 channels in 16 bytes, one
-// position per 16-byte row, so a tap shift along K is again the descriptor
-// moved by 16 t bytes.  M = 128 stacks copies of the input tile, copy q
+// the position the MMA's K and keeps both operands in the MN-major layout: 8
+// channels in 16 bytes, one position per 16-byte row, so a tap shift along K
+// is again the descriptor moved by 16 t bytes.  M = 128 stacks copies of the input tile, copy q
 // shifted by q rows, so that one MMA covers taps (g NCOPY + q); N is the
 // output channels of dy.  Each CTA accumulates a chunk of rows in TMEM and
 // writes its partial sums; k_wgrad_reduce adds the chunks in a fixed order.
@@ -1181,8 +1181,8 @@ __device__ __forceinline__ uint64_t tc_desc_mn(uint32_t addr, uint32_t mn_stride
 constexpr int TRN_SLOTS = 4;
 constexpr int TRN_THREADS = 128 * TRN_SLOTS;
 
-// 16-byte global -> shared copies that complete asynchronously (L2 only):
-// the next row's tiles load while the current row's MMAs run
+// 16-byte global -> shared copies that complete asynchronously (L2 only), for
+// the 16-channel layers' rows
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
                "l"(src)
@@ -1613,7 +1613,8 @@ struct vg_corrector {
   // BF16 GEMM operands
   __nv_bfloat16 *w1f, *w2f, *w3f, *w4f;  // fwd [5][rows][cin]
   __nv_bfloat16 *w2b, *w3b, *w4b;        // bwd [5][cin][cols]
-  // activations and gradients, channels-last [rows][128][C]
+  // activations and gradients: engine 0 has the 64-channel ones by channel groups
+  // ([rows][8][128][8]), the rest lie channels-last [rows][128][C]
   __nv_bfloat16 *x0, *a1, *a2, *a3, *dy4, *d3, *d2, *d1;
   float *pred, *scale, *part, *bpart, *loss_part;
   float2 *gmean, *tmean, *pmean;  // group means [groups][128] as double-float pairs

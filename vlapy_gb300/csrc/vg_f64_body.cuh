@@ -1,8 +1,8 @@
 // FP64 device bodies shared by the single-run kernels (vg_reduce_f64.cu,
-// vg_advect_f64.cu) and the batched FP64 sweep (vg_sweep_f64.cu): NumPy's
-// pairwise summation, the driver pulses, the spectral Poisson solve of one
-// run, the Thomas solve of one row and the x-drift of one column tile.  A run
-// of the batch goes through the same code as a single run.
+// vg_advect_f64.cu, vg_thomas_f64.cu) and the batched step (vg_batch_f64.cu):
+// NumPy's pairwise summation, the driver pulses, the spectral Poisson solve of
+// one run, the Thomas solve of one row and the x-drift of one column tile in
+// doubles.
 #pragma once
 
 #include "vg_internal.cuh"

@@ -50,6 +50,7 @@ struct vg_plan {
   int* pw_v;   // NumPy pairwise tree over nv-1 trapz terms
   int* pw_x;   // NumPy pairwise tree over nx values (x-means)
   int pw_v_leaves, pw_x_leaves, pw_v_words, pw_x_words;
+  int pw_v_levels;  // pw_v ends with the additions by height (pairwise_table)
   // scratch
   double* dens;   // [nx]
   double* mom;    // [nx][MOM_STRIDE]

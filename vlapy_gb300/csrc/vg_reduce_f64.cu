@@ -109,7 +109,7 @@ __global__ void k_row_moments_f64(const double* __restrict__ f, int nv, const do
 // factor of two commutes with every rounding above the subnormal range).
 // p: nv products in shared memory, or the row itself in global memory.
 __device__ __forceinline__ double trapz_exact(const double* p, int nv, double dv, const int* __restrict__ table,
-                                              double* term, double* leaf, double* result) {
+                                              int by_level, double* term, double* leaf, double* result) {
   for (int j = threadIdx.x; j < nv - 1; j += blockDim.x) term[j] = mul_rn(dv, add_rn(p[j + 1], p[j]));
   __syncthreads();
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -142,8 +142,26 @@ __device__ __forceinline__ double trapz_exact(const double* p, int nv, double dv
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const int* prog = leaves + 2 * nl;
+  const int* prog = leaves + 2 * nl;
+  if (by_level) {
+    // the tree's additions level by level, side by side (one thread running the
+    // program waited some 10,000 cycles for 31 leaves: density 77 -> 66 us, DG moments
+    // 261 -> 234 us at 2048 x 4096)
+    if (w == 0) {
+      const int* lv = prog + np;
+      const int levels = *lv++;
+      for (int l = 0; l < levels; ++l) {
+        const int n = *lv++;
+        for (int i = lane; i < n; i += 32) {
+          const int dst = lv[2 * i], src = lv[2 * i + 1];
+          leaf[dst] = add_rn(leaf[dst], leaf[src]);
+        }
+        lv += 2 * n;
+        __syncwarp();
+      }
+      if (lane == 0) *result = nv > 1 ? leaf[0] * 0.5 : 0.0;
+    }
+  } else if (threadIdx.x == 0) {
     int sp = 0;
     for (int i = 0; i < np; ++i) {
       const int op = prog[i];
@@ -169,7 +187,7 @@ __device__ __forceinline__ double trapz_exact(const double* p, int nv, double dv
 template <int OP>
 __global__ void __launch_bounds__(256) k_trapz_f64(const double* __restrict__ f, int nv, const double* __restrict__ v,
                                                    const double* __restrict__ v2, const int* __restrict__ table,
-                                                   double dv, double* __restrict__ out, int stride) {
+                                                   int by_level, double dv, double* __restrict__ out, int stride) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double res[2];
   double* term = reinterpret_cast<double*>(smem_raw);  // [nv]
@@ -178,23 +196,23 @@ __global__ void __launch_bounds__(256) k_trapz_f64(const double* __restrict__ f,
   const double* fr = f + (size_t)blockIdx.x * nv;
   double* o = out + (size_t)blockIdx.x * stride;
   if constexpr (OP == TRAPZ_DENSITY) {
-    const double n = trapz_exact(fr, nv, dv, table, term, leaf, &res[0]);
+    const double n = trapz_exact(fr, nv, dv, table, by_level, term, leaf, &res[0]);
     if (threadIdx.x == 0) o[0] = n;
   } else if constexpr (OP == TRAPZ_LB) {
     for (int j = threadIdx.x; j < nv; j += blockDim.x) prod[j] = mul_rn(fr[j], v2[j]);
     __syncthreads();
-    const double t = trapz_exact(prod, nv, dv, table, term, leaf, &res[0]);
+    const double t = trapz_exact(prod, nv, dv, table, by_level, term, leaf, &res[0]);
     if (threadIdx.x == 0) o[1] = t;
   } else {
     for (int j = threadIdx.x; j < nv; j += blockDim.x) prod[j] = mul_rn(fr[j], v[j]);
     __syncthreads();
-    const double vbar = trapz_exact(prod, nv, dv, table, term, leaf, &res[0]);
+    const double vbar = trapz_exact(prod, nv, dv, table, by_level, term, leaf, &res[0]);
     for (int j = threadIdx.x; j < nv; j += blockDim.x) {
       const double d = sub_rn(v[j], vbar);
       prod[j] = mul_rn(fr[j], mul_rn(d, d));
     }
     __syncthreads();
-    const double t = trapz_exact(prod, nv, dv, table, term, leaf, &res[1]);
+    const double t = trapz_exact(prod, nv, dv, table, by_level, term, leaf, &res[1]);
     if (threadIdx.x == 0) {
       o[0] = vbar;
       o[1] = t;
@@ -219,11 +237,11 @@ cudaError_t launch_trapz_f64(const vg_plan& p, int op, const double* f, double* 
   if (err != cudaSuccess) return err;
   const int block = p.nv >= 1024 ? 256 : p.nv >= 512 ? 128 : 64;
   if (op == TRAPZ_DENSITY)
-    k_trapz_f64<TRAPZ_DENSITY><<<p.nx, block, smem, s>>>(f, p.nv, p.v, p.v_pow, p.pw_v, p.dv, out, stride);
+    k_trapz_f64<TRAPZ_DENSITY><<<p.nx, block, smem, s>>>(f, p.nv, p.v, p.v_pow, p.pw_v, p.pw_v_levels, p.dv, out, stride);
   else if (op == TRAPZ_DG)
-    k_trapz_f64<TRAPZ_DG><<<p.nx, block, smem, s>>>(f, p.nv, p.v, p.v_pow, p.pw_v, p.dv, out, stride);
+    k_trapz_f64<TRAPZ_DG><<<p.nx, block, smem, s>>>(f, p.nv, p.v, p.v_pow, p.pw_v, p.pw_v_levels, p.dv, out, stride);
   else
-    k_trapz_f64<TRAPZ_LB><<<p.nx, block, smem, s>>>(f, p.nv, p.v, p.v_pow, p.pw_v, p.dv, out, stride);
+    k_trapz_f64<TRAPZ_LB><<<p.nx, block, smem, s>>>(f, p.nv, p.v, p.v_pow, p.pw_v, p.pw_v_levels, p.dv, out, stride);
   return cudaGetLastError();
 }
 
@@ -393,12 +411,13 @@ __global__ void __launch_bounds__(256) k_fields_series_f64(const double* __restr
 }
 
 // stored_f[i][slot][v] = complex64(sum_x f[x][v] exp(-2 pi i m x / nx)).  A CTA
-// takes 32 columns; its eight warps take every eighth row and the partial sums
-// are added in warp order.  MODES_AT_ONCE modes share one pass over f (their
+// takes 32 columns; its sixteen warps take every sixteenth row, eight loads in
+// flight, and the partial sums are added in warp order.  MODES_AT_ONCE modes share one pass over f (their
 // cosines and sines come from a table of the nx angles in shared memory, or, for
 // long columns, straight from the plan's table or sincospi).  One thread per
 // column had run 32 CTAs of serial loops: 2.01 ms at 2048 x 4096 with two modes,
-// now bound by the three FP64 operations per cell.
+// 136 us with eight warps and four loads, now 60 (the three FP64 operations a
+// cell take 47).
 constexpr int MODES_AT_ONCE = 2;
 constexpr int MODES_TABLE_NX = 4096;
 __device__ __forceinline__ cx<double> mode_angle(int q, int nx, int nx_pow2, const cx<double>* __restrict__ tw) {
@@ -414,11 +433,12 @@ __device__ __forceinline__ cx<double> mode_angle(int q, int nx, int nx_pow2, con
   sincospi(2.0 * (double)q / (double)nx, &sn, &cs);
   return {cs, -sn};
 }
-__global__ void __launch_bounds__(256) k_store_modes_f64(const double* __restrict__ f, int nx, int nv, int n_modes,
+constexpr int MODES_WARPS = 16;
+__global__ void __launch_bounds__(32 * MODES_WARPS) k_store_modes_f64(const double* __restrict__ f, int nx, int nv, int n_modes,
                                                          int n_slots, int nx_pow2, const cx<double>* __restrict__ tw,
                                                          int i, cx<float>* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double part[2 * MODES_AT_ONCE][8][32];
+  __shared__ double part[2 * MODES_AT_ONCE][MODES_WARPS][32];
   cx<double>* angles = reinterpret_cast<cx<double>*>(smem_raw);
   const bool table = nx <= MODES_TABLE_NX && n_modes > 1;
   if (table)
@@ -435,12 +455,10 @@ __global__ void __launch_bounds__(256) k_store_modes_f64(const double* __restric
     for (int u = 0; u < MODES_AT_ONCE; ++u) {
       zr[u] = zi[u] = 0.0;
       at[u] = (int)(((long long)(m0 + u) * w) % nx);
-      step[u] = (int)(((long long)(m0 + u) * 8) % nx);
+      step[u] = (int)(((long long)(m0 + u) * MODES_WARPS) % nx);
     }
     if (j < nv) {
-#pragma unroll 4
-      for (int x = w; x < nx; x += 8) {
-        const double fv = f[(size_t)x * nv + j];
+      auto add = [&](double fv) {
 #pragma unroll
         for (int u = 0; u < MODES_AT_ONCE; ++u) {
           if (m0 + u >= nm) continue;
@@ -454,7 +472,16 @@ __global__ void __launch_bounds__(256) k_store_modes_f64(const double* __restric
           at[u] += step[u];
           if (at[u] >= nx) at[u] -= nx;
         }
+      };
+      int x = w;
+      for (; x + 7 * MODES_WARPS < nx; x += 8 * MODES_WARPS) {
+        double fv[8];  // eight loads in flight
+#pragma unroll
+        for (int u = 0; u < 8; ++u) fv[u] = f[(size_t)(x + u * MODES_WARPS) * nv + j];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) add(fv[u]);
       }
+      for (; x < nx; x += MODES_WARPS) add(f[(size_t)x * nv + j]);
     }
 #pragma unroll
     for (int u = 0; u < MODES_AT_ONCE; ++u) {
@@ -464,7 +491,7 @@ __global__ void __launch_bounds__(256) k_store_modes_f64(const double* __restric
     __syncthreads();
     if (w < 2 * MODES_AT_ONCE && m0 + w / 2 < nm && j < nv) {
       double z = part[w][0][lane];
-      for (int q = 1; q < 8; ++q) z += part[w][q][lane];
+      for (int q = 1; q < MODES_WARPS; ++q) z += part[w][q][lane];
       const float zf = __double2float_rn(z);
       const int m = m0 + w / 2;
       for (int sl = n_modes == 1 ? 0 : m; sl < (n_modes == 1 ? n_slots : m + 1); ++sl)
@@ -506,7 +533,7 @@ cudaError_t launch_storage_f64(const vg_plan& p, const double* f, const double* 
       const size_t tab = p.nx <= MODES_TABLE_NX && h.n_modes > 1 ? (size_t)p.nx * sizeof(cx<double>) : 0;
       err = ensure_smem((const void*)k_store_modes_f64, tab);
       if (err != cudaSuccess) return err;
-      k_store_modes_f64<<<div_up(p.nv, 32), 256, tab, s>>>(f, p.nx, p.nv, h.n_modes, h.n_slots,
+      k_store_modes_f64<<<div_up(p.nv, 32), 32 * MODES_WARPS, tab, s>>>(f, p.nx, p.nv, h.n_modes, h.n_slots,
                                                            p.nx_pow2 && p.nx <= FFT_NMAX, p.tw64, i,
                                                            static_cast<cx<float>*>(h.stored_f));
       err = cudaGetLastError();
