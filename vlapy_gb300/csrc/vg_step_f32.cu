@@ -358,10 +358,14 @@ template <int N, bool KICK>
 cudaError_t row_nk(const vg_plan& p, RowArgs a, cudaStream_t s) {
   constexpr int R = row32_radix(N);
   constexpr int G = N / R;
-  const int block = row32_block(N, R);
-  const int P = block / G;
   const int npairs = (p.nx + 1) / 2;
-  const int ngroups = (npairs + P - 1) / P;
+  // Row-pair groups per CTA: fewer where the pairs do not give every SM a CTA (whole
+  // warps).  A CTA's groups share its barriers and take turns at the modes: two groups a
+  // CTA, 16 CTAs, 33 us a step of a driven 64 x 1024 run; one, 32 CTAs, 30.
+  int P = row32_block(N, R) / G;
+  while (P > 1 && (P / 2) * G >= 32 && div_up(npairs, P) < p.f32->n_sm) P /= 2;
+  const int block = P * G;
+  const int ngroups = div_up(npairs, P);
   const size_t mode_bytes = (size_t)(a.want_mom ? a.n_modes : 0) * N * sizeof(cx<float>);
   a.macc_global = (size_t)P * row32_group_bytes(N, R) + mode_bytes > ((size_t)100 << 10) ? 1 : 0;
   const size_t smem = (size_t)P * row32_group_bytes(N, R) + (a.macc_global ? 0 : mode_bytes);
