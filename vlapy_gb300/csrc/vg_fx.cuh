@@ -564,8 +564,8 @@ struct FxLine {
   bool on, bad;
 };
 // The pair in doubles, for the lines that fx_shift_back turns away.  Each line is
-// brought to order one by its own power of two (exact), so that neither takes the
-// other's rounding.  Out of line: it must not take registers from the
+// brought to order one (below it, if subnormal) by its own power of two (exact), so
+// that neither takes the other's rounding.  Out of line: it must not take registers from the
 // fixed-point path.
 template <int N, typename Sync>
 __device__ __noinline__ void fx_pair_f64(FxLine a, FxLine b, long long es, cx<double>* s, int t,
@@ -573,7 +573,9 @@ __device__ __noinline__ void fx_pair_f64(FxLine a, FxLine b, long long es, cx<do
                                          Sync sync) {
   constexpr int R = fx_radix(N), G = fx_threads(N);
   const bool use_a = a.on && !a.bad, use_b = b.on && !b.bad;
-  const double da = ldexp(1.0, 1023 - a.E), db = ldexp(1.0, 1023 - b.E);
+  // (a line of subnormal values has E < 0: 2^1023 is the largest factor there is)
+  const int sa = a.E > 0 ? 1023 - a.E : 1023, sb = b.E > 0 ? 1023 - b.E : 1023;
+  const double da = ldexp(1.0, sa), db = ldexp(1.0, sb);
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const long long n = (long long)(t + i * G) * es;
@@ -588,7 +590,7 @@ __device__ __noinline__ void fx_pair_f64(FxLine a, FxLine b, long long es, cx<do
   });
   sync();
   block_fft<double, N, true, R>(s, t, tw, sync);
-  const double sc = 1.0 / N, ua = ldexp(1.0, a.E - 1023), ub = ldexp(1.0, b.E - 1023);
+  const double sc = 1.0 / N, ua = ldexp(1.0, -sa), ub = ldexp(1.0, -sb);
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
 #pragma unroll
   for (int i = 0; i < R; ++i) {
