@@ -106,7 +106,7 @@ __device__ __forceinline__ bool pulse_amplitude(const vg_pulse& q, double t, dou
 // spent 31 us at nx = 64 with one pulse; with the density launch that this kernel
 // takes over 35, now 9).
 constexpr int FIELD32_WIDE_NX = 1024;
-constexpr int FIELD32_PULSES = 32;  // pulses whose envelopes are held at a time
+constexpr int FIELD32_PULSES = 32;  // pulses whose envelopes are held at a time, one a lane
 __host__ __device__ constexpr int field32_block(int nx) {
   return nx <= FIELD32_WIDE_NX ? 256 : fft_threads<float>(nx);
 }
@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(field32_block(NX)) k_field_f32(
   constexpr int B = field32_block(NX);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double amp[FIELD32_PULSES];
+  __shared__ unsigned sounding;  // bit i: pulse i adds to the field (a NaN amplitude does)
   cx<float>* s = reinterpret_cast<cx<float>*>(smem_raw);
   float* drv = reinterpret_cast<float*>(s + sp_len<float>(NX));  // [NX]
   const int t = threadIdx.x;
@@ -135,17 +136,20 @@ __global__ void __launch_bounds__(field32_block(NX)) k_field_f32(
   if (pulses)
     for (int p0 = 0; p0 < np; p0 += FIELD32_PULSES) {
       const int n_here = min(FIELD32_PULSES, np - p0);
-      // (a silent pulse: its amplitude is NaN here and it adds nothing)
-      if (t >= B - 32 && t - (B - 32) < n_here) {
-        double a;
-        amp[t - (B - 32)] = pulse_amplitude(P[p0 + t - (B - 32)], tt, &a) ? a : __longlong_as_double(0x7ff8000000000000ll);
+      if (t >= B - 32) {
+        const int i = t - (B - 32);
+        double a = 0.0;
+        const bool on = i < n_here && pulse_amplitude(P[p0 + i], tt, &a);
+        amp[i] = a;
+        const unsigned mask = __ballot_sync(0xffffffffu, on);
+        if (i == 0) sounding = mask;
       }
       __syncthreads();
       for (int n = t; n < NX; n += B) {
         float total = drv[n];
         for (int i = 0; i < n_here; ++i) {
+          if (!(sounding >> i & 1)) continue;  // a silent pulse adds nothing
           const double a = amp[i];
-          if (isnan(a)) continue;
           const vg_pulse& q = P[p0 + i];
           double arg = q.k0 * x[n] - q.w0 * tt;
           arg -= 6.283185307179586 * rint(arg * 0.15915494309189535);
