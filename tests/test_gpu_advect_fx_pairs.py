@@ -60,3 +60,37 @@ def test_subnormal_columns_beside_a_spike(nx, tiny):
     got = g.cpu().numpy()
     for c in range(nv):
         _within(got[:, c:c + 1], ref[:, c:c + 1], bound[c:c + 1], 0)
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-6, 1e6, 1e-307, 1e290])
+@pytest.mark.parametrize("n", [2048, 4096, 8192])
+def test_spike_beside_a_smooth_line(n, scale):
+    """A line in doubles beside one of far more of its maximum in its RMS: each errs by its own RMS only."""
+    p, x, v, kx, kv = plan(4, n)
+    f = np.zeros((4, n))
+    f[0] = scale * np.exp(-v ** 2 / 2.0)
+    f[3] = f[0]
+    f[1, n // 3] = f[2, n // 5] = 1.0
+    e = np.array([0.03, -0.05, 0.05, -0.02])
+    g = torch.as_tensor(f, device="cuda")
+    p.edfdv(g, torch.as_tensor(e, device="cuda"), 0.05)
+    ref, bound = advected(f, kv, e, 0.05, 1)
+    got = g.cpu().numpy()
+    for r in range(4):
+        _within(got[r:r + 1], ref[r:r + 1], bound[r:r + 1], 1)
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-6, 1e6, 1e-307, 1e290])
+@pytest.mark.parametrize("nx", [1024, 4096, 8192])
+def test_spiked_column_beside_a_smooth_one(nx, scale):
+    nv = 6
+    p, x, v, kx, kv = plan(nx, nv)
+    f = np.repeat(scale * (1.0 + 0.5 * np.cos(0.3 * x))[:, None], nv, axis=1)
+    f[:, 2:5] = 0.0
+    f[nx // 3, 2] = f[nx // 7, 4] = 1.0
+    g = torch.as_tensor(f, device="cuda")
+    p.vdfdx(g, 0.1)
+    ref, bound = advected(f, kx, v, 0.1, 0)
+    got = g.cpu().numpy()
+    for c in range(nv):
+        _within(got[:, c:c + 1], ref[:, c:c + 1], bound[c:c + 1], 0)

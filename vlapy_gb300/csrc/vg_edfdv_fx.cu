@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(fx_row_block(N), fx_row_block(N) > 256 ? 1 : 2
   const int h = fx_shift_back<N>(n, bad_a || Ea <= 1, bad_b || Eb <= 1);
   if (h < 0) {
     sync();
-    fx_pair_f64<N>({fa, ea, Ea, true, bad_a}, {fb, eb, Eb, vb, bad_b}, 1, reinterpret_cast<cx<double>*>(s), t, kv, dt,
+    fx_pair_f64<N>({fa, ea, fx_up(Ea, n.a2), true, bad_a}, {fb, eb, fx_up(Eb, n.b2), vb, bad_b}, 1, reinterpret_cast<cx<double>*>(s), t, kv, dt,
                    tw64, sync);
     return;
   }

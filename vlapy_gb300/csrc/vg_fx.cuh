@@ -478,7 +478,8 @@ __device__ __forceinline__ fxc fx_turn_by(fxc a, const fxw& w) {
 
 // What the rotation learns about the bins it leaves: an upper bound of the sum
 // of their moduli in units of 2^38, and the sums of the squares of line a's and
-// b's bins in units of 2^94, rounded down
+// b's bins in units of 2^88, rounded down (by Parseval's theorem a sum is the line's
+// mean square, below 2^31 units)
 struct FxNorms {
   unsigned l1, a2, b2;
 };
@@ -490,7 +491,7 @@ __device__ __forceinline__ unsigned fx_mod(fx z) {
   return max(x, y) + lo - (lo >> 1) - (lo >> 4);  // (1 - 1/2 - 1/16) lo
 }
 __device__ __forceinline__ unsigned fx_sq(long long a) {
-  const unsigned q = fx_abs_hi(a) >> 15;
+  const unsigned q = fx_abs_hi(a) >> 12;
   return q * q;
 }
 
@@ -548,34 +549,40 @@ __device__ __forceinline__ int fx_shift_back(const FxNorms& n, bool no_a, bool n
   int h = 0;
   while (h < 16 && (n.l1 >> h) >= lim) ++h;
   constexpr float dbl = 1e-16f * (1.f + 0.2f * ilog2(N));
-  // rms^2 = q 2^94 >= N (FX_NOISE 2^h / dbl)^2
-  const float need = FX_NOISE * (float)(1 << h) / (dbl * 140737488355328.f);  // 2^47
+  // rms^2 = q 2^88 >= N (FX_NOISE 2^h / dbl)^2
+  const float need = FX_NOISE * (float)(1 << h) / (dbl * 17592186044416.f);  // 2^44
   const float least = (float)N * need * need;
   if ((!no_a && (float)n.a2 < least) || (!no_b && (float)n.b2 < least)) return -1;
   return h;
 }
 
-// One line of a pair and its phase: elements f[n es], the scale E of its fixed
-// point, the double c of its phase ((-k) dt) c; bad: it comes out as NaN
+// One line of a pair and its phase: elements f[n es], the power of two that brings
+// it to an RMS of order one, the double c of its phase ((-k) dt) c; bad: it comes out
+// as NaN
 struct FxLine {
   double* f;
   double c;
-  int E;
+  int up;
   bool on, bad;
 };
+// that power of two for a line of scale E whose bins' squares add up to q (FxNorms).
+// It and its inverse are doubles: at most 2^1023 (a line of subnormal values has E < 0
+// and stays below order one), at least 2^-1023.
+__device__ __forceinline__ int fx_up(int E, unsigned q) {
+  return max(-1023, min(FX_SCALE - 44 - E - (32 - __clz((int)q)) / 2, 1023));
+}
 // The pair in doubles, for the lines that fx_shift_back turns away.  Each line is
-// brought to order one (below it, if subnormal) by its own power of two (exact), so
-// that neither takes the other's rounding.  Out of line: it must not take registers from the
-// fixed-point path.
+// brought to the same RMS by its own power of two (exact): what one of them rounds at
+// reaches the other, which must not take more than its own.  (Brought to the same
+// maximum, a spike beside a smooth line took five times the error it has alone at 2048.)
+// Out of line: it must not take registers from the fixed-point path.
 template <int N, typename Sync>
 __device__ __noinline__ void fx_pair_f64(FxLine a, FxLine b, long long es, cx<double>* s, int t,
                                          const double* __restrict__ kw, double dt, const cx<double>* __restrict__ tw,
                                          Sync sync) {
   constexpr int R = fx_radix(N), G = fx_threads(N);
   const bool use_a = a.on && !a.bad, use_b = b.on && !b.bad;
-  // (a line of subnormal values has E < 0: 2^1023 is the largest factor there is)
-  const int sa = a.E > 0 ? 1023 - a.E : 1023, sb = b.E > 0 ? 1023 - b.E : 1023;
-  const double da = ldexp(1.0, sa), db = ldexp(1.0, sb);
+  const double da = ldexp(1.0, a.up), db = ldexp(1.0, b.up);
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const long long n = (long long)(t + i * G) * es;
@@ -590,7 +597,7 @@ __device__ __noinline__ void fx_pair_f64(FxLine a, FxLine b, long long es, cx<do
   });
   sync();
   block_fft<double, N, true, R>(s, t, tw, sync);
-  const double sc = 1.0 / N, ua = ldexp(1.0, -sa), ub = ldexp(1.0, -sb);
+  const double sc = 1.0 / N, ua = ldexp(1.0, -a.up), ub = ldexp(1.0, -b.up);
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
 #pragma unroll
   for (int i = 0; i < R; ++i) {

@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(fx_col_block(NX), fx_col_block(NX) > 256 ? 1 :
   if (__syncthreads_or(h < 0)) {
     // a column the fixed-point transform is not exact enough for: the tile's pairs in doubles
     cx<double>* sd = reinterpret_cast<cx<double>*>(smem_raw) + (size_t)p * (sp_len<double>(NX) + COL_PAD);
-    fx_pair_f64<NX>({fc, ca, Ea, va, bad_a}, {fc + 1, cb, Eb, vb, bad_b}, nv, sd, t, r.kx, dt, tw64, sync);
+    fx_pair_f64<NX>({fc, ca, fx_up(Ea, n.a2), va, bad_a}, {fc + 1, cb, fx_up(Eb, n.b2), vb, bad_b}, nv, sd, t, r.kx, dt, tw64, sync);
     return;
   }
   fx_fft<NX, true, false, true>(s, t, tw, sync, io, h);
