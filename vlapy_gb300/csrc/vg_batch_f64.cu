@@ -121,10 +121,10 @@ struct vg_batch {
     int* pw_v;
   };
   std::vector<Cls> cls;
-  // nx classes: x-drift items and Poisson run lists
+  // classes of nx and transform: x-drift items and Poisson run lists
   struct XCls {
     int nx, W;
-    bool fx;  // every run's kx is uniform: the fixed-point x-drift
+    bool fx;  // the runs' kx are uniform: the fixed-point x-drift
     int2* items;
     int n_items;
     int n_ids;
@@ -471,33 +471,35 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
     tmp.tw32 = b->tw32;
     B_TRY(cuda_status(launch_twiddles(tmp, 0), "twiddles"));
   }
-  // x classes: (run, column tile) items of the x-drift and the Poisson run lists
-  std::map<int, std::pair<std::vector<int2>, std::vector<int>>> by_nx;
-  std::map<int, long long> pairs_of;  // column pairs of each nx class
-  std::map<int, bool> fx_of;
+  // x classes: (run, column tile) items of the x-drift and the Poisson run lists, by nx
+  // and by whether the run's kx is uniform, as a single run's choice of transform is
+  using XKey = std::pair<int, bool>;
+  std::map<XKey, std::pair<std::vector<int2>, std::vector<int>>> by_nx;
+  std::map<XKey, long long> pairs_of;  // column pairs of each class
+  std::vector<XKey> key_of(n_runs);
   std::vector<FxColRun> fx_runs(n_runs);
   for (int i = 0; i < n_runs; ++i) {
     const vg_run_desc& d = runs[i];
     fx_runs[i] = {rd[i].f_off, d.nv, rd[i].v, rd[i].kx, {}};
     const bool ok = fx_uniform(d.kx, d.nx) && fx_make_turn(d.kx[1], d.dt, &fx_runs[i].turn);
-    if (!fx_of.count(d.nx)) fx_of[d.nx] = true;
-    fx_of[d.nx] = fx_of[d.nx] && ok;
-    pairs_of[d.nx] += (d.nv + 1) / 2;
+    key_of[i] = XKey(d.nx, ok);
+    pairs_of[key_of[i]] += (d.nv + 1) / 2;
   }
   B_TRY(b_alloc(b, &b->fx_runs, fx_runs.size(), fx_runs.data(), "batch runs"));
-  auto tile_w = [&](int nx) { return 2 * (fx_of[nx] ? fx_col_pairs(nx, pairs_of[nx]) : col_seqs<double>(nx)); };
+  auto tile_w = [&](const XKey& k) {
+    return 2 * (k.second ? fx_col_pairs(k.first, pairs_of[k]) : col_seqs<double>(k.first));
+  };
   for (int i = 0; i < n_runs; ++i) {
-    const int nx = rd[i].nx;
-    const int W = tile_w(nx);
-    auto& e = by_nx[nx];
+    const int W = tile_w(key_of[i]);
+    auto& e = by_nx[key_of[i]];
     for (int t = 0; t * W < rd[i].nv; ++t) e.first.push_back(make_int2(i, t));
     e.second.push_back(i);
   }
   for (auto& kv : by_nx) {
     vg_batch::XCls xc;
-    xc.nx = kv.first;
+    xc.nx = kv.first.first;
     xc.W = tile_w(kv.first);
-    xc.fx = fx_of[kv.first];
+    xc.fx = kv.first.second;
     xc.n_items = (int)kv.second.first.size();
     xc.n_ids = (int)kv.second.second.size();
     B_TRY(b_alloc(b, &xc.items, kv.second.first.size(), kv.second.first.data(), "batch work list"));

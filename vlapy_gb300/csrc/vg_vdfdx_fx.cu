@@ -111,19 +111,16 @@ __global__ void __launch_bounds__(fx_col_block(NX), fx_col_block(NX) > 256 ? 1 :
   }
   // (E <= 1: a column of zeros, or of values that small)
   const int h = fx_shift_back<NX>(n, bad_a || Ea <= 1, bad_b || Eb <= 1);
-  if (__syncthreads_or(h < 0)) {
-    // a column the fixed-point transform is not exact enough for: the tile's pairs in doubles
-    cx<double>* sd = reinterpret_cast<cx<double>*>(smem_raw) + (size_t)p * (sp_len<double>(NX) + COL_PAD);
-    fx_pair_f64<NX>({fc, ca, fx_up(Ea, n.a2), va, bad_a}, {fc + 1, cb, fx_up(Eb, n.b2), vb, bad_b}, nv, sd, t, r.kx, dt, tw64, sync);
-    return;
-  }
-  fx_fft<NX, true, false, true>(s, t, tw, sync, io, h);
+  const bool turned = h < 0;  // a pair that fixed point is not exact enough for
+  const bool any_turned = __syncthreads_or(turned);
+  fx_fft<NX, true, false, true>(s, t, tw, sync, io, turned ? 16 : h);
   // lines of zeros stay so: the partner's rounding does not reach them
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
   const bool set_a = bad_a || zero_a, set_b = bad_b || zero_b;
   const double val_a = bad_a ? nan : 0.0, val_b = bad_b ? nan : 0.0;
 #pragma unroll
   for (int i = 0; i < R; ++i) {
+    if (turned) break;
     double* q = fc + (size_t)(t + i * G) * nv;
     const double xa = set_a ? val_a : fx_to_double(io[i].x, Ea - FX_SCALE + h);
     const double xb = set_b ? val_b : fx_to_double(io[i].y, Eb - FX_SCALE + h);
@@ -133,6 +130,15 @@ __global__ void __launch_bounds__(fx_col_block(NX), fx_col_block(NX) > 256 ? 1 :
       if (va) q[0] = xa;
       if (vb) q[1] = xb;
     }
+  }
+  if (any_turned) {
+    // Pair by pair: a column comes out the same whatever its tile holds (a batch and a
+    // single run have different tiles).  The tile's other pairs go along with nothing
+    // to load or store, for the barriers.
+    __syncthreads();
+    cx<double>* sd = reinterpret_cast<cx<double>*>(smem_raw) + (size_t)p * (sp_len<double>(NX) + COL_PAD);
+    fx_pair_f64<NX>({fc, ca, fx_up(Ea, n.a2), va && turned, bad_a}, {fc + 1, cb, fx_up(Eb, n.b2), vb && turned, bad_b}, nv,
+                    sd, t, r.kx, dt, tw64, sync);
   }
 }
 
