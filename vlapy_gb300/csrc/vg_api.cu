@@ -708,11 +708,7 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
     if (dx || dv)
       TRY(dev_copy<unsigned char>(p, reinterpret_cast<unsigned char**>(&p->dft_work), nullptr,
                                   dft_fx_scratch(d->nx, d->nv, dx, dv), "DFT scratch", true));
-    std::vector<int2> vp;
-    if (d->nv <= FX_MOMENTS_NV && fx_powers_host(d->v, d->v_pow, d->nv, &vp, &p->fx_pw)) {
-      TRY(dev_copy(p, &p->fx_vp, vp.data(), vp.size(), "velocity powers"));
-      p->fx_log = p->fx_tables->log;
-    }
+    p->fx_log = p->fx_tables->log;
   }
   std::vector<int> tv = pairwise_table(d->nv - 1), tx = pairwise_table(d->nx);
   p->pw_v_leaves = tv[0];
@@ -727,10 +723,15 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
   TRY(dev_copy<double>(p, &p->rho, nullptr, nx, "scratch"));
   TRY(dev_copy<double>(p, &p->etmp, nullptr, 4 * nx + 4, "scratch"));
   TRY(dev_copy<int>(p, &p->flags, nullptr, 1, "status"));
+  if (d->precision == VG_F64) TRY(cuda_status(static_cast<DevArena*>(p->arena)->flush(), "plan setup"));
+  if (d->precision == VG_F64 && d->nv <= FX_MOMENTS_NV && fx_powers_scale(d->v, d->v_pow, d->nv, &p->fx_pw)) {
+    unsigned char* mem = nullptr;
+    TRY(dev_copy<unsigned char>(p, &mem, nullptr, fx_powers_bytes(d->nv), "velocity powers", true));
+    TRY(cuda_status(build_fx_powers(p->v, p->v_pow, d->nv, mem, &p->fx_pw, 0), "velocity powers"));
+  }
   if (d->nx <= POISSON_FX_NX && d->precision == VG_F64) {
     TRY(dev_copy<int2>(p, &p->green, nullptr, nx, "Green's function"));
     TRY(dev_copy<int>(p, &p->green_e, nullptr, 1, "Green's function"));
-    TRY(cuda_status(static_cast<DevArena*>(p->arena)->flush(), "plan setup"));
     TRY(cuda_status(build_poisson_fx(p->inv_kx, d->nx, 1, p->green, p->green_e, p->etmp, 0), "Green's function"));
   }
   if (d->precision == VG_F64 && d->collision != VG_COLL_NONE)

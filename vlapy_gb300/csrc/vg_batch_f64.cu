@@ -116,7 +116,6 @@ struct vg_batch {
     int kv_uniform;
     double *v, *kv, *v_pow;
     fxw* dft_v;  // nv not a power of two: its angles
-    int2* fx_vp;  // null: the storage moments in doubles
     FxPowers fx_pw;
     int* pw_v;
   };
@@ -197,7 +196,6 @@ vg_plan class_view(const vg_batch* b, const vg_batch::Cls& c) {
   v.kv_uniform = c.kv_uniform;
   v.dft_v = c.dft_v;
   v.dft_work = b->dft_work;
-  v.fx_vp = c.fx_vp;
   v.fx_pw = c.fx_pw;
   v.fx_log = b->fx_tables->log;
   return v;
@@ -403,12 +401,14 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
       c.dv_sq = d.dv_sq;
       c.kv1 = d.kv[1];
       c.kv_uniform = fx_uniform(d.kv, d.nv);
-      std::vector<int2> vp;
-      if (d.nv <= FX_MOMENTS_NV && fx_powers_host(d.v, d.v_pow, d.nv, &vp, &c.fx_pw))
-        B_TRY(b_alloc(b, &c.fx_vp, vp.size(), vp.data(), "batch grids"));
       B_TRY(b_alloc(b, &c.v, d.nv, d.v, "batch grids"));
       B_TRY(b_alloc(b, &c.kv, d.nv, d.kv, "batch grids"));
       B_TRY(b_alloc(b, &c.v_pow, 5 * (size_t)d.nv, d.v_pow, "batch grids"));
+      if (d.nv <= FX_MOMENTS_NV && fx_powers_scale(d.v, d.v_pow, d.nv, &c.fx_pw)) {
+        unsigned char* mem = nullptr;
+        B_TRY(b_alloc<unsigned char>(b, &mem, fx_powers_bytes(d.nv), nullptr, "batch grids"));
+        B_TRY(cuda_status(build_fx_powers(c.v, c.v_pow, d.nv, mem, &c.fx_pw, 0), "batch grids"));
+      }
       const std::vector<int> tv = pairwise_table(d.nv - 1);
       c.pw_v_leaves = tv[0];
       B_TRY(b_alloc(b, &c.pw_v, tv.size(), tv.data(), "batch tables"));

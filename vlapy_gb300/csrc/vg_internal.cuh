@@ -40,8 +40,6 @@ struct vg_plan {
   vg::fxw* dft_x;
   void* dft_work;
   // fixed-point storage moments: the velocity powers and the logarithm's table
-  // (null: the moments in doubles)
-  int2* fx_vp;
   vg::FxPowers fx_pw;
   vg::FxLogEntry* fx_log;
   // Green's function of the Poisson solve (null: by transforms)

@@ -3,18 +3,26 @@
 //
 // In doubles these eight moments are some 60 FP64 instructions per cell (a log is
 // 30 of them), 64 cycles each and scheduler: 1.32 ms at 2048 x 4096 with the
-// memory system idle.  Here a row is scaled to 64-bit integers by its own power of
-// two (vg_fx.cuh), the velocity powers are Q62 fractions of their largest value,
-// every product is three wide multiplies and every sum is exact (96 bits), so that
-// only the products round, at 2^-60 of the row's maximum times the power's
-// (NumPy's pairwise sums round at 2^-53 of the partial sums).  The density that the Poisson solve takes and the
-// moments of the collision operator stay NumPy's own sums, bit for bit
-// (k_row_moments_f64).
+// memory system idle, here 0.16 (0.127 with one scale for a row and a power, see below;
+// a row close to one: 0.58).
+//
+// Precision.  A factor is its mantissa, brought to [2^61, 2^62), and its exponent, so
+// that a product (three wide multiplies) rounds at 2^-58 of itself; it is then shifted
+// to the scale of the largest product of its row and power, which a first pass over the
+// exponents finds, and added exactly (96 bits).  An error of a sum is therefore a few
+// times 2^-59 of its own largest term, whatever the shape of the row, where a product
+// of doubles rounds at 2^-53 of itself and NumPy's pairwise sums at 2^-53 of the
+// partial sums.  (With one scale for a row and one for a power, max f max|v|^p, the
+// fifth moment of a row of vth 0.3 on |v| < 6.4 was known to 1e-13 only.)  The values
+// are not NumPy's bit for bit; the density that the Poisson solve takes and the moments
+// of the collision operator are (k_trapz_f64).
 //
 // log f: f = m 2^e with 1 <= m < 2; c = one of 1024 16-bit reciprocals of m, so
 // that r = m c - 1 (exact in 64 bits) is below 2^-10.9, and log m = -log c + r -
 // r^2 (1/2 - r/3 + r^2/4), the rest below 2^-57 (a table-driven logarithm in the
-// manner of P. T. P. Tang, ACM Trans. Math. Softw. 16, 1990).
+// manner of P. T. P. Tang, ACM Trans. Math. Softw. 16, 1990).  It is good to some
+// 2^-56, so a row whose f is close to one (sum f |log f| below a quarter of sum f)
+// takes its entropy in doubles.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -41,18 +49,42 @@ __device__ __forceinline__ double sum_to_double(Sum96 s) {
   return fma((double)s.hi, 281474976710656.0, (double)s.lo);  // 2^48
 }
 
-// log f - (E - 1023) log 2 in Q56 for f > 0 of a row of scale E, f >= 2^-60 of the largest
-__device__ __forceinline__ long long log_q56(double f, int E, const FxLogEntry* __restrict__ table) {
-  unsigned long long u = (unsigned long long)__double_as_longlong(f);
-  int e = (int)(u >> 52);
+// A double as n 2^(e - 1084), |n| in [2^61, 2^62), or n = 0 with an exponent below all others
+struct FxNum {
+  long long n;
+  int e;
+};
+constexpr int FX_ZERO_E = -16384;
+__device__ __forceinline__ FxNum fx_num(double x) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+  int e = (int)((u >> 52) & 0x7ff);
   unsigned long long m = u & 0xfffffffffffffull;
-  if (e == 0) {  // subnormal: bring the leading one to the implicit place
-    const int z = __clzll((long long)m) - 11;
-    m = (m << z) & 0xfffffffffffffull;
+  if (e) {
+    m |= 1ull << 52;
+  } else {
+    if (m == 0) return {0, FX_ZERO_E};
+    const int z = __clzll((long long)m) - 11;  // subnormal
+    m <<= z;
     e = 1 - z;
   }
-  const FxLogEntry t = table[(unsigned)(m >> 42)];
-  m |= 1ull << 52;
+  const long long n = (long long)(m << 9);
+  return {(long long)u < 0 ? -n : n, e};
+}
+// the exponent alone
+__device__ __forceinline__ int fx_num_e(double x) {
+  const int e = (__double2hiint(x) >> 20) & 0x7ff;
+  return e ? e : fx_num(x).e;
+}
+// a / 2^k rounded, k >= 0
+__device__ __forceinline__ long long fx_shr(long long a, int k) {
+  k = min(k, 62);
+  return (a + ((1ll << k) >> 1)) >> k;
+}
+
+// log f - (e0 - 1023) log 2 in Q56 of f = num > 0
+__device__ __forceinline__ long long log_q56(FxNum num, int e0, const FxLogEntry* __restrict__ table) {
+  const unsigned long long m = (unsigned long long)num.n >> 9;  // 53 bits
+  const FxLogEntry t = table[(unsigned)(m >> 42) & 1023u];
   const long long r = (long long)(m * (unsigned long long)t.c);  // (m c - 1) 2^67 modulo 2^64
   const long long r6 = r << 6;                                   // Q73
   const int rh = fx_hi(r6), rl = fx_lo(r6);
@@ -60,41 +92,60 @@ __device__ __forceinline__ long long log_q56(double f, int E, const FxLogEntry* 
   const long long third = fx_rmul<0>(r6, fx_hi(1537228672809129301ll), fx_lo(1537228672809129301ll));  // r / 3, Q71
   const long long p = (1ll << 61) - (third >> 9) + (r2 >> 22);   // 1/2 - r/3 + r^2/4, Q62
   const long long q = fx_rmul<0>(r2, fx_hi(p), fx_lo(p));        // r^2 p, Q80
-  return t.l + (r >> 11) - (q >> 24) + (long long)(e - E) * 49946518145322874ll;  // log 2 in Q56
+  return t.l + (r >> 11) - (q >> 24) + (long long)(num.e - e0) * 49946518145322874ll;  // log 2 in Q56
 }
 
+constexpr double LN2 = 0.69314718055994530942;
+
 // One CTA per row.  FULL: slots n, j, v^2 .. v^5, f^2, f log f; else n, j, v^2, f^2, f log f.
+// v, v_pow: the powers as doubles, for rows that are not finite.
 template <bool FULL>
-__global__ void __launch_bounds__(256) k_moments_fx(const double* __restrict__ f, int nv, const int2* __restrict__ vp,
-                                                    FxPowers pw, const FxLogEntry* __restrict__ table, double dv,
+__global__ void __launch_bounds__(256) k_moments_fx(const double* __restrict__ f, int nv, FxPowers pw,
+                                                    const FxLogEntry* __restrict__ table, double dv,
+                                                    const double* __restrict__ v, const double* __restrict__ v_pow,
                                                     double* __restrict__ out, int stride) {
   constexpr int NP = FULL ? 6 : 3;       // velocity powers
   constexpr int NQ = NP + 2;
-  __shared__ unsigned smax[8], sbad[8];
+  __shared__ int smax[NP][8];
+  __shared__ unsigned sbad[8];
+  __shared__ float ssize[8];
   __shared__ Sum96 part[NQ][8];
+  __shared__ double red[8];
+  __shared__ int redo;
   const double* fr = f + (size_t)blockIdx.x * nv;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  // scale of the row; a value that is not above zero makes the entropy NaN, as log f does
-  unsigned mx = 0;
+  // the largest exponent of f and of its products with the powers; a value that is not
+  // above zero makes the entropy NaN, as log f does
+  int mx[NP];
+#pragma unroll
+  for (int p = 0; p < NP; ++p) mx[p] = 2 * FX_ZERO_E;
   bool low = false;
   for (int j = threadIdx.x; j < nv; j += blockDim.x) {
     const double x = fr[j];
-    mx = max(mx, fx_exp_bits(x));
+    const int e = fx_num_e(x);
     low = low || !(__double_as_longlong(x) > 0);
+    mx[0] = max(mx[0], e);
+    const int4 d = pw.drop[j];
+    const int dd[3] = {d.x, d.y, d.z};
+#pragma unroll
+    for (int p = 1; p < NP; ++p) mx[p] = max(mx[p], e - ((dd[(p - 1) / 2] >> (16 * ((p - 1) & 1))) & 0xffff));
   }
-  mx = __reduce_max_sync(0xffffffffu, mx);
   const unsigned anylow = __any_sync(0xffffffffu, low);
-  if (lane == 0) {
-    smax[w] = mx;
-    sbad[w] = anylow;
+#pragma unroll
+  for (int p = 0; p < NP; ++p) {
+    mx[p] = __reduce_max_sync(0xffffffffu, mx[p]);
+    if (lane == 0) smax[p][w] = mx[p];
   }
+  if (lane == 0) sbad[w] = anylow;
+  if (threadIdx.x == 0) redo = 0;
   __syncthreads();
   unsigned bad = 0;
   for (int q = 0; q < nw; ++q) {
-    mx = max(mx, smax[q]);
+#pragma unroll
+    for (int p = 0; p < NP; ++p) mx[p] = max(mx[p], smax[p][q]);
     bad |= sbad[q];
   }
-  const int E = fx_exp(mx);
+  const int E = mx[0];
   double* o = out + (size_t)blockIdx.x * stride;
   if (E == FX_NONFINITE) {
     // plain sums, for the infinities' and NaNs' sake: a thread per moment
@@ -104,7 +155,7 @@ __global__ void __launch_bounds__(256) k_moments_fx(const double* __restrict__ f
       for (int j = 0; j < nv; ++j) {
         const double x = fr[j];
         double t = x;
-        if (q >= 1 && q < NP) t = x * ldexp((double)(((long long)vp[(size_t)(q - 1) * nv + j].x << 32) + vp[(size_t)(q - 1) * nv + j].y), pw.e[q - 1] - 62);
+        if (q >= 1 && q < NP) t = x * (q == 1 ? v[j] : v_pow[(size_t)(q - 1) * nv + j]);
         else if (q == NP) t = x * x;
         else if (q == NP + 1) t = x * log(x);
         acc += (j == 0 || j == nv - 1) ? 0.5 * t : t;
@@ -113,54 +164,111 @@ __global__ void __launch_bounds__(256) k_moments_fx(const double* __restrict__ f
     }
     return;
   }
+  // logarithms against 2^(e0 - 1023): log f itself unless f is far from one.  All
+  // f |log| <= 2^(E + 1 - 1023) (0.7 |E - e0| + 1.07) <= 2^(E - 1022 + up)
+  const int far = abs(E - 1023) <= 40 ? abs(E - 1023) : 0, e0 = abs(E - 1023) <= 40 ? 1023 : E;
+  const int up = far == 0 ? 1 : far <= 1 ? 1 : far <= 4 ? 2 : far <= 9 ? 3 : far <= 21 ? 4 : 5;
   Acc96 s[NQ];
 #pragma unroll
   for (int q = 0; q < NQ; ++q) s[q] = {0, 0};
+  float size = 0.f;  // sum of f |log|, in units of 2^32 of its sum
   for (int j = threadIdx.x; j < nv; j += blockDim.x) {
-    const double x = fr[j];
-    const long long F = fx_from_double(x, E);
-    const long long lg = (bad || F == 0) ? 0 : log_q56(x, E, table);
+    const FxNum F = fx_num(fr[j]);
     const int half = (j == 0 || j == nv - 1) ? 1 : 0;  // the trapz weight of the ends
-    acc_add(s[0], (F << 3) >> half);
+    const int down = E - F.e;
+    acc_add(s[0], fx_shr(F.n, down + half));
+    const int4 d = pw.drop[j];
+    const int dd[3] = {d.x, d.y, d.z};
 #pragma unroll
     for (int p = 1; p < NP; ++p) {
-      const int2 c = vp[(size_t)(p - 1) * nv + j];
-      acc_add(s[p], fx_rmul<3>(F, c.x, c.y) >> half);
+      const int2 c = pw.mant[(size_t)(p - 1) * nv + j];
+      const int drop = (dd[(p - 1) / 2] >> (16 * ((p - 1) & 1))) & 0xffff;
+      acc_add(s[p], fx_shr(fx_rmul<0>(F.n, c.x, c.y), mx[p] - (F.e - drop) + half));
     }
-    acc_add(s[NP], fx_rmul<3>(F, fx_hi(F), fx_lo(F)) >> half);
-    acc_add(s[NP + 1], fx_rmul<3>(F, fx_hi(lg), fx_lo(lg)) >> half);
+    acc_add(s[NP], fx_shr(fx_rmul<0>(F.n, fx_hi(F.n), fx_lo(F.n)), 2 * down + half));
+    if (!bad && down <= 70) {
+      const long long lg = log_q56(F, e0, table);
+      const int z = __clzll(lg < 0 ? -lg : lg) - 2;  // (62: lg is zero)
+      const long long ln = z >= 0 ? lg << z : lg >> 1;
+      const long long t = fx_rmul<0>(F.n, fx_hi(ln), fx_lo(ln));  // at least 2^58
+      const int k = down + z - (8 - up) + half;                   // (-4 or more)
+      const long long u = fx_shr(t << max(-k, 0), max(k, 0));     // at most 2^62
+      acc_add(s[NP + 1], u);
+      size += fabsf((float)(int)(u >> 32));
+    }
   }
 #pragma unroll
   for (int q = 0; q < NQ; ++q) {
     const Sum96 t = warp_sum(s[q]);
     if (lane == 0) part[q][w] = t;
   }
+#pragma unroll
+  for (int m = 16; m > 0; m >>= 1) size += __shfl_xor_sync(0xffffffffu, size, m);
+  if (lane == 0) ssize[w] = size;
   __syncthreads();
-  if (threadIdx.x >= NQ) return;
-  const int q = threadIdx.x;
-  Sum96 t = part[q][0];
-  for (int k = 1; k < nw; ++k) {
-    t.hi += part[q][k].hi;
-    t.lo += part[q][k].lo;
-  }
-  const double sum = nv < 2 ? 0.0 : dv * sum_to_double(t);
-  // sums of 8 F, and of F V, F^2, F L over 2^61 (V in Q62 of 2^e, L in Q56)
-  double r;
-  if (q == 0) r = ldexp(sum, E - FX_SCALE - 3);
-  else if (q < NP) r = ldexp(sum, E - FX_SCALE - 1 + pw.e[q - 1]);
-  else if (q == NP) r = ldexp(ldexp(sum, E - FX_SCALE + 30), E - FX_SCALE + 31);
-  else {
-    Sum96 n = part[0][0];
+  if (threadIdx.x < NQ) {
+    const int q = threadIdx.x;
+    Sum96 t = part[q][0];
     for (int k = 1; k < nw; ++k) {
-      n.hi += part[0][k].hi;
-      n.lo += part[0][k].lo;
+      t.hi += part[q][k].hi;
+      t.lo += part[q][k].lo;
     }
-    const double nsum = dv * sum_to_double(n) * 0.125;
-    r = ldexp(fma(nsum, (double)(E - 1023) * 0.69314718055994530942, sum * 32.0), E - FX_SCALE);
-    if (nv < 2) r = 0.0;
-    else if (bad) r = __longlong_as_double(0x7ff8000000000000ll);
+    const double sum = nv < 2 ? 0.0 : dv * sum_to_double(t);
+    // f = F 2^(e - 1084), a product of two such numbers was divided by 2^64
+    double r;
+    if (q == 0) r = ldexp(sum, E - 1084);
+    else if (q < NP) r = ldexp(sum, mx[q] + pw.e[q - 1] - 2104);
+    else if (q == NP) r = ldexp(sum, 2 * E - 2104);
+    else {
+      // F times a logarithm in Q56, divided by 2^64, times 2^(8 - up)
+      r = ldexp(sum, E - 1084 + 64 - 56 - (8 - up));
+      Sum96 n = part[0][0];
+      for (int k = 1; k < nw; ++k) {
+        n.hi += part[0][k].hi;
+        n.lo += part[0][k].lo;
+      }
+      const double nsum = ldexp(dv * sum_to_double(n), E - 1084);
+      if (e0 != 1023) r = fma(nsum, (double)(e0 - 1023) * LN2, r);
+      if (nv < 2) r = 0.0;
+      else if (bad) r = __longlong_as_double(0x7ff8000000000000ll);
+      else if (e0 == 1023) {
+        // the sum of f |log f| against a quarter of f's
+        float a = 0.f;
+        for (int k = 0; k < nw; ++k) a += ssize[k];
+        redo = ldexp((double)a, 32 + 8 - (8 - up)) < 0.25 * fabs(sum_to_double(n));
+      }
+    }
+    o[q] = r;
   }
-  o[q] = r;
+  __syncthreads();
+  if (!redo) return;
+  // (logarithms near zero: the entropy in doubles)
+  double acc = 0.0;
+  for (int j = threadIdx.x; j < nv; j += blockDim.x) {
+    const double x = fr[j], t = x * log(x);
+    acc += (j == 0 || j == nv - 1) ? 0.5 * t : t;
+  }
+  for (int m = 16; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+  if (lane == 0) red[w] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < nw; ++k) acc += red[k];
+    o[NP + 1] = dv * acc;
+  }
+}
+
+// the powers' mantissas and by how much their exponents are below the largest
+__global__ void k_powers(const double* __restrict__ v, const double* __restrict__ v_pow, int nv, FxPowers pw, int4* drop,
+                         int2* mant) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= nv) return;
+  int d[6] = {};
+  for (int p = 0; p < 5; ++p) {
+    const FxNum a = fx_num(p == 0 ? v[j] : v_pow[(size_t)p * nv + j]);
+    mant[(size_t)p * nv + j] = make_int2(fx_hi(a.n), fx_lo(a.n));
+    d[p] = min(pw.e[p] - a.e, 0xffff);
+  }
+  drop[j] = make_int4(d[0] | d[1] << 16, d[2] | d[3] << 16, d[4], 0);
 }
 
 // log(c / 2^15) by the series of 2 atanh((c - 2^15) / (c + 2^15)) in double-double
@@ -208,36 +316,43 @@ const FxLogEntry* fx_log_host() {
   return table.data();
 }
 
-bool fx_powers_host(const double* v, const double* v_pow, int nv, std::vector<int2>* out, FxPowers* pw) {
-  out->assign(5 * (size_t)nv, make_int2(0, 0));
+bool fx_powers_scale(const double* v, const double* v_pow, int nv, FxPowers* pw) {
   // v, then v^2, v^3, v^4, v^5 as v_pow's rows 1 .. 4 hold them
   for (int p = 0; p < 5; ++p) {
     const double* a = p == 0 ? v : v_pow + (size_t)p * nv;
     double mx = 0.0;
+    bool finite = true;
     for (int j = 0; j < nv; ++j) {
-      if (!std::isfinite(a[j])) return false;
+      finite = finite && std::isfinite(a[j]);
       mx = std::max(mx, std::fabs(a[j]));
     }
+    if (!finite) return false;
     int e = 0;
     std::frexp(mx, &e);
     if (mx == 0.0) e = 0;
     if (e > 900 || e < -900) return false;
-    pw->e[p] = e;
-    const double up = std::ldexp(1.0, 62 - e);
-    for (int j = 0; j < nv; ++j) {
-      const long long q = (long long)std::llrint(a[j] * up);
-      (*out)[(size_t)p * nv + j] = make_int2(fx_hi(q), fx_lo(q));
-    }
+    pw->e[p] = e + 1022;  // the largest exponent field
   }
   return true;
 }
 
-cudaError_t launch_moments_fx(const double* f, int nrows, int nv, const int2* vp, const FxPowers& pw,
+size_t fx_powers_bytes(int nv) { return (size_t)nv * (sizeof(int4) + 5 * sizeof(int2)); }
+
+cudaError_t build_fx_powers(const double* v, const double* v_pow, int nv, void* mem, FxPowers* pw, cudaStream_t s) {
+  int4* drop = static_cast<int4*>(mem);
+  int2* mant = reinterpret_cast<int2*>(drop + nv);
+  pw->drop = drop;
+  pw->mant = mant;
+  k_powers<<<div_up(nv, 128), 128, 0, s>>>(v, v_pow, nv, *pw, drop, mant);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_moments_fx(const double* f, int nrows, int nv, const double* v, const double* v_pow, const FxPowers& pw,
                               const FxLogEntry* table, double dv, double* out, int stride, bool full, cudaStream_t s) {
   // four to eight elements a thread, whole warps
   const int block = nv >= 1024 ? 256 : nv >= 512 ? 128 : 64;
-  if (full) k_moments_fx<true><<<nrows, block, 0, s>>>(f, nv, vp, pw, table, dv, out, stride);
-  else k_moments_fx<false><<<nrows, block, 0, s>>>(f, nv, vp, pw, table, dv, out, stride);
+  if (full) k_moments_fx<true><<<nrows, block, 0, s>>>(f, nv, pw, table, dv, v, v_pow, out, stride);
+  else k_moments_fx<false><<<nrows, block, 0, s>>>(f, nv, pw, table, dv, v, v_pow, out, stride);
   return cudaGetLastError();
 }
 

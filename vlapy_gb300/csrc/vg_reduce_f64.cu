@@ -1,13 +1,15 @@
 // FP64 reductions, field solve and storage step.
 //
-// Every trapz over v and every mean over x is evaluated with NumPy's pairwise
-// summation tree (a table built at plan creation): leaves of <= 128 terms are
+// The density, the collision operators' moments and every mean over x are evaluated
+// with NumPy's pairwise summation tree (a table built at plan creation): leaves of <= 128 terms are
 // summed with eight interleaved accumulators (one thread per accumulator chain
 // in the row moments), and one thread per moment replays the post-order
 // combine program.  Products use
 // explicitly rounded intrinsics so nvcc cannot contract them into FMAs.  With
-// f equal, densities and moments are then bit-identical to the reference's
-// np.trapz (vlapy/core/field.py:36, vlapy/core/step.py:164-223).
+// f equal, they are then bit-identical to the reference's np.trapz and np.mean
+// (vlapy/core/field.py:36, vlapy/core/collisions.py, vlapy/core/step.py:174-229).
+// The moments that a step stores are nearer to the exact sums than np.trapz's, and
+// not its bits (vg_moments_fx.cu).
 #include "vg_internal.cuh"
 #include "vg_f64_body.cuh"
 
@@ -503,8 +505,8 @@ __global__ void __launch_bounds__(32 * MODES_WARPS) k_store_modes_f64(const doub
 
 cudaError_t launch_storage_moments_f64(const vg_plan& p, const double* f, double* out, int stride, bool full,
                                        cudaStream_t s) {
-  if (p.fx_vp && p.nv <= FX_MOMENTS_NV)
-    return launch_moments_fx(f, p.nx, p.nv, p.fx_vp, p.fx_pw, p.fx_log, p.dv, out, stride, full, s);
+  if (p.fx_pw.drop)
+    return launch_moments_fx(f, p.nx, p.nv, p.v, p.v_pow, p.fx_pw, p.fx_log, p.dv, out, stride, full, s);
   MomSpec spec;
   const int kinds[8] = {MOM_ONE, MOM_V, MOM_W, MOM_W, MOM_W, MOM_W, MOM_SQ, MOM_FLOGF};
   const int args[8] = {0, 0, 1, 2, 3, 4, 0, 0};

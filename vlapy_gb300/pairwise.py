@@ -5,9 +5,10 @@ vlapy/core/field.py:36) forms ``t_j = (dx * (y[j+1] + y[j])) / 2`` and sums the
 ``n = len(y) - 1`` terms with NumPy's pairwise reduction: blocks of at most
 128 terms are summed with eight interleaved accumulators, larger ranges are
 split at ``n/2`` rounded down to a multiple of 8 and the halves added.  The
-FP64 mode of the CUDA kernels evaluates the same tree so that densities and
-moments agree with the reference bit for bit when f does; with ``1 - n``
-cancelling in the Poisson solve, that is what keeps the field within 1e-12.
+FP64 mode of the CUDA kernels evaluates the same tree so that the density, the
+collision operators' moments and the means over x agree with the reference bit for
+bit when f does; with ``1 - n`` cancelling in the Poisson solve, that is what keeps
+the field within 1e-12.  (The stored moments are summed exactly instead.)
 
 ``leaf_program(n)`` returns the leaves (start, length) and a post-order
 program: an entry ``k >= 0`` pushes leaf k's sum, ``-1`` pops two values and
