@@ -2,6 +2,8 @@
 // vg_vdfdx_fx.cu; the arithmetic is in vg_fx.cuh).
 #pragma once
 
+#include <vector>
+
 #include "vg_fx.cuh"
 #include "vg_moments_fx.cuh"
 
@@ -18,12 +20,20 @@ struct FxTables {
 };
 cudaError_t fx_tables_acquire(FxTables** out);
 void fx_tables_release(FxTables* t);
+// the step k1 of a wavenumber grid k[m] = m k1, h + l
+struct FxStep {
+  double h, l;
+};
 // turns per index and unit field or velocity of the phase ((-k) dt) c with k =
 // m k1: A = -k1 dt / (2 pi) to 62 bits; false when it is not finite
-bool fx_make_turn(double k1, double dt, FxTurn* out);
-// true when k[m] is m k[1] to a few roundings for m <= n / 2 (fftfreq's grid):
-// the fixed-point phases step from index to index
-bool fx_uniform(const double* k, int n);
+bool fx_make_turn(FxStep k1, double dt, FxTurn* out);
+// true when k[m] is m k[1] to a few roundings for m <= n / 2 (fftfreq's grid): the
+// fixed-point phases step from index to index, by the grid's least-squares step
+// (k[1]'s own rounding, taken m times, would be an error of up to 2^-53 of every phase
+// beside those that the k[m] have)
+bool fx_uniform(const double* k, int n, FxStep* k1);
+// what is left of the wavenumbers k[0 .. n / 2] past the step, (k[m] - m k1) 2^64 / (2 pi)
+std::vector<float> fx_step_rest(const double* k, int n, FxStep k1);
 
 // v-advection of nrows rows of nv (a power of two <= 8192); kv, dt and tw64 for
 // the row pairs that go through doubles
@@ -46,12 +56,12 @@ cudaError_t launch_vdfdx_fx(double* f, int nx, const FxColRun* runs, const int2*
                             double dt, const fxw* tw, const cx<double>* tw64, cudaStream_t s);
 
 // Lines whose length N is not a power of two (vg_dft_fx.cu): n_lines lines of N
-// elements es apart, line l at l ls with the phase's double c[l]; angles: the N
-// angles' table; scratch: dft_fx_scratch bytes for the larger of the directions
+// elements es apart, line l at l ls with the phase ((-k) dt) c of its double c[l];
+// angles: the N angles' table; rest: fx_step_rest's; scratch: dft_fx_scratch bytes for the larger of the directions
 // a plan uses
 size_t dft_fx_scratch(int nx, int nv, bool x, bool v);
 cudaError_t build_dft_table(int N, const fxw* tw, fxw* out, cudaStream_t s);
 cudaError_t launch_dft_fx(double* f, int N, int n_lines, long long es, long long ls, const double* c, FxTurn turn,
-                          const fxw* tw, const fxw* angles, void* scratch, cudaStream_t s);
+                          const float* rest, double dt, const fxw* tw, const fxw* angles, void* scratch, cudaStream_t s);
 
 }  // namespace vg

@@ -692,18 +692,18 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
   if (d->precision == VG_F64) {
     TRY(cuda_status(fx_tables_acquire(&p->fx_tables), "fixed-point tables"));
     p->tw_fx = p->fx_tables->tw;
-    p->kv1 = d->kv[1];
-    p->kx1 = d->kx[1];
-    p->kv_uniform = fx_uniform(d->kv, d->nv);
-    p->kx_uniform = fx_uniform(d->kx, d->nx);
+    p->kv_uniform = fx_uniform(d->kv, d->nv, &p->kv1);
+    p->kx_uniform = fx_uniform(d->kx, d->nx, &p->kx1);
     const bool dx = !p->nx_pow2 && d->nx <= DFT_ADVECT_NMAX, dv = !p->nv_pow2 && d->nv <= DFT_ADVECT_NMAX;
     if (dv) {
       TRY(dev_copy<fxw>(p, &p->dft_v, nullptr, nv, "DFT angles"));
       TRY(cuda_status(build_dft_table(d->nv, p->tw_fx, p->dft_v, 0), "DFT angles"));
+      TRY(upload(p, &p->dft_rest_v, fx_step_rest(d->kv, d->nv, p->kv1), "DFT angles"));
     }
     if (dx) {
       TRY(dev_copy<fxw>(p, &p->dft_x, nullptr, nx, "DFT angles"));
       TRY(cuda_status(build_dft_table(d->nx, p->tw_fx, p->dft_x, 0), "DFT angles"));
+      TRY(upload(p, &p->dft_rest_x, fx_step_rest(d->kx, d->nx, p->kx1), "DFT angles"));
     }
     if (dx || dv)
       TRY(dev_copy<unsigned char>(p, reinterpret_cast<unsigned char**>(&p->dft_work), nullptr,

@@ -112,10 +112,12 @@ struct vg_batch {
     long long f_off;
     int x_off, rows;
     int pw_v_leaves;
-    double dv, dv_sq, kv1;
+    double dv, dv_sq;
+    FxStep kv1;
     int kv_uniform;
     double *v, *kv, *v_pow;
-    fxw* dft_v;  // nv not a power of two: its angles
+    fxw* dft_v;  // nv not a power of two: its angles, and what kv is off its step by
+    float* dft_rest_v;
     FxPowers fx_pw;
     int* pw_v;
   };
@@ -195,6 +197,7 @@ vg_plan class_view(const vg_batch* b, const vg_batch::Cls& c) {
   v.kv1 = c.kv1;
   v.kv_uniform = c.kv_uniform;
   v.dft_v = c.dft_v;
+  v.dft_rest_v = c.dft_rest_v;
   v.dft_work = b->dft_work;
   v.fx_pw = c.fx_pw;
   v.fx_log = b->fx_tables->log;
@@ -399,8 +402,11 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
       c.x_off = xoff;
       c.dv = d.dv;
       c.dv_sq = d.dv_sq;
-      c.kv1 = d.kv[1];
-      c.kv_uniform = fx_uniform(d.kv, d.nv);
+      c.kv_uniform = fx_uniform(d.kv, d.nv, &c.kv1);
+      if (!is_pow2(d.nv)) {
+        const std::vector<float> rest = fx_step_rest(d.kv, d.nv, c.kv1);
+        B_TRY(b_alloc(b, &c.dft_rest_v, rest.size(), rest.data(), "batch grids"));
+      }
       B_TRY(b_alloc(b, &c.v, d.nv, d.v, "batch grids"));
       B_TRY(b_alloc(b, &c.kv, d.nv, d.kv, "batch grids"));
       B_TRY(b_alloc(b, &c.v_pow, 5 * (size_t)d.nv, d.v_pow, "batch grids"));
@@ -481,7 +487,8 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
   for (int i = 0; i < n_runs; ++i) {
     const vg_run_desc& d = runs[i];
     fx_runs[i] = {rd[i].f_off, d.nv, rd[i].v, rd[i].kx, {}};
-    const bool ok = fx_uniform(d.kx, d.nx) && fx_make_turn(d.kx[1], d.dt, &fx_runs[i].turn);
+    FxStep k1;
+    const bool ok = fx_uniform(d.kx, d.nx, &k1) && fx_make_turn(k1, d.dt, &fx_runs[i].turn);
     key_of[i] = XKey(d.nx, ok);
     pairs_of[key_of[i]] += (d.nv + 1) / 2;
   }

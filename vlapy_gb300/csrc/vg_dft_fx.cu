@@ -65,6 +65,7 @@ struct __align__(16) Fold {
 // scale into scale[line])
 __global__ void __launch_bounds__(DFT_BLOCK) k_dft_fwd_fx(const double* __restrict__ f, int N, int n_lines, long long es,
                                                           long long ls, const double* __restrict__ c, FxTurn turn,
+                                                          const float* __restrict__ rest, float dt,
                                                           const fxw* __restrict__ tw, const fxw* __restrict__ angles,
                                                           fx* __restrict__ G, int* __restrict__ scale) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -151,7 +152,9 @@ __global__ void __launch_bounds__(DFT_BLOCK) k_dft_fwd_fx(const double* __restri
   for (int u = 0; u < DFT_LINES; ++u) {
     if (part != u || k >= K || l0 + u >= n_lines) continue;
     const double cl = bad[u] ? 0.0 : c[l0 + u];
-    const fxw p = fx_mult(fx_sincos((unsigned long long)k * fx_turn(turn, cl), tw));
+    // (the wavenumber's own rounding, some 2^-53 of the phase, in FP32)
+    const long long own = __float2ll_rn(-rest[k] * dt * (float)cl);
+    const fxw p = fx_mult(fx_sincos((unsigned long long)k * fx_turn(turn, cl) + (unsigned long long)own, tw));
     fx z = fx_cmul<0, false>({re[u], -im[u]}, p);
     // half weight for the bins that have no mirror image
     if (k == 0 || 2 * k == N) z = fx_down<1>(z);
@@ -261,7 +264,7 @@ cudaError_t build_dft_table(int N, const fxw* tw, fxw* out, cudaStream_t s) {
 }
 
 cudaError_t launch_dft_fx(double* f, int N, int n_lines, long long es, long long ls, const double* c, FxTurn turn,
-                          const fxw* tw, const fxw* angles, void* scratch, cudaStream_t s) {
+                          const float* rest, double dt, const fxw* tw, const fxw* angles, void* scratch, cudaStream_t s) {
   const int K = dft_bins(N);
   const size_t smem = (size_t)N * sizeof(fxw) + (size_t)DFT_LINES * K * sizeof(Fold);
   cudaError_t err = ensure_smem((const void*)k_dft_fwd_fx, smem);
@@ -275,7 +278,8 @@ cudaError_t launch_dft_fx(double* f, int N, int n_lines, long long es, long long
     const int n = std::min(n_lines - l0, 2 * 65535);
     const dim3 grid(tiles, div_up(n, DFT_LINES));
     double* fl = f + (long long)l0 * ls;
-    k_dft_fwd_fx<<<grid, DFT_BLOCK, smem, s>>>(fl, N, n, es, ls, c + l0, turn, tw, angles, G + (size_t)l0 * K, scale + l0);
+    k_dft_fwd_fx<<<grid, DFT_BLOCK, smem, s>>>(fl, N, n, es, ls, c + l0, turn, rest, (float)dt, tw, angles, G + (size_t)l0 * K,
+                                               scale + l0);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     k_dft_inv_fx<<<grid, DFT_BLOCK, smem, s>>>(fl, N, n, es, ls, angles, G + (size_t)l0 * K, scale + l0);

@@ -255,10 +255,10 @@ void fx_tables_release(FxTables* t) {
   delete t;
 }
 
-bool fx_make_turn(double k1, double dt, FxTurn* out) {
-  const double p = k1 * dt;
+bool fx_make_turn(FxStep k1, double dt, FxTurn* out) {
+  const double p = k1.h * dt;
   if (!std::isfinite(p) || std::fabs(p) > 1e280 || (p != 0.0 && std::fabs(p) < 1e-280)) return false;
-  const dd a = dd_mul(dd_norm(p, std::fma(k1, dt, -p)), kInv2Pi);
+  const dd a = dd_mul(dd_norm(p, std::fma(k1.h, dt, -p) + k1.l * dt), kInv2Pi);
   int e = 0;
   const double m = std::frexp(a.h, &e);
   out->am = -((long long)std::ldexp(m, 62) + (long long)std::llrint(std::ldexp(a.l, 62 - e)));
@@ -266,13 +266,35 @@ bool fx_make_turn(double k1, double dt, FxTurn* out) {
   return true;
 }
 
-bool fx_uniform(const double* k, int n) {
+bool fx_uniform(const double* k, int n, FxStep* k1) {
+  *k1 = {k[n > 1 ? 1 : 0], 0.0};
   for (int m = 0; m <= n / 2; ++m) {
     const double want = m * k[n > 1 ? 1 : 0], tol = 1e-15 * std::fabs(want);
     if (!(std::fabs(std::fabs(k[m % n]) - std::fabs(want)) <= tol)) return false;
     if (2 * m != n && m > 0 && want != 0.0 && (k[m] < 0.0) != (want < 0.0)) return false;
   }
+  // sum m k[m] / sum m^2 (the Nyquist bin's sign is the other way round)
+  dd num = {0.0, 0.0};
+  double den = 0.0;
+  for (int m = 1; m <= n / 2; ++m) {
+    const double km = std::copysign(k[m], k1->h), p = m * km;
+    num = dd_add(num, {p, std::fma((double)m, km, -p)});
+    den += (double)m * m;
+  }
+  // (far from the ends of the range, where the parts are doubles)
+  if (std::fabs(num.h) > 1e-250 && std::fabs(num.h) < 1e250) {
+    const double q = num.h / den;
+    const dd s = dd_norm(q, (std::fma(-q, den, num.h) + num.l) / den);
+    *k1 = {s.h, s.l};
+  }
   return true;
+}
+
+std::vector<float> fx_step_rest(const double* k, int n, FxStep k1) {
+  std::vector<float> r(n / 2 + 1, 0.f);
+  for (int m = 1; m <= n / 2; ++m)
+    r[m] = (float)((std::fma(-(double)m, k1.h, std::copysign(k[m], k1.h)) - m * k1.l) * std::ldexp(kInv2Pi.h, 64));
+  return r;
 }
 
 #define VG_FX_CASES(M) M(1) M(2) M(3) M(4) M(5) M(6) M(7) M(8) M(9) M(10) M(11) M(12) M(13)

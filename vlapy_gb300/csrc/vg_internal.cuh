@@ -29,15 +29,18 @@ struct vg_plan {
   vg_pulse* pulses;  // [n_pulses]
   vg::cx<double>* tw64;  // [FFT_NMAX]
   vg::cx<float>* tw32;   // [FFT_NMAX]
-  // fixed-point advection: its table (null: none), kv[1] and kx[1], and whether
+  // fixed-point advection: its table (null: none), the grids' steps, and whether
   // each wavenumber grid is uniform (else the transforms in doubles)
   vg::FxTables* fx_tables;
   vg::fxw* tw_fx;
-  double kv1, kx1;
+  vg::FxStep kv1, kx1;
   int kv_uniform, kx_uniform;
-  // lengths that are not powers of two: their angle tables and the bins' scratch
+  // lengths that are not powers of two: their angle tables, what the wavenumbers
+  // are off the grid's step by, and the bins' scratch
   vg::fxw* dft_v;
   vg::fxw* dft_x;
+  float* dft_rest_v;
+  float* dft_rest_x;
   void* dft_work;
   // fixed-point storage moments: the velocity powers and the logarithm's table
   vg::FxPowers fx_pw;
