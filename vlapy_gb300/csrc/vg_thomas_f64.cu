@@ -23,7 +23,8 @@
 // the serial one bit for bit.  The k-th sweep leaves at least k lanes exact,
 // so there are never more sweeps than lanes; contraction makes it two
 // (the pivots forget their start by a factor a c / p^2 per element, below 0.6
-// for c = nu dt vth / dv^2 up to 13).  Measured: 64 x 1024 from 1.59 to 0.03 ms,
+// for c = nu dt vth / dv^2 up to 13; strongly collisional rows of a full chip are left
+// to one thread each, see launch_thomas_f64).  Measured: 64 x 1024 from 1.59 to 0.03 ms,
 // 2048 x 4096 from 6.4 to 1.07 ms, against one thread per row.
 //
 // Divisions that share a divisor (by 2 dv, by a pivot) go through its
@@ -41,6 +42,8 @@
 // that is some 90 cycles an element on the FP32 and integer pipes, where the FP64
 // sweep takes 130 to 600, and leaves about nine elements to sweep again: two sweeps
 // instead of two to eight, 2048 x 4096 from 1.31 to 1.07 ms, 64 x 1024 from 45 to 33 us.
+#include <cmath>
+
 #include "vg_internal.cuh"
 #include "vg_f32.cuh"
 #include "vg_f64_body.cuh"
@@ -124,10 +127,25 @@ struct ThomasArgs {
   const double* nudt_row;  // per row (0: leave the row as it is), or null: nudt
   double dv, dv_sq;
   double* scratch;
+  // either: both kernels run, and the rows' collisionality says which of them solves
+  // (all_stiff); stiff: 32 times the limit of the mean of sqrt(nudt vth)
+  bool either;
+  float stiff;
 };
+// Whether the launch is k_thomas_serial's: the same answer in every warp of both
+// kernels, from 32 rows spread over all (whole warps call it)
+__device__ __forceinline__ bool all_stiff(const ThomasArgs& a) {
+  const size_t row = (size_t)((long long)(threadIdx.x & 31) * a.nrows / 32);
+  const double nudt = a.nudt_row ? a.nudt_row[row] : a.nudt;
+  float q = __fsqrt_rn(__double2float_rn(__dmul_rn(nudt, a.mom[row * a.mstride + a.vth_col])));
+#pragma unroll
+  for (int m = 16; m > 0; m >>= 1) q = __fadd_rn(q, __shfl_xor_sync(0xffffffffu, q, m));
+  return q > a.stiff;  // (NaN: no)
+}
 
 __global__ void k_thomas_serial(ThomasArgs a) {
   const int row = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a.either && !all_stiff(a)) return;
   if (row >= a.nrows) return;
   const double nudt = a.nudt_row ? a.nudt_row[row] : a.nudt;
   if (a.nudt_row && nudt == 0.0) return;
@@ -167,6 +185,7 @@ __global__ void __launch_bounds__(WIDE ? 512 : 32) k_thomas_chunks(ThomasArgs g,
   // rows of collisionless runs are left as they are (the lanes stay for the exchanges)
   const bool live_row = valid && !(g.nudt_row && nudt == 0.0);
   if (WIDE && !live_row) return;
+  if (g.either && all_stiff(g)) return;
   const int j0 = t * L, j1 = live_row ? min(j0 + L, N) : 0;
   const int n = max(j1 - j0, 0);  // this lane's elements
   double* fr = g.f + (size_t)(live_row ? row : 0) * N;
@@ -462,21 +481,38 @@ cudaError_t chunks(const ThomasArgs& a, cudaStream_t s) {
 cudaError_t launch_thomas_f64(double* f, int nrows, int nv, const double* v, const double* mom, int mstride,
                               int vbar_col, int vth_col, int dougherty, double nudt, const double* nudt_row, double dv,
                               double dv_sq, double* scratch, cudaStream_t s) {
-  const ThomasArgs a = {f, nrows, nv, v, mom, mstride, vbar_col, vth_col, dougherty, nudt, nudt_row, dv, dv_sq,
-                        scratch};
+  ThomasArgs a = {f, nrows, nv, v, mom, mstride, vbar_col, vth_col, dougherty, nudt, nudt_row, dv, dv_sq,
+                  scratch, false, 0.f};
   if (nv > THOMAS_CHUNK_NV || nv < 16 || nrows >= THOMAS_SERIAL_ROWS) {
     k_thomas_serial<<<div_up(nrows, 64), 64, 0, s>>>(a);
     return cudaGetLastError();
   }
+  // Rows of strong collisions (c = nudt vth / dv^2) forget a guess over some 20 sqrt(c)
+  // elements, so the sweeps over a full chip's rows cost 4e-5 us a cell and sqrt(c),
+  // where one thread a row takes 1.6 us an element whatever c.  They meet near sqrt(c)
+  // = 40000 / rows: 2048 x 4096 at c = 320 (6.8 ms; 45 ms in chunks at c = 1e5), 2048 x
+  // 1024 at 340, 8192 x 1024 at 31, 11000 x 512 at 16.  Below a million cells the
+  // chunks fit the chip and are never the slower (1024 x 1024: 1.8 against 1.6 ms at c
+  // = 1e5; 300 x 2048: 2.2 against 3.1), except for the longest rows, one of which
+  // fills an SM (4 x 4096 meets at 2e4, 64 x 8192 at 6e4).  vth is only known on the
+  // device: both kernels are launched and one of them returns (an idle launch is 2 us).
+  // The mean of sqrt(c) decides for all rows: the serial kernel takes as long for a few.
+  const long long cells = (long long)nrows * nv;
+  a.either = cells >= (1 << 20) || nv >= 4096;
+  double root = 40000.0 / nrows;
+  if (cells < (1 << 20) || (nv >= 4096 && root > 200.0)) root = 200.0;
+  a.stiff = (float)(32.0 * root * std::sqrt(dv_sq));
   // The shortest chunk that still gives every scheduler at most two warps (152
   // x 8 = 1216): a lane's share of the parallel work falls with L, while the
   // elements swept again do not depend on it, so once the schedulers are full
   // longer chunks waste less (32: five arrays of a warp's chunks take 42 KB, and
   // four warps must fit an SM)
-  const long long cells = (long long)nrows * nv;
-  if (nv <= 4096 && cells < 32LL * 8 * 1216) return chunks<8>(a, s);
-  if (cells < 32LL * 16 * 1216) return chunks<16>(a, s);
-  return chunks<32>(a, s);
+  const cudaError_t err = nv <= 4096 && cells < 32LL * 8 * 1216 ? chunks<8>(a, s)
+                          : cells < 32LL * 16 * 1216            ? chunks<16>(a, s)
+                                                                : chunks<32>(a, s);
+  if (err != cudaSuccess || !a.either) return err;
+  k_thomas_serial<<<div_up(nrows, 64), 64, 0, s>>>(a);
+  return cudaGetLastError();
 }
 
 }  // namespace vg
