@@ -32,20 +32,21 @@ bool fx_make_turn(FxStep k1, double dt, FxTurn* out);
 // (k[1]'s own rounding, taken m times, would be an error of up to 2^-53 of every phase
 // beside those that the k[m] have)
 bool fx_uniform(const double* k, int n, FxStep* k1);
-// what is left of the wavenumbers k[0 .. n / 2] past the step, (k[m] - m k1) 2^64 / (2 pi)
+// what is left of the wavenumbers k[1 .. n / 2] past the step, (k[m] - m k1) 2^64 / (2 pi),
+// and at 0 (where nothing is) the largest modulus of these
 std::vector<float> fx_step_rest(const double* k, int n, FxStep k1);
 
-// v-advection of nrows rows of nv (a power of two <= 8192); kv, dt and tw64 for
-// the row pairs that go through doubles
-cudaError_t launch_edfdv_fx(double* f, int nrows, int nv, const double* e, FxTurn turn, const fxw* tw, const double* kv,
-                            double dt, const cx<double>* tw64, cudaStream_t s);
+// v-advection of nrows rows of nv (a power of two <= 8192) by dt; rest: fx_step_rest's
+// of kv; tw64 for the row pairs that go through doubles
+cudaError_t launch_edfdv_fx(double* f, int nrows, int nv, const double* e, FxTurn turn, double dt, const float* rest,
+                            const fxw* tw, const cx<double>* tw64, cudaStream_t s);
 
 // One run of the x-advection: f[nx][nv] at f + f_off
 struct FxColRun {
   long long f_off;
   int nv;
   const double* v;
-  const double* kx;
+  const float* rest;  // fx_step_rest's of kx
   FxTurn turn;
 };
 // column pairs per CTA for nx (a power of two <= 8192) when `pairs` pairs are advanced together

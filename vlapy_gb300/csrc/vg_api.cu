@@ -694,16 +694,16 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
     p->tw_fx = p->fx_tables->tw;
     p->kv_uniform = fx_uniform(d->kv, d->nv, &p->kv1);
     p->kx_uniform = fx_uniform(d->kx, d->nx, &p->kx1);
+    if (p->kv_uniform) TRY(upload(p, &p->rest_v, fx_step_rest(d->kv, d->nv, p->kv1), "kv"));
+    if (p->kx_uniform) TRY(upload(p, &p->rest_x, fx_step_rest(d->kx, d->nx, p->kx1), "kx"));
     const bool dx = !p->nx_pow2 && d->nx <= DFT_ADVECT_NMAX, dv = !p->nv_pow2 && d->nv <= DFT_ADVECT_NMAX;
     if (dv) {
       TRY(dev_copy<fxw>(p, &p->dft_v, nullptr, nv, "DFT angles"));
       TRY(cuda_status(build_dft_table(d->nv, p->tw_fx, p->dft_v, 0), "DFT angles"));
-      TRY(upload(p, &p->dft_rest_v, fx_step_rest(d->kv, d->nv, p->kv1), "DFT angles"));
     }
     if (dx) {
       TRY(dev_copy<fxw>(p, &p->dft_x, nullptr, nx, "DFT angles"));
       TRY(cuda_status(build_dft_table(d->nx, p->tw_fx, p->dft_x, 0), "DFT angles"));
-      TRY(upload(p, &p->dft_rest_x, fx_step_rest(d->kx, d->nx, p->kx1), "DFT angles"));
     }
     if (dx || dv)
       TRY(dev_copy<unsigned char>(p, reinterpret_cast<unsigned char**>(&p->dft_work), nullptr,

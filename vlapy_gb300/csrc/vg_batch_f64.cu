@@ -116,8 +116,8 @@ struct vg_batch {
     FxStep kv1;
     int kv_uniform;
     double *v, *kv, *v_pow;
-    fxw* dft_v;  // nv not a power of two: its angles, and what kv is off its step by
-    float* dft_rest_v;
+    float* rest_v;  // what kv is off its step by
+    fxw* dft_v;  // nv not a power of two: its angles
     FxPowers fx_pw;
     int* pw_v;
   };
@@ -197,7 +197,7 @@ vg_plan class_view(const vg_batch* b, const vg_batch::Cls& c) {
   v.kv1 = c.kv1;
   v.kv_uniform = c.kv_uniform;
   v.dft_v = c.dft_v;
-  v.dft_rest_v = c.dft_rest_v;
+  v.rest_v = c.rest_v;
   v.dft_work = b->dft_work;
   v.fx_pw = c.fx_pw;
   v.fx_log = b->fx_tables->log;
@@ -403,9 +403,9 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
       c.dv = d.dv;
       c.dv_sq = d.dv_sq;
       c.kv_uniform = fx_uniform(d.kv, d.nv, &c.kv1);
-      if (!is_pow2(d.nv)) {
+      if (c.kv_uniform) {
         const std::vector<float> rest = fx_step_rest(d.kv, d.nv, c.kv1);
-        B_TRY(b_alloc(b, &c.dft_rest_v, rest.size(), rest.data(), "batch grids"));
+        B_TRY(b_alloc(b, &c.rest_v, rest.size(), rest.data(), "batch grids"));
       }
       B_TRY(b_alloc(b, &c.v, d.nv, d.v, "batch grids"));
       B_TRY(b_alloc(b, &c.kv, d.nv, d.kv, "batch grids"));
@@ -484,14 +484,24 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
   std::map<XKey, long long> pairs_of;  // column pairs of each class
   std::vector<XKey> key_of(n_runs);
   std::vector<FxColRun> fx_runs(n_runs);
+  std::vector<float> rest;  // of all runs' kx
+  std::vector<size_t> rest_off;
   for (int i = 0; i < n_runs; ++i) {
     const vg_run_desc& d = runs[i];
-    fx_runs[i] = {rd[i].f_off, d.nv, rd[i].v, rd[i].kx, {}};
+    fx_runs[i] = {rd[i].f_off, d.nv, rd[i].v, nullptr, {}};
     FxStep k1;
     const bool ok = fx_uniform(d.kx, d.nx, &k1) && fx_make_turn(k1, d.dt, &fx_runs[i].turn);
+    rest_off.push_back(rest.size());
+    if (ok) {
+      const std::vector<float> one = fx_step_rest(d.kx, d.nx, k1);
+      rest.insert(rest.end(), one.begin(), one.end());
+    }
     key_of[i] = XKey(d.nx, ok);
     pairs_of[key_of[i]] += (d.nv + 1) / 2;
   }
+  float* rest_d = nullptr;
+  B_TRY(b_alloc(b, &rest_d, rest.size(), rest.data(), "batch grids"));
+  for (int i = 0; i < n_runs; ++i) fx_runs[i].rest = rest_d + rest_off[i];
   B_TRY(b_alloc(b, &b->fx_runs, fx_runs.size(), fx_runs.data(), "batch runs"));
   auto tile_w = [&](const XKey& k) {
     return 2 * (k.second ? fx_col_pairs(k.first, pairs_of[k]) : col_seqs<double>(k.first));

@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(DFT_BLOCK) k_dft_fwd_fx(const double* __restri
     if (part != u || k >= K || l0 + u >= n_lines) continue;
     const double cl = bad[u] ? 0.0 : c[l0 + u];
     // (the wavenumber's own rounding, some 2^-53 of the phase, in FP32)
-    const long long own = __float2ll_rn(-rest[k] * dt * (float)cl);
+    const long long own = k ? __float2ll_rn(-rest[k] * dt * (float)cl) : 0;
     const fxw p = fx_mult(fx_sincos((unsigned long long)k * fx_turn(turn, cl) + (unsigned long long)own, tw));
     fx z = fx_cmul<0, false>({re[u], -im[u]}, p);
     // half weight for the bins that have no mirror image

@@ -28,8 +28,8 @@ __host__ __device__ constexpr int fx_row_block(int n) { return fx_threads(n) > 2
 
 template <int N>
 __global__ void __launch_bounds__(fx_row_block(N), fx_row_block(N) > 256 ? 1 : 2)
-    k_edfdv_fx(double* __restrict__ f, int nrows, const double* __restrict__ e, FxTurn turn,
-               const fxw* __restrict__ tw, const double* __restrict__ kv, double dt, const cx<double>* __restrict__ tw64) {
+    k_edfdv_fx(double* __restrict__ f, int nrows, const double* __restrict__ e, FxTurn turn, double dt,
+               const float* __restrict__ rest, const fxw* __restrict__ tw, const cx<double>* __restrict__ tw64) {
   constexpr int R = fx_radix(N), G = fx_threads(N);
   constexpr int DOWN = ilog2(N) - fx_shift<N>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -83,7 +83,11 @@ __global__ void __launch_bounds__(fx_row_block(N), fx_row_block(N) > 256 ? 1 : 2
       io[i] = {bad_a ? 0 : fx_from_double(da[i], Ea), bad_b ? 0 : fx_from_double(db[i], Eb)};
   }
   fx_fft<N, false, true, false>(s, t, tw, sync, io);
-  FxNorms n = fx_rotate<N, DOWN>(s, t, fx_turn(turn, bad_a ? 0.0 : ea), fx_turn(turn, bad_b ? 0.0 : eb), tw);
+  const unsigned long long ta = fx_turn(turn, bad_a ? 0.0 : ea), tb = fx_turn(turn, bad_b ? 0.0 : eb);
+  const float oa = bad_a ? 0.f : fx_own_scale(dt, ea), ob = bad_b ? 0.f : fx_own_scale(dt, eb);
+  // (entry 0 of rest: the largest)
+  const bool own = rest[0] * fmaxf(fabsf(oa), fabsf(ob)) > FX_OWN_LEAST;
+  FxNorms n = fx_rotate<N, DOWN>(s, t, ta, tb, own, oa, ob, rest, tw);
   n.l1 = __reduce_add_sync(mask, n.l1);
   n.a2 = __reduce_add_sync(mask, n.a2);
   n.b2 = __reduce_add_sync(mask, n.b2);
@@ -105,8 +109,8 @@ __global__ void __launch_bounds__(fx_row_block(N), fx_row_block(N) > 256 ? 1 : 2
   const int h = fx_shift_back<N>(n, bad_a || Ea <= 1, bad_b || Eb <= 1);
   if (h < 0) {
     sync();
-    fx_pair_f64<N>({fa, ea, fx_up(Ea, n.a2), true, bad_a}, {fb, eb, fx_up(Eb, n.b2), vb, bad_b}, 1, reinterpret_cast<cx<double>*>(s), t, kv, dt,
-                   tw64, sync);
+    fx_pair_f64<N>({fa, ta, oa, fx_up(Ea, n.a2), true, bad_a}, {fb, tb, ob, fx_up(Eb, n.b2), vb, bad_b}, 1,
+                   reinterpret_cast<cx<double>*>(s), t, rest, tw, tw64, sync);
     return;
   }
   fx_fft<N, true, false, true>(s, t, tw, sync, io, h);
@@ -122,7 +126,7 @@ __global__ void __launch_bounds__(fx_row_block(N), fx_row_block(N) > 256 ? 1 : 2
 }
 
 template <int N>
-cudaError_t edfdv_fx_n(double* f, int nrows, const double* e, FxTurn turn, const fxw* tw, const double* kv, double dt,
+cudaError_t edfdv_fx_n(double* f, int nrows, const double* e, FxTurn turn, double dt, const float* rest, const fxw* tw,
                        const cx<double>* tw64, cudaStream_t s) {
   constexpr int G = fx_threads(N);
   const int pairs = (nrows + 1) / 2;
@@ -133,7 +137,7 @@ cudaError_t edfdv_fx_n(double* f, int nrows, const double* e, FxTurn turn, const
   const size_t smem = (size_t)P * sp_len<double>(N) * sizeof(fx);
   cudaError_t err = ensure_smem((const void*)k_edfdv_fx<N>, smem);
   if (err != cudaSuccess) return err;
-  k_edfdv_fx<N><<<div_up(pairs, P), P * G, smem, s>>>(f, nrows, e, turn, tw, kv, dt, tw64);
+  k_edfdv_fx<N><<<div_up(pairs, P), P * G, smem, s>>>(f, nrows, e, turn, dt, rest, tw, tw64);
   return cudaGetLastError();
 }
 
@@ -292,18 +296,20 @@ bool fx_uniform(const double* k, int n, FxStep* k1) {
 
 std::vector<float> fx_step_rest(const double* k, int n, FxStep k1) {
   std::vector<float> r(n / 2 + 1, 0.f);
-  for (int m = 1; m <= n / 2; ++m)
+  for (int m = 1; m <= n / 2; ++m) {
     r[m] = (float)((std::fma(-(double)m, k1.h, std::copysign(k[m], k1.h)) - m * k1.l) * std::ldexp(kInv2Pi.h, 64));
+    r[0] = std::max(r[0], std::fabs(r[m]));
+  }
   return r;
 }
 
 #define VG_FX_CASES(M) M(1) M(2) M(3) M(4) M(5) M(6) M(7) M(8) M(9) M(10) M(11) M(12) M(13)
 
-cudaError_t launch_edfdv_fx(double* f, int nrows, int nv, const double* e, FxTurn turn, const fxw* tw, const double* kv,
-                            double dt, const cx<double>* tw64, cudaStream_t s) {
+cudaError_t launch_edfdv_fx(double* f, int nrows, int nv, const double* e, FxTurn turn, double dt, const float* rest,
+                            const fxw* tw, const cx<double>* tw64, cudaStream_t s) {
   switch (ilog2(nv)) {
 #define CASE(L) \
-  case L: return edfdv_fx_n<(1 << L)>(f, nrows, e, turn, tw, kv, dt, tw64, s);
+  case L: return edfdv_fx_n<(1 << L)>(f, nrows, e, turn, dt, rest, tw, tw64, s);
     VG_FX_CASES(CASE)
 #undef CASE
     default: return cudaErrorInvalidValue;

@@ -19,10 +19,14 @@
 //    still fits, the bins are used as they are (shifted by h).  A distribution
 //    function's spectrum is compact: h is 0 or 1.
 //  * The error of the result is then about 0.6 sqrt(N) 2^h units, and the lines
-//    for which that is more than 2^-52 of their RMS (a noise-like or spiked
-//    line of a long transform) are transformed in doubles instead, inside the
-//    same kernel.  So the error is below that of the transform in doubles on
-//    every input (measured against 128-bit arithmetic, see the kernels).
+//    for which that is more than the error of a transform in doubles are
+//    transformed in doubles instead, inside the same kernel, so that the error
+//    is at or below that of the doubles on every input (measured against 128-bit
+//    arithmetic).  These are the lines whose RMS is below 0.002 to 0.005 sqrt(N)
+//    of their maximum, by the maximum's mantissa: of Maxwellians on |v| < 8, at N =
+//    1024 some of vth 0.1, at 4096 half of vth 0.3 (a third of vth 1 on |v| < 16), at
+//    8192 a fifth of vth 1 (two thirds on |v| < 16); and lines whose spectrum is
+//    broad (h > 0): noise from N = 256 on, filaments and fronts of the longest grids.
 // Lines that hold a NaN or infinity come out as NaN, as from a transform in
 // doubles.
 //
@@ -476,6 +480,20 @@ __device__ __forceinline__ fxc fx_turn_by(fxc a, const fxw& w) {
   return {(long long)((unsigned long long)p.x << 2), (long long)((unsigned long long)p.y << 2)};
 }
 
+// A grid's wavenumbers are m k1 to their own rounding only, which is some 2^-53 of the
+// phase: what wavenumber m is off by (rest of fx_step_rest, here in FP32) times
+// fx_own_scale, a small angle in Q64, is turned on top of the m steps.  (Without it the
+// phases' errors are those of the doubles ((-k) dt) c, twice to thirty times the
+// transform's on lines with all wavenumbers in them.)  It is 3 % of the x-drift; below
+// 2^-53, the wavenumbers' rounding of phases of a radian or two, it is left out: a small
+// part of the transform's own error.
+__device__ __forceinline__ float fx_own_scale(double dt, double c) { return -6.28318531f * (float)dt * (float)c; }
+__device__ __forceinline__ fxc fx_own(fxc p, float own) {
+  const int d = __float2int_rn(own);
+  return {p.c - __mulhi((int)(p.s >> 32), d), p.s + __mulhi((int)(p.c >> 32), d)};
+}
+constexpr float FX_OWN_LEAST = 2048.f;  // 2^-53 in Q64
+
 // What the rotation learns about the bins it leaves: an upper bound of the sum
 // of their moduli in units of 2^38, and the sums of the squares of line a's and
 // b's bins in units of 2^88, rounded down (by Parseval's theorem a sum is the line's
@@ -497,10 +515,11 @@ __device__ __forceinline__ unsigned fx_sq(long long a) {
 
 // Rotation of a packed line pair in the bins (two_real_rotate of vg_fft.cuh):
 // the sequence in s is the transform of a + i b, still to be divided by 2^DOWN;
-// bin k of a is multiplied by exp(2 pi i k fa / 2^64), of b likewise.  The G
-// threads of the sequence take the bins t, t + G, ... <= N/2.
+// bin k of a is multiplied by exp(2 pi i k fa / 2^64) and, if own, turned by rest[k]
+// oa, of b likewise.  The G threads of the sequence take the bins t, t + G, ... <= N/2.
 template <int N, int DOWN>
-__device__ __forceinline__ FxNorms fx_rotate(fx* s, int t, unsigned long long fa, unsigned long long fb,
+__device__ __forceinline__ FxNorms fx_rotate(fx* s, int t, unsigned long long fa, unsigned long long fb, bool own,
+                                             float oa, float ob, const float* __restrict__ rest,
                                              const fxw* __restrict__ tw) {
   constexpr int G = fx_threads(N);
   FxNorms n = {0, 0, 0};
@@ -508,7 +527,13 @@ __device__ __forceinline__ FxNorms fx_rotate(fx* s, int t, unsigned long long fa
   const fxw ga = fx_mult(fx_sincos_call((unsigned long long)G * fa, tw));
   const fxw gb = fx_mult(fx_sincos_call((unsigned long long)G * fb, tw));
   for (int k = t; k <= N / 2; k += G) {
-    const fxw wa = fx_mult(pa), wb = fx_mult(pb);
+    fxc qa = pa, qb = pb;
+    if (own) {
+      const float r = rest[k];
+      qa = fx_own(pa, r * oa);
+      qb = fx_own(pb, r * ob);
+    }
+    const fxw wa = fx_mult(qa), wb = fx_mult(qb);
     const fx zk = fx_down<DOWN>(s[fx_sp(k)]);
     if (k == 0 || 2 * k == N) {
       // the bins of both lines are real: only the real part of the rotation acts
@@ -556,55 +581,71 @@ __device__ __forceinline__ int fx_shift_back(const FxNorms& n, bool no_a, bool n
   return h;
 }
 
+inline __device__ __noinline__ double fx_scale_far(double x, int k) { return ldexp(x, k); }
+// x 2^k without an FP64 instruction where x and the result are ordinary
+__device__ __forceinline__ double fx_scale(double x, int k) {
+  const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
+  if ((unsigned)(e - 1) < 2046u && (unsigned)(e + k - 1) < 2046u) return __hiloint2double(hi + (k << 20), __double2loint(x));
+  return x == 0.0 ? x : fx_scale_far(x, k);
+}
+
 // One line of a pair and its phase: elements f[n es], the power of two that brings
-// it to an RMS of order one, the double c of its phase ((-k) dt) c; bad: it comes out
+// it to an RMS of order one, its turns per index and fx_own_scale; bad: it comes out
 // as NaN
 struct FxLine {
   double* f;
-  double c;
+  unsigned long long turn;
+  float own;
   int up;
   bool on, bad;
 };
 // that power of two for a line of scale E whose bins' squares add up to q (FxNorms).
-// It and its inverse are doubles: at most 2^1023 (a line of subnormal values has E < 0
-// and stays below order one), at least 2^-1023.
-__device__ __forceinline__ int fx_up(int E, unsigned q) {
-  return max(-1023, min(FX_SCALE - 44 - E - (32 - __clz((int)q)) / 2, 1023));
-}
+__device__ __forceinline__ int fx_up(int E, unsigned q) { return FX_SCALE - 44 - E - (32 - __clz((int)q)) / 2; }
 // The pair in doubles, for the lines that fx_shift_back turns away.  Each line is
 // brought to the same RMS by its own power of two (exact): what one of them rounds at
 // reaches the other, which must not take more than its own.  (Brought to the same
 // maximum, a spike beside a smooth line took five times the error it has alone at 2048.)
+// The phases are the fixed-point ones (their sines were a quarter of the FP64
+// instructions) and the scaling moves exponents, since the pair has paid for the
+// fixed-point forward transform as well: a half kick of 2048 x 4096 of noise takes 1.01
+// ms, 1.23 with sines and products in doubles, 1.02 with no fixed point at all (0.24 for
+// smooth rows); 4096 x 4096 columns 2.17, 2.55, 2.13.
 // Out of line: it must not take registers from the fixed-point path.
 template <int N, typename Sync>
 __device__ __noinline__ void fx_pair_f64(FxLine a, FxLine b, long long es, cx<double>* s, int t,
-                                         const double* __restrict__ kw, double dt, const cx<double>* __restrict__ tw,
-                                         Sync sync) {
+                                         const float* __restrict__ rest, const fxw* __restrict__ angles,
+                                         const cx<double>* __restrict__ tw, Sync sync) {
   constexpr int R = fx_radix(N), G = fx_threads(N);
   const bool use_a = a.on && !a.bad, use_b = b.on && !b.bad;
-  const double da = ldexp(1.0, a.up), db = ldexp(1.0, b.up);
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const long long n = (long long)(t + i * G) * es;
-    s[sp<double>(t + i * G)] = {use_a ? a.f[n] * da : 0.0, use_b ? b.f[n] * db : 0.0};
+    s[sp<double>(t + i * G)] = {use_a ? fx_scale(a.f[n], a.up) : 0.0, use_b ? fx_scale(b.f[n], b.up) : 0.0};
   }
   sync();
   block_fft<double, N, false, R>(s, t, tw, sync);
+  fxc pa = fx_sincos_call((unsigned long long)t * a.turn, angles), pb = fx_sincos_call((unsigned long long)t * b.turn, angles);
+  const fxw ga = fx_mult(fx_sincos_call((unsigned long long)G * a.turn, angles));
+  const fxw gb = fx_mult(fx_sincos_call((unsigned long long)G * b.turn, angles));
   two_real_rotate<double>(s, N, t, G, [&](int k, double& ca, double& sa, double& cb, double& sb) {
-    const double ph = -kw[k] * dt;
-    sincos(use_a ? ph * a.c : 0.0, &sa, &ca);
-    sincos(use_b ? ph * b.c : 0.0, &sb, &cb);
+    const float own = rest[k];
+    const fxc qa = fx_own(pa, own * a.own), qb = fx_own(pb, own * b.own);
+    ca = fx_to_double(qa.c, -62);
+    sa = fx_to_double(qa.s, -62);
+    cb = fx_to_double(qb.c, -62);
+    sb = fx_to_double(qb.s, -62);
+    pa = fx_turn_by(pa, ga);
+    pb = fx_turn_by(pb, gb);
   });
   sync();
   block_fft<double, N, true, R>(s, t, tw, sync);
-  const double sc = 1.0 / N, ua = ldexp(1.0, -a.up), ub = ldexp(1.0, -b.up);
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const long long n = (long long)(t + i * G) * es;
     const cx<double> z = s[sp<double>(t + i * G)];
-    if (a.on) a.f[n] = a.bad ? nan : (z.x * sc) * ua;
-    if (b.on) b.f[n] = b.bad ? nan : (z.y * sc) * ub;
+    if (a.on) a.f[n] = a.bad ? nan : fx_scale(z.x, -a.up - ilog2(N));
+    if (b.on) b.f[n] = b.bad ? nan : fx_scale(z.y, -b.up - ilog2(N));
   }
 }
 

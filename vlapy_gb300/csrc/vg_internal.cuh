@@ -35,12 +35,12 @@ struct vg_plan {
   vg::fxw* tw_fx;
   vg::FxStep kv1, kx1;
   int kv_uniform, kx_uniform;
-  // lengths that are not powers of two: their angle tables, what the wavenumbers
-  // are off the grid's step by, and the bins' scratch
+  // what the wavenumbers are off their grid's step by
+  float* rest_v;
+  float* rest_x;
+  // lengths that are not powers of two: their angle tables and the bins' scratch
   vg::fxw* dft_v;
   vg::fxw* dft_x;
-  float* dft_rest_v;
-  float* dft_rest_x;
   void* dft_work;
   // fixed-point storage moments: the velocity powers and the logarithm's table
   vg::FxPowers fx_pw;

@@ -101,7 +101,11 @@ __global__ void __launch_bounds__(fx_col_block(NX), fx_col_block(NX) > 256 ? 1 :
   }
   const CtaSync sync;
   fx_fft<NX, false, true, false>(s, t, tw, sync, io);
-  FxNorms n = fx_rotate<NX, DOWN>(s, t, fx_turn(r.turn, bad_a ? 0.0 : ca), fx_turn(r.turn, bad_b ? 0.0 : cb), tw);
+  const unsigned long long ta = fx_turn(r.turn, bad_a ? 0.0 : ca), tb = fx_turn(r.turn, bad_b ? 0.0 : cb);
+  const float oa = bad_a ? 0.f : fx_own_scale(dt, ca), ob = bad_b ? 0.f : fx_own_scale(dt, cb);
+  // (entry 0 of rest: the largest)
+  const bool own = r.rest[0] * fmaxf(fabsf(oa), fabsf(ob)) > FX_OWN_LEAST;
+  FxNorms n = fx_rotate<NX, DOWN>(s, t, ta, tb, own, oa, ob, r.rest, tw);
   if constexpr (G > 1) {
     atomicAdd(&red[5 * p + 2], n.l1);
     atomicAdd(&red[5 * p + 3], n.a2);
@@ -111,8 +115,21 @@ __global__ void __launch_bounds__(fx_col_block(NX), fx_col_block(NX) > 256 ? 1 :
   }
   // (E <= 1: a column of zeros, or of values that small)
   const int h = fx_shift_back<NX>(n, bad_a || Ea <= 1, bad_b || Eb <= 1);
-  const bool turned = h < 0;  // a pair that fixed point is not exact enough for
-  const bool any_turned = __syncthreads_or(turned);
+  // Pairs that fixed point is not exact enough for go through doubles, pair by pair: a
+  // column comes out the same whatever its tile holds (a batch and a single run have
+  // different tiles).  The tile's other pairs go along with nothing to load or store,
+  // for the barriers.
+  const bool turned = h < 0;
+  const int n_turned = __syncthreads_count(turned);  // threads
+  auto in_doubles = [&]() {
+    cx<double>* sd = reinterpret_cast<cx<double>*>(smem_raw) + (size_t)p * (sp_len<double>(NX) + COL_PAD);
+    fx_pair_f64<NX>({fc, ta, oa, fx_up(Ea, n.a2), va && turned, bad_a}, {fc + 1, tb, ob, fx_up(Eb, n.b2), vb && turned, bad_b},
+                    nv, sd, t, r.rest, tw, tw64, sync);
+  };
+  if (n_turned == (int)blockDim.x) {
+    in_doubles();
+    return;
+  }
   fx_fft<NX, true, false, true>(s, t, tw, sync, io, turned ? 16 : h);
   // lines of zeros stay so: the partner's rounding does not reach them
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
@@ -131,14 +148,9 @@ __global__ void __launch_bounds__(fx_col_block(NX), fx_col_block(NX) > 256 ? 1 :
       if (vb) q[1] = xb;
     }
   }
-  if (any_turned) {
-    // Pair by pair: a column comes out the same whatever its tile holds (a batch and a
-    // single run have different tiles).  The tile's other pairs go along with nothing
-    // to load or store, for the barriers.
+  if (n_turned > 0) {
     __syncthreads();
-    cx<double>* sd = reinterpret_cast<cx<double>*>(smem_raw) + (size_t)p * (sp_len<double>(NX) + COL_PAD);
-    fx_pair_f64<NX>({fc, ca, fx_up(Ea, n.a2), va && turned, bad_a}, {fc + 1, cb, fx_up(Eb, n.b2), vb && turned, bad_b}, nv,
-                    sd, t, r.kx, dt, tw64, sync);
+    in_doubles();
   }
 }
 
