@@ -45,7 +45,8 @@ __global__ void __launch_bounds__(128) k_green(const double* __restrict__ inv_kx
     dd_acc(h, l, oh, ol);
   }
   if (lane != 0) return;
-  const double g = -(h + l) / (double)nx;
+  // (the bins 0 and nx / 2 of a real rho do not act, unless they are no numbers)
+  const double g = -(h + l) / (double)nx + 0.0 * (inv[0] + (nx % 2 ? 0.0 : inv[nx / 2]));
   double* o = out + (size_t)blockIdx.y * nx;
   o[n] = g;
   if (n > 0 && 2 * n != nx) o[nx - n] = -g;
