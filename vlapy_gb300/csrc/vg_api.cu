@@ -169,17 +169,23 @@ using namespace vg;
 
 namespace {
 
-// A plan's device memory: blocks of a megabyte that are zeroed once and handed
-// out in pieces, so that its twenty-odd arrays cost one or two allocations (they
-// were most of the time of making a small plan)
+// A plan's device memory: blocks that are zeroed once and handed out in pieces, so that
+// its twenty-odd arrays cost one or two allocations (they were most of the time of
+// making a small plan).  Blocks of a quarter of a megabyte for an FP64 plan's grids and
+// tables: the driver hands such blocks out of what it holds in 2 MB pages, and a new
+// page takes some 70 us.  An FP32 plan's constants and partial sums fill larger ones.
 struct DevArena {
-  static constexpr size_t BLOCK = (size_t)1 << 20, ALIGN = 256;
+  static constexpr size_t ALIGN = 256;
+  const size_t BLOCK;
   std::vector<void*> blocks;
   char* cur = nullptr;
   size_t left = 0;
   // what is copied in waits in `stage` and goes in one copy: every copy from
   // pageable memory is a wait of some 6 us (plans hold ten to twenty of them)
-  static constexpr size_t STAGE = (size_t)256 << 10;
+  static constexpr size_t STAGE_MAX = (size_t)256 << 10;
+  const size_t STAGE;
+  DevArena(size_t block, size_t copied)
+      : BLOCK(block), STAGE(std::min(STAGE_MAX, (copied + ALIGN - 1) / ALIGN * ALIGN)) {}
   std::vector<char> stage;
   char* stage_dst = nullptr;
   ~DevArena() {
@@ -654,7 +660,9 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
   }
   vg_plan* p = new vg_plan();
   std::memset(p, 0, sizeof(vg_plan));
-  p->arena = new DevArena();
+  // (grids, their powers, the summation trees, and FP32's constants)
+  p->arena = new DevArena(d->precision == VG_F64 ? (size_t)256 << 10 : (size_t)1 << 20,
+                          ((size_t)d->nx * 5 + (size_t)d->nv * 13 + 2048) * sizeof(double));
   p->nx = d->nx;
   p->nv = d->nv;
   p->precision = d->precision;
@@ -688,7 +696,7 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
   if (d->f_background) TRY(dev_copy(p, &p->f_bg, d->f_background, nv, "f_background"));
   if (d->n_pulses > 0) TRY(dev_copy(p, &p->pulses, d->pulses, (size_t)d->n_pulses, "pulses"));
   TRY(dev_copy<cx<double>>(p, &p->tw64, nullptr, FFT_NMAX, "twiddles"));
-  TRY(dev_copy<cx<float>>(p, &p->tw32, nullptr, FFT_NMAX, "twiddles"));
+  if (d->precision == VG_F32_DELTA_F) TRY(dev_copy<cx<float>>(p, &p->tw32, nullptr, FFT_NMAX, "twiddles"));
   if (d->precision == VG_F64) {
     TRY(cuda_status(fx_tables_acquire(&p->fx_tables), "fixed-point tables"));
     p->tw_fx = p->fx_tables->tw;
@@ -705,9 +713,6 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
       TRY(dev_copy<fxw>(p, &p->dft_x, nullptr, nx, "DFT angles"));
       TRY(cuda_status(build_dft_table(d->nx, p->tw_fx, p->dft_x, 0), "DFT angles"));
     }
-    if (dx || dv)
-      TRY(dev_copy<unsigned char>(p, reinterpret_cast<unsigned char**>(&p->dft_work), nullptr,
-                                  dft_fx_scratch(d->nx, d->nv, dx, dv), "DFT scratch", true));
     p->fx_log = p->fx_tables->log;
   }
   std::vector<int> tv = pairwise_table(d->nv - 1), tx = pairwise_table(d->nx);
@@ -734,8 +739,15 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
     TRY(dev_copy<int>(p, &p->green_e, nullptr, 1, "Green's function"));
     TRY(cuda_status(build_poisson_fx(p->inv_kx, d->nx, 1, p->green, p->green_e, p->etmp, 0), "Green's function"));
   }
-  if (d->precision == VG_F64 && d->collision != VG_COLL_NONE)
-    TRY(dev_copy<double>(p, &p->bb, nullptr, 2 * nx * thomas_pad(d->nv), "thomas scratch", true));
+  if (d->precision == VG_F64) {
+    // one scratch for the DFTs and the tridiagonal solve, which take turns
+    const size_t solve = d->collision == VG_COLL_NONE ? 0 : thomas_scratch(d->nx, d->nv) * sizeof(double);
+    const size_t dft = p->dft_x || p->dft_v ? dft_fx_scratch(d->nx, d->nv, p->dft_x, p->dft_v) : 0;
+    unsigned char* mem = nullptr;
+    TRY(dev_copy<unsigned char>(p, &mem, nullptr, std::max(solve, dft), "scratch", true));
+    p->bb = reinterpret_cast<double*>(mem);
+    p->dft_work = mem;
+  }
   if (d->precision == VG_F32_DELTA_F) TRY(setup_f32(p, d));
   TRY(cuda_status(static_cast<DevArena*>(p->arena)->flush(), "plan setup"));
   TRY(cuda_status(launch_twiddles(*p, 0), "twiddles"));

@@ -103,7 +103,7 @@ struct vg_batch {
   double* mom = nullptr;       // [x_points][BATCH_MOMS]
   double* fpmom = nullptr;     // [x_points][2]
   double* nudt_row = nullptr;  // [x_points]
-  double* bb = nullptr;        // [max class rows][2][nv]
+  double* bb = nullptr;        // thomas_scratch of the largest class
   int* flags = nullptr;        // status bits raised on the device (VG_FLAG_*)
   int max_pw_x_leaves = 0;
   // nv classes: a contiguous block of runs each
@@ -422,7 +422,7 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
     }
     vg_batch::Cls& c = b->cls.back();
     c.rows += d.nx;
-    bb_need = std::max(bb_need, (size_t)c.rows * 2 * thomas_pad(c.nv));
+    bb_need = std::max(bb_need, thomas_scratch(c.rows, c.nv));
     if (!pw_x_of.count(d.nx)) {
       const std::vector<int> tx = pairwise_table(d.nx);
       int* p = nullptr;
@@ -530,7 +530,7 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
     double *inv_x = nullptr, *work = nullptr;
     B_TRY(b_alloc(b, &xc.x_offs, offs.size(), offs.data(), "batch work list"));
     B_TRY(b_alloc(b, &inv_x, inv.size(), inv.data(), "batch grids"));
-    B_TRY(b_alloc<double>(b, &work, inv.size(), nullptr, "batch grids"));
+    B_TRY(b_alloc<double>(b, &work, inv.size() + xc.nx, nullptr, "batch grids"));
     B_TRY(b_alloc<int2>(b, &xc.green, inv.size(), nullptr, "batch grids"));
     B_TRY(b_alloc<int>(b, &xc.green_e, offs.size(), nullptr, "batch grids"));
     for (int r0 = 0; r0 < xc.n_ids; r0 += 65535)

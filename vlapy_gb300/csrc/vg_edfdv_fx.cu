@@ -14,6 +14,7 @@
 // (smooth lines), in doubles 3.0e-16 and 3.2e-16.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <mutex>
 #include <vector>
 
@@ -211,9 +212,16 @@ std::vector<fxw> build_table() {
   return out;
 }
 
-const std::vector<fxw>& twiddles_host() {
-  static const std::vector<fxw> table = build_table();
-  return table;
+// both tables as they lie on the device, so that they go in one copy
+const std::vector<unsigned char>& tables_host() {
+  static const std::vector<unsigned char> bytes = [] {
+    const std::vector<fxw> tw = build_table();
+    std::vector<unsigned char> b(tw.size() * sizeof(fxw) + FX_LOG_ENTRIES * sizeof(FxLogEntry));
+    std::memcpy(b.data(), tw.data(), tw.size() * sizeof(fxw));
+    std::memcpy(b.data() + tw.size() * sizeof(fxw), fx_log_host(), FX_LOG_ENTRIES * sizeof(FxLogEntry));
+    return b;
+  }();
+  return bytes;
 }
 
 std::mutex tables_mu;
@@ -234,13 +242,11 @@ cudaError_t fx_tables_acquire(FxTables** out) {
       return cudaSuccess;
     }
   FxTables t = {dev, 1, nullptr, nullptr};
-  const std::vector<fxw>& tw = twiddles_host();
-  err = cudaMalloc(&t.tw, tw.size() * sizeof(fxw) + FX_LOG_ENTRIES * sizeof(FxLogEntry));
+  const std::vector<unsigned char>& host = tables_host();
+  err = cudaMalloc(&t.tw, host.size());
   if (err != cudaSuccess) return err;
-  t.log = reinterpret_cast<FxLogEntry*>(t.tw + tw.size());
-  err = cudaMemcpy(t.tw, tw.data(), tw.size() * sizeof(fxw), cudaMemcpyHostToDevice);
-  if (err == cudaSuccess)
-    err = cudaMemcpy(t.log, fx_log_host(), FX_LOG_ENTRIES * sizeof(FxLogEntry), cudaMemcpyHostToDevice);
+  t.log = reinterpret_cast<FxLogEntry*>(t.tw + FX_TABLE);
+  err = cudaMemcpy(t.tw, host.data(), host.size(), cudaMemcpyHostToDevice);
   if (err != cudaSuccess) {
     cudaFree(t.tw);
     return err;

@@ -55,7 +55,7 @@ struct vg_plan {
   // scratch
   double* dens;   // [nx]
   double* mom;    // [nx][MOM_STRIDE]
-  double* bb;     // [nx][2][nv] Thomas elimination scratch (pivots, upper diagonal; FP64 mode)
+  double* bb;     // Thomas elimination scratch, thomas_scratch doubles (null: none is needed; FP64 mode)
   double* rho;    // [nx]
   double* etmp;   // [nx]
   int* flags;     // status bits raised on the device (VG_FLAG_*; null: none kept)
@@ -167,7 +167,7 @@ struct FieldTime {
 };
 cudaError_t launch_poisson_f64(const vg_plan& p, const double* dens, int dens_is_density,
                                const double* driver, const FieldTime& ft, double* e, cudaStream_t s);
-// tridiagonal solve of rows with scratch of 2 thomas_pad(nv) doubles per row;
+// tridiagonal solve of rows with scratch of thomas_scratch doubles (it grows with nrows);
 // nudt_row (per row, 0: leave the row as it is) or nudt for all
 cudaError_t launch_thomas_f64(double* f, int nrows, int nv, const double* v, const double* mom, int mstride,
                               int vbar_col, int vth_col, int dougherty, double nudt, const double* nudt_row, double dv,
@@ -184,6 +184,13 @@ constexpr int THOMAS_CHUNK_NV = 8192;
 constexpr int THOMAS_SERIAL_ROWS = 12288;
 // doubles per scratch array of a row: whole chunks of 32 for a whole number of warps
 __host__ __device__ constexpr size_t thomas_pad(int nv) { return ((size_t)nv + 1023) / 1024 * 1024; }
+// rows that may go either way, by their collisionality (see launch_thomas_f64)
+constexpr bool thomas_either(int nrows, int nv) { return (long long)nrows * nv >= (1 << 20) || nv >= 4096; }
+constexpr size_t thomas_scratch(int nrows, int nv) {
+  return nv > THOMAS_SMEM_NV ? 2 * (size_t)nrows * thomas_pad(nv)
+         : nv < 16 || nrows >= THOMAS_SERIAL_ROWS || thomas_either(nrows, nv) ? 2 * (size_t)nrows * nv
+                                                                              : 0;
+}
 cudaError_t launch_storage_f64(const vg_plan& p, const double* f, const double* e, const double* de,
                                const vg_history& h, int i, cudaStream_t s);
 cudaError_t launch_driver(const vg_plan& p, const FieldTime& ft, double* out, cudaStream_t s);

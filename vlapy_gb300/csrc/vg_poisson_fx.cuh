@@ -14,7 +14,7 @@ struct PoissonFx {
   const int* e;
 };
 // Builds n_runs tables of one nx: inv_kx[r] are DEVICE arrays of nx, g and e the
-// runs' tables, work DEVICE scratch of nx doubles per run
+// runs' tables, work DEVICE scratch of nx doubles per run and nx more
 cudaError_t build_poisson_fx(const double* inv_kx, int nx, int n_runs, int2* g, int* e, double* work, cudaStream_t s);
 
 }  // namespace vg

@@ -556,7 +556,7 @@ __global__ void k_twiddles(cx<double>* __restrict__ t64, cx<float>* __restrict__
   double sn, cs;
   sincospi((double)k / (double)h, &sn, &cs);
   t64[q] = {cs, -sn};
-  t32[q] = {(float)cs, (float)-sn};
+  if (t32) t32[q] = {(float)cs, (float)-sn};
 }
 
 cudaError_t launch_twiddles(vg_plan& p, cudaStream_t s) {

@@ -498,7 +498,7 @@ cudaError_t launch_thomas_f64(double* f, int nrows, int nv, const double* v, con
   // device: both kernels are launched and one of them returns (an idle launch is 2 us).
   // The mean of sqrt(c) decides for all rows: the serial kernel takes as long for a few.
   const long long cells = (long long)nrows * nv;
-  a.either = cells >= (1 << 20) || nv >= 4096;
+  a.either = thomas_either(nrows, nv);
   double root = 40000.0 / nrows;
   if (cells < (1 << 20) || (nv >= 4096 && root > 200.0)) root = 200.0;
   a.stiff = (float)(32.0 * root * std::sqrt(dv_sq));
