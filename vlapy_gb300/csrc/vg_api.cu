@@ -509,7 +509,7 @@ int setup_f32(vg_plan* p, const vg_run_desc* d) {
   for (int k = 0; k < 7; ++k) q->rc.f0m[k] = mom[k];
   q->rc.dv2f = split_f2(dv);
   q->rc.idv2f = split_f2(1.0 / dv2);
-  for (int k = 0; k < 7; ++k) q->rc.f0m2f[k] = split_f2(mom[k]);
+  for (int k = 0; k < 3; ++k) q->rc.f0m2f[k] = split_f2(mom[k]);
   VG_CHECK(upload(p, &q->rc_dev, std::vector<RowConsts>(1, q->rc), "f32 constants"));
   int dev = 0, nsm = 1;
   cudaGetDevice(&dev);

@@ -137,10 +137,10 @@ __device__ __forceinline__ double row_moment(const double* __restrict__ slots, i
   return q < 7 ? rc.dv * sum + rc.f0m[q] : rc.dv * sum;
 }
 
-// the same in double-float (7e-15 relative), off the FP64 pipe
-__device__ __forceinline__ df32 row_moment_df(const double* __restrict__ slots, int q, const RowConsts& rc) {
-  const df32 m = df_mul({rc.dv2f.x, rc.dv2f.y}, reinterpret_cast<const df32*>(slots)[q]);
-  return q < 7 ? df_add(m, {rc.f0m2f[q].x, rc.f0m2f[q].y}) : m;
+// the same without the background's share (slot 7 has none apart) in double-float (7e-15
+// relative), off the FP64 pipe
+__device__ __forceinline__ df32 row_deviation_df(const double* __restrict__ slots, int q, const RowConsts& rc) {
+  return df_mul({rc.dv2f.x, rc.dv2f.y}, reinterpret_cast<const df32*>(slots)[q]);
 }
 
 // rotation of one packed row pair with the delta-f background term; the 1/N of

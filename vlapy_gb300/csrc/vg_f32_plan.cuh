@@ -22,7 +22,7 @@ struct RowConsts {
   // the same in double-float, for the per-row collision scalars (the FP64
   // pipe of this part is 1/64 of FP32, so a row's scalars stay off it)
   float2 dv2f, idv2f;  // dv and 1 / dv^2 split (hi, lo)
-  float2 f0m2f[7];     // f0m split
+  float2 f0m2f[3];     // f0m[0..2] split
 };
 
 struct RowArgs {

@@ -534,9 +534,10 @@ __global__ void __launch_bounds__(sweep_row_block(N), KICK ? (sweep_row_radix(N)
 
 // e history row and the seven series of every run (one CTA per run, one
 // row per thread): each warp adds its rows' double-float sums by
-// transposition, then seven threads add the four warps' totals in order.  The
-// moments are formed in double-float as well (in FP64 they were some 60
-// instructions a row at 64 cycles each: 42 us for 4096 runs, now 18).
+// transposition, then seven threads add the four warps' totals in order.  The rows'
+// deviations from the background are formed in double-float as well (in FP64 they
+// were some 60 instructions a row at 64 cycles each: 42 us for 4096 runs, now 18); the
+// background's share, by far the larger part, is added once, in FP64.
 __global__ void __launch_bounds__(128) k_sweep_store(const SweepRunDev* __restrict__ runs, int n_runs,
                                                      const SweepConsts* __restrict__ scp,
                                                      const double* __restrict__ mom, const float* __restrict__ e32,
@@ -555,9 +556,9 @@ __global__ void __launch_bounds__(128) k_sweep_store(const SweepRunDev* __restri
     const double* slots = mom + (size_t)(r.x_off + x) * MOM_STRIDE;
     // e^2 exactly (the field is an FP32 value); no driver
     const float e2 = ex * ex;
-    const df32 src[7] = {row_moment_df(slots, 0, rc), row_moment_df(slots, 1, rc), row_moment_df(slots, 2, rc),
-                         {e2, fmaf(ex, ex, -e2)},     {0.f, 0.f},                  row_moment_df(slots, 6, rc),
-                         row_moment_df(slots, 7, rc)};
+    const df32 src[7] = {row_deviation_df(slots, 0, rc), row_deviation_df(slots, 1, rc), row_deviation_df(slots, 2, rc),
+                         {e2, fmaf(ex, ex, -e2)},        {0.f, 0.f},                     row_deviation_df(slots, 6, rc),
+                         row_deviation_df(slots, 7, rc)};
 #pragma unroll
     for (int q = 0; q < 7; ++q) acc[q] = df_add(acc[q], src[q]);
   }
@@ -569,7 +570,8 @@ __global__ void __launch_bounds__(128) k_sweep_store(const SweepRunDev* __restri
   if (s_row && threadIdx.x < 7) {
     df32 t = red[0][threadIdx.x];
     for (int w = 1; w < 4; ++w) t = df_add(t, red[w][threadIdx.x]);
-    s_row[(size_t)blockIdx.x * 7 + threadIdx.x] = df_to_double(t) / r.nx;
+    const double back = threadIdx.x < 3 ? rc.f0m[threadIdx.x] : threadIdx.x == 5 ? rc.f0m[6] : 0.0;
+    s_row[(size_t)blockIdx.x * 7 + threadIdx.x] = df_to_double(t) / r.nx + back;
   }
 }
 
@@ -873,7 +875,7 @@ int sweep_class(vg_sweep* s, int cls, int nv) {
   for (int k = 0; k < 7; ++k) rc.f0m[k] = mom[k];
   rc.dv2f = split_f2(dv);
   rc.idv2f = split_f2(1.0 / dv2);
-  for (int k = 0; k < 7; ++k) rc.f0m2f[k] = split_f2(mom[k]);
+  for (int k = 0; k < 3; ++k) rc.f0m2f[k] = split_f2(mom[k]);
   s->consts_h.F0[cls] = dF0;
   s->consts_h.v64[cls] = dv64;
   s->consts_h.c0[cls] = split_f2(mom[0] - 1.0);
