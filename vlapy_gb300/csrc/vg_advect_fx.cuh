@@ -23,6 +23,7 @@ void fx_tables_release(FxTables* t);
 // the step k1 of a wavenumber grid k[m] = m k1, h + l
 struct FxStep {
   double h, l;
+  float own;  // the largest modulus of fx_step_rest's
 };
 // turns per index and unit field or velocity of the phase ((-k) dt) c with k =
 // m k1: A = -k1 dt / (2 pi) to 62 bits; false when it is not finite
@@ -32,9 +33,8 @@ bool fx_make_turn(FxStep k1, double dt, FxTurn* out);
 // (k[1]'s own rounding, taken m times, would be an error of up to 2^-53 of every phase
 // beside those that the k[m] have)
 bool fx_uniform(const double* k, int n, FxStep* k1);
-// what is left of the wavenumbers k[1 .. n / 2] past the step, (k[m] - m k1) 2^64 / (2 pi),
-// and at 0 (where nothing is) the largest modulus of these
-std::vector<float> fx_step_rest(const double* k, int n, FxStep k1);
+// what is left of the wavenumbers k[0 .. n / 2] past the step, (k[m] - m k1) 2^64 / (2 pi)
+std::vector<float> fx_step_rest(const double* k, int n, FxStep* k1);
 
 // v-advection of nrows rows of nv (a power of two <= 8192) by dt; rest: fx_step_rest's
 // of kv; tw64 for the row pairs that go through doubles

@@ -320,7 +320,8 @@ int collision_f64(vg_plan* p, double* f, cudaStream_t s) {
                        "collision moments"));
   return cuda_status(prof_run(p, PK_FP_SOLVE, s, [&] {
                        return launch_thomas_f64(f, p->nx, p->nv, p->v, p->mom, MOM_STRIDE, 0, 1,
-                                                p->collision == VG_COLL_DG, p->nudt, nullptr, p->dv, p->dv_sq, p->bb, s);
+                                                p->collision == VG_COLL_DG, p->nudt, nullptr, p->root_most, p->dv, p->dv_sq, p->bb,
+                                                s);
                      }),
                      "tridiagonal solve");
 }
@@ -675,6 +676,7 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
   p->dv = d->dv;
   p->dv_sq = d->dv_sq;
   p->nudt = d->nu * d->dt;
+  p->root_most = thomas_root_most(std::sqrt(p->nudt), d->v, d->nv);
   p->nx_pow2 = is_pow2(d->nx);
   p->nv_pow2 = is_pow2(d->nv);
   const size_t nx = d->nx, nv = d->nv;
@@ -702,8 +704,8 @@ int vg_plan_create(const vg_run_desc* d, vg_plan** out) {
     p->tw_fx = p->fx_tables->tw;
     p->kv_uniform = fx_uniform(d->kv, d->nv, &p->kv1);
     p->kx_uniform = fx_uniform(d->kx, d->nx, &p->kx1);
-    if (p->kv_uniform) TRY(upload(p, &p->rest_v, fx_step_rest(d->kv, d->nv, p->kv1), "kv"));
-    if (p->kx_uniform) TRY(upload(p, &p->rest_x, fx_step_rest(d->kx, d->nx, p->kx1), "kx"));
+    if (p->kv_uniform) TRY(upload(p, &p->rest_v, fx_step_rest(d->kv, d->nv, &p->kv1), "kv"));
+    if (p->kx_uniform) TRY(upload(p, &p->rest_x, fx_step_rest(d->kx, d->nx, &p->kx1), "kx"));
     const bool dx = !p->nx_pow2 && d->nx <= DFT_ADVECT_NMAX, dv = !p->nv_pow2 && d->nv <= DFT_ADVECT_NMAX;
     if (dv) {
       TRY(dev_copy<fxw>(p, &p->dft_v, nullptr, nv, "DFT angles"));

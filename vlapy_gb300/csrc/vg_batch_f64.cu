@@ -112,7 +112,7 @@ struct vg_batch {
     long long f_off;
     int x_off, rows;
     int pw_v_leaves;
-    double dv, dv_sq;
+    double dv, dv_sq, root_most;
     FxStep kv1;
     int kv_uniform;
     double *v, *kv, *v_pow;
@@ -289,7 +289,8 @@ int batch_sequence(vg_batch* b, double* f, double* e, int nsteps, double* e_hist
                           for (const auto& c : b->cls) {
                             const cudaError_t err = launch_thomas_f64(
                                 f + c.f_off, c.rows, c.nv, c.v, b->fpmom + (size_t)c.x_off * 2, 2, 0, 1,
-                                b->collision == VG_COLL_DG, 0.0, b->nudt_row + c.x_off, c.dv, c.dv_sq, b->bb, s);
+                                b->collision == VG_COLL_DG, 0.0, b->nudt_row + c.x_off, c.root_most, c.dv, c.dv_sq,
+                                b->bb, s);
                             if (err != cudaSuccess) return err;
                           }
                           return cudaSuccess;
@@ -404,7 +405,7 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
       c.dv_sq = d.dv_sq;
       c.kv_uniform = fx_uniform(d.kv, d.nv, &c.kv1);
       if (c.kv_uniform) {
-        const std::vector<float> rest = fx_step_rest(d.kv, d.nv, c.kv1);
+        const std::vector<float> rest = fx_step_rest(d.kv, d.nv, &c.kv1);
         B_TRY(b_alloc(b, &c.rest_v, rest.size(), rest.data(), "batch grids"));
       }
       B_TRY(b_alloc(b, &c.v, d.nv, d.v, "batch grids"));
@@ -441,9 +442,15 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
     kx_all.insert(kx_all.end(), d.kx, d.kx + d.nx);
     // nu * dt as vg_plan_create forms it; 0 leaves the run's rows as they are
     const double nudt = (d.collision != VG_COLL_NONE && d.nu > 0.0) ? d.nu * d.dt : 0.0;
+    c.root_most += d.nx * std::sqrt(nudt);  // (a sum over the class's rows so far)
     nudt_row.insert(nudt_row.end(), (size_t)d.nx, nudt);
     cells += (long long)d.nx * d.nv;
     xoff += d.nx;
+  }
+  for (auto& c : b->cls) {
+    const vg_run_desc* d = runs;
+    while (d->nv != c.nv) ++d;
+    c.root_most = thomas_root_most(c.root_most / c.rows, d->v, c.nv);
   }
   b->cells = cells;
   b->x_points = xoff;
@@ -490,12 +497,13 @@ int vg_batch_create(const vg_run_desc* runs, int32_t n_runs, vg_batch** out) {
     const vg_run_desc& d = runs[i];
     fx_runs[i] = {rd[i].f_off, d.nv, rd[i].v, nullptr, {}};
     FxStep k1;
-    const bool ok = fx_uniform(d.kx, d.nx, &k1) && fx_make_turn(k1, d.dt, &fx_runs[i].turn);
+    const bool uniform = fx_uniform(d.kx, d.nx, &k1);
     rest_off.push_back(rest.size());
-    if (ok) {
-      const std::vector<float> one = fx_step_rest(d.kx, d.nx, k1);
+    if (uniform) {
+      const std::vector<float> one = fx_step_rest(d.kx, d.nx, &k1);
       rest.insert(rest.end(), one.begin(), one.end());
     }
+    const bool ok = uniform && fx_make_turn(k1, d.dt, &fx_runs[i].turn);
     key_of[i] = XKey(d.nx, ok);
     pairs_of[key_of[i]] += (d.nv + 1) / 2;
   }

@@ -131,7 +131,7 @@ __device__ __forceinline__ void dft_fwd(const double* __restrict__ f, int N, int
   if (rot) {
     const double cl = (part ? bad[1] : bad[0]) ? 0.0 : c[l0 + part];
     // (the wavenumber's own rounding, some 2^-53 of the phase, in FP32)
-    const long long own = k ? __float2ll_rn(-rest[k] * dt * (float)cl) : 0;
+    const long long own = __float2ll_rn(-rest[k] * dt * (float)cl);
     p = fx_mult(fx_sincos((unsigned long long)k * fx_turn(turn, cl) + (unsigned long long)own, tw));
   }
   __syncthreads();

@@ -86,8 +86,7 @@ __global__ void __launch_bounds__(fx_row_block(N), fx_row_block(N) > 256 ? 1 : 2
   fx_fft<N, false, true, false>(s, t, tw, sync, io);
   const unsigned long long ta = fx_turn(turn, bad_a ? 0.0 : ea), tb = fx_turn(turn, bad_b ? 0.0 : eb);
   const float oa = bad_a ? 0.f : fx_own_scale(dt, ea), ob = bad_b ? 0.f : fx_own_scale(dt, eb);
-  // (entry 0 of rest: the largest)
-  const bool own = rest[0] * fmaxf(fabsf(oa), fabsf(ob)) > FX_OWN_LEAST;
+  const bool own = turn.own * fmaxf(fabsf(oa), fabsf(ob)) > FX_OWN_LEAST;
   FxNorms n = fx_rotate<N, DOWN>(s, t, ta, tb, own, oa, ob, rest, tw);
   n.l1 = __reduce_add_sync(mask, n.l1);
   n.a2 = __reduce_add_sync(mask, n.a2);
@@ -273,11 +272,12 @@ bool fx_make_turn(FxStep k1, double dt, FxTurn* out) {
   const double m = std::frexp(a.h, &e);
   out->am = -((long long)std::ldexp(m, 62) + (long long)std::llrint(std::ldexp(a.l, 62 - e)));
   out->ae = e - 62;
+  out->own = k1.own;
   return true;
 }
 
 bool fx_uniform(const double* k, int n, FxStep* k1) {
-  *k1 = {k[n > 1 ? 1 : 0], 0.0};
+  *k1 = {k[n > 1 ? 1 : 0], 0.0, 0.f};
   for (int m = 0; m <= n / 2; ++m) {
     const double want = m * k[n > 1 ? 1 : 0], tol = 1e-15 * std::fabs(want);
     if (!(std::fabs(std::fabs(k[m % n]) - std::fabs(want)) <= tol)) return false;
@@ -295,16 +295,16 @@ bool fx_uniform(const double* k, int n, FxStep* k1) {
   if (std::fabs(num.h) > 1e-250 && std::fabs(num.h) < 1e250) {
     const double q = num.h / den;
     const dd s = dd_norm(q, (std::fma(-q, den, num.h) + num.l) / den);
-    *k1 = {s.h, s.l};
+    *k1 = {s.h, s.l, 0.f};
   }
   return true;
 }
 
-std::vector<float> fx_step_rest(const double* k, int n, FxStep k1) {
+std::vector<float> fx_step_rest(const double* k, int n, FxStep* k1) {
   std::vector<float> r(n / 2 + 1, 0.f);
   for (int m = 1; m <= n / 2; ++m) {
-    r[m] = (float)((std::fma(-(double)m, k1.h, std::copysign(k[m], k1.h)) - m * k1.l) * std::ldexp(kInv2Pi.h, 64));
-    r[0] = std::max(r[0], std::fabs(r[m]));
+    r[m] = (float)((std::fma(-(double)m, k1->h, std::copysign(k[m], k1->h)) - m * k1->l) * std::ldexp(kInv2Pi.h, 64));
+    k1->own = std::max(k1->own, std::fabs(r[m]));
   }
   return r;
 }

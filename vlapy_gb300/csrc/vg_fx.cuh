@@ -430,6 +430,7 @@ __device__ __forceinline__ double fx_to_double(long long v, int k) {
 struct FxTurn {
   long long am;
   int ae;
+  float own;  // the largest modulus of fx_step_rest's
 };
 __device__ __forceinline__ unsigned long long fx_turn(FxTurn A, double c) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(c);
@@ -485,14 +486,14 @@ __device__ __forceinline__ fxc fx_turn_by(fxc a, const fxw& w) {
 // fx_own_scale, a small angle in Q64, is turned on top of the m steps.  (Without it the
 // phases' errors are those of the doubles ((-k) dt) c, twice to thirty times the
 // transform's on lines with all wavenumbers in them.)  It is 3 % of the x-drift; below
-// 2^-53, the wavenumbers' rounding of phases of a radian or two, it is left out: a small
-// part of the transform's own error.
+// 2^-51, what the wavenumbers' rounding makes of phases of ten radians or so, it is left
+// out: the transform's own error is as large.
 __device__ __forceinline__ float fx_own_scale(double dt, double c) { return -6.28318531f * (float)dt * (float)c; }
 __device__ __forceinline__ fxc fx_own(fxc p, float own) {
   const int d = __float2int_rn(own);
   return {p.c - __mulhi((int)(p.s >> 32), d), p.s + __mulhi((int)(p.c >> 32), d)};
 }
-constexpr float FX_OWN_LEAST = 2048.f;  // 2^-53 in Q64
+constexpr float FX_OWN_LEAST = 8192.f;  // 2^-51 in Q64
 
 // What the rotation learns about the bins it leaves: an upper bound of the sum
 // of their moduli in units of 2^38, and the sums of the squares of line a's and

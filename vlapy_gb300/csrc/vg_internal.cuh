@@ -16,7 +16,7 @@ struct vg_plan {
   void* arena;  // the plan's device memory (all arrays below but the spline's)
   // scalars of the run
   int nx, nv, precision, collision, integrator, n_pulses;
-  double dt, nu, dx, dv, dv_sq, nudt;
+  double dt, nu, dx, dv, dv_sq, nudt, root_most;
   int nx_pow2, nv_pow2;
   // device constants
   double* x;
@@ -168,10 +168,13 @@ struct FieldTime {
 cudaError_t launch_poisson_f64(const vg_plan& p, const double* dens, int dens_is_density,
                                const double* driver, const FieldTime& ft, double* e, cudaStream_t s);
 // tridiagonal solve of rows with scratch of thomas_scratch doubles (it grows with nrows);
-// nudt_row (per row, 0: leave the row as it is) or nudt for all
+// nudt_row (per row, 0: leave the row as it is) or nudt for all; root_most: an upper
+// estimate of the rows' mean of sqrt(nudt vth) (speed only)
 cudaError_t launch_thomas_f64(double* f, int nrows, int nv, const double* v, const double* mom, int mstride,
-                              int vbar_col, int vth_col, int dougherty, double nudt, const double* nudt_row, double dv,
-                              double dv_sq, double* scratch, cudaStream_t s);
+                              int vbar_col, int vth_col, int dougherty, double nudt, const double* nudt_row,
+                              double root_most, double dv, double dv_sq, double* scratch, cudaStream_t s);
+// root_most of rows with a mean square root of nudt of `root`: 2 max|v| of it (vth <= n v^2, n <= 4)
+double thomas_root_most(double root, const double* v, int nv);
 // longest row whose chunked solve keeps all its arrays in shared memory, and
 // longest row it takes at all
 constexpr int THOMAS_SMEM_NV = 4096;

@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(field32_block(NX)) k_field_f32(
   constexpr int B = field32_block(NX);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double amp[FIELD32_PULSES];
-  __shared__ unsigned sounding;  // bit i: pulse i adds to the field (a NaN amplitude does)
+  __shared__ bool sounding[FIELD32_PULSES];  // the pulse adds to the field (a NaN amplitude does)
   cx<float>* s = reinterpret_cast<cx<float>*>(smem_raw);
   float* drv = reinterpret_cast<float*>(s + sp_len<float>(NX));  // [NX]
   const int t = threadIdx.x;
@@ -136,19 +136,17 @@ __global__ void __launch_bounds__(field32_block(NX)) k_field_f32(
   if (pulses)
     for (int p0 = 0; p0 < np; p0 += FIELD32_PULSES) {
       const int n_here = min(FIELD32_PULSES, np - p0);
-      if (t >= B - 32) {
+      if (t >= B - 32 && t - (B - 32) < n_here) {
         const int i = t - (B - 32);
         double a = 0.0;
-        const bool on = i < n_here && pulse_amplitude(P[p0 + i], tt, &a);
+        sounding[i] = pulse_amplitude(P[p0 + i], tt, &a);
         amp[i] = a;
-        const unsigned mask = __ballot_sync(0xffffffffu, on);
-        if (i == 0) sounding = mask;
       }
       __syncthreads();
       for (int n = t; n < NX; n += B) {
         float total = drv[n];
         for (int i = 0; i < n_here; ++i) {
-          if (!(sounding >> i & 1)) continue;  // a silent pulse adds nothing
+          if (!sounding[i]) continue;  // a silent pulse adds nothing
           const double a = amp[i];
           const vg_pulse& q = P[p0 + i];
           double arg = q.k0 * x[n] - q.w0 * tt;

@@ -42,6 +42,7 @@
 // that is some 90 cycles an element on the FP32 and integer pipes, where the FP64
 // sweep takes 130 to 600, and leaves about nine elements to sweep again: two sweeps
 // instead of two to eight, 2048 x 4096 from 1.31 to 1.07 ms, 64 x 1024 from 45 to 33 us.
+#include <algorithm>
 #include <cmath>
 
 #include "vg_internal.cuh"
@@ -135,7 +136,7 @@ struct ThomasArgs {
 // Whether the launch is k_thomas_serial's: the same answer in every warp of both
 // kernels, from 32 rows spread over all (whole warps call it)
 __device__ __forceinline__ bool all_stiff(const ThomasArgs& a) {
-  const size_t row = (size_t)((long long)(threadIdx.x & 31) * a.nrows / 32);
+  const size_t row = (size_t)((threadIdx.x & 31) * (unsigned)a.nrows / 32);
   const double nudt = a.nudt_row ? a.nudt_row[row] : a.nudt;
   float q = __fsqrt_rn(__double2float_rn(__dmul_rn(nudt, a.mom[row * a.mstride + a.vth_col])));
 #pragma unroll
@@ -478,9 +479,15 @@ cudaError_t chunks(const ThomasArgs& a, cudaStream_t s) {
 
 }  // namespace
 
+double thomas_root_most(double root, const double* v, int nv) {
+  double vmax = 0.0;
+  for (int j = 0; j < nv; ++j) vmax = std::max(vmax, std::fabs(v[j]));
+  return 2.0 * root * vmax;
+}
+
 cudaError_t launch_thomas_f64(double* f, int nrows, int nv, const double* v, const double* mom, int mstride,
-                              int vbar_col, int vth_col, int dougherty, double nudt, const double* nudt_row, double dv,
-                              double dv_sq, double* scratch, cudaStream_t s) {
+                              int vbar_col, int vth_col, int dougherty, double nudt, const double* nudt_row,
+                              double root_most, double dv, double dv_sq, double* scratch, cudaStream_t s) {
   ThomasArgs a = {f, nrows, nv, v, mom, mstride, vbar_col, vth_col, dougherty, nudt, nudt_row, dv, dv_sq,
                   scratch, false, 0.f};
   if (nv > THOMAS_CHUNK_NV || nv < 16 || nrows >= THOMAS_SERIAL_ROWS) {
@@ -497,11 +504,14 @@ cudaError_t launch_thomas_f64(double* f, int nrows, int nv, const double* v, con
   // fills an SM (4 x 4096 meets at 2e4, 64 x 8192 at 6e4).  vth is only known on the
   // device: both kernels are launched and one of them returns (an idle launch is 2 us).
   // The mean of sqrt(c) decides for all rows: the serial kernel takes as long for a few.
+  // Where root_most, from the largest vth that a density of four or less has on the
+  // grid, is below the line, the serial kernel is not launched.
   const long long cells = (long long)nrows * nv;
-  a.either = thomas_either(nrows, nv);
   double root = 40000.0 / nrows;
   if (cells < (1 << 20) || (nv >= 4096 && root > 200.0)) root = 200.0;
-  a.stiff = (float)(32.0 * root * std::sqrt(dv_sq));
+  root *= std::sqrt(dv_sq);
+  a.either = thomas_either(nrows, nv) && !(root_most < root);
+  a.stiff = (float)(32.0 * root);
   // The shortest chunk that still gives every scheduler at most two warps (152
   // x 8 = 1216): a lane's share of the parallel work falls with L, while the
   // elements swept again do not depend on it, so once the schedulers are full

@@ -103,8 +103,7 @@ __global__ void __launch_bounds__(fx_col_block(NX), fx_col_block(NX) > 256 ? 1 :
   fx_fft<NX, false, true, false>(s, t, tw, sync, io);
   const unsigned long long ta = fx_turn(r.turn, bad_a ? 0.0 : ca), tb = fx_turn(r.turn, bad_b ? 0.0 : cb);
   const float oa = bad_a ? 0.f : fx_own_scale(dt, ca), ob = bad_b ? 0.f : fx_own_scale(dt, cb);
-  // (entry 0 of rest: the largest)
-  const bool own = r.rest[0] * fmaxf(fabsf(oa), fabsf(ob)) > FX_OWN_LEAST;
+  const bool own = r.turn.own * fmaxf(fabsf(oa), fabsf(ob)) > FX_OWN_LEAST;
   FxNorms n = fx_rotate<NX, DOWN>(s, t, ta, tb, own, oa, ob, r.rest, tw);
   if constexpr (G > 1) {
     atomicAdd(&red[5 * p + 2], n.l1);
@@ -126,9 +125,13 @@ __global__ void __launch_bounds__(fx_col_block(NX), fx_col_block(NX) > 256 ? 1 :
     fx_pair_f64<NX>({fc, ta, oa, fx_up(Ea, n.a2), va && turned, bad_a}, {fc + 1, tb, ob, fx_up(Eb, n.b2), vb && turned, bad_b},
                     nv, sd, t, r.rest, tw, tw64, sync);
   };
-  if (n_turned == (int)blockDim.x) {
-    in_doubles();
-    return;
+  // (short columns are hardly ever turned away, and a second copy of the call is 2 us of
+  // a cold launch)
+  if constexpr (NX >= 256) {
+    if (n_turned == (int)blockDim.x) {
+      in_doubles();
+      return;
+    }
   }
   fx_fft<NX, true, false, true>(s, t, tw, sync, io, turned ? 16 : h);
   // lines of zeros stay so: the partner's rounding does not reach them
