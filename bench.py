@@ -1016,7 +1016,7 @@ def main():
 def main_sweep(args, w, rank, world):
     cfg = {"workload": "sweep", "n_runs": w["n_runs"], "seed": w["seed"], "nx": [32, 64, 128],
            "nv": [256, 512, 1024], "vmax": w["vmax"], "dt": w["dt"], "collision": "dg (25% of runs nu=0)",
-           "integrator": "leapfrog", "precision": "fp32-deltaf (FP64 moment/zero-mode reductions)",
+           "integrator": "leapfrog", "precision": "fp32-deltaf (double-float moment/zero-mode reductions)",
            "storage": "per run and step: field e[nx] + 7 series", "run_steps": SWEEP_STEPS}
     if args.impl == "reference":
         if rank != 0:

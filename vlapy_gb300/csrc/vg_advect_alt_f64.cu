@@ -108,7 +108,9 @@ __global__ void k_sl_solve_x(const double* __restrict__ f, double* __restrict__ 
 // backward) are composed for it, and it replays its chunk from the value that gives.
 // The maps contract (|w_q| < 0.27), so the reassociation changes only rounding.  It is
 // twice the FP64 instructions of one thread a line, each 64 cycles a warp whatever the
-// number of warps, so it pays as long as schedulers are idle.
+// number of warps, so for the x step it pays as long as schedulers are idle.  The v step
+// is split over a row's lanes in any case (its columns lie side by side in memory); more
+// warps a row add little to that and never took longer (8192 x 512: 390 -> 369 us).
 
 // x step, SL_X_SPLIT warps per 32 columns, each with a chunk of the nx unknowns.  One
 // thread a column took 33 us at 64 x 1024 (32 warps on the whole chip), now 14.
@@ -355,7 +357,7 @@ __global__ void k_edfdv_cd2(const double* __restrict__ fin, double* __restrict__
 
 int cell_blocks(size_t cells) {
   const size_t b = (cells + 255) / 256;
-  return (int)(b < 152 * 16 ? (b ? b : 1) : 152 * 16);
+  return (int)(b < GB300_SMS * 16 ? (b ? b : 1) : GB300_SMS * 16);
 }
 
 }  // namespace
@@ -387,8 +389,8 @@ cudaError_t ensure_sl_scratch(vg_plan& p) {
 
 cudaError_t launch_vdfdx_sl_f64(const vg_plan& p, const double* fin, double* fout, double dt, cudaStream_t s) {
   // one-warp CTAs (each column's chain is bound by its warp's FP64 issue, not by the CTA shape)
-  // split while its warps are no more than two a scheduler (152 x 8)
-  if (p.nx >= 4 * SL_X_SPLIT && div_up(p.nv, 32) * SL_X_SPLIT <= 1216)
+  // split while its warps are no more than two a scheduler
+  if (p.nx >= 4 * SL_X_SPLIT && div_up(p.nv, 32) * SL_X_SPLIT <= 8 * GB300_SMS)
     k_sl_solve_x_split<<<div_up(p.nv, 32), 32 * SL_X_SPLIT, 0, s>>>(fin, p.sl_m, p.nx, p.nv, p.x, p.sl_w);
   else
     k_sl_solve_x<<<div_up(p.nv, 32), 32, 0, s>>>(fin, p.sl_m, p.nx, p.nv, p.x, p.sl_w);

@@ -1,6 +1,6 @@
-// FP64 advection kernels in doubles (wavenumber grids that are not uniform, and
-// lengths that are not powers of two): the exponential integrators in v (rows) and x
-// (columns) of vlapy/core/vlasov.py:83-140, as shared-memory FFTs.
+// FP64 advection kernels in doubles, for wavenumber grids that are not uniform: the
+// exponential integrators in v (rows) and x (columns) of vlapy/core/vlasov.py:83-140, as
+// shared-memory FFTs or, for lengths that are not powers of two, direct DFTs.
 //
 // v-advection (rows).  One group of N/R threads owns a PAIR of rows packed as
 // z = f[a] + i f[b]; one complex FFT of length nv transforms both rows, the

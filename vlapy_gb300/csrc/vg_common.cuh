@@ -7,6 +7,8 @@
 
 namespace vg {
 
+constexpr int GB300_SMS = 152;  // four schedulers each
+
 template <typename T>
 struct __align__(2 * sizeof(T)) cx {
   T x, y;

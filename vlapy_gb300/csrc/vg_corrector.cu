@@ -101,14 +101,6 @@ __device__ __forceinline__ void zero_rows(unsigned char* tile, int r0, int rows)
   }
 }
 
-// The 64-channel tensors of this engine lie as [row][group of 8 channels][position]
-// [8]: a group is the 2 KB run that a tile's group is, so a row comes by eight bulk
-// copies that one thread issues, and the epilogue's store of a group is 512 contiguous
-// bytes a warp.  (With a position's channels together, every load and store of a warp
-// touched 32 lines: 97 us for 64 to 64 channels over 8192 rows and 113 for their
-// gradient, now 50 and 65.)  The 16-channel ones (features, the loss's gradient) are
-// [row][position][16], as the mma.sync engine has all of them.
-//
 // MODE 0: out = relu(conv + b) (bf16); MODE 1: out[p] = conv + b, channel 0
 // only (fp32); MODE 2: out = conv * (mask > 0) (bf16, no bias).
 // Weights W: bf16 [5][COUT][CIN] (for MODE 2: transposed, tap-flipped).

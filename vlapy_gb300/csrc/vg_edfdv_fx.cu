@@ -5,8 +5,10 @@
 // One group of N / 8 threads (N / 16 at 8192) owns a pair of rows as one complex
 // sequence; f is read once and written once.
 //
-// Measured against the transforms in doubles (FP64 pipe 84 % busy): 4096 x 8192
-// 4.44 -> 0.88 ms, 2048 x 4096 1.02 -> 0.23 ms, 64 x 1024 70 -> 16 us.  Bound by
+// Measured against the transforms in doubles (FP64 pipe 84 % busy), smooth rows:
+// 4096 x 8192 4.44 -> 0.88 ms, 2048 x 4096 1.02 -> 0.24 ms, 64 x 1024 70 -> 16 us one
+// launch after another (25 with cold caches).  Rows that go through doubles after all
+// (vg_fx.cuh): 2048 x 4096 of noise 1.01 ms.  Bound by
 // integer issue: a complex product is 12 wide multiplies at a quarter of the
 // add rate.  Radix 16 (3 passes instead of 4 at 4096) takes 0.21 ms there but
 // 34 us at 64 x 1024, where half as many threads carry the latency.  RMS error
@@ -19,6 +21,7 @@
 #include <vector>
 
 #include "vg_advect_fx.cuh"
+#include "vg_dd.cuh"
 #include "vg_internal.cuh"
 
 namespace vg {
@@ -133,7 +136,7 @@ cudaError_t edfdv_fx_n(double* f, int nrows, const double* e, FxTurn turn, doubl
   // groups per CTA: fewer when the pairs would not give every SM two CTAs
   // (a scheduler runs the integer work of one CTA's warps with gaps), whole warps
   int P = fx_row_block(N) / G;
-  while (P > 1 && (P / 2) * G >= 32 && div_up(pairs, P) < 304) P /= 2;
+  while (P > 1 && (P / 2) * G >= 32 && div_up(pairs, P) < 2 * GB300_SMS) P /= 2;
   const size_t smem = (size_t)P * sp_len<double>(N) * sizeof(fx);
   cudaError_t err = ensure_smem((const void*)k_edfdv_fx<N>, smem);
   if (err != cudaSuccess) return err;
@@ -142,22 +145,6 @@ cudaError_t edfdv_fx_n(double* f, int nrows, const double* e, FxTurn turn, doubl
 }
 
 // ---- host tables -------------------------------------------------------------
-// double-double arithmetic by exact products (fma) and two-sums
-struct dd {
-  double h, l;
-};
-dd dd_norm(double a, double b) {
-  const double s = a + b, t = s - a;
-  return {s, (a - (s - t)) + (b - t)};
-}
-dd dd_mul(dd a, dd b) {
-  const double p = a.h * b.h;
-  return dd_norm(p, std::fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h));
-}
-dd dd_add(dd a, dd b) {
-  const dd s = dd_norm(a.h, b.h);
-  return dd_norm(s.h, s.l + (a.l + b.l));
-}
 const dd kPi = {3.141592653589793116, 1.2246467991473532072e-16};
 const dd kInv2Pi = {0.15915494309189534561, -9.8393383375912127e-18};
 
@@ -170,9 +157,8 @@ void dd_cos_sin(int j, dd* c, dd* s) {
   for (int n = 1; n < 16; ++n) {
     const dd pc = dd_mul(tc, x2), ps = dd_mul(ts, x2);
     const double dc = -(2.0 * n - 1.0) * (2.0 * n), ds = -(2.0 * n) * (2.0 * n + 1.0);
-    const double qc = pc.h / dc, qs = ps.h / ds;
-    tc = dd_norm(qc, (std::fma(-qc, dc, pc.h) + pc.l) / dc);
-    ts = dd_norm(qs, (std::fma(-qs, ds, ps.h) + ps.l) / ds);
+    tc = dd_div(pc, dc);
+    ts = dd_div(ps, ds);
     *c = dd_add(*c, tc);
     *s = dd_add(*s, ts);
   }
@@ -293,8 +279,7 @@ bool fx_uniform(const double* k, int n, FxStep* k1) {
   }
   // (far from the ends of the range, where the parts are doubles)
   if (std::fabs(num.h) > 1e-250 && std::fabs(num.h) < 1e250) {
-    const double q = num.h / den;
-    const dd s = dd_norm(q, (std::fma(-q, den, num.h) + num.l) / den);
+    const dd s = dd_div(num, den);
     *k1 = {s.h, s.l, 0.f};
   }
   return true;

@@ -566,9 +566,7 @@ __device__ __forceinline__ FxNorms fx_rotate(fx* s, int t, unsigned long long fa
 // fx_cmul<2> overflow), or -1 where the error of the result, FX_NOISE sqrt(N)
 // 2^h units, exceeds that of the transform in doubles, 1e-16 (1 + log2(N) / 5)
 // of a line's RMS.  A line that is zero (no_a, no_b) has no error to speak of.
-#ifndef FX_NOISE
-#define FX_NOISE 0.6f
-#endif
+constexpr float FX_NOISE = 0.6f;
 template <int N>
 __device__ __forceinline__ int fx_shift_back(const FxNorms& n, bool no_a, bool no_b) {
   constexpr unsigned lim = 7827145u;  // 2^22.9

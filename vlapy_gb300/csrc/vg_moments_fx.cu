@@ -27,6 +27,7 @@
 #include <cmath>
 #include <vector>
 
+#include "vg_dd.cuh"
 #include "vg_internal.cuh"
 #include "vg_moments_fx.cuh"
 
@@ -275,29 +276,12 @@ __global__ void k_powers(const double* __restrict__ v, const double* __restrict_
 }
 
 // log(c / 2^15) by the series of 2 atanh((c - 2^15) / (c + 2^15)) in double-double
-struct dd {
-  double h, l;
-};
-dd dd_norm(double a, double b) {
-  const double s = a + b, t = s - a;
-  return {s, (a - (s - t)) + (b - t)};
-}
-dd dd_mul(dd a, dd b) {
-  const double p = a.h * b.h;
-  return dd_norm(p, std::fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h));
-}
-dd dd_div(double a, double b) {
-  const double q = a / b;
-  return dd_norm(q, std::fma(-q, b, a) / b);
-}
 long long log_of(int c) {
-  const dd z = dd_div((double)(c - 32768), (double)(c + 32768)), z2 = dd_mul(z, z);
+  const dd z = dd_div({(double)(c - 32768), 0.0}, (double)(c + 32768)), z2 = dd_mul(z, z);
   dd term = z, sum = z;
   for (int n = 3; n < 60; n += 2) {
     term = dd_mul(term, z2);
-    const dd t = dd_mul(term, dd_div(1.0, (double)n));
-    const dd s = dd_norm(sum.h, t.h);
-    sum = dd_norm(s.h, s.l + (sum.l + t.l));
+    sum = dd_add(sum, dd_mul(term, dd_div({1.0, 0.0}, (double)n)));
   }
   return 2 * ((long long)std::llrint(std::ldexp(sum.h, 56)) + (long long)std::llrint(std::ldexp(sum.l, 56)));
 }
@@ -355,7 +339,7 @@ cudaError_t launch_moments_fx(const double* f, int nrows, int nv, const double* 
   // four to eight elements a thread, whole warps; two where the rows do not fill the chip
   // (64 x 1024: 15.4 -> 14.4 us)
   int block = nv >= 1024 ? 256 : nv >= 512 ? 128 : 64;
-  if (nrows <= 152) block *= 2;
+  if (nrows <= GB300_SMS) block *= 2;
   if (full) k_moments_fx<true><<<nrows, block, 0, s>>>(f, nv, pw, table, dv, v, v_pow, out, stride);
   else k_moments_fx<false><<<nrows, block, 0, s>>>(f, nv, pw, table, dv, v, v_pow, out, stride);
   return cudaGetLastError();

@@ -512,13 +512,12 @@ cudaError_t launch_thomas_f64(double* f, int nrows, int nv, const double* v, con
   root *= std::sqrt(dv_sq);
   a.either = thomas_either(nrows, nv) && !(root_most < root);
   a.stiff = (float)(32.0 * root);
-  // The shortest chunk that still gives every scheduler at most two warps (152
-  // x 8 = 1216): a lane's share of the parallel work falls with L, while the
+  // The shortest chunk that still gives every scheduler at most two warps: a lane's share of the parallel work falls with L, while the
   // elements swept again do not depend on it, so once the schedulers are full
   // longer chunks waste less (32: five arrays of a warp's chunks take 42 KB, and
   // four warps must fit an SM)
-  const cudaError_t err = nv <= 4096 && cells < 32LL * 8 * 1216 ? chunks<8>(a, s)
-                          : cells < 32LL * 16 * 1216            ? chunks<16>(a, s)
+  const cudaError_t err = nv <= 4096 && cells < 32LL * 8 * (8 * GB300_SMS) ? chunks<8>(a, s)
+                          : cells < 32LL * 16 * (8 * GB300_SMS)            ? chunks<16>(a, s)
                                                                 : chunks<32>(a, s);
   if (err != cudaSuccess || !a.either) return err;
   k_thomas_serial<<<div_up(nrows, 64), 64, 0, s>>>(a);

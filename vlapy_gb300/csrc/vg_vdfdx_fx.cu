@@ -7,8 +7,9 @@
 // read one row segment of 16 S bytes; every element goes from global memory to
 // registers and back once, and shared memory carries only the passes between.
 //
-// Measured against the transforms in doubles: 4096 x 8192 4.26 -> 1.01 ms, 2048
-// x 4096 0.98 -> 0.23 ms, 64 x 1024 57 -> 15 us.  Bound as the v-advection
+// Measured against the transforms in doubles, smooth columns: 4096 x 8192 4.26 ->
+// 1.04 ms, 2048 x 4096 0.98 -> 0.23 ms, 64 x 1024 57 -> 14 us one launch after another
+// (17 with cold caches); of noise 2048 x 4096 0.96 ms.  Bound as the v-advection
 // (vg_edfdv_fx.cu); 128-bit check: 0.8e-16 of the column's RMS at nx = 1024, in
 // doubles 2.6e-16.
 #include <algorithm>
@@ -174,7 +175,7 @@ cudaError_t vdfdx_fx_n(double* f, const FxColRun* runs, const int2* items, int n
 template <int NX>
 int col_pairs_n(long long pairs) {
   int S = fx_col_max_pairs(NX);
-  while (S > 1 && (S / 2) * fx_threads(NX) >= 32 && (pairs + S - 1) / S < 304) S /= 2;
+  while (S > 1 && (S / 2) * fx_threads(NX) >= 32 && (pairs + S - 1) / S < 2 * GB300_SMS) S /= 2;
   return S;
 }
 
