@@ -180,7 +180,7 @@ cudaError_t vdfdx_n(const vg_plan& p, double* f, double dt, cudaStream_t s) {
 cudaError_t launch_edfdv_f64(const vg_plan& p, double* f, const double* e, double dt, cudaStream_t s) {
   FxTurn turn;
   if (p.nv_pow2 && p.tw_fx && p.kv_uniform && fx_make_turn(p.kv1, dt, &turn))
-    return launch_edfdv_fx(f, p.nx, p.nv, e, turn, dt, p.rest_v, p.tw_fx, p.tw64, s);
+    return launch_edfdv_fx(f, p.nx, p.nv, e, turn, p.rest_v, p.tw_fx, p.tw64, s);
   if (!p.nv_pow2 && p.dft_v && p.kv_uniform && fx_make_turn(p.kv1, dt, &turn))
     return launch_dft_fx(f, p.nv, p.nx, 1, p.nv, e, turn, p.rest_v, dt, p.tw_fx, p.dft_v, p.dft_work, s);
   if (!p.nv_pow2) return dft_advect(f, p.nv, p.nx, 1, p.nv, p.kv, e, dt, s);
@@ -195,7 +195,7 @@ cudaError_t launch_edfdv_f64(const vg_plan& p, double* f, const double* e, doubl
 cudaError_t launch_vdfdx_f64(const vg_plan& p, double* f, double dt, cudaStream_t s) {
   FxColRun run = {0, p.nv, p.v, p.rest_x, {}};
   if (p.nx_pow2 && p.tw_fx && p.kx_uniform && fx_make_turn(p.kx1, dt, &run.turn))
-    return launch_vdfdx_fx(f, p.nx, nullptr, nullptr, 0, run, fx_col_pairs(p.nx, (p.nv + 1) / 2), dt, p.tw_fx, p.tw64, s);
+    return launch_vdfdx_fx(f, p.nx, nullptr, nullptr, 0, run, fx_col_pairs(p.nx, (p.nv + 1) / 2), p.tw_fx, p.tw64, s);
   if (!p.nx_pow2 && p.dft_x && p.kx_uniform && fx_make_turn(p.kx1, dt, &run.turn))
     return launch_dft_fx(f, p.nx, p.nv, p.nv, 1, p.v, run.turn, p.rest_x, dt, p.tw_fx, p.dft_x, p.dft_work, s);
   if (!p.nx_pow2) return dft_advect(f, p.nx, p.nv, p.nv, 1, p.kx, p.v, dt, s);

@@ -36,9 +36,9 @@ bool fx_uniform(const double* k, int n, FxStep* k1);
 // what is left of the wavenumbers k[0 .. n / 2] past the step, (k[m] - m k1) 2^64 / (2 pi)
 std::vector<float> fx_step_rest(const double* k, int n, FxStep* k1);
 
-// v-advection of nrows rows of nv (a power of two <= 8192) by dt; rest: fx_step_rest's
+// v-advection of nrows rows of nv (a power of two <= 8192); rest: fx_step_rest's
 // of kv; tw64 for the row pairs that go through doubles
-cudaError_t launch_edfdv_fx(double* f, int nrows, int nv, const double* e, FxTurn turn, double dt, const float* rest,
+cudaError_t launch_edfdv_fx(double* f, int nrows, int nv, const double* e, FxTurn turn, const float* rest,
                             const fxw* tw, const cx<double>* tw64, cudaStream_t s);
 
 // One run of the x-advection: f[nx][nv] at f + f_off
@@ -54,7 +54,7 @@ int fx_col_pairs(int nx, long long pairs);
 // x-advection: items null: run `one`, all its tiles; else (run, tile) items of
 // one nx over runs, tiles of S pairs
 cudaError_t launch_vdfdx_fx(double* f, int nx, const FxColRun* runs, const int2* items, int n_items, FxColRun one, int S,
-                            double dt, const fxw* tw, const cx<double>* tw64, cudaStream_t s);
+                            const fxw* tw, const cx<double>* tw64, cudaStream_t s);
 
 // Lines whose length N is not a power of two (vg_dft_fx.cu): n_lines lines of N
 // elements es apart, line l at l ls with the phase ((-k) dt) c of its double c[l];

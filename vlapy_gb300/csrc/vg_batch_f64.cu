@@ -223,7 +223,7 @@ cudaError_t batch_vdfdx_all(const vg_batch* b, double* f, double dt, cudaStream_
   for (const auto& xc : b->xcls) {
     cudaError_t err = cudaErrorInvalidValue;
     if (xc.fx) {
-      err = launch_vdfdx_fx(f, xc.nx, b->fx_runs, xc.items, xc.n_items, FxColRun{}, xc.W / 2, dt, b->fx_tables->tw, b->tw64, s);
+      err = launch_vdfdx_fx(f, xc.nx, b->fx_runs, xc.items, xc.n_items, FxColRun{}, xc.W / 2, b->fx_tables->tw, b->tw64, s);
       if (err != cudaSuccess) return err;
       continue;
     }

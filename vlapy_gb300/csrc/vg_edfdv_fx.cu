@@ -32,7 +32,7 @@ __host__ __device__ constexpr int fx_row_block(int n) { return fx_threads(n) > 2
 
 template <int N>
 __global__ void __launch_bounds__(fx_row_block(N), fx_row_block(N) > 256 ? 1 : 2)
-    k_edfdv_fx(double* __restrict__ f, int nrows, const double* __restrict__ e, FxTurn turn, double dt,
+    k_edfdv_fx(double* __restrict__ f, int nrows, const double* __restrict__ e, FxTurn turn,
                const float* __restrict__ rest, const fxw* __restrict__ tw, const cx<double>* __restrict__ tw64) {
   constexpr int R = fx_radix(N), G = fx_threads(N);
   constexpr int DOWN = ilog2(N) - fx_shift<N>();
@@ -88,8 +88,12 @@ __global__ void __launch_bounds__(fx_row_block(N), fx_row_block(N) > 256 ? 1 : 2
   }
   fx_fft<N, false, true, false>(s, t, tw, sync, io);
   const unsigned long long ta = fx_turn(turn, bad_a ? 0.0 : ea), tb = fx_turn(turn, bad_b ? 0.0 : eb);
-  const float oa = bad_a ? 0.f : fx_own_scale(dt, ea), ob = bad_b ? 0.f : fx_own_scale(dt, eb);
-  const bool own = turn.own * fmaxf(fabsf(oa), fabsf(ob)) > FX_OWN_LEAST;
+  const bool own = fx_has_own(turn, ea) || fx_has_own(turn, eb);
+  float oa = 0.f, ob = 0.f;
+  if (own) {
+    oa = bad_a ? 0.f : turn.own * (float)ea;
+    ob = bad_b ? 0.f : turn.own * (float)eb;
+  }
   FxNorms n = fx_rotate<N, DOWN>(s, t, ta, tb, own, oa, ob, rest, tw);
   n.l1 = __reduce_add_sync(mask, n.l1);
   n.a2 = __reduce_add_sync(mask, n.a2);
@@ -129,7 +133,7 @@ __global__ void __launch_bounds__(fx_row_block(N), fx_row_block(N) > 256 ? 1 : 2
 }
 
 template <int N>
-cudaError_t edfdv_fx_n(double* f, int nrows, const double* e, FxTurn turn, double dt, const float* rest, const fxw* tw,
+cudaError_t edfdv_fx_n(double* f, int nrows, const double* e, FxTurn turn, const float* rest, const fxw* tw,
                        const cx<double>* tw64, cudaStream_t s) {
   constexpr int G = fx_threads(N);
   const int pairs = (nrows + 1) / 2;
@@ -140,7 +144,7 @@ cudaError_t edfdv_fx_n(double* f, int nrows, const double* e, FxTurn turn, doubl
   const size_t smem = (size_t)P * sp_len<double>(N) * sizeof(fx);
   cudaError_t err = ensure_smem((const void*)k_edfdv_fx<N>, smem);
   if (err != cudaSuccess) return err;
-  k_edfdv_fx<N><<<div_up(pairs, P), P * G, smem, s>>>(f, nrows, e, turn, dt, rest, tw, tw64);
+  k_edfdv_fx<N><<<div_up(pairs, P), P * G, smem, s>>>(f, nrows, e, turn, rest, tw, tw64);
   return cudaGetLastError();
 }
 
@@ -258,7 +262,10 @@ bool fx_make_turn(FxStep k1, double dt, FxTurn* out) {
   const double m = std::frexp(a.h, &e);
   out->am = -((long long)std::ldexp(m, 62) + (long long)std::llrint(std::ldexp(a.l, 62 - e)));
   out->ae = e - 62;
-  out->own = k1.own;
+  out->own = (float)(-6.283185307179586 * dt);
+  // |c| < 2^(e - 1022): own |c| times the largest rest above the least that counts
+  const double most = std::fabs(k1.own * 6.283185307179586 * dt);
+  out->own_e = most > 0.0 ? std::max(0, 1023 + std::ilogb(FX_OWN_LEAST / most)) : 4096;
   return true;
 }
 
@@ -296,11 +303,11 @@ std::vector<float> fx_step_rest(const double* k, int n, FxStep* k1) {
 
 #define VG_FX_CASES(M) M(1) M(2) M(3) M(4) M(5) M(6) M(7) M(8) M(9) M(10) M(11) M(12) M(13)
 
-cudaError_t launch_edfdv_fx(double* f, int nrows, int nv, const double* e, FxTurn turn, double dt, const float* rest,
+cudaError_t launch_edfdv_fx(double* f, int nrows, int nv, const double* e, FxTurn turn, const float* rest,
                             const fxw* tw, const cx<double>* tw64, cudaStream_t s) {
   switch (ilog2(nv)) {
 #define CASE(L) \
-  case L: return edfdv_fx_n<(1 << L)>(f, nrows, e, turn, dt, rest, tw, tw64, s);
+  case L: return edfdv_fx_n<(1 << L)>(f, nrows, e, turn, rest, tw, tw64, s);
     VG_FX_CASES(CASE)
 #undef CASE
     default: return cudaErrorInvalidValue;

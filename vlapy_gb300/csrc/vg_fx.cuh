@@ -430,7 +430,8 @@ __device__ __forceinline__ double fx_to_double(long long v, int k) {
 struct FxTurn {
   long long am;
   int ae;
-  float own;  // the largest modulus of fx_step_rest's
+  float own;  // what fx_step_rest's are to be multiplied with, besides c, for fx_own
+  int own_e;  // from which exponent of c on that is worth while
 };
 __device__ __forceinline__ unsigned long long fx_turn(FxTurn A, double c) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(c);
@@ -482,18 +483,21 @@ __device__ __forceinline__ fxc fx_turn_by(fxc a, const fxw& w) {
 }
 
 // A grid's wavenumbers are m k1 to their own rounding only, which is some 2^-53 of the
-// phase: what wavenumber m is off by (rest of fx_step_rest, here in FP32) times
-// fx_own_scale, a small angle in Q64, is turned on top of the m steps.  (Without it the
+// phase: what wavenumber m is off by (rest of fx_step_rest, here in FP32) times -2 pi
+// dt c, a small angle in Q64, is turned on top of the m steps.  (Without it the
 // phases' errors are those of the doubles ((-k) dt) c, twice to thirty times the
 // transform's on lines with all wavenumbers in them.)  It is 3 % of the x-drift; below
 // 2^-51, what the wavenumbers' rounding makes of phases of ten radians or so, it is left
 // out: the transform's own error is as large.
-__device__ __forceinline__ float fx_own_scale(double dt, double c) { return -6.28318531f * (float)dt * (float)c; }
+// (by its exponent: a conversion takes as long as some thirty other instructions)
+__device__ __forceinline__ bool fx_has_own(const FxTurn& t, double c) {
+  return ((__double2hiint(c) >> 20) & 0x7ff) >= t.own_e;
+}
 __device__ __forceinline__ fxc fx_own(fxc p, float own) {
   const int d = __float2int_rn(own);
   return {p.c - __mulhi((int)(p.s >> 32), d), p.s + __mulhi((int)(p.c >> 32), d)};
 }
-constexpr float FX_OWN_LEAST = 8192.f;  // 2^-51 in Q64
+constexpr double FX_OWN_LEAST = 8192.0;  // 2^-51 in Q64
 
 // What the rotation learns about the bins it leaves: an upper bound of the sum
 // of their moduli in units of 2^38, and the sums of the squares of line a's and
@@ -589,8 +593,8 @@ __device__ __forceinline__ double fx_scale(double x, int k) {
 }
 
 // One line of a pair and its phase: elements f[n es], the power of two that brings
-// it to an RMS of order one, its turns per index and fx_own_scale; bad: it comes out
-// as NaN
+// it to an RMS of order one, its turns per index and what its fx_own angles are the
+// rest's multiples of; bad: it comes out as NaN
 struct FxLine {
   double* f;
   unsigned long long turn;

@@ -102,19 +102,18 @@ constexpr double LN2 = 0.69314718055994530942;
 
 // One CTA per row.  FULL: slots n, j, v^2 .. v^5, f^2, f log f; else n, j, v^2, f^2, f log f.
 // v, v_pow: the powers as doubles, for rows that are not finite.
-constexpr int MOMENTS_WARPS = 16;
-template <bool FULL>
-__global__ void __launch_bounds__(32 * MOMENTS_WARPS) k_moments_fx(const double* __restrict__ f, int nv, FxPowers pw,
+template <bool FULL, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) k_moments_fx(const double* __restrict__ f, int nv, FxPowers pw,
                                                     const FxLogEntry* __restrict__ table, double dv,
                                                     const double* __restrict__ v, const double* __restrict__ v_pow,
                                                     double* __restrict__ out, int stride) {
   constexpr int NP = FULL ? 6 : 3;       // velocity powers
   constexpr int NQ = NP + 2;
-  __shared__ int smax[NP][MOMENTS_WARPS];
-  __shared__ unsigned sbad[MOMENTS_WARPS];
-  __shared__ float ssize[MOMENTS_WARPS];
-  __shared__ Sum96 part[NQ][MOMENTS_WARPS];
-  __shared__ double red[MOMENTS_WARPS];
+  __shared__ int smax[NP][WARPS];
+  __shared__ unsigned sbad[WARPS];
+  __shared__ float ssize[WARPS];
+  __shared__ Sum96 part[NQ][WARPS];
+  __shared__ double red[WARPS];
   __shared__ int redo;
   const double* fr = f + (size_t)blockIdx.x * nv;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -340,8 +339,9 @@ cudaError_t launch_moments_fx(const double* f, int nrows, int nv, const double* 
   // (64 x 1024: 15.4 -> 14.4 us)
   int block = nv >= 1024 ? 256 : nv >= 512 ? 128 : 64;
   if (nrows <= GB300_SMS) block *= 2;
-  if (full) k_moments_fx<true><<<nrows, block, 0, s>>>(f, nv, pw, table, dv, v, v_pow, out, stride);
-  else k_moments_fx<false><<<nrows, block, 0, s>>>(f, nv, pw, table, dv, v, v_pow, out, stride);
+  auto run = [&](auto kernel) { kernel<<<nrows, block, 0, s>>>(f, nv, pw, table, dv, v, v_pow, out, stride); };
+  if (block > 256) run(full ? k_moments_fx<true, 16> : k_moments_fx<false, 16>);
+  else run(full ? k_moments_fx<true, 8> : k_moments_fx<false, 8>);
   return cudaGetLastError();
 }
 

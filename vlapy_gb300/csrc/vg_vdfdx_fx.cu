@@ -40,7 +40,7 @@ __host__ __device__ constexpr int fx_col_ld(int nx, int S) {
 template <int NX>
 __global__ void __launch_bounds__(fx_col_block(NX), fx_col_block(NX) > 256 ? 1 : 2)
     k_vdfdx_fx(double* __restrict__ f, const FxColRun* __restrict__ runs, const int2* __restrict__ items, FxColRun one,
-               int s_log, int ld, double dt, const fxw* __restrict__ tw, const cx<double>* __restrict__ tw64) {
+               int s_log, int ld, const fxw* __restrict__ tw, const cx<double>* __restrict__ tw64) {
   constexpr int R = fx_radix(NX), G = fx_threads(NX);
   constexpr int DOWN = ilog2(NX) - fx_shift<NX>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -103,8 +103,12 @@ __global__ void __launch_bounds__(fx_col_block(NX), fx_col_block(NX) > 256 ? 1 :
   const CtaSync sync;
   fx_fft<NX, false, true, false>(s, t, tw, sync, io);
   const unsigned long long ta = fx_turn(r.turn, bad_a ? 0.0 : ca), tb = fx_turn(r.turn, bad_b ? 0.0 : cb);
-  const float oa = bad_a ? 0.f : fx_own_scale(dt, ca), ob = bad_b ? 0.f : fx_own_scale(dt, cb);
-  const bool own = r.turn.own * fmaxf(fabsf(oa), fabsf(ob)) > FX_OWN_LEAST;
+  const bool own = fx_has_own(r.turn, ca) || fx_has_own(r.turn, cb);
+  float oa = 0.f, ob = 0.f;
+  if (own) {
+    oa = bad_a ? 0.f : r.turn.own * (float)ca;
+    ob = bad_b ? 0.f : r.turn.own * (float)cb;
+  }
   FxNorms n = fx_rotate<NX, DOWN>(s, t, ta, tb, own, oa, ob, r.rest, tw);
   if constexpr (G > 1) {
     atomicAdd(&red[5 * p + 2], n.l1);
@@ -160,7 +164,7 @@ __global__ void __launch_bounds__(fx_col_block(NX), fx_col_block(NX) > 256 ? 1 :
 
 template <int NX>
 cudaError_t vdfdx_fx_n(double* f, const FxColRun* runs, const int2* items, int n_items, const FxColRun& one, int S,
-                       double dt, const fxw* tw, const cx<double>* tw64, cudaStream_t s) {
+                       const fxw* tw, const cx<double>* tw64, cudaStream_t s) {
   constexpr int G = fx_threads(NX);
   const int ld = fx_col_ld(NX, S);
   const size_t smem = std::max((size_t)S * ld * sizeof(fx) + (size_t)S * 5 * sizeof(unsigned),
@@ -168,7 +172,7 @@ cudaError_t vdfdx_fx_n(double* f, const FxColRun* runs, const int2* items, int n
   cudaError_t err = ensure_smem((const void*)k_vdfdx_fx<NX>, smem);
   if (err != cudaSuccess) return err;
   const int blocks = items ? n_items : div_up((one.nv + 1) / 2, S);
-  k_vdfdx_fx<NX><<<blocks, S * G, smem, s>>>(f, runs, items, one, ilog2(S), ld, dt, tw, tw64);
+  k_vdfdx_fx<NX><<<blocks, S * G, smem, s>>>(f, runs, items, one, ilog2(S), ld, tw, tw64);
   return cudaGetLastError();
 }
 
@@ -194,10 +198,10 @@ int fx_col_pairs(int nx, long long pairs) {
 }
 
 cudaError_t launch_vdfdx_fx(double* f, int nx, const FxColRun* runs, const int2* items, int n_items, FxColRun one, int S,
-                            double dt, const fxw* tw, const cx<double>* tw64, cudaStream_t s) {
+                            const fxw* tw, const cx<double>* tw64, cudaStream_t s) {
   switch (ilog2(nx)) {
 #define CASE(L) \
-  case L: return vdfdx_fx_n<(1 << L)>(f, runs, items, n_items, one, S, dt, tw, tw64, s);
+  case L: return vdfdx_fx_n<(1 << L)>(f, runs, items, n_items, one, S, tw, tw64, s);
     VG_FX_CASES(CASE)
 #undef CASE
     default: return cudaErrorInvalidValue;
