@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(fx_row_block(N), fx_row_block(N) > 256 ? 1 : 2
   }
   fx_fft<N, false, true, false>(s, t, tw, sync, io);
   const unsigned long long ta = fx_turn(turn, bad_a ? 0.0 : ea), tb = fx_turn(turn, bad_b ? 0.0 : eb);
-  const bool own = fx_has_own(turn, ea) || fx_has_own(turn, eb);
+  const bool own = N >= FX_OWN_N && (fx_has_own(turn, ea) || fx_has_own(turn, eb));
   float oa = 0.f, ob = 0.f;
   if (own) {
     oa = bad_a ? 0.f : turn.own * (float)ea;

@@ -498,6 +498,8 @@ __device__ __forceinline__ fxc fx_own(fxc p, float own) {
   return {p.c - __mulhi((int)(p.s >> 32), d), p.s + __mulhi((int)(p.c >> 32), d)};
 }
 constexpr double FX_OWN_LEAST = 8192.0;  // 2^-51 in Q64
+// (shorter lines hardly have such phases: the code is left out for the cold launches' sake)
+constexpr int FX_OWN_N = 128;
 
 // What the rotation learns about the bins it leaves: an upper bound of the sum
 // of their moduli in units of 2^38, and the sums of the squares of line a's and

@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_moments_fx(const double* __restr
   __shared__ float ssize[WARPS];
   __shared__ Sum96 part[NQ][WARPS];
   __shared__ double red[WARPS];
-  __shared__ int redo;
+  __shared__ int redo, top[NP];
   const double* fr = f + (size_t)blockIdx.x * nv;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   // the largest exponent of f and of its products with the powers; a value that is not
@@ -148,6 +148,10 @@ __global__ void __launch_bounds__(32 * WARPS) k_moments_fx(const double* __restr
     for (int p = 0; p < NP; ++p) mx[p] = max(mx[p], smax[p][q]);
     bad |= sbad[q];
   }
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int p = 0; p < NP; ++p) top[p] = mx[p];
+  }
   const int E = mx[0];
   double* o = out + (size_t)blockIdx.x * stride;
   if (E == FX_NONFINITE) {
@@ -174,9 +178,11 @@ __global__ void __launch_bounds__(32 * WARPS) k_moments_fx(const double* __restr
   Acc96 s[NQ];
 #pragma unroll
   for (int q = 0; q < NQ; ++q) s[q] = {0, 0};
+  double xn = threadIdx.x < nv ? fr[threadIdx.x] : 0.0;  // (the next element, on its way)
   float size = 0.f;  // sum of f |log|, in units of 2^32 of its sum
   for (int j = threadIdx.x; j < nv; j += blockDim.x) {
-    const FxNum F = fx_num(fr[j]);
+    const FxNum F = fx_num(xn);
+    xn = fr[min(j + (int)blockDim.x, nv - 1)];
     const int half = (j == 0 || j == nv - 1) ? 1 : 0;  // the trapz weight of the ends
     const int down = E - F.e;
     acc_add(s[0], fx_shr(F.n, down + half));
@@ -220,7 +226,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_moments_fx(const double* __restr
     // f = F 2^(e - 1084), a product of two such numbers was divided by 2^64
     double r;
     if (q == 0) r = ldexp(sum, E - 1084);
-    else if (q < NP) r = ldexp(sum, mx[q] + pw.e[q - 1] - 2104);
+    else if (q < NP) r = ldexp(sum, top[q] + pw.e[q - 1] - 2104);
     else if (q == NP) r = ldexp(sum, 2 * E - 2104);
     else {
       // F times a logarithm in Q56, divided by 2^64, times 2^(8 - up)

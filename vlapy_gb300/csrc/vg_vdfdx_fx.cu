@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(fx_col_block(NX), fx_col_block(NX) > 256 ? 1 :
   const CtaSync sync;
   fx_fft<NX, false, true, false>(s, t, tw, sync, io);
   const unsigned long long ta = fx_turn(r.turn, bad_a ? 0.0 : ca), tb = fx_turn(r.turn, bad_b ? 0.0 : cb);
-  const bool own = fx_has_own(r.turn, ca) || fx_has_own(r.turn, cb);
+  const bool own = NX >= FX_OWN_N && (fx_has_own(r.turn, ca) || fx_has_own(r.turn, cb));
   float oa = 0.f, ob = 0.f;
   if (own) {
     oa = bad_a ? 0.f : r.turn.own * (float)ca;
